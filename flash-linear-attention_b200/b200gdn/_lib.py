@@ -1,6 +1,8 @@
-"""ctypes binding of libb200gdn.so (the C ABI declared in include/b200gdn.h).
+"""Bindings of libb200gdn.so (the C ABI declared in include/b200gdn.h): ctypes for the context-parallel path and for
+callers that drive single stages, and the native host path (``host()``, built from csrc/host.cpp) that the operators go
+through.
 
-The library is the only compute path of this package: when it cannot be loaded every operator
+The library is the only compute path of this package: when it or the host extension cannot be loaded every operator
 raises, there is no fallback.
 """
 from __future__ import annotations
@@ -34,7 +36,7 @@ class ChunkArgs(C.Structure):
         ('dq', _p), ('dk', _p), ('dv', _p), ('dg', _p), ('dbeta', _p), ('dh0', _p),
         ('dh', _p), ('dv2', _p), ('dw', _p), ('dk_part', _p), ('dG', _p), ('dq_acc', _p),
         ('options', C.c_uint32), ('A_log', _p), ('dt_bias', _p), ('gate_partials', _p), ('dA_log', _p), ('ddt_bias', _p),
-        ('cp_M', _p), ('cp_dM', _p), ('qk', _p), ('rstd_q', _p), ('rstd_k', _p),
+        ('cp_M', _p), ('cp_dM', _p), ('qk', _p), ('rstd_q', _p), ('rstd_k', _p), ('gb_dtype', C.c_int32),
     ]
 
 
@@ -45,6 +47,7 @@ class RecurrentArgs(C.Structure):
         ('qkv_dtype', C.c_int32),
         ('cu_seqlens', _p), ('q', _p), ('k', _p), ('v', _p), ('g', _p), ('beta', _p), ('A_log', _p),
         ('dt_bias', _p), ('h0', _p), ('o', _p), ('ht', _p), ('state_indices', _p), ('n_slots', C.c_int32),
+        ('gb_dtype', C.c_int32),
     ]
 
 
@@ -79,6 +82,7 @@ class ConvArgs(C.Structure):
         ('tile_meta', _p), ('seq_meta', _p), ('x', _p), ('weight', _p), ('bias', _p), ('residual', _p),
         ('initial_state', _p), ('y', _p), ('final_state', _p),
         ('dy', _p), ('dx', _p), ('dweight', _p), ('dbias', _p), ('dinitial_state', _p), ('partials', _p),
+        ('param_dtype', C.c_int32),
     ]
 
 
@@ -88,6 +92,7 @@ class NormGateArgs(C.Structure):
         ('dtype', C.c_int32), ('eps', C.c_float),
         ('x', _p), ('g', _p), ('weight', _p), ('bias', _p), ('y', _p), ('rstd', _p),
         ('dy', _p), ('dx', _p), ('dg', _p), ('dweight', _p), ('dbias', _p), ('partials', _p),
+        ('param_dtype', C.c_int32),
     ]
 
 
@@ -165,12 +170,34 @@ def load():
     return _lib
 
 
+_host = None
+
+
+def host():
+    """The native host path (csrc/host.cpp), loaded once."""
+    global _host
+    if _host is None:
+        load()   # the kernels' library first: a missing or stale build is reported as such
+        with _lock:
+            if _host is None:
+                import torch   # noqa: F401  (its shared libraries must be in the process)
+                try:
+                    from . import _host as mod
+                except ImportError as e:
+                    raise B200GDNError(f'the native host path cannot be loaded ({e}): build it with '
+                                       '`make -C flash-linear-attention_b200/csrc` (or __graft_entry__.build()). '
+                                       'There is no fallback path.') from e
+                mod.set_error_class(B200GDNError)
+                _host = mod
+    return _host
+
+
 _launches = 0
 
 
 def launch_count() -> int:
-    """Kernels enqueued through this binding since import (benchmark bookkeeping)."""
-    return _launches
+    """Kernels enqueued through these bindings since import (benchmark bookkeeping)."""
+    return _launches + (_host.launch_count() if _host is not None else 0)
 
 
 def call(name: str, args: C.Structure, stream: int) -> None:

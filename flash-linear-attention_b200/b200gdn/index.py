@@ -7,6 +7,8 @@ from typing import Optional, Sequence, Tuple
 import numpy as np
 import torch
 
+from . import _lib
+
 CHUNK = 64
 _cache: dict = {}
 
@@ -14,8 +16,14 @@ _cache: dict = {}
 class Tables(tuple):
     """(chunk_meta, seq_meta, (n_chunks, n_seq)) plus ``covered``: False when token rows before the first or after
     the last sequence belong to no sequence (a padded packed buffer).  The kernels never write such rows, so the
-    caller zero-fills its intermediates then."""
+    caller zero-fills its intermediates then.  ``native()`` is the same as one handle for the native host path."""
     covered = True
+    _native = None
+
+    def native(self):
+        if self._native is None:
+            self._native = _lib.host().plan(self[0], self[1], self[2][0], self[2][1], self.covered)
+        return self._native
 
 
 def build_tables(bounds: Sequence[Tuple[int, int]]):
@@ -44,13 +52,13 @@ def tables_for(B: int, T: int, cu_seqlens: Optional[torch.Tensor], cu_seqlens_cp
     ``cu_seqlens`` (the reference memoises its index tensors the same way, fla/utils/_decorators.py:33-80).
     A packed batch without ``cu_seqlens_cpu`` costs one device-to-host copy on first use."""
     if cu_seqlens is None:
-        key = ('dense', B, T, str(device))
+        key = ('dense', B, T, device)
         hit = _cache.get(key)
         if hit is not None:
             return hit[0]
         bounds = [(b * T, (b + 1) * T) for b in range(B)]
     else:
-        key = ('varlen', id(cu_seqlens), B * T, str(device))
+        key = ('varlen', id(cu_seqlens), B * T, device)
         hit = _cache.get(key)
         if hit is not None and hit[1] is cu_seqlens:
             return hit[0]
@@ -84,7 +92,15 @@ _split_cache: dict = {}
 class SplitPlan:
     """Virtual-sequence tables and the index tensors that tie the pieces of a sequence together."""
     __slots__ = ('tables', 'n_pieces', 'n_pre', 'chains', 'n_chains', 'pre_fwd', 'pre_bwd', 'first_piece', 'last_piece',
-                 'pieces_per_seq')
+                 'pieces_per_seq', '_native')
+
+    def native(self):
+        """The plan as one handle for the native host path."""
+        if self._native is None:
+            t = self.tables
+            self._native = _lib.host().plan(t[0], t[1], t[2][0], t[2][1], t.covered, self.chains, self.pre_fwd, self.pre_bwd,
+                                            self.first_piece, self.last_piece, self.n_chains, self.n_pre)
+        return self._native
 
 
 def piece_counts(chunks_per_seq, HV: int, slices: int):
@@ -134,19 +150,20 @@ def split_plan(bounds, HV: int, slices: int, device, rows: int) -> Optional[Spli
     plan.first_piece = torch.tensor(first_piece, dtype=torch.long).to(device)
     plan.last_piece = torch.tensor(last_piece, dtype=torch.long).to(device)
     plan.pieces_per_seq = pieces
+    plan._native = None
     return plan
 
 
 def split_plan_for(B: int, T: int, cu_seqlens, cu_seqlens_cpu, device, HV: int, slices: int) -> Optional[SplitPlan]:
     """Memoised like tables_for (by shape, or by the identity of ``cu_seqlens``)."""
     if cu_seqlens is None:
-        key = ('dense', B, T, HV, slices, FORCE_PIECES, str(device))
+        key = ('dense', B, T, HV, slices, FORCE_PIECES, device)
         hit = _split_cache.get(key)
         if hit is not None:
             return hit[0]
         bounds = [(b * T, (b + 1) * T) for b in range(B)]
     else:
-        key = ('varlen', id(cu_seqlens), B * T, HV, slices, FORCE_PIECES, str(device))
+        key = ('varlen', id(cu_seqlens), B * T, HV, slices, FORCE_PIECES, device)
         hit = _split_cache.get(key)
         if hit is not None and hit[1] is cu_seqlens:
             return hit[0]
@@ -158,3 +175,9 @@ def split_plan_for(B: int, T: int, cu_seqlens, cu_seqlens_cpu, device, HV: int, 
         _split_cache.clear()
     _split_cache[key] = (plan, cu_seqlens)
     return plan
+
+
+def native_plan(B: int, T: int, cu_seqlens, cu_seqlens_cpu, device, HV: int, slices: int):
+    """Handle of the split plan of these sequences, or of their chunk tables when none is worth cutting."""
+    plan = split_plan_for(B, T, cu_seqlens, cu_seqlens_cpu, device, HV, slices)
+    return (plan if plan is not None else tables_for(B, T, cu_seqlens, cu_seqlens_cpu, device)).native()

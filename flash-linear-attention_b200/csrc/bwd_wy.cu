@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_wy_kernel(const b200gdn_chunk
     }
     if (tid < BT) {
       const bool ok = tid < cm.len;
-      float b = ok ? a.beta[(row0 + tid) * a.HV + hv] : 0.f;
+      float b = ok ? ld_param(a.beta, (row0 + tid) * a.HV + hv, a.gb_dtype) : 0.f;
       if (a.options & B200GDN_PREP_BETA_SIGMOID) {   // raw beta: the kernels work with (1|2) sigmoid(beta)
         const float sg = 1.f / (1.f + expf(-b));
         sgm[tid] = sg;
@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_wy_kernel(const b200gdn_chunk
       }
       bet[tid] = b;
       if (a.options & B200GDN_PREP_GATE)
-        gx[tid] = (ok ? a.g[(row0 + tid) * a.HV + hv] : 0.f) + (a.dt_bias ? a.dt_bias[hv] : 0.f);
+        gx[tid] = (ok ? ld_param(a.g, (row0 + tid) * a.HV + hv, a.gb_dtype) : 0.f) + (a.dt_bias ? a.dt_bias[hv] : 0.f);
       dGin[tid] = ok ? a.dG[(row0 + tid) * a.HV + hv] : 0.f;
     }
     if (!tc5::mbar_wait(bar_ld, gi & 1)) failed = true;
@@ -432,7 +432,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_wy_kernel(const b200gdn_chunk
         float db = ckbg * eg[i] + cvb + rmk;
         if (a.options & B200GDN_PREP_BETA_SIGMOID)   // chain rule through (1|2) sigmoid
           db *= ((a.options & B200GDN_PREP_NEG_EIGVAL) ? 2.f : 1.f) * sgm[i] * (1.f - sgm[i]);
-        a.dbeta[(row0 + i) * a.HV + hv] = db;
+        st_param(a.dbeta, (row0 + i) * a.HV + hv, a.gb_dtype, db);
       }
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -443,7 +443,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_wy_kernel(const b200gdn_chunk
     }
     if (__syncthreads_or(!ph.wait())) { failed = true; break; }
     if (!(a.options & B200GDN_PREP_GATE)) {
-      if (tid < cm.len) a.dg[(row0 + tid) * a.HV + hv] = dGs[tid] + (tid < 32 ? dGs[32] : 0.f);
+      if (tid < cm.len) st_param(a.dg, (row0 + tid) * a.HV + hv, a.gb_dtype, dGs[tid] + (tid < 32 ? dGs[32] : 0.f));
     } else {
       // fused gate: g = -exp(A_log) softplus(x), x = g_raw + dt_bias.  dg_raw = dg (-exp(A_log)) sigmoid(x);
       // dA_log += dg g and ddt_bias += dg_raw, summed over the chunk here and over the chunks by a second kernel
@@ -453,7 +453,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_wy_kernel(const b200gdn_chunk
           const float dgi = dGs[tid] + (tid < 32 ? dGs[32] : 0.f);
           const float x = gx[tid], negA = -expf(a.A_log[hv]);
           const float draw = dgi * negA / (1.f + expf(-x));
-          a.dg[(row0 + tid) * a.HV + hv] = draw;
+          st_param(a.dg, (row0 + tid) * a.HV + hv, a.gb_dtype, draw);
           sA = dgi * negA * (x > 20.f ? x : log1pf(expf(x)));
           sB = draw;
         }

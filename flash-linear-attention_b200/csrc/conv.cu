@@ -150,8 +150,8 @@ __global__ void __launch_bounds__(CT) conv_fwd_kernel(const b200gdn_conv_args a)
 #pragma unroll
   for (int c = 0; c < C; ++c) {
 #pragma unroll
-    for (int j = 0; j < W; ++j) w[j][c] = a.weight[(int64_t)(d0 + c) * W + j];
-    b[c] = a.bias ? a.bias[d0 + c] : 0.f;
+    for (int j = 0; j < W; ++j) w[j][c] = ld_param(a.weight, (int64_t)(d0 + c) * W + j, a.param_dtype);
+    b[c] = a.bias ? ld_param(a.bias, d0 + c, a.param_dtype) : 0.f;
   }
   load_history<T, W, C>(a, ti, d0, hist);
   // one token; FULL: the token is known to lie inside the share, so nothing in the body is conditional and the
@@ -239,8 +239,8 @@ __global__ void __launch_bounds__(CT) conv_bwd_kernel(const b200gdn_conv_args a)
 #pragma unroll
   for (int c = 0; c < C; ++c) {
 #pragma unroll
-    for (int j = 0; j < W; ++j) w[j][c] = a.weight[(int64_t)(d0 + c) * W + j];
-    b[c] = a.bias ? a.bias[d0 + c] : 0.f;
+    for (int j = 0; j < W; ++j) w[j][c] = ld_param(a.weight, (int64_t)(d0 + c) * W + j, a.param_dtype);
+    b[c] = a.bias ? ld_param(a.bias, d0 + c, a.param_dtype) : 0.f;
   }
   load_history<T, W, C>(a, ti, d0, hist);
   float ring[W][C];   // ring[k]: dx of token (u - k) so far, u the token being processed
@@ -364,8 +364,8 @@ __global__ void __launch_bounds__(32 * RW) conv_param_reduce_kernel(const b200gd
 #pragma unroll
   for (int r = 1; r < RW; ++r) s += part[r][lane];
   const int d = (int)(i / (a.W + 1)), j = (int)(i % (a.W + 1));
-  if (j < a.W) a.dweight[(int64_t)d * a.W + j] = s;
-  else if (a.dbias != nullptr) a.dbias[d] = s;
+  if (j < a.W) st_param(a.dweight, (int64_t)d * a.W + j, a.param_dtype, s);
+  else if (a.dbias != nullptr) st_param(a.dbias, d, a.param_dtype, s);
 }
 
 // channels per thread: four in both passes.  With eight (16-byte accesses for bf16) the per-channel state of the backward

@@ -3,6 +3,7 @@
 // (The tensor-core / TMEM / TMA primitives live in tc5.cuh, tc5_tile.cuh and tma.cuh.)
 #pragma once
 #include <cuda_bf16.h>
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -25,10 +26,7 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
-// ---- small asynchronous global -> shared copies (4 bytes per thread) --------------------------------------
-__device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(smem_u32(smem)), "l"(gmem));
-}
+// ---- asynchronous global -> shared copies: group bookkeeping ------------------------------------------------
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() {
@@ -43,6 +41,18 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 __device__ __forceinline__ float2 unpack_bf16(uint32_t v) {
   __nv_bfloat162 b = *reinterpret_cast<__nv_bfloat162*>(&v);
   return __bfloat1622float2(b);
+}
+
+// ---- tensors read / written in the caller's precision (B200GDN_F32 / BF16 / F16) ----------------------------
+__device__ __forceinline__ float ld_param(const void* p, int64_t i, int code) {
+  if (code == B200GDN_F32) return static_cast<const float*>(p)[i];
+  if (code == B200GDN_BF16) return __bfloat162float(static_cast<const __nv_bfloat16*>(p)[i]);
+  return __half2float(static_cast<const __half*>(p)[i]);
+}
+__device__ __forceinline__ void st_param(void* p, int64_t i, int code, float x) {
+  if (code == B200GDN_F32) static_cast<float*>(p)[i] = x;
+  else if (code == B200GDN_BF16) static_cast<__nv_bfloat16*>(p)[i] = __float2bfloat16_rn(x);
+  else static_cast<__half*>(p)[i] = __float2half_rn(x);
 }
 
 // Shared address of the 16-byte chunk holding (row r, columns col8 .. col8+7) of a bf16 tile of `rows` rows in the
@@ -103,8 +113,23 @@ int set_error(int code, const char* fmt, ...);
 int check_launch(const char* what);
 void reset_launch_count();
 
+// Whether this thread has set the attribute for (kernel, device) before: the driver call costs about half a microsecond,
+// which a decoding step would pay on every launch.
+inline bool smem_attr_set_before(const void* kern) {
+  struct Entry { const void* kern; int dev; };
+  static thread_local Entry seen[64];
+  static thread_local int n = 0;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  for (int i = 0; i < n; ++i)
+    if (seen[i].kern == kern && seen[i].dev == dev) return true;
+  if (n < 64) seen[n++] = Entry{kern, dev};
+  return false;
+}
+
 template <typename Kern>
-int ensure_smem(Kern kern, size_t bytes) {
+int ensure_smem(Kern kern, size_t bytes) {   // `bytes` is a constant of the kernel's instantiation
+  if (smem_attr_set_before(reinterpret_cast<const void*>(kern))) return 0;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   if (e != cudaSuccess) return set_error(B200GDN_ERR_CUDA, "cudaFuncSetAttribute(%zu B): %s", bytes, cudaGetErrorString(e));
   return 0;

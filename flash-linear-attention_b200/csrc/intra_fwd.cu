@@ -136,15 +136,11 @@ __global__ void __launch_bounds__(NTHREADS, 4) intra_fwd_kernel(const b200gdn_ch
     tma::prefetch_3d(&maps.v, cm.row, (hv * DV) / 64);   // V is loaded late (it reuses L's place): have it in L2 by then
   }
   if (warp == 1) tc5::tmem_alloc(tmem_slot, 128);
-  if (tid < BT) {   // asynchronous copies: nobody stalls on the DRAM latency of the gates before the first barrier
-    if (tid < cm.len) {
-      cp_async4(graw + tid, a.g + (row0 + tid) * a.HV + hv);
-      cp_async4(bet + tid, a.beta + (row0 + tid) * a.HV + hv);
-    } else {
-      graw[tid] = 0.f;
-      bet[tid] = 0.f;
-    }
-    cp_async_commit();
+  // the gates of this thread's token: the loads are issued here and first used behind the barrier below
+  float g_raw = 0.f, b_raw = 0.f;
+  if (tid < cm.len) {
+    g_raw = ld_param(a.g, (row0 + tid) * a.HV + hv, a.gb_dtype);
+    b_raw = ld_param(a.beta, (row0 + tid) * a.HV + hv, a.gb_dtype);
   }
   // zero the fp32 inverse (the merges and the final conversion read the untouched blocks as zeros)
   for (int i = tid; i < BT * LDF / 4; i += NTHREADS) reinterpret_cast<float4*>(Af)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -157,16 +153,16 @@ __global__ void __launch_bounds__(NTHREADS, 4) intra_fwd_kernel(const b200gdn_ch
 
   if (tid < BT) {
     // inclusive scan of g over the chunk: shuffle scan inside each of the two warps, carry added below
-    cp_async_wait<0>();   // this thread's own g and beta
     if (a.options != 0 && tid < cm.len) {   // the layer's gate / beta activations, fused (rows past the end stay 0)
       if (a.options & B200GDN_PREP_GATE) {
-        const float x = graw[tid] + (a.dt_bias ? a.dt_bias[hv] : 0.f);
-        graw[tid] = -expf(a.A_log[hv]) * (x > 20.f ? x : log1pf(expf(x)));
+        const float x = g_raw + (a.dt_bias ? a.dt_bias[hv] : 0.f);
+        g_raw = -expf(a.A_log[hv]) * (x > 20.f ? x : log1pf(expf(x)));
       }
       if (a.options & B200GDN_PREP_BETA_SIGMOID)
-        bet[tid] = ((a.options & B200GDN_PREP_NEG_EIGVAL) ? 2.f : 1.f) / (1.f + expf(-bet[tid]));
+        b_raw = ((a.options & B200GDN_PREP_NEG_EIGVAL) ? 2.f : 1.f) / (1.f + expf(-b_raw));
     }
-    float s = graw[tid];
+    bet[tid] = b_raw;
+    float s = g_raw;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const float y = __shfl_up_sync(0xffffffffu, s, o);
@@ -179,11 +175,11 @@ __global__ void __launch_bounds__(NTHREADS, 4) intra_fwd_kernel(const b200gdn_ch
     if (successor_cta(pf_dist, c2, h2)) {   // L2 look-ahead for the CTA that will follow this one
       const int row2 = load_chunk_meta(a.chunk_meta, c2).row;
       tma::prefetch_3d(&maps.k, row2, ((h2 / G) * DK) / 64);
-      // g and beta of a chunk are [64][HV] fp32 blocks: the HV CTAs of a chunk pull two lines each
-      const int lines = BT * a.HV * 4 / 128;
+      // g and beta of a chunk are [64][HV] blocks: the HV CTAs of a chunk pull (up to) two lines each
+      const int gb_bytes = a.gb_dtype == B200GDN_F32 ? 4 : 2, lines = BT * a.HV * gb_bytes / 128;
       for (int l = h2 * 2; l < h2 * 2 + 2 && l < lines; ++l) {
-        tma::prefetch_line(a.g + (int64_t)row2 * a.HV + l * 32);
-        tma::prefetch_line(a.beta + (int64_t)row2 * a.HV + l * 32);
+        tma::prefetch_line(static_cast<const char*>(a.g) + (int64_t)row2 * a.HV * gb_bytes + l * 128);
+        tma::prefetch_line(static_cast<const char*>(a.beta) + (int64_t)row2 * a.HV * gb_bytes + l * 128);
       }
     }
   }

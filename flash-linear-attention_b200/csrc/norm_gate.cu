@@ -42,8 +42,8 @@ __global__ void __launch_bounds__(NT) norm_gate_fwd_kernel(const b200gdn_norm_ga
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const int d = (v * LPV + sub) * 8 + i;
-      w[v][i] = a.weight ? a.weight[d] : 1.f;
-      b[v][i] = a.bias ? a.bias[d] : 0.f;
+      w[v][i] = a.weight ? ld_param(a.weight, d, a.param_dtype) : 1.f;
+      b[v][i] = a.bias ? ld_param(a.bias, d, a.param_dtype) : 0.f;
     }
   const int64_t stride = (int64_t)gridDim.x * (NT / 32) * RW;
   // the loop bound is the warp's first row, so that every lane takes part in the shuffles of a round
@@ -103,8 +103,8 @@ __global__ void __launch_bounds__(NT) norm_gate_bwd_kernel(const b200gdn_norm_ga
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const int d = (v * LPV + sub) * 8 + i;
-      w[v][i] = a.weight ? a.weight[d] : 1.f;
-      b[v][i] = a.bias ? a.bias[d] : 0.f;
+      w[v][i] = a.weight ? ld_param(a.weight, d, a.param_dtype) : 1.f;
+      b[v][i] = a.bias ? ld_param(a.bias, d, a.param_dtype) : 0.f;
       dw[v][i] = 0.f;
       db[v][i] = 0.f;
     }
@@ -204,8 +204,8 @@ __global__ void __launch_bounds__(32 * RW) norm_gate_param_reduce_kernel(const b
   if (q != 0) return;
 #pragma unroll
   for (int r = 1; r < RW; ++r) s += part[r][lane];
-  if (which == 0) { if (a.dweight) a.dweight[d] = s; }
-  else if (a.dbias) a.dbias[d] = s;
+  if (which == 0) { if (a.dweight) st_param(a.dweight, d, a.param_dtype, s); }
+  else if (a.dbias) st_param(a.dbias, d, a.param_dtype, s);
 }
 
 template <typename T, int LPV, int NV>

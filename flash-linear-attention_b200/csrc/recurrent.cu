@@ -99,12 +99,12 @@ __global__ void __launch_bounds__(NTHREADS, (DK <= 128 ? 8 : 4)) recurrent_kerne
     }
     if (tid < VS) vs[tid] = ld_elem(a.v, (row * a.HV + hv) * DV + v0 + tid, a.qkv_dtype);
     if (tid == 0) {
-      float gg = a.g ? a.g[row * a.HV + hv] : 0.f;
+      float gg = a.g ? ld_param(a.g, row * a.HV + hv, a.gb_dtype) : 0.f;
       if (a.flags & B200GDN_REC_GATE) {
         if (a.dt_bias) gg += a.dt_bias[hv];
         gg = -expf(a.A_log[hv]) * softplus_f(gg);
       }
-      float bb = a.beta[row * a.HV + hv];
+      float bb = ld_param(a.beta, row * a.HV + hv, a.gb_dtype);
       if (a.flags & B200GDN_REC_BETA_SIGMOID) {
         bb = 1.f / (1.f + expf(-bb));
         if (a.flags & B200GDN_REC_NEG_EIGVAL) bb *= 2.f;
@@ -266,12 +266,12 @@ __global__ void __launch_bounds__(256, 2) recurrent_rows_kernel(const b200gdn_re
       vs[tid - DK] = ld_elem(a.v, (row * a.HV + hv) * DV + tid - DK, a.qkv_dtype);
     }
     if (tid == NT - 1) {
-      float gg = a.g ? a.g[row * a.HV + hv] : 0.f;
+      float gg = a.g ? ld_param(a.g, row * a.HV + hv, a.gb_dtype) : 0.f;
       if (a.flags & B200GDN_REC_GATE) {
         if (a.dt_bias) gg += a.dt_bias[hv];
         gg = -expf(a.A_log[hv]) * softplus_f(gg);
       }
-      float bb = a.beta[row * a.HV + hv];
+      float bb = ld_param(a.beta, row * a.HV + hv, a.gb_dtype);
       if (a.flags & B200GDN_REC_BETA_SIGMOID) {
         bb = 1.f / (1.f + expf(-bb));
         if (a.flags & B200GDN_REC_NEG_EIGVAL) bb *= 2.f;
@@ -407,12 +407,12 @@ __global__ void __launch_bounds__(288, 1) decode_stream_kernel(const b200gdn_rec
           const int item = (int)blockIdx.x + jj * (int)gridDim.x;
           const int n = item / a.HV, hv = item % a.HV, hq = hv / G;
           const int64_t row = n;   // one token per sequence
-          float gg = a.g ? a.g[row * a.HV + hv] : 0.f;
+          float gg = a.g ? ld_param(a.g, row * a.HV + hv, a.gb_dtype) : 0.f;
           if (a.flags & B200GDN_REC_GATE) {
             if (a.dt_bias) gg += a.dt_bias[hv];
             gg = -expf(a.A_log[hv]) * softplus_f(gg);
           }
-          float bb = a.beta[row * a.HV + hv];
+          float bb = ld_param(a.beta, row * a.HV + hv, a.gb_dtype);
           if (a.flags & B200GDN_REC_BETA_SIGMOID) {
             bb = 1.f / (1.f + expf(-bb));
             if (a.flags & B200GDN_REC_NEG_EIGVAL) bb *= 2.f;

@@ -37,6 +37,12 @@ extern "C" {
 #define B200GDN_ABI_VERSION 1
 #define B200GDN_CHUNK 64
 
+/* element type of small per-head / per-channel tensors that are read (or written) in the caller's own precision:
+ * gates and betas, convolution and norm parameters.  0 is fp32, so that a zeroed argument block means fp32. */
+#define B200GDN_F32 0
+#define B200GDN_BF16 1
+#define B200GDN_F16 2
+
 typedef enum b200gdn_status {
   B200GDN_OK = 0,
   B200GDN_ERR_BAD_ARGUMENT = -1,   /* null pointer, wrong struct size, zero size */
@@ -73,8 +79,8 @@ typedef struct b200gdn_chunk_args {
   const void* q;                 /* bf16 [rows,H,K] */
   const void* k;                 /* bf16 [rows,H,K] */
   const void* v;                 /* bf16 [rows,HV,V] */
-  const float* g;                /* [rows,HV] log-space decay per token (forward only) */
-  const float* beta;             /* [rows,HV] */
+  const void* g;                 /* [rows,HV] log-space decay per token (forward only), element type gb_dtype */
+  const void* beta;              /* [rows,HV], element type gb_dtype */
   const float* h0;               /* [n_seq,HV,K,V] or NULL */
   /* forward outputs */
   void* o;                       /* bf16 [rows,HV,V] */
@@ -95,8 +101,8 @@ typedef struct b200gdn_chunk_args {
   void* dk;                      /* bf16 [rows,H,K]; between B200GDN_BWD_DQKWG and B200GDN_BWD_WY it holds the
                                     chunk-local part of dk, to which the WY stage adds its terms in place */
   void* dv;                      /* bf16 [rows,HV,V] */
-  float* dg;                     /* [rows,HV] */
-  float* dbeta;                  /* [rows,HV] */
+  void* dg;                      /* [rows,HV], element type gb_dtype */
+  void* dbeta;                   /* [rows,HV], element type gb_dtype */
   float* dh0;                    /* [n_seq,HV,K,V] or NULL */
   /* backward workspace */
   void* dh;                      /* bf16 [n_chunks,HV,K,V] */
@@ -131,6 +137,7 @@ typedef struct b200gdn_chunk_args {
    * (replaces l2norm_bwd, fla/modules/l2norm.py:200-251).  NULL: dq / dk are gradients w.r.t. q / k as passed. */
   const float* rstd_q;
   const float* rstd_k;
+  int32_t gb_dtype;              /* B200GDN_F32 / BF16 / F16: element type of g, beta, dg and dbeta */
 } b200gdn_chunk_args;
 
 /* Replaces chunk_gated_delta_rule_fwd (fla/ops/gated_delta_rule/chunk.py:33-123):
@@ -168,8 +175,8 @@ typedef struct b200gdn_recurrent_args {
   const void* q;                 /* [B,T,H,K] */
   const void* k;                 /* [B,T,H,K] */
   const void* v;                 /* [B,T,HV,V] */
-  const float* g;                /* [B,T,HV] or NULL */
-  const float* beta;             /* [B,T,HV] */
+  const void* g;                 /* [B,T,HV] or NULL, element type gb_dtype */
+  const void* beta;              /* [B,T,HV], element type gb_dtype */
   const float* A_log;            /* [HV] (gate in kernel) or NULL */
   const float* dt_bias;          /* [HV] or NULL */
   const float* h0;               /* [n_seq,HV,K,V] ([.,.,V,K] when V-first) or NULL */
@@ -182,6 +189,7 @@ typedef struct b200gdn_recurrent_args {
   int32_t n_slots;               /* slots in the pool (with state_indices); an index outside [0, n_slots) marks a
                                     padding sequence: its state is neither taken from its slot nor written back and its
                                     output row is meaningless.  0 = unknown, indices are then trusted */
+  int32_t gb_dtype;              /* B200GDN_F32 / BF16 / F16: element type of g and beta */
 } b200gdn_recurrent_args;
 
 #define B200GDN_REC_L2NORM 1u         /* q, k <- x * rsqrt(sum x^2 + 1e-6) */
@@ -307,8 +315,8 @@ typedef struct b200gdn_conv_args {
   const int32_t* tile_meta;      /* device [n_tiles][4], as chunk_meta */
   const int32_t* seq_meta;       /* device [n_seq][2], as seq_meta */
   const void* x;                 /* [rows, D] */
-  const float* weight;           /* [D, W] */
-  const float* bias;             /* [D] or NULL */
+  const void* weight;            /* [D, W], element type param_dtype */
+  const void* bias;              /* [D] or NULL, element type param_dtype */
   const void* residual;          /* [rows, D] or NULL (forward) */
   const void* initial_state;     /* [n_seq, D, W] or NULL */
   void* y;                       /* [rows, D] (forward) */
@@ -316,10 +324,11 @@ typedef struct b200gdn_conv_args {
   /* backward */
   const void* dy;                /* [rows, D] */
   void* dx;                      /* [rows, D] */
-  float* dweight;                /* [D, W] or NULL */
-  float* dbias;                  /* [D] or NULL */
+  void* dweight;                 /* [D, W] or NULL, element type param_dtype */
+  void* dbias;                   /* [D] or NULL, element type param_dtype */
   void* dinitial_state;          /* [n_seq, D, W] or NULL */
   float* partials;               /* workspace fp32 [2 n_tiles, D, W + 1]; required with dweight */
+  int32_t param_dtype;           /* B200GDN_F32 / BF16 / F16 */
 } b200gdn_conv_args;
 int b200gdn_conv_fwd(const b200gdn_conv_args* args, void* stream);
 int b200gdn_conv_bwd(const b200gdn_conv_args* args, void* stream);
@@ -339,16 +348,17 @@ typedef struct b200gdn_norm_gate_args {
   float eps;
   const void* x;                 /* [rows, D] */
   const void* g;                 /* [rows, D] */
-  const float* weight;           /* [D] or NULL */
-  const float* bias;             /* [D] or NULL */
+  const void* weight;            /* [D] or NULL, element type param_dtype */
+  const void* bias;              /* [D] or NULL, element type param_dtype */
   void* y;                       /* [rows, D] (forward) */
   float* rstd;                   /* [rows]: written by the forward pass, read by the backward pass */
   const void* dy;
   void* dx;
   void* dg;
-  float* dweight;                /* [D] or NULL */
-  float* dbias;                  /* [D] or NULL */
+  void* dweight;                 /* [D] or NULL, element type param_dtype */
+  void* dbias;                   /* [D] or NULL, element type param_dtype */
   float* partials;
+  int32_t param_dtype;           /* B200GDN_F32 / BF16 / F16 */
 } b200gdn_norm_gate_args;
 int b200gdn_norm_gate_fwd(const b200gdn_norm_gate_args* args, void* stream);
 int b200gdn_norm_gate_bwd(const b200gdn_norm_gate_args* args, void* stream);

@@ -221,3 +221,17 @@ def test_slab_hands_out_aligned_addresses_and_null_for_absent_pieces():
     assert Slab.addresses(slab.buf, list(slab.offs)) == addr
     assert int(slab.buf.sum()) == 0                      # zero=True fills the allocation
     assert Slab(torch.device('cpu'), False, (0, 0)).buf.numel() >= 256   # never an empty allocation
+
+
+def test_native_host_path_declines_what_it_does_not_serve():
+    """The direct call leaves tensors it does not serve to the checks of the Python wrapper, and a plan handle is
+    required where the chunk tables are."""
+    from b200gdn import _lib
+    host = _lib.host()
+    q, g = torch.zeros(1, 4, 2, 64), torch.zeros(1, 4, 2)
+    assert host.recurrent(q, q, q, g, g, None, None, None, None, False, 0, None, False, None) is NotImplemented   # CPU tensors
+    assert host.recurrent(q, q, q, g, 'x', None, None, None, None, False, 0, None, False, None) is NotImplemented
+    with pytest.raises(TypeError):
+        host.recurrent(q)
+    with pytest.raises(ValueError):
+        host.chunk(q, q, q, g, g, None, None, None, 1.0, False, 0, object())
