@@ -213,3 +213,27 @@ def test_state_pool_addressed_by_indices(B, T):
     assert out_pool.data_ptr() == pool.data_ptr()
     assert torch.equal(o, o_ref)
     assert torch.equal(pool, want)
+
+
+@pytest.mark.parametrize('K,V', [(128, 128), (64, 64), (32, 32), (256, 64)])
+@pytest.mark.parametrize('T', [1, 2, 16, 33, 65])
+@pytest.mark.parametrize('misaligned', [False, True])
+def test_token_blocks_and_unaligned_rows(K, V, T, misaligned):
+    """The token walk at the edges of its blocks (8 to 32 tokens by K), the single-token step, and q / k / v that do not
+    start on a 16-byte boundary (read element by element)."""
+    from b200gdn import fused_recurrent_gated_delta_rule
+    dev, H, HV = 'cuda', 2, 4
+    q, k, v, graw, braw, A_log, dt_bias, gen = _inputs(2, T, H, HV, K, V, 5, torch.bfloat16)
+    h0 = torch.randn(2, HV, K, V, generator=gen) * 0.5
+    ref_o, ref_ht = O.recurrent_step_options(q.float(), k.float(), v.float(), graw, braw, None, h0, True, True, True, A_log, dt_bias,
+                                             True, True, False)
+
+    def place(x):
+        x = x.to(dev)
+        return torch.cat([x.new_zeros(1), x.flatten()])[1:].view(x.shape) if misaligned else x
+    o, ht = fused_recurrent_gated_delta_rule(
+        place(q), place(k), place(v), graw.to(dev), beta=braw.to(dev), initial_state=h0.to(dev), output_final_state=True,
+        use_qk_l2norm_in_kernel=True, use_gate_in_kernel=True, A_log=A_log.to(dev), dt_bias=dt_bias.to(dev),
+        use_beta_sigmoid_in_kernel=True, allow_neg_eigval=True)
+    O.assert_close('o', ref_o, o.float().cpu(), 0.004)
+    O.assert_close('ht', ref_ht, ht.cpu(), 1e-5)
