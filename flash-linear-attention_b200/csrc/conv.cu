@@ -6,15 +6,18 @@
 // (k = 1..W-1) or are zero; final_state[n, d, :] holds the last W inputs of the sequence (cache entries shifted in when
 // the sequence is shorter than W).
 //
-// Pure HBM streaming: a thread owns four consecutive channels (one 8-byte access per token for bf16) and walks 32
-// consecutive tokens of one sequence (half a tile of the mixer's chunk table) with the W-1 previous inputs in
-// registers, so x is read once (plus W-1 rows of overlap per share) and y written once.  The rows reach the thread
-// through a private ring of asynchronous 8- or 16-byte copies in shared memory (sixteen tokens, twelve of them in flight
-// while four are consumed): the DRAM latency is paid once per share, not once per round of loads, and the registers
-// hold no look-ahead.  The backward pass recomputes the pre-activation, forms dx with a register ring over the W taps
-// (the W-1 tokens after the share are re-evaluated for their contribution to its dx), writes the gradient of the
-// cache for a sequence's first share, and leaves per-share partial sums of dweight / dbias that a second kernel adds
-// in a fixed order (no atomics: results are bit-reproducible).
+// HBM streaming: a thread owns four consecutive channels and walks the tokens of its share with the W-1 previous inputs in
+// registers, so x is read once (plus W-1 rows of overlap per share) and y written once.  Channels are handled in pairs by
+// two-wide fp32 instructions, loads run four to eight tokens ahead in registers, and groups of four tokens are unrolled so
+// that the history is renamed, not moved.  The backward pass recomputes the pre-activation, forms dx with a register ring
+// over the W taps (the W-1 tokens after the share are evaluated again for their contribution to its dx), writes the
+// gradient of the cache for a sequence's first share, and leaves per-share sums of dweight / dbias that a second kernel
+// adds in a fixed order (no atomics: results are bit-reproducible).
+// One token per sequence (a decoding step) has a kernel of its own: no walk, the cache as whole words.
+// bf16, W = 4, SiLU, [4, 4096, 2048]: forward 32.7 us (4.1 TB/s of x and y; 35.3 with scalar instructions behind a ring of
+// asynchronous copies), backward 61.8 us (80.9) + 4.6 (6.7) for the parameter sums; what is left to the copy rate is the
+// loads in flight per SM (an eighth forward CTA spills: 40.6 us; 16-byte accesses with eight channels a thread: 40.9).
+// A decoding step of 32 users: 2.3 us (4.9).
 #include <type_traits>
 
 #include "gdn_common.cuh"
@@ -23,315 +26,379 @@
 namespace gdn {
 namespace {
 
-constexpr int CT = 64;    // threads per CTA: 512 channels
-constexpr int SUB = 32;   // tokens per CTA: a 64-token tile is walked by two CTAs (blockIdx.z)
-constexpr int NSUB = 64 / SUB;
-constexpr int GRP = 4;    // tokens per copy group
-constexpr int NGRP = 4;   // copy groups in the ring: three in flight, one being consumed
-constexpr int RING = GRP * NGRP;
+constexpr int CT = 128;    // threads per CTA
+constexpr int C = 4;       // channels per thread
+constexpr int GRP = 4;     // tokens per group: one group is computed while one or two are being loaded
 
-__device__ __forceinline__ float silu_f(float x) { return x * fast_sigmoid(x); }
-__device__ __forceinline__ float dsilu_f(float x) {
-  const float s = fast_sigmoid(x);
-  return s * (1.f + x * (1.f - s));
-}
-
-__device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(smem_u32(smem)), "l"(gmem) : "memory");
-}
-
-// A thread's ring of rows in shared memory: slot s holds the thread's C channels of one token as PIECES pieces of
-// PB = 8 or 16 bytes, laid out [slot][piece][thread] so that the threads of a warp touch consecutive words.
-template <typename T, int C>
-struct RowRing {
-  static constexpr int BYTES = C * (int)sizeof(T);            // 8, 16 or 32
-  static constexpr int PB = BYTES < 16 ? BYTES : 16;
-  static constexpr int PIECES = BYTES / PB;
-  static constexpr size_t bytes = (size_t)RING * PIECES * CT * PB;
-  unsigned char* base;   // this thread's word of slot 0, piece 0
-  __device__ __forceinline__ unsigned char* word(int slot, int piece) const { return base + (size_t)(slot * PIECES + piece) * CT * PB; }
-  __device__ __forceinline__ void fetch(int slot, const void* src, int64_t idx) const {
-    const unsigned char* p = reinterpret_cast<const unsigned char*>(static_cast<const T*>(src) + idx);
+// the thread's channels of one token as loaded (8 bytes, 16 for fp32)
+template <typename T>
+struct Raw {
+  static constexpr int N = C * (int)sizeof(T) / 4;   // 32-bit words
+  uint32_t w[N];
+  __device__ __forceinline__ void load(const void* base, int64_t idx) {
+    const T* p = static_cast<const T*>(base) + idx;
+    if constexpr (N == 4) *reinterpret_cast<uint4*>(w) = __ldg(reinterpret_cast<const uint4*>(p));
+    else *reinterpret_cast<uint2*>(w) = __ldg(reinterpret_cast<const uint2*>(p));
+  }
+  __device__ __forceinline__ void get(uint64_t (&x)[C / 2]) const {
 #pragma unroll
-    for (int h = 0; h < PIECES; ++h) {
-      if constexpr (PB == 16) cp_async16(word(slot, h), p + h * 16);
-      else cp_async8(word(slot, h), p);
+    for (int i = 0; i < C / 2; ++i) {
+      if constexpr (sizeof(T) == 2) x[i] = widen2<T>(w[i]);
+      else x[i] = pack2(__uint_as_float(w[2 * i]), __uint_as_float(w[2 * i + 1]));
     }
   }
-  __device__ __forceinline__ void read(int slot, float (&x)[C]) const {
-    if constexpr (BYTES == 8) {
-      const uint2 u = *reinterpret_cast<const uint2*>(word(slot, 0));
-      float y[8];
-      unpack8<T>(make_uint4(u.x, u.y, 0u, 0u), y);
+};
+template <typename T>
+__device__ __forceinline__ void store_pairs(void* base, int64_t idx, const uint64_t (&x)[C / 2]) {
+  Raw<T> r;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) x[i] = y[i];
-    } else if constexpr (sizeof(T) == 2) {
-      unpack8<T>(*reinterpret_cast<const uint4*>(word(slot, 0)), x);
+  for (int i = 0; i < C / 2; ++i) {
+    if constexpr (sizeof(T) == 2) {
+      r.w[i] = narrow2<T>(x[i]);
     } else {
-#pragma unroll
-      for (int h = 0; h < PIECES; ++h) {
-        const uint4 u = *reinterpret_cast<const uint4*>(word(slot, h));
-        x[4 * h] = __uint_as_float(u.x); x[4 * h + 1] = __uint_as_float(u.y);
-        x[4 * h + 2] = __uint_as_float(u.z); x[4 * h + 3] = __uint_as_float(u.w);
-      }
+      const float2 f = unpack2(x[i]);
+      r.w[2 * i] = __float_as_uint(f.x);
+      r.w[2 * i + 1] = __float_as_uint(f.y);
     }
   }
-};
+  T* p = static_cast<T*>(base) + idx;
+  if constexpr (Raw<T>::N == 4) *reinterpret_cast<uint4*>(p) = *reinterpret_cast<const uint4*>(r.w);
+  else *reinterpret_cast<uint2*>(p) = *reinterpret_cast<const uint2*>(r.w);
+}
 
-// One CTA's share of a tile: `row` is its first token, `len` its token count, `first` / `last` say whether it starts /
-// ends its sequence, `after` how many tokens of the sequence follow it (capped at 3, the largest overlap needed).
-struct TileInfo {
-  int n, row, len;
-  bool first, last;
-  int after;
+// One CTA's share of a tile: `row` is its first token, `len` its token count, `pos` that token's place in its sequence,
+// `last` whether the share ends the sequence, `after` how many tokens of the sequence follow it (capped at 3, the
+// largest overlap needed).
+struct Share {
+  int n, row, len, pos, after;
+  bool last;
 };
-__device__ __forceinline__ TileInfo load_tile(const b200gdn_conv_args& a, int tile, int sub) {
+__device__ __forceinline__ Share load_share(const b200gdn_conv_args& a, int tile, int sub, int tokens) {
   const int4 m = reinterpret_cast<const int4*>(a.tile_meta)[tile];
   const int ntiles = a.seq_meta[2 * m.x + 1];
-  const int start = sub * SUB;
-  TileInfo ti;
-  ti.n = m.x;
-  ti.row = m.y + start;
-  ti.len = m.z - start < SUB ? m.z - start : SUB;   // <= 0: nothing to do for this CTA
-  ti.first = m.w == 0 && sub == 0;
-  const int rest = m.z - start - ti.len;            // tokens of the tile behind this share
-  ti.last = m.w == ntiles - 1 && rest <= 0;
+  const int start = sub * tokens;
+  Share s;
+  s.n = m.x;
+  s.row = m.y + start;
+  s.len = m.z - start < tokens ? m.z - start : tokens;   // <= 0: nothing to do for this CTA
+  s.pos = m.w * BT + start;
+  const int rest = m.z - start - s.len;                  // tokens of the tile behind this share
+  s.last = m.w == ntiles - 1 && rest <= 0;
   int after = rest;
   if (after < 3 && m.w < ntiles - 1) after += a.tile_meta[4 * (tile + 1) + 2];
-  ti.after = after < 3 ? (after < 0 ? 0 : after) : 3;
-  return ti;
+  s.after = after < 3 ? (after < 0 ? 0 : after) : 3;
+  return s;
 }
 
-// the W inputs before token `row` of sequence n for channels d0..d0+C-1: hist[W-1] is x[row-1]; from the rows of x for a
-// later tile, from the cache (or zeros) for a sequence's first tile
-template <typename T, int W, int C>
-__device__ __forceinline__ void load_history(const b200gdn_conv_args& a, const TileInfo& ti, int d0, float (&hist)[W][C]) {
+// x of channels d0.. at place `pos` of sequence n (row0: the row of place 0): a row of x, a cache entry, or zero
+template <typename T, int W>
+__device__ __forceinline__ void input_at(const b200gdn_conv_args& a, int n, int64_t row0, int pos, int d0, uint64_t (&x)[C / 2]) {
+  if (pos >= 0) {
+    Raw<T> r;
+    r.load(a.x, (row0 + pos) * a.D + d0);
+    r.get(x);
+  } else {
 #pragma unroll
-  for (int k = 1; k <= W; ++k) {
-    float (&h)[C] = hist[W - k];
-    if (!ti.first) {
-      load_c<T, C>(a.x, (int64_t)(ti.row - k) * a.D + d0, h);
-    } else if (a.initial_state != nullptr && k < W) {
+    for (int i = 0; i < C / 2; ++i) {
+      float v[2] = {0.f, 0.f};
+      if (a.initial_state != nullptr && pos >= -W)
 #pragma unroll
-      for (int c = 0; c < C; ++c) h[c] = Io<T>::ld(a.initial_state, ((int64_t)ti.n * a.D + d0 + c) * W + (W - k));
-    } else if (a.initial_state != nullptr) {   // k == W: the cache's oldest entry (only ever copied into the final state)
-#pragma unroll
-      for (int c = 0; c < C; ++c) h[c] = Io<T>::ld(a.initial_state, ((int64_t)ti.n * a.D + d0 + c) * W);
-    } else {
-#pragma unroll
-      for (int c = 0; c < C; ++c) h[c] = 0.f;
+        for (int e = 0; e < 2; ++e) v[e] = Io<T>::ld(a.initial_state, ((int64_t)n * a.D + d0 + 2 * i + e) * W + (W + pos));
+      x[i] = pack2(v[0], v[1]);
     }
   }
 }
 
-template <typename T, int W, int C>
-__global__ void __launch_bounds__(CT) conv_fwd_kernel(const b200gdn_conv_args a) {
-  extern __shared__ __align__(16) unsigned char ring_mem[];
+template <int W>
+struct Taps {
+  uint64_t w[W][C / 2], b[C / 2];
+  __device__ __forceinline__ void load(const b200gdn_conv_args& a, int d0) {
+#pragma unroll
+    for (int i = 0; i < C / 2; ++i) {
+      const int d = d0 + 2 * i;
+#pragma unroll
+      for (int j = 0; j < W; ++j)
+        w[j][i] = pack2(ld_param(a.weight, (int64_t)d * W + j, a.param_dtype), ld_param(a.weight, (int64_t)(d + 1) * W + j, a.param_dtype));
+      b[i] = a.bias ? pack2(ld_param(a.bias, d, a.param_dtype), ld_param(a.bias, d + 1, a.param_dtype)) : 0ull;
+    }
+  }
+  // bias + sum of the taps; hist[j] is x[t - (W-1) + j]
+  __device__ __forceinline__ uint64_t pre(const uint64_t (&hist)[W - 1][C / 2], const uint64_t (&cur)[C / 2], int i) const {
+    uint64_t acc = fma2(w[W - 1][i], cur[i], b[i]);
+#pragma unroll
+    for (int j = 0; j < W - 1; ++j) acc = fma2(w[j][i], hist[j][i], acc);
+    return acc;
+  }
+};
+
+template <typename T, int W>
+__global__ void __launch_bounds__(CT, sizeof(T) == 4 ? 5 : 7) conv_fwd_kernel(const b200gdn_conv_args a, const int tokens) {
   const int d0 = (blockIdx.y * CT + threadIdx.x) * C;
-  if (d0 >= a.D) return;   // no barrier below: every thread works on its own slots only
-  const TileInfo ti = load_tile(a, blockIdx.x, blockIdx.z);
-  if (ti.len <= 0) return;
-  const RowRing<T, C> rx{ring_mem + threadIdx.x * RowRing<T, C>::PB};
-  auto issue = [&](int gi) {   // one group: tokens 4 gi .. 4 gi + 3 of the share (an empty group past its end)
+  if (d0 >= a.D) return;
+  const Share s = load_share(a, blockIdx.x, blockIdx.z, tokens);
+  if (s.len <= 0) return;
+  const bool act = a.flags & B200GDN_CONV_SILU;
+  const int64_t base = (int64_t)s.row * a.D + d0;
+  Raw<T> buf[2][GRP];
+  auto fetch = [&](int t0, Raw<T> (&r)[GRP]) {
+#pragma unroll
+    for (int u = 0; u < GRP; ++u)
+      if (t0 + u < s.len) r[u].load(a.x, base + (int64_t)(t0 + u) * a.D);
+  };
+  fetch(0, buf[0]);
+  fetch(GRP, buf[1]);
+  Taps<W> k;
+  k.load(a, d0);
+  uint64_t hist[W - 1][C / 2];
+#pragma unroll
+  for (int j = 0; j < W - 1; ++j) input_at<T, W>(a, s.n, s.row - s.pos, s.pos - (W - 1) + j, d0, hist[j]);
+  auto group = [&](int t0, Raw<T> (&r)[GRP], auto full) {
 #pragma unroll
     for (int u = 0; u < GRP; ++u) {
-      const int t = gi * GRP + u;
-      if (t < ti.len) rx.fetch(t % RING, a.x, (int64_t)(ti.row + t) * a.D + d0);
+      if (!decltype(full)::value && t0 + u >= s.len) return;
+      uint64_t cur[C / 2], y[C / 2];
+      r[u].get(cur);
+#pragma unroll
+      for (int i = 0; i < C / 2; ++i) {
+        y[i] = k.pre(hist, cur, i);
+        if (act) y[i] = mul2(y[i], fast_sigmoid2(y[i]));
+      }
+      const int64_t off = base + (int64_t)(t0 + u) * a.D;
+      if (a.residual) {
+        Raw<T> q;
+        uint64_t res[C / 2];
+        q.load(a.residual, off);
+        q.get(res);
+#pragma unroll
+        for (int i = 0; i < C / 2; ++i) y[i] = add2(y[i], res[i]);
+      }
+      store_pairs<T>(a.y, off, y);
+#pragma unroll
+      for (int j = 0; j < W - 2; ++j)
+#pragma unroll
+        for (int i = 0; i < C / 2; ++i) hist[j][i] = hist[j + 1][i];
+#pragma unroll
+      for (int i = 0; i < C / 2; ++i) hist[W - 2][i] = cur[i];
     }
-    cp_async_commit();
   };
+  for (int t0 = 0; t0 < s.len; t0 += 2 * GRP) {
 #pragma unroll
-  for (int gi = 0; gi < NGRP - 1; ++gi) issue(gi);
-  const bool act = a.flags & B200GDN_CONV_SILU;
-  float w[W][C], b[C], hist[W][C];
-#pragma unroll
-  for (int c = 0; c < C; ++c) {
-#pragma unroll
-    for (int j = 0; j < W; ++j) w[j][c] = ld_param(a.weight, (int64_t)(d0 + c) * W + j, a.param_dtype);
-    b[c] = a.bias ? ld_param(a.bias, d0 + c, a.param_dtype) : 0.f;
-  }
-  load_history<T, W, C>(a, ti, d0, hist);
-  // one token; FULL: the token is known to lie inside the share, so nothing in the body is conditional and the
-  // compiler renames the history registers across the unrolled tokens of a group instead of moving them
-  auto token = [&](int t, auto full) {
-    if (!decltype(full)::value && t >= ti.len) return;
-    float cur[C], y[C];
-    rx.read(t % RING, cur);
-#pragma unroll
-    for (int c = 0; c < C; ++c) {
-      float acc = b[c] + w[W - 1][c] * cur[c];
-#pragma unroll
-      for (int j = 0; j < W - 1; ++j) acc += w[j][c] * hist[j + 1][c];
-      y[c] = act ? silu_f(acc) : acc;
-    }
-    const int64_t off = (int64_t)(ti.row + t) * a.D + d0;
-    if (a.residual) {
-      float r[C];
-      load_c<T, C>(a.residual, off, r);
-#pragma unroll
-      for (int c = 0; c < C; ++c) y[c] += r[c];
-    }
-    store_c<T, C>(a.y, off, y);
-#pragma unroll
-    for (int j = 0; j < W - 1; ++j)
-#pragma unroll
-      for (int c = 0; c < C; ++c) hist[j][c] = hist[j + 1][c];
-#pragma unroll
-    for (int c = 0; c < C; ++c) hist[W - 1][c] = cur[c];
-  };
-  const int n_grp = (ti.len + GRP - 1) / GRP;
-  for (int gi = 0; gi < n_grp; ++gi) {
-    issue(gi + NGRP - 1);          // into the slots the previous round has consumed
-    cp_async_wait<NGRP - 1>();     // all but the youngest three groups have landed: group gi is there
-    if ((gi + 1) * GRP <= ti.len) {
-#pragma unroll
-      for (int u = 0; u < GRP; ++u) token(gi * GRP + u, std::true_type{});
-    } else {
-#pragma unroll
-      for (int u = 0; u < GRP; ++u) token(gi * GRP + u, std::false_type{});
+    for (int h = 0; h < 2; ++h) {
+      const int t = t0 + h * GRP;
+      if (t + GRP <= s.len) group(t, buf[h], std::true_type{});
+      else if (t < s.len) group(t, buf[h], std::false_type{});
+      fetch(t + 2 * GRP, buf[h]);
     }
   }
-  cp_async_wait<0>();
-  if (a.final_state != nullptr && ti.last) {
+  if (a.final_state != nullptr && s.last) {
+    uint64_t fin[W][C / 2];   // read completely before it is written: the cache may be updated in place
 #pragma unroll
-    for (int j = 0; j < W; ++j)
+    for (int j = 0; j < W; ++j) input_at<T, W>(a, s.n, s.row - s.pos, s.pos + s.len - W + j, d0, fin[j]);
 #pragma unroll
-      for (int c = 0; c < C; ++c) Io<T>::st(a.final_state, ((int64_t)ti.n * a.D + d0 + c) * W + j, hist[j][c]);
+    for (int i = 0; i < C / 2; ++i)
+#pragma unroll
+      for (int j = 0; j < W; ++j) {
+        const float2 f = unpack2(fin[j][i]);
+        Io<T>::st(a.final_state, ((int64_t)s.n * a.D + d0 + 2 * i) * W + j, f.x);
+        Io<T>::st(a.final_state, ((int64_t)s.n * a.D + d0 + 2 * i + 1) * W + j, f.y);
+      }
   }
 }
 
-template <typename T, int W, int C>
-__global__ void __launch_bounds__(CT) conv_bwd_kernel(const b200gdn_conv_args a) {
-  extern __shared__ __align__(16) unsigned char ring_mem[];
+// One token per sequence (row n = sequence n): latency of one round of loads.  With W = 4 a thread's 16 cache entries are
+// whole 16-byte words.
+template <typename T, int W>
+__global__ void __launch_bounds__(CT) conv_step_kernel(const b200gdn_conv_args a) {
+  const int d0 = (blockIdx.x * CT + threadIdx.x) * C, n = blockIdx.y;
+  if (d0 >= a.D) return;
+  const int64_t off = (int64_t)n * a.D + d0;
+  const bool words = W == 4 && ((reinterpret_cast<uintptr_t>(a.initial_state) | reinterpret_cast<uintptr_t>(a.final_state)) & 15) == 0;
+  Raw<T> raw;
+  raw.load(a.x, off);
+  float c[C * W];   // the cache, channel after channel
+#pragma unroll
+  for (int i = 0; i < C * W; ++i) c[i] = 0.f;
+  if (a.initial_state != nullptr) {
+    if (words) {
+#pragma unroll
+      for (int i = 0; i < C * W / 8; ++i) {
+        float z[8];
+        load8<T>(a.initial_state, off * W + 8 * i, z);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) c[8 * i + e] = z[e];
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < C * W; ++i) c[i] = Io<T>::ld(a.initial_state, off * W + i);
+    }
+  }
+  Taps<W> k;
+  k.load(a, d0);
+  uint64_t cur[C / 2], y[C / 2], hist[W - 1][C / 2];
+  raw.get(cur);
+#pragma unroll
+  for (int j = 0; j < W - 1; ++j)
+#pragma unroll
+    for (int i = 0; i < C / 2; ++i) hist[j][i] = pack2(c[2 * i * W + j + 1], c[(2 * i + 1) * W + j + 1]);
+#pragma unroll
+  for (int i = 0; i < C / 2; ++i) {
+    y[i] = k.pre(hist, cur, i);
+    if (a.flags & B200GDN_CONV_SILU) y[i] = mul2(y[i], fast_sigmoid2(y[i]));
+  }
+  if (a.residual) {
+    Raw<T> q;
+    uint64_t res[C / 2];
+    q.load(a.residual, off);
+    q.get(res);
+#pragma unroll
+    for (int i = 0; i < C / 2; ++i) y[i] = add2(y[i], res[i]);
+  }
+  store_pairs<T>(a.y, off, y);
+  if (a.final_state == nullptr) return;
+#pragma unroll
+  for (int i = 0; i < C; ++i) {   // shift the token in
+    const float2 f = unpack2(cur[i / 2]);
+#pragma unroll
+    for (int j = 0; j < W - 1; ++j) c[i * W + j] = c[i * W + j + 1];
+    c[i * W + W - 1] = i & 1 ? f.y : f.x;
+  }
+  if (words) {
+#pragma unroll
+    for (int i = 0; i < C * W / 8; ++i) {
+      float z[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) z[e] = c[8 * i + e];
+      store8<T>(a.final_state, off * W + 8 * i, z);
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < C * W; ++i) Io<T>::st(a.final_state, off * W + i, c[i]);
+  }
+}
+
+template <typename T, int W>
+__global__ void __launch_bounds__(CT, sizeof(T) == 4 ? 3 : 4) conv_bwd_kernel(const b200gdn_conv_args a, const int tokens) {
   const int d0 = (blockIdx.y * CT + threadIdx.x) * C;
-  if (d0 >= a.D) return;   // no barrier below: every thread works on its own slots only
-  const int tile = blockIdx.x;
-  const TileInfo ti = load_tile(a, tile, blockIdx.z);
+  if (d0 >= a.D) return;
+  const Share s = load_share(a, blockIdx.x, blockIdx.z, tokens);
   const bool act = a.flags & B200GDN_CONV_SILU;
-  float* const part = a.partials ? a.partials + (((int64_t)tile * NSUB + blockIdx.z) * a.D + d0) * (W + 1) : nullptr;
-  if (ti.len <= 0) {   // no token in this share: its partial sums are zeros
+  // sums of this share: [W + 1][D], taps then bias
+  float* const part = a.partials ? a.partials + ((int64_t)blockIdx.x * gridDim.z + blockIdx.z) * (W + 1) * a.D + d0 : nullptr;
+  auto put = [&](int j, const uint64_t (&x)[C / 2]) {
+    const float2 p = unpack2(x[0]), q = unpack2(x[1]);
+    *reinterpret_cast<float4*>(part + (int64_t)j * a.D) = make_float4(p.x, p.y, q.x, q.y);
+  };
+  if (s.len <= 0) {   // no token in this share: its sums are zeros
+    const uint64_t zero[C / 2] = {};
     if (part != nullptr)
-      for (int i = 0; i < C * (W + 1); ++i) part[i] = 0.f;
+      for (int j = 0; j <= W; ++j) put(j, zero);
     return;
   }
   // tokens of the same sequence after this share whose pre-activation gradient reaches its dx
-  const int nxt = ti.after < W - 1 ? ti.after : W - 1;
-  const int n_tok = ti.len + nxt;
-  const RowRing<T, C> rx{ring_mem + threadIdx.x * RowRing<T, C>::PB}, rdy{ring_mem + RowRing<T, C>::bytes + threadIdx.x * RowRing<T, C>::PB};
-  auto issue = [&](int gi) {
+  const int n_tok = s.len + (s.after < W - 1 ? s.after : W - 1);
+  const int64_t base = (int64_t)s.row * a.D + d0;
+  Raw<T> bx[2][GRP], by[2][GRP];
+  auto fetch = [&](int t0, Raw<T> (&rx)[GRP], Raw<T> (&ry)[GRP]) {
 #pragma unroll
-    for (int u = 0; u < GRP; ++u) {
-      const int t = gi * GRP + u;
-      if (t < n_tok) {
-        const int64_t off = (int64_t)(ti.row + t) * a.D + d0;
-        rx.fetch(t % RING, a.x, off);
-        rdy.fetch(t % RING, a.dy, off);
+    for (int u = 0; u < GRP; ++u)
+      if (t0 + u < n_tok) {
+        rx[u].load(a.x, base + (int64_t)(t0 + u) * a.D);
+        ry[u].load(a.dy, base + (int64_t)(t0 + u) * a.D);
       }
-    }
-    cp_async_commit();
   };
+  fetch(0, bx[0], by[0]);
+  fetch(GRP, bx[1], by[1]);
+  Taps<W> k;
+  k.load(a, d0);
+  uint64_t hist[W - 1][C / 2];
 #pragma unroll
-  for (int gi = 0; gi < NGRP - 1; ++gi) issue(gi);
-  float w[W][C], b[C], hist[W][C];
+  for (int j = 0; j < W - 1; ++j) input_at<T, W>(a, s.n, s.row - s.pos, s.pos - (W - 1) + j, d0, hist[j]);
+  uint64_t ring[W - 1][C / 2];   // ring[m]: dx of token (u - 1 - m) so far, u the token being processed
+  uint64_t dw[W][C / 2], db[C / 2];
 #pragma unroll
-  for (int c = 0; c < C; ++c) {
+  for (int i = 0; i < C / 2; ++i) {
+    db[i] = 0ull;
 #pragma unroll
-    for (int j = 0; j < W; ++j) w[j][c] = ld_param(a.weight, (int64_t)(d0 + c) * W + j, a.param_dtype);
-    b[c] = a.bias ? ld_param(a.bias, d0 + c, a.param_dtype) : 0.f;
+    for (int j = 0; j < W; ++j) dw[j][i] = 0ull;
+#pragma unroll
+    for (int j = 0; j < W - 1; ++j) ring[j][i] = 0ull;
   }
-  load_history<T, W, C>(a, ti, d0, hist);
-  float ring[W][C];   // ring[k]: dx of token (u - k) so far, u the token being processed
-  float dw[W][C], db[C];
-#pragma unroll
-  for (int j = 0; j < W; ++j)
-#pragma unroll
-    for (int c = 0; c < C; ++c) { ring[j][c] = 0.f; dw[j][c] = 0.f; }
-#pragma unroll
-  for (int c = 0; c < C; ++c) db[c] = 0.f;
-  const int lo = (ti.first && a.dinitial_state != nullptr) ? -(W - 1) : 0;   // first token whose dx this share emits
+  const bool to_cache = s.pos == 0 && a.dinitial_state != nullptr;
   const int last = n_tok - 1 + (W - 1);   // the extra steps only flush the ring
-  // one step; FULL: the token is known to lie inside the share (it is loaded, counted for the parameters, and no
-  // step of its group is past the end), so only the store is conditional and the compiler renames the history and
-  // ring registers across the unrolled steps of a group instead of moving them
-  auto step = [&](int u, auto full) {
+  const uint64_t one = pack2(1.f, 1.f), mone = pack2(-1.f, -1.f);
+  // one step; FULL: the token is known to lie inside the share (it is loaded and counted for the parameters), so only the
+  // store is conditional and the compiler renames the history and ring registers across the unrolled steps of a group
+  auto step = [&](int u, const Raw<T>& rx, const Raw<T>& ry, auto full) {
     constexpr bool FULL = decltype(full)::value;
     if (!FULL && u > last) return;
-    float dpre[C];
+    uint64_t dpre[C / 2];
     if (FULL || u < n_tok) {
-      float cur[C], dy[C];
-      rx.read(u % RING, cur);
-      rdy.read(u % RING, dy);
+      uint64_t cur[C / 2];
+      rx.get(cur);
+      ry.get(dpre);
 #pragma unroll
-      for (int c = 0; c < C; ++c) {
-        float acc = b[c] + w[W - 1][c] * cur[c];
-#pragma unroll
-        for (int j = 0; j < W - 1; ++j) acc += w[j][c] * hist[j + 1][c];
-        dpre[c] = act ? dy[c] * dsilu_f(acc) : dy[c];
-      }
-      if (FULL || u < ti.len) {   // the parameters' gradients: every token is counted by the share that owns it
-#pragma unroll
-        for (int c = 0; c < C; ++c) {
-          db[c] += dpre[c];
-          dw[W - 1][c] += dpre[c] * cur[c];
-#pragma unroll
-          for (int j = 0; j < W - 1; ++j) dw[j][c] += dpre[c] * hist[j + 1][c];
+      for (int i = 0; i < C / 2; ++i) {
+        if (act) {   // d silu(p) = s (1 + p (1 - s))
+          const uint64_t p = k.pre(hist, cur, i), sg = fast_sigmoid2(p);
+          dpre[i] = mul2(dpre[i], mul2(sg, fma2(p, fma2(sg, mone, one), one)));
         }
+        if (FULL || u < s.len) {   // the parameters' gradients: every token is counted by the share that owns it
+          db[i] = add2(db[i], dpre[i]);
+          dw[W - 1][i] = fma2(dpre[i], cur[i], dw[W - 1][i]);
+#pragma unroll
+          for (int j = 0; j < W - 1; ++j) dw[j][i] = fma2(dpre[i], hist[j][i], dw[j][i]);
+        }
+#pragma unroll
+        for (int j = 0; j < W - 2; ++j) hist[j][i] = hist[j + 1][i];
+        hist[W - 2][i] = cur[i];
       }
-#pragma unroll
-      for (int j = 0; j < W - 1; ++j)
-#pragma unroll
-        for (int c = 0; c < C; ++c) hist[j][c] = hist[j + 1][c];
-#pragma unroll
-      for (int c = 0; c < C; ++c) hist[W - 1][c] = cur[c];
     } else {
 #pragma unroll
-      for (int c = 0; c < C; ++c) dpre[c] = 0.f;
+      for (int i = 0; i < C / 2; ++i) dpre[i] = 0ull;
     }
-    // dpre[u] reaches token u - k through tap W - 1 - k
+    // dpre[u] reaches token u - m through tap W - 1 - m; token u - (W - 1) is complete with it
+    uint64_t done[C / 2];
 #pragma unroll
-    for (int k = 0; k < W; ++k)
+    for (int i = 0; i < C / 2; ++i) {
+      done[i] = fma2(k.w[0][i], dpre[i], ring[W - 2][i]);
 #pragma unroll
-      for (int c = 0; c < C; ++c) ring[k][c] += w[W - 1 - k][c] * dpre[c];
-    const int s = u - (W - 1);   // this token has now received every contribution
-    if (s >= lo && s < ti.len) {
-      if (s >= 0) {
-        store_c<T, C>(a.dx, (int64_t)(ti.row + s) * a.D + d0, ring[W - 1]);
-      } else {   // an input before the sequence start: gradient of the cache entry x[s] = initial_state[n, d, W + s]
+      for (int m = W - 2; m > 0; --m) ring[m][i] = fma2(k.w[W - 1 - m][i], dpre[i], ring[m - 1][i]);
+      ring[0][i] = mul2(k.w[W - 1][i], dpre[i]);
+    }
+    const int e = u - (W - 1);
+    if (e >= 0) {
+      if (e < s.len) store_pairs<T>(a.dx, base + (int64_t)e * a.D, done);
+    } else if (to_cache) {   // an input before the sequence start: gradient of the cache entry x[e] = initial_state[n, d, W + e]
 #pragma unroll
-        for (int c = 0; c < C; ++c) Io<T>::st(a.dinitial_state, ((int64_t)ti.n * a.D + d0 + c) * W + (W + s), ring[W - 1][c]);
+      for (int i = 0; i < C / 2; ++i) {
+        const float2 f = unpack2(done[i]);
+        Io<T>::st(a.dinitial_state, ((int64_t)s.n * a.D + d0 + 2 * i) * W + (W + e), f.x);
+        Io<T>::st(a.dinitial_state, ((int64_t)s.n * a.D + d0 + 2 * i + 1) * W + (W + e), f.y);
       }
     }
-#pragma unroll
-    for (int k = W - 1; k > 0; --k)
-#pragma unroll
-      for (int c = 0; c < C; ++c) ring[k][c] = ring[k - 1][c];
-#pragma unroll
-    for (int c = 0; c < C; ++c) ring[0][c] = 0.f;
   };
-  for (int gi = 0; gi * GRP <= last; ++gi) {
-    issue(gi + NGRP - 1);          // into the slots the previous round has consumed
-    cp_async_wait<NGRP - 1>();     // group gi is there
-    if ((gi + 1) * GRP <= ti.len) {
+  for (int t0 = 0; t0 <= last; t0 += 2 * GRP) {
 #pragma unroll
-      for (int v = 0; v < GRP; ++v) step(gi * GRP + v, std::true_type{});
-    } else {
+    for (int h = 0; h < 2; ++h) {
+      const int t = t0 + h * GRP;
+      if (t + GRP <= s.len) {
 #pragma unroll
-      for (int v = 0; v < GRP; ++v) step(gi * GRP + v, std::false_type{});
+        for (int v = 0; v < GRP; ++v) step(t + v, bx[h][v], by[h][v], std::true_type{});
+      } else {
+#pragma unroll
+        for (int v = 0; v < GRP; ++v) step(t + v, bx[h][v], by[h][v], std::false_type{});
+      }
+      fetch(t + 2 * GRP, bx[h], by[h]);
     }
   }
-  cp_async_wait<0>();
-  if (ti.first && a.dinitial_state != nullptr) {   // the cache's oldest entry never enters the convolution
+  if (to_cache) {   // the cache's oldest entry never enters the convolution
 #pragma unroll
-    for (int c = 0; c < C; ++c) Io<T>::st(a.dinitial_state, ((int64_t)ti.n * a.D + d0 + c) * W, 0.f);
+    for (int c = 0; c < C; ++c) Io<T>::st(a.dinitial_state, ((int64_t)s.n * a.D + d0 + c) * W, 0.f);
   }
   if (part != nullptr) {
-    float* p = part;
 #pragma unroll
-    for (int c = 0; c < C; ++c) {
-#pragma unroll
-      for (int j = 0; j < W; ++j) p[c * (W + 1) + j] = dw[j][c];
-      p[c * (W + 1) + W] = db[c];
-    }
+    for (int j = 0; j < W; ++j) put(j, dw[j]);
+    put(W, db);
   }
 }
 
@@ -339,54 +406,58 @@ __global__ void __launch_bounds__(CT) conv_bwd_kernel(const b200gdn_conv_args a)
 // consecutive outputs (four interleaved running sums, so that the loads overlap), then the sixteen sums are added in
 // warp order
 constexpr int RW = 16;
-__global__ void __launch_bounds__(32 * RW) conv_param_reduce_kernel(const b200gdn_conv_args a) {
+__global__ void __launch_bounds__(32 * RW) conv_param_reduce_kernel(const b200gdn_conv_args a, const int n) {
   __shared__ float part[RW][32];
   const int lane = threadIdx.x & 31, q = threadIdx.x >> 5;
-  const int64_t per_tile = (int64_t)a.D * (a.W + 1);
+  const int64_t per_share = (int64_t)a.D * (a.W + 1);
   const int64_t i = (int64_t)blockIdx.x * 32 + lane;
   float s4[4] = {0.f, 0.f, 0.f, 0.f};
-  if (i < per_tile) {
-    const int n = a.n_tiles * NSUB;
+  if (i < per_share) {
     int t = q;
     for (; t + 3 * RW < n; t += 4 * RW) {
 #pragma unroll
-      for (int e = 0; e < 4; ++e) s4[e] += a.partials[(int64_t)(t + e * RW) * per_tile + i];
+      for (int e = 0; e < 4; ++e) s4[e] += a.partials[(int64_t)(t + e * RW) * per_share + i];
     }
-    for (; t < n; t += RW) s4[0] += a.partials[(int64_t)t * per_tile + i];
+    for (; t < n; t += RW) s4[0] += a.partials[(int64_t)t * per_share + i];
   }
   float s = (s4[0] + s4[1]) + (s4[2] + s4[3]);
   part[q][lane] = s;
   __syncthreads();
-  if (q != 0 || i >= per_tile) return;
+  if (q != 0 || i >= per_share) return;
 #pragma unroll
   for (int r = 1; r < RW; ++r) s += part[r][lane];
-  const int d = (int)(i / (a.W + 1)), j = (int)(i % (a.W + 1));
+  const int j = (int)(i / a.D), d = (int)(i % a.D);
   if (j < a.W) st_param(a.dweight, (int64_t)d * a.W + j, a.param_dtype, s);
   else if (a.dbias != nullptr) st_param(a.dbias, d, a.param_dtype, s);
 }
 
-// channels per thread: four in both passes.  With eight (16-byte accesses for bf16) the per-channel state of the backward
-// pass (taps, history, dx ring, parameter sums) caps the SM at eight warps, and the forward pass at sixteen; the kernels
-// are bound by instruction issue and dependent chains, not by access width, so the extra warps win (measured).
-constexpr int C_FWD = 4, C_BWD = 4;
+// Tokens per share: a whole tile of 64 while that still gives the SMs twelve warps each, else 32 (and 16 forward; a
+// backward share also costs a row of parameter sums, and the workspace holds two per tile).
+int share_tokens(const b200gdn_conv_args& a, int least) {
+  int64_t warps = (int64_t)a.n_tiles * ((a.D / C + 31) / 32);
+  int tokens = 64;
+  for (; tokens > least && warps < 148 * 12; warps *= 2) tokens /= 2;
+  return tokens;
+}
 
 template <typename T, int W>
 int launch_t(const b200gdn_conv_args& a, cudaStream_t st, bool bwd) {
+  const unsigned y = (a.D / C + CT - 1) / CT;
   if (!bwd) {
-    dim3 grid(a.n_tiles, (a.D / C_FWD + CT - 1) / CT, NSUB);
-    constexpr size_t smem = RowRing<T, C_FWD>::bytes;
-    if (int e = ensure_smem(conv_fwd_kernel<T, W, C_FWD>, smem)) return e;
-    conv_fwd_kernel<T, W, C_FWD><<<grid, CT, smem, st>>>(a);
+    if (a.rows == a.n_tiles && a.n_seq == a.n_tiles && a.n_seq <= 65535) {   // every sequence is one token
+      conv_step_kernel<T, W><<<dim3(y, a.n_seq), CT, 0, st>>>(a);
+      return check_launch("conv_step");
+    }
+    const int tokens = share_tokens(a, 16);
+    conv_fwd_kernel<T, W><<<dim3(a.n_tiles, y, 64 / tokens), CT, 0, st>>>(a, tokens);
     return check_launch("conv_fwd");
   }
-  dim3 grid(a.n_tiles, (a.D / C_BWD + CT - 1) / CT, NSUB);
-  constexpr size_t smem = 2 * RowRing<T, C_BWD>::bytes;
-  if (int e = ensure_smem(conv_bwd_kernel<T, W, C_BWD>, smem)) return e;
-  conv_bwd_kernel<T, W, C_BWD><<<grid, CT, smem, st>>>(a);
+  const int tokens = share_tokens(a, 32);
+  conv_bwd_kernel<T, W><<<dim3(a.n_tiles, y, 64 / tokens), CT, 0, st>>>(a, tokens);
   if (int e = check_launch("conv_bwd")) return e;
   if (a.partials != nullptr && a.dweight != nullptr) {
     const int64_t n = (int64_t)a.D * (a.W + 1);
-    conv_param_reduce_kernel<<<(unsigned)((n + 31) / 32), 32 * RW, 0, st>>>(a);
+    conv_param_reduce_kernel<<<(unsigned)((n + 31) / 32), 32 * RW, 0, st>>>(a, a.n_tiles * (64 / tokens));
     return check_launch("conv_param_reduce");
   }
   return 0;

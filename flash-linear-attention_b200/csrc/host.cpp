@@ -58,13 +58,15 @@ Tensor new_tensor(at::IntArrayRef sizes, at::ScalarType t, const at::Device& dev
   if (zero) x.zero_();
   return x;
 }
-// the tensor itself when it has that type and is contiguous already
-Tensor dense(const Tensor& x, at::ScalarType t) {
+// the tensor itself when it has that type, is contiguous and starts on the 16-byte boundary the kernels' copies need
+Tensor dense(const Tensor& x) {
   if (!x.defined()) return x;
-  const Tensor y = x.scalar_type() == t ? x : x.to(t);
-  return y.is_contiguous() ? y : y.contiguous();
+  const Tensor y = x.is_contiguous() ? x : x.contiguous();
+  return (reinterpret_cast<uintptr_t>(y.data_ptr()) & 15) ? y.clone() : y;
 }
-Tensor dense(const Tensor& x) { return !x.defined() || x.is_contiguous() ? x : x.contiguous(); }
+Tensor dense(const Tensor& x, at::ScalarType t) { return !x.defined() || x.scalar_type() == t ? dense(x) : dense(x.to(t)); }
+// a state that may be updated in place is never moved (the kernels take a slower path, or say that they do not serve it)
+Tensor dense_state(const Tensor& x, at::ScalarType t) { return !x.defined() ? x : x.to(t).contiguous(); }
 Tensor cast(const Tensor& x, at::ScalarType t) { return !x.defined() || x.scalar_type() == t ? x : x.to(t); }
 void* ptr(const Tensor& x) { return x.defined() ? x.data_ptr() : nullptr; }
 float* fptr(const Tensor& x) { return static_cast<float*>(ptr(x)); }
@@ -153,7 +155,7 @@ std::pair<Tensor, Tensor> recurrent(Tensor q, Tensor k, Tensor v, Tensor g, Tens
   Tensor cu = cu_seqlens;
   if (cu.defined()) cu = cu.to(dev, at::kInt).contiguous();
   a.gb_dtype = gate_types(g, beta);
-  const Tensor A = dense(A_log, at::kFloat), bias = dense(dt_bias, at::kFloat), h0 = dense(initial_state, at::kFloat);
+  const Tensor A = dense(A_log, at::kFloat), bias = dense(dt_bias, at::kFloat), h0 = dense_state(initial_state, at::kFloat);
   a.cu_seqlens = iptr(cu);
   a.q = ptr(q);
   a.k = ptr(k);
@@ -520,7 +522,7 @@ ConvForward conv_forward(const Tensor& x, const Tensor& weight, const Tensor& bi
   r.b = bias;
   s->param_dtype = gate_types(r.w, r.b);   // weight and bias in one element type the kernels read
   const Tensor res = dense(residual, t);
-  r.h0 = dense(initial_state, t);
+  r.h0 = dense_state(initial_state, t);
   if (initial_state.defined()) s->ht = initial_state.scalar_type();
   const int64_t D = x.size(2);
   r.y = new_tensor(r.x.sizes(), t, dev, !plan->covered);

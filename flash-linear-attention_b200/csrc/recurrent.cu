@@ -43,28 +43,6 @@ __device__ __forceinline__ int64_t state_slot(const b200gdn_recurrent_args& a, i
   return slot;
 }
 
-// two fp32 multiply-adds in one instruction
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
-  uint64_t d;
-  asm("mul.rn.f32x2 %0, %1, %2;\n" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
-  uint64_t d;
-  asm("mov.b64 %0, {%1, %2};\n" : "=l"(d) : "f"(lo), "f"(hi));
-  return d;
-}
-__device__ __forceinline__ float2 unpack2(uint64_t v) {
-  float2 f;
-  asm("mov.b64 {%0, %1}, %2;\n" : "=f"(f.x), "=f"(f.y) : "l"(v));
-  return f;
-}
-
 // RPL consecutive elements (a lane's rows of q or k) as fp32 pairs
 template <typename T, int RPL>
 __device__ __forceinline__ void load_pairs(const void* base, int64_t idx, bool wide, uint64_t (&x)[RPL / 2]) {
@@ -81,14 +59,7 @@ __device__ __forceinline__ void load_pairs(const void* base, int64_t idx, bool w
         w[0] = *reinterpret_cast<const uint32_t*>(p);
       }
 #pragma unroll
-      for (int i = 0; i < RPL / 2; ++i) {
-        if constexpr (!std::is_same<T, __half>::value) {
-          x[i] = pack2(__uint_as_float(w[i] << 16), __uint_as_float(w[i] & 0xffff0000u));
-        } else {
-          const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
-          x[i] = pack2(f.x, f.y);
-        }
-      }
+      for (int i = 0; i < RPL / 2; ++i) x[i] = widen2<T>(w[i]);
       return;
     }
   } else if (wide) {

@@ -110,6 +110,54 @@ __device__ __forceinline__ void store_c(void* base, int64_t idx, const float (&x
   }
 }
 
+// ---- two fp32 operations in one instruction (channel or row pairs; each half rounds like the scalar instruction) ------
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;\n" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;\n" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+  uint64_t d;
+  asm("mov.b64 %0, {%1, %2};\n" : "=l"(d) : "f"(lo), "f"(hi));
+  return d;
+}
+__device__ __forceinline__ float2 unpack2(uint64_t v) {
+  float2 f;
+  asm("mov.b64 {%0, %1}, %2;\n" : "=f"(f.x), "=f"(f.y) : "l"(v));
+  return f;
+}
+// one 32-bit word of two 16-bit elements <-> an fp32 pair
+template <typename T>
+__device__ __forceinline__ uint64_t widen2(uint32_t w) {
+  if constexpr (!std::is_same<T, __half>::value) {
+    return pack2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
+  } else {
+    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w));
+    return pack2(f.x, f.y);
+  }
+}
+template <typename T>
+__device__ __forceinline__ uint32_t narrow2(uint64_t v) {
+  const float2 f = unpack2(v);
+  if constexpr (!std::is_same<T, __half>::value) {
+    const __nv_bfloat162 p = __floats2bfloat162_rn(f.x, f.y);
+    return *reinterpret_cast<const uint32_t*>(&p);
+  } else {
+    const __half2 p = __floats2half2_rn(f.x, f.y);
+    return *reinterpret_cast<const uint32_t*>(&p);
+  }
+}
+
 // sigmoid with two MUFU instructions (ex2.approx.ftz, rcp.approx.ftz: about 2 ulp each; the library forms of exp and
 // division add range handling that costs more instructions than the rest of an element's work in these kernels)
 __device__ __forceinline__ float fast_sigmoid(float x) {
@@ -117,6 +165,17 @@ __device__ __forceinline__ float fast_sigmoid(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;\n" : "=f"(e) : "f"(x * -1.4426950408889634f));
   asm("rcp.approx.ftz.f32 %0, %1;\n" : "=f"(r) : "f"(1.f + e));
   return r;
+}
+// the same for a pair
+__device__ __forceinline__ uint64_t fast_sigmoid2(uint64_t x) {
+  const float2 z = unpack2(mul2(x, pack2(-1.4426950408889634f, -1.4426950408889634f)));
+  float2 e, r;
+  asm("ex2.approx.ftz.f32 %0, %1;\n" : "=f"(e.x) : "f"(z.x));
+  asm("ex2.approx.ftz.f32 %0, %1;\n" : "=f"(e.y) : "f"(z.y));
+  const float2 d = unpack2(add2(pack2(e.x, e.y), pack2(1.f, 1.f)));
+  asm("rcp.approx.ftz.f32 %0, %1;\n" : "=f"(r.x) : "f"(d.x));
+  asm("rcp.approx.ftz.f32 %0, %1;\n" : "=f"(r.y) : "f"(d.y));
+  return pack2(r.x, r.y);
 }
 
 }  // namespace gdn

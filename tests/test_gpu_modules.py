@@ -135,3 +135,23 @@ def test_module_errors():
         rms_norm_gated(x, x, None, residual=x)
     with pytest.raises(B200GDNError, match='are built'):
         rms_norm_gated(torch.zeros(4, 96, device='cuda'), torch.zeros(4, 96, device='cuda'), None)
+
+
+@pytest.mark.parametrize('W', [2, 3, 4])
+@pytest.mark.parametrize('misaligned', [False, True])
+def test_conv_single_token_step(W, misaligned):
+    """One token per sequence: the same output and shifted cache as the general walk, in place, also for a cache that does
+    not start on a 16-byte boundary."""
+    from b200gdn.modules import causal_conv1d
+    gen = torch.Generator(device='cuda').manual_seed(W)
+    rn = lambda *s: torch.randn(*s, device='cuda', generator=gen).to(torch.bfloat16)
+    N, D = 5, 520
+    x, w, b, r, c = rn(N, 1, D), rn(D, W), rn(D), rn(N, 1, D), rn(N, D, W)
+    want = (c[..., 1:].float() * w[:, :-1].float()).sum(-1) + x[:, 0].float() * w[:, -1].float() + b.float()
+    want = want * torch.sigmoid(want) + r[:, 0].float()
+    cache = torch.cat([c.new_zeros(1), c.flatten()])[1:].view(c.shape) if misaligned else c.clone()
+    with torch.no_grad():
+        y, new = causal_conv1d(x, w, b, r, cache, True, 'silu', inplace_state=True)
+    assert new.data_ptr() == cache.data_ptr()
+    O.assert_close('y', want.cpu(), y[:, 0].float().cpu(), 4e-3)
+    assert torch.equal(new, torch.cat([c[..., 1:], x[:, 0, :, None]], -1))
