@@ -67,7 +67,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_dqk_kernel(const b200gdn_chun
   uint64_t* bar_c = bar + 3;   // q, k (once)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar + 4);
 
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int q = warp & 3, hc = warp >> 2;
   const int g = lane >> 2, t = lane & 3;
   const int c = blockIdx.x, hq = blockIdx.y;
@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_dqk_kernel(const b200gdn_chun
     if (__syncthreads_or(failed)) { failed = true; break; }
 
     // ---- phase 1: dP = do v_new^T
-    if (tid == 0) {
+    if (warp == 0) {
       tc5::fence_after_sync();
       issue_mma_t<DV / 16>(TM_DP, Operand{tc5::smem_addr(Do), BT, 0}, Operand{tc5::smem_addr(Vn), BT, 0}, 64, 64, 0);
       ph.commit();
@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_dqk_kernel(const b200gdn_chun
         par_b ^= 1u;
         if (__syncthreads_or(failed)) { failed = true; break; }
       }
-      if (tid == 0) {
+      if (warp == 0) {
         tc5::fence_after_sync();
         issue_mma_t<4>(TM_DQ, Operand{tc5::smem_addr(Do) + p * BT * 128, BT, 0}, Operand{tc5::smem_addr(Hp), DK, 0}, 64, DK, p > 0);
         issue_mma_t<4>(TM_DKS, Operand{tc5::smem_addr(Vn) + p * BT * 128, BT, 0}, Operand{tc5::smem_addr(dHp), DK, 0}, 64, DK,
@@ -315,7 +315,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_dqk_kernel(const b200gdn_chun
     __syncthreads();  // every warp has drained the dq columns; staging tile complete
 
     // ---- phase 3: dk_intra = dP~^T q (into the columns dq just left)
-    if (tid == 0) {
+    if (warp == 0) {
       tc5::fence_after_sync();
       issue_mma_t<4>(TM_DKI, opPm, opQ, 64, DK, 0);
       ph.commit();

@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_wy_kernel(const b200gdn_chunk
   uint64_t* bar_ld = bar + 1;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_ld + 1);
 
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int q = warp & 3, hc = warp >> 2;
   const int g = lane >> 2, t = lane & 3;
   const int c = blockIdx.x, hq = blockIdx.y;
@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_wy_kernel(const b200gdn_chunk
     if (__syncthreads_or(failed)) { failed = true; break; }
 
     // ---- phase 1: dW = -dU h^T | dA2 = dU V^T | KK = K K^T
-    if (tid == 0) {
+    if (warp == 0) {
       tc5::fence_after_sync();
       issue_mma_t<DV / 16>(TM_BIG, opdU_k, Operand{tc5::smem_addr(Hs), DK, 0}, 64, DK, 0, /*neg_a=*/1);
       issue_mma_t<DV / 16>(TM_S1, opdU_k, Operand{tc5::smem_addr(Vs), BT, 0}, 64, 64, 0);
@@ -237,7 +237,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_wy_kernel(const b200gdn_chunk
     __syncthreads();
 
     // ---- phase 2: dA1 = dW K^T | dVb = A^T dU
-    if (tid == 0) {
+    if (warp == 0) {
       tc5::fence_after_sync();
       issue_mma_t<DK / 16>(TM_S1, opdW_k, opK_k, 64, 64, 0);
       issue_mma_t<BT / 16>(TM_BIG, opA_mn, opdU_mn, 64, DV, 0);
@@ -285,7 +285,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_wy_kernel(const b200gdn_chunk
       __syncthreads();
 
       // ---- phase 3: Y = dA A^T | dk = (A beta 2^gamma)^T dW
-      if (tid == 0) {
+      if (warp == 0) {
         tc5::fence_after_sync();
         issue_mma_t<BT / 16>(TM_S1, Operand{tc5::smem_addr(dAs), BT, 0}, opA_k, 64, 64, 0);
         issue_mma_t<BT / 16>(TM_BIG, opAb_mn, opdW_mn, 64, DK, 0);
@@ -341,7 +341,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_wy_kernel(const b200gdn_chunk
     __syncthreads();
 
     // ---- phase 4: X = A^T Y
-    if (tid == 0) {
+    if (warp == 0) {
       tc5::fence_after_sync();
       issue_mma_t<BT / 16>(TM_S1, opA_mn, Operand{tc5::smem_addr(Ys), BT, 1}, 64, 64, 0);
       ph.commit();
@@ -373,7 +373,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_wy_kernel(const b200gdn_chunk
     __syncthreads();
 
     // ---- phase 5: dk += M2 K + M2^T K
-    if (tid == 0) {
+    if (warp == 0) {
       tc5::fence_after_sync();
       issue_mma_t<BT / 16>(TM_BIG, Operand{tc5::smem_addr(M2s), BT, 0}, opK_mn, 64, DK, 1);
       issue_mma_t<BT / 16>(TM_BIG, Operand{tc5::smem_addr(M2s), BT, 1}, opK_mn, 64, DK, 1);

@@ -42,7 +42,7 @@ __global__ void __launch_bounds__(NTHREADS, 4) dv_local_kernel(const b200gdn_chu
   uint64_t* bar_mma = bar_ld + 1;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_mma + 1);
 
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int g = lane >> 2, t = lane & 3;
   const int c = blockIdx.x, hv = blockIdx.y;
   const int G = a.HV / a.H, hq = hv / G;
@@ -82,7 +82,7 @@ __global__ void __launch_bounds__(NTHREADS, 4) dv_local_kernel(const b200gdn_chu
   }
   if (!tc5::mbar_wait(bar_ld, 0)) failed = true;
 
-  if (tid == 0 && !failed) {
+  if (warp == 0 && __all_sync(0xffffffffu, !failed)) {
     tc5::fence_after_sync();
     issue_mma_t<DK / 16>(TM_P, Operand{tc5::smem_addr(Qs), BT, 0}, Operand{tc5::smem_addr(Ks), BT, 0}, 64, 64, 0);
     ph.commit();
@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(NTHREADS, 4) dv_local_kernel(const b200gdn_chu
     tc5::fence_before_sync();
     __syncthreads();
     // dv_local = P^T do
-    if (tid == 0) {
+    if (warp == 0) {
       tc5::fence_after_sync();
       issue_mma_t<BT / 16>(TM_D, Operand{tc5::smem_addr(Ps), BT, 1}, Operand{tc5::smem_addr(Ds), BT, 1}, 64, DV, 0);
       ph.commit();

@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(NTHREADS, 4) intra_fwd_kernel(const b200gdn_ch
   uint64_t* bar_v = bar + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar + 3);
 
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int q = warp & 3, hc = warp >> 2;
   const int g = lane >> 2, t = lane & 3;
   const int c = blockIdx.x, hv = blockIdx.y;
@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(NTHREADS, 4) intra_fwd_kernel(const b200gdn_ch
   if (__syncthreads_or(failed)) {
     failed = true;
   } else {
-    if (tid == 0) {
+    if (warp == 0) {
       tc5::fence_after_sync();
       issue_mma_t<DK / 16>(tm, Operand{tc5::smem_addr(Ks), BT, 0}, Operand{tc5::smem_addr(Ks), BT, 0}, 64, 64, 0);
       if (with_qk) issue_mma_t<DK / 16>(tm + 64, Operand{tc5::smem_addr(Qs), BT, 0}, Operand{tc5::smem_addr(Ks), BT, 0}, 64, 64, 0);
@@ -322,7 +322,7 @@ __global__ void __launch_bounds__(NTHREADS, 4) intra_fwd_kernel(const b200gdn_ch
     __syncthreads();
 
     // ---- W = Aw K   (K as an MN-major B operand: contraction over the token rows)
-    if (tid == 0) {
+    if (warp == 0) {
       tc5::fence_after_sync();
       issue_mma_t<BT / 16>(tm, Operand{tc5::smem_addr(Aw), BT, 0}, Operand{tc5::smem_addr(Ks), BT, 1}, 64, DK, 0);
       ph.commit();
@@ -343,7 +343,7 @@ __global__ void __launch_bounds__(NTHREADS, 4) intra_fwd_kernel(const b200gdn_ch
       tc5::fence_before_sync();
       __syncthreads();   // W has left tensor memory, K is no longer an operand
       // ---- U = Au V into the same columns, while W is converted and staged over the K tile
-      if (tid == 0) {
+      if (warp == 0) {
         tc5::fence_after_sync();
         issue_mma_t<BT / 16>(tm, Operand{tc5::smem_addr(Au), BT, 0}, Operand{tc5::smem_addr(Vs), BT, 1}, 64, DV, 0);
         ph.commit();

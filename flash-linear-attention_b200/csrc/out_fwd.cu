@@ -48,7 +48,7 @@ __global__ void __launch_bounds__(NTHREADS, 3) out_fwd_kernel(const b200gdn_chun
   uint64_t* bar_mma = bar_qk + 3;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_qk + 4);
 
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int g = lane >> 2, t = lane & 3;
   const int c = blockIdx.x, hv = blockIdx.y;
   const int G = a.HV / a.H, hq = hv / G;
@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(NTHREADS, 3) out_fwd_kernel(const b200gdn_chun
   if (!tc5::mbar_wait(bar_qk, 0)) failed = true;
 
   // ---- phase 1a: P = Q K^T
-  if (tid == 0 && !failed) {
+  if (warp == 0 && __all_sync(0xffffffffu, !failed)) {
     tc5::fence_after_sync();
     issue_mma_t<DK / 16>(tm, Operand{tc5::smem_addr(Qs), BT, 0}, Operand{tc5::smem_addr(Ks), BT, 0}, 64, 64, 0);
     ph.commit();
@@ -130,10 +130,12 @@ __global__ void __launch_bounds__(NTHREADS, 3) out_fwd_kernel(const b200gdn_chun
       failed = true;
     } else {
       // ---- phase 1b: O = Q h (over the columns P has left); v_new arrives over K meanwhile
-      if (tid == 0) {
+      if (warp == 0) {
         tc5::fence_after_sync();
         issue_mma_t<DK / 16>(tm, Operand{tc5::smem_addr(Qs), BT, 0}, Operand{tc5::smem_addr(Hs), DK, 1}, 64, DV, 0);
         ph.commit();
+      }
+      if (tid == 0) {
         tc5::mbar_expect_tx(bar_v, (uint32_t)(BT * DV * 2));
         tma::load_3d(Vn, &maps.vn, cm.row, (hv * DV) / 64, bar_v);
       }
@@ -163,7 +165,7 @@ __global__ void __launch_bounds__(NTHREADS, 3) out_fwd_kernel(const b200gdn_chun
           failed = true;
         } else {
           // ---- phase 2: O += P v_new
-          if (tid == 0) {
+          if (warp == 0) {
             tc5::fence_after_sync();
             issue_mma_t<BT / 16>(tm, Operand{tc5::smem_addr(Ps), BT, 0}, Operand{tc5::smem_addr(Vn), BT, 1}, 64, DV, 1);
             ph.commit();

@@ -10,9 +10,10 @@
 //
 // Same organisation as the forward scan: one CTA per 64-column slice of one state; a producer thread feeds
 // a ring of stages with TMA (Q, K, W tiles, the do slice, gamma; the qk tile with DVL, the dv_local slice without);
-// one thread issues tcgen05.mma  acc = K dS_bf16  and  dS += Q^T do_s - W^T dv2  with accumulators in TMEM and the
-// TMA stores of dh_c and dv2; eight epilogue warps move dS between TMEM and shared memory and form dv2.
-// DVL: the MMA thread also issues  L = qk^T do  of the NEXT chunk right after a step's last product (it only needs
+// the chain MMA warp issues  acc = K dS_bf16  and  dS += Q^T do_s - W^T dv2  with accumulators in TMEM; a store warp
+// issues the TMA stores of dh_c and dv2; eight epilogue warps move dS between TMEM and shared memory and form dv2.
+// B4 T4096 H16 K=V=128: 95 us (107 with products and stores issued by one thread in turn).
+// DVL: the chain MMA warp also issues  L = qk^T do  of the NEXT chunk right after a step's last product (it only needs
 // loaded tiles and runs while the epilogue warps convert dS); qk = tril(Q K^T 2^(gamma_i-gamma_j)) comes ready-made
 // from the forward pass; the epilogue warps add scale L where they form dv2.
 // Rows of a ragged last chunk (the first step of the reverse walk) that lie past its end are zeroed in the do and qk
@@ -30,7 +31,8 @@ namespace {
 
 constexpr int BV = 64;
 constexpr int NEPI = 256;
-constexpr int WARP_PROD = NEPI / 32, WARP_MMA = NEPI / 32 + 1;
+constexpr int WARP_PROD = NEPI / 32, WARP_MMA = WARP_PROD + 1, WARP_STORE = WARP_MMA + 1;
+constexpr int NTHREADS = 32 * (WARP_STORE + 1);
 __device__ int g_scan_bwd_timeout = 0;
 
 template <int DK, int NSTAGE, bool DVL>
@@ -44,7 +46,7 @@ struct ScanBwdSmem {
   static constexpr size_t o_dos = o_d2 + 2 * s_bytes;       // do scale 2^gamma [64][64]
   static constexpr size_t o_gam = o_dos + s_bytes;
   static constexpr size_t o_bar = o_gam + NSTAGE * BT * 4;
-  static constexpr size_t bytes = o_bar + (3 * NSTAGE + 5) * 8 + 16 + 1024;
+  static constexpr size_t bytes = o_bar + (4 * NSTAGE + 5) * 8 + 16 + 1024;
 };
 
 struct ScanBwdMaps {
@@ -52,7 +54,7 @@ struct ScanBwdMaps {
 };
 
 template <int DK, int DV, int NSTAGE, bool DVL>
-__global__ void __launch_bounds__(NEPI + 64)
+__global__ void __launch_bounds__(NTHREADS)
     scan_bwd_kernel(const b200gdn_chunk_args a, const __grid_constant__ ScanBwdMaps maps) {
   using S = ScanBwdSmem<DK, NSTAGE, DVL>;
   constexpr int NH = DK / 64;
@@ -61,15 +63,16 @@ __global__ void __launch_bounds__(NEPI + 64)
   float* gam_all = reinterpret_cast<float*>(smem + S::o_gam);
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + S::o_bar);   // K, do, gamma (+ qk | dv_local): what a step needs first
   uint64_t* full2 = full + NSTAGE;      // Q, W: operands of the step's last products
-  uint64_t* empty = full2 + NSTAGE;
-  uint64_t* s_ready = empty + NSTAGE;   // dS accumulated (last product of a step done)
-  uint64_t* sb_ready = s_ready + 1;     // bf16 snapshot in shared memory
-  uint64_t* v_ready = sb_ready + 1;     // acc = K dS done
-  uint64_t* vt_ready = v_ready + 1;     // dv2 / do_s tiles written, decayed dS back in TMEM
-  uint64_t* l_ready = vt_ready + 1;     // DVL: L = qk^T do done
+  // (barriers that a warp off the chain waits for come per stage or per buffer, see the forward scan)
+  uint64_t* v_done = full2 + NSTAGE;    // acc = K dS done
+  uint64_t* s_done = v_done + NSTAGE;   // dS accumulated (last product of a step done): the stage's tiles are free
+  uint64_t* sb_ready = s_done + NSTAGE; // bf16 snapshot in shared memory
+  uint64_t* vt_ready = sb_ready + 1;    // dv2 / do_s tiles written, decayed dS back in TMEM
+  uint64_t* st_free = vt_ready + 1;     // [2] the TMA stores have read the snapshot and the dv2 tile
+  uint64_t* l_ready = st_free + 2;      // DVL: L = qk^T do done
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(l_ready + 1);
 
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   // CTAs past the DV / 64 value slices (launched only when cp_dM is given) scan the backward transition matrix of the
   // sequence instead: zero do and dv_local, identity end gradient, V := K, nothing stored but the final "gradient" dM
   const bool m_mode = (int)blockIdx.x >= DV / BV;
@@ -91,12 +94,13 @@ __global__ void __launch_bounds__(NEPI + 64)
     for (int s = 0; s < NSTAGE; ++s) {
       tc5::mbar_init(&full[s], 1);
       tc5::mbar_init(&full2[s], 1);
-      tc5::mbar_init(&empty[s], 1);
+      tc5::mbar_init(&v_done[s], 1);
+      tc5::mbar_init(&s_done[s], 1);
     }
-    tc5::mbar_init(s_ready, 1);
     tc5::mbar_init(sb_ready, NEPI / 32);
-    tc5::mbar_init(v_ready, 1);
     tc5::mbar_init(vt_ready, NEPI / 32);
+    tc5::mbar_init(&st_free[0], 1);
+    tc5::mbar_init(&st_free[1], 1);
     tc5::mbar_init(l_ready, 1);
     tc5::fence_mbar_init();
   }
@@ -129,7 +133,7 @@ __global__ void __launch_bounds__(NEPI + 64)
           tma::prefetch_3d(&maps.q, row_pf, (hq * DK) / 64);
           tma::prefetch_3d(&maps.w, row_pf, (hv * DK) / 64);
         }
-        if (ic >= NSTAGE && !tc5::mbar_wait(&empty[s], ((ic / NSTAGE) - 1) & 1)) { failed = true; break; }
+        if (ic >= NSTAGE && !tc5::mbar_wait(&s_done[s], ((ic / NSTAGE) - 1) & 1)) { failed = true; break; }
         unsigned char* base = smem + (size_t)s * S::stage_bytes;
         // in the order the step needs them, on two barriers: the first product does not wait for Q and W
         tc5::mbar_expect_tx(&full[s], tx1);
@@ -144,59 +148,63 @@ __global__ void __launch_bounds__(NEPI + 64)
       }
     }
   } else if (warp == WARP_MMA) {
-    // ================= MMA thread =================
-    if (lane == 0) {
+    // ================= chain MMA warp =================
+    {
       const uint32_t dos_addr = tc5::smem_addr(smem + S::o_dos);
-      ChunkMeta cm_next = nc > 0 ? load_chunk_meta(a.chunk_meta, c_last) : ChunkMeta{0, 0, 0, 0};   // an empty sequence owns no chunk
-      for (int ic = 0; ic < nc && !failed; ++ic) {
-        const int c = c_last - ic, s = ic % NSTAGE, buf = ic & 1;
-        const ChunkMeta cm = cm_next;
-        if (ic + 1 < nc) cm_next = load_chunk_meta(a.chunk_meta, c - 1);
+      for (int ic = 0; ic < nc; ++ic) {
+        const int s = ic % NSTAGE, par = (ic / NSTAGE) & 1, buf = ic & 1;
         const uint32_t q_addr = tc5::smem_addr(smem + (size_t)s * S::stage_bytes);
         const uint32_t k_addr = q_addr + (uint32_t)S::t_bytes, w_addr = q_addr + 2 * (uint32_t)S::t_bytes;
         const uint32_t do_addr = q_addr + 3 * (uint32_t)S::t_bytes, pq_addr = do_addr + (uint32_t)S::s_bytes;
-        unsigned char* sb_ptr = smem + S::o_sb + buf * S::sb_bytes;
-        unsigned char* d2_ptr = smem + S::o_d2 + buf * S::s_bytes;
-        if (!tc5::mbar_wait(&full[s], (ic / NSTAGE) & 1) || !tc5::mbar_wait(sb_ready, ic & 1)) { failed = true; break; }
+        const uint32_t sb_addr = tc5::smem_addr(smem + S::o_sb + buf * S::sb_bytes), d2_addr = tc5::smem_addr(smem + S::o_d2 + buf * S::s_bytes);
+        if (!tc5::mbar_wait_warp(&full[s], par) || !tc5::mbar_wait_warp(sb_ready, ic & 1)) { failed = true; break; }
         tc5::fence_after_sync();
         // acc = K dS_bf16
-        issue_mma_t<DK / 16>(TM_V, Operand{k_addr, BT, 0}, Operand{tc5::smem_addr(sb_ptr), DK, 1}, 64, BV, 0);
-        tc5::mma_commit(v_ready);
+        issue_mma_t<DK / 16>(TM_V, Operand{k_addr, BT, 0}, Operand{sb_addr, DK, 1}, 64, BV, 0);
+        tc5::mma_commit(&v_done[s]);
         if (dvl && ic == 0) {
           // L = qk^T do of the first step (the tails of a ragged chunk's tiles were zeroed before sb_ready)
           issue_mma_t<BT / 16>(TM_L, Operand{pq_addr, BT, 1}, Operand{do_addr, BT, 1}, 64, BV, 0);
           tc5::mma_commit(l_ready);
         }
-        if (st_dh) {
-          tma::store_2d(&maps.dh, v0, (c * a.HV + hv) * DK, sb_ptr);
-          tma::store_commit();
-          tma::store_wait_read<1>();   // older stores have released their tiles (re-written next step)
-        } else {
-          tma::store_wait_read<0>();
-        }
-        if (!tc5::mbar_wait(&full2[s], (ic / NSTAGE) & 1) || !tc5::mbar_wait(vt_ready, ic & 1)) { failed = true; break; }
+        if (!tc5::mbar_wait_warp(&full2[s], par) || !tc5::mbar_wait_warp(vt_ready, ic & 1)) { failed = true; break; }
         tc5::fence_after_sync();
         // dS += Q^T do_s - W^T dv2
         if (has_do) issue_mma_t<BT / 16>(TM_S, Operand{q_addr, BT, 1}, Operand{dos_addr, BT, 1}, DK, BV, 1);
-        issue_mma_t<BT / 16>(TM_S, Operand{w_addr, BT, 1}, Operand{tc5::smem_addr(d2_ptr), BT, 1}, DK, BV, 1, /*neg_a=*/1);
-        tc5::mma_commit(s_ready);
-        tc5::mma_commit(&empty[s]);   // every product that reads this stage's tiles has been issued before this commit
-        if (store_d2 && cm.len == BT) {
-          tma::store_2d(&maps.dv2, hv * DV + v0, cm.row, d2_ptr);
-          tma::store_commit();
-        }
+        issue_mma_t<BT / 16>(TM_S, Operand{w_addr, BT, 1}, Operand{d2_addr, BT, 1}, DK, BV, 1, /*neg_a=*/1);
+        tc5::mma_commit(&s_done[s]);
         if (dvl && ic + 1 < nc) {
           // L = qk^T do of the next step: it needs loaded tiles only and runs while the epilogue warps convert dS.
           // Waiting for those tiles here costs nothing, the next product of the chain needs them as well.
           const int s2 = (ic + 1) % NSTAGE;
-          if (!tc5::mbar_wait(&full[s2], ((ic + 1) / NSTAGE) & 1)) { failed = true; break; }
+          if (!tc5::mbar_wait_warp(&full[s2], ((ic + 1) / NSTAGE) & 1)) { failed = true; break; }
           tc5::fence_after_sync();
           const uint32_t do2 = tc5::smem_addr(smem + (size_t)s2 * S::stage_bytes) + 3 * (uint32_t)S::t_bytes;
           issue_mma_t<BT / 16>(TM_L, Operand{do2 + (uint32_t)S::s_bytes, BT, 1}, Operand{do2, BT, 1}, 64, BV, 0);
           tc5::mma_commit(l_ready);
         }
       }
-      tma::store_wait_all<0>();
+    }
+  } else if (warp == WARP_STORE) {
+    // ================= store warp: the snapshot dh_c and dv2 leave by TMA =================
+    if (lane == 0 && (st_dh || store_d2)) {
+      for (int ic = 0; ic < nc; ++ic) {
+        const int c = c_last - ic, s = ic % NSTAGE, par = (ic / NSTAGE) & 1, buf = ic & 1;
+        const ChunkMeta cm = load_chunk_meta(a.chunk_meta, c);
+        if (!tc5::mbar_wait(&v_done[s], par)) { failed = true; break; }   // the snapshot is complete, and the chain has read it
+        if (st_dh) {
+          tma::store_2d(&maps.dh, v0, (c * a.HV + hv) * DK, smem + S::o_sb + buf * S::sb_bytes);
+          tma::store_commit();
+        }
+        if (!tc5::mbar_wait(&s_done[s], par)) { failed = true; break; }   // ... and dv2 likewise
+        if (store_d2 && cm.len == BT) {
+          tma::store_2d(&maps.dv2, hv * DV + v0, cm.row, smem + S::o_d2 + buf * S::s_bytes);
+          tma::store_commit();
+        }
+        tma::store_wait_read<0>();
+        tc5::mbar_arrive(&st_free[buf]);
+      }
+      tma::store_wait_all<0>();   // shared tiles must outlive the stores that read them
     }
   } else if (warp < WARP_PROD) {
     // ================= epilogue warps =================
@@ -232,8 +240,10 @@ __global__ void __launch_bounds__(NEPI + 64)
       const uint32_t sb_tile = sb_base + buf * (uint32_t)S::sb_bytes;
       const uint32_t d2_tile = d2_base + buf * (uint32_t)S::s_bytes;
 
+      // the snapshot and dv2 tiles of two chunks ago have left (waited for in the shadow of the last product)
+      if (ic >= 2 && (st_dh || store_d2) && !tc5::mbar_wait(&st_free[buf], ((ic >> 1) - 1) & 1)) { failed = true; break; }
       if (ic > 0) {
-        if (!tc5::mbar_wait(s_ready, (ic - 1) & 1)) { failed = true; break; }
+        if (!tc5::mbar_wait(&s_done[(ic - 1) % NSTAGE], ((ic - 1) / NSTAGE) & 1)) { failed = true; break; }
         tc5::fence_after_sync();
 #pragma unroll
         for (int hf = 0; hf < NH; ++hf) tc5::tmem_ld_16x256b_x4(TM_S + s_lane + ((uint32_t)(16 * hf) << 16) + 32 * hc, Sr[hf]);
@@ -301,7 +311,7 @@ __global__ void __launch_bounds__(NEPI + 64)
         }
       }
       tc5::tmem_st_wait();
-      if (!tc5::mbar_wait(v_ready, ic & 1)) { failed = true; break; }
+      if (!tc5::mbar_wait(&v_done[s], (ic / NSTAGE) & 1)) { failed = true; break; }
       if (dvl && !tc5::mbar_wait(l_ready, ic & 1)) { failed = true; break; }
       tc5::fence_after_sync();
       float acc[16];
@@ -346,7 +356,7 @@ __global__ void __launch_bounds__(NEPI + 64)
 
     if (!failed && dh0_out != nullptr) {
       if (nc > 0) {
-        if (tc5::mbar_wait(s_ready, (nc - 1) & 1)) {
+        if (tc5::mbar_wait(&s_done[(nc - 1) % NSTAGE], ((nc - 1) / NSTAGE) & 1)) {
           tc5::fence_after_sync();
 #pragma unroll
           for (int hf = 0; hf < NH; ++hf) tc5::tmem_ld_16x256b_x4(TM_S + s_lane + ((uint32_t)(16 * hf) << 16) + 32 * hc, Sr[hf]);
@@ -402,7 +412,7 @@ int launch(const b200gdn_chunk_args& a, cudaStream_t st) {
   if (DVL) rc |= tma::encode_bf16_2d(&m.pq, a.qk, a.rows, (uint64_t)a.HV * BT, (uint64_t)a.HV * BT, BT); else m.pq = dummy;
   if (rc != 0) return set_error(B200GDN_ERR_CUDA, "scan_bwd: cuTensorMapEncodeTiled failed (%d)", rc);
   dim3 grid(DV / BV + (a.cp_dM != nullptr ? DK / BV : 0), a.HV, a.n_seq);
-  scan_bwd_kernel<DK, DV, NSTAGE, DVL><<<grid, NEPI + 64, S::bytes, st>>>(a, m);
+  scan_bwd_kernel<DK, DV, NSTAGE, DVL><<<grid, NTHREADS, S::bytes, st>>>(a, m);
   return check_launch(DVL ? "scan_dvl_bwd" : "scan_bwd");
 }
 

@@ -9,14 +9,14 @@
 // neither h nor v_new is read back from HBM for the output (they are still written for the backward pass).
 //
 // The recurrence is a chain of 64-row steps, so what matters is the latency of one step.  One CTA owns a
-// 64-column slice of one state and is specialised by warp:
+// 64-column slice of one state and is specialised by warp, so that nothing off the chain can delay it:
 //   * producer warp: TMA (cp.async.bulk.tensor, 128-byte swizzle) fills a ring of NSTAGE stages with
 //     W [64 x K], K [64 x K], the U slice [64 x 64] (and Q [64 x K]) of the chunks ahead; full/empty mbarriers;
 //     in the OUT form the tiles of the chunk that will take a stage next are pulled into L2 at the same time;
-//   * MMA warp (one thread): tcgen05.mma  V_acc = W S_bf16  (64 x 64 x K) and  S += K^T V~  (K x 64 x 64),
-//     operands straight from the swizzled tiles, accumulators in TMEM; it also issues the TMA stores of
-//     the state snapshot h_c and of v_new from double-buffered shared tiles.  OUT: the two products of the output
-//     are off the chain: O1 = Q S_bf16 goes behind the first product (it runs while the epilogue warps form v_new)
+//   * chain MMA warp: tcgen05.mma  V_acc = W S_bf16  (64 x 64 x K) and  S += K^T V~  (K x 64 x 64), operands straight
+//     from the swizzled tiles, accumulators in TMEM, and nothing else;
+//   * store warp: TMA stores of the state snapshot h_c and of v_new from double-buffered shared tiles;
+//   * output MMA warp (OUT): O1 = Q S_bf16 behind the chain's first product (it runs while the epilogue warps form v_new)
 //     and O2 = P~ v_new behind the second (it runs while they convert S), with P~ = tril(Q K^T 2^(gamma_i-gamma_j))
 //     loaded ready-made (the intra-chunk kernel emits it), so nothing of the output waits on the chain's warps;
 //   * eight epilogue warps: read S from TMEM, round it to bf16 into shared memory, write it back scaled
@@ -24,8 +24,10 @@
 //   * OUT: four output warps (one per TMEM lane quadrant) read O1 and O2, form scale (O1 2^gamma_i + O2) and store
 //     o (one TMA store per warp, 16 rows).
 // Per step the chain is  S -> bf16 -> MMA -> v_new -> MMA, with four mbarrier hand-offs; everything of the output
-// runs in the shadow of that chain.  A tcgen05.mma of these shapes (N = 64) occupies the tensor pipe for about 45
-// cycles per 16-deep step whatever M is, so the chain's products cost ~550 cycles per chunk and the output's ~540.
+// runs in the shadow of that chain.  Measured by clock stamps at K = V = 128: 1.94 k cycles a step (3.17 k when one thread
+// inside a divergent branch issued chain, output and stores in turn: 75-80 cycles per tcgen05.mma, waits for stores on the
+// chain).  With h and v_new stored the bound is the SM's TMA traffic, 64 KB in and 32 KB out a step: 2.39 k cycles.
+// B4 T4096 H16 K=V=128: 98 us with h and v_new stored (113), 78 us without (112).
 // A ragged last chunk is loaded as a full box (rows of the next sequence or zero fill); its extra rows
 // are selected away where v_new is formed, and its v_new / o rows are written with plain predicated stores.
 //
@@ -42,8 +44,10 @@ namespace {
 
 constexpr int BV = 64;          // state columns per CTA
 constexpr int NEPI = 256;       // 8 epilogue warps
-constexpr int WARP_PROD = NEPI / 32, WARP_MMA = NEPI / 32 + 1;
-constexpr int NOUT = 4;         // output warps (OUT form): warps WARP_MMA + 1 ..
+constexpr int WARP_PROD = NEPI / 32, WARP_MMA = WARP_PROD + 1, WARP_STORE = WARP_MMA + 1;
+constexpr int NOUT = 4;         // output warps (OUT form): warps WARP_STORE + 1 .., then the warp that issues their products
+constexpr int WARP_OMMA = WARP_STORE + 1 + NOUT;
+constexpr int threads_of(bool out) { return 32 * (out ? WARP_OMMA + 1 : WARP_STORE + 1); }
 __device__ int g_scan_fwd_timeout = 0;
 
 template <int DK, int NSTAGE, bool OUT>
@@ -58,9 +62,9 @@ struct ScanFwdSmem {
   static constexpr size_t o_vn = o_sb + 2 * sb_bytes;       // 2 x v_new slice [64][64]
   static constexpr size_t o_vt = o_vn + 2 * u_bytes;        // gated v_new slice
   static constexpr size_t o_os = o_vt + u_bytes;            // OUT: 2 x o staging [64][64]
-  static constexpr size_t o_gam = o_os + (OUT ? 2 * u_bytes : 0);  // NSTAGE x 64 floats
-  static constexpr size_t o_bar = o_gam + NSTAGE * BT * 4;
-  static constexpr size_t bytes = o_bar + (3 * NSTAGE + 8) * 8 + 16 + 1024;  // + alignment slack
+  static constexpr size_t o_gam = o_os + (OUT ? 2 * u_bytes : 0);  // 2 NSTAGE x 64 floats
+  static constexpr size_t o_bar = o_gam + 2 * NSTAGE * BT * 4;
+  static constexpr size_t bytes = o_bar + (6 * NSTAGE + 10) * 8 + 16 + 1024;  // + alignment slack
 };
 
 struct ScanFwdMaps {
@@ -68,7 +72,7 @@ struct ScanFwdMaps {
 };
 
 template <int DK, int DV, int NSTAGE, bool OUT>
-__global__ void __launch_bounds__(NEPI + 64 + (OUT ? NOUT * 32 : 0))
+__global__ void __launch_bounds__(threads_of(OUT))
     scan_fwd_kernel(const b200gdn_chunk_args a, const __grid_constant__ ScanFwdMaps maps) {
   using S = ScanFwdSmem<DK, NSTAGE, OUT>;
   constexpr int NH = DK / 64;   // 16-row halves of the state per epilogue warp
@@ -76,19 +80,23 @@ __global__ void __launch_bounds__(NEPI + 64 + (OUT ? NOUT * 32 : 0))
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   float* gam_all = reinterpret_cast<float*>(smem + S::o_gam);
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + S::o_bar);   // W, U, gamma of a stage (what the step needs first)
-  uint64_t* full2 = full + NSTAGE;      // K (and Q, P~) of a stage
-  uint64_t* empty = full2 + NSTAGE;
-  uint64_t* s_ready = empty + NSTAGE;   // S accumulated (MMA 2 done)
-  uint64_t* sb_ready = s_ready + 1;     // bf16 snapshot in shared memory
-  uint64_t* v_ready = sb_ready + 1;     // V_acc done (MMA 1)
-  uint64_t* vt_ready = v_ready + 1;     // v_new / V~ tiles written, decayed S back in TMEM
-  // OUT, one pair of barriers per accumulator pair (chunk parity): a single barrier could complete two phases while a
-  // slow output warp still waits for the first, and a parity wait cannot tell a phase from the one two later
-  uint64_t* grp_ready = vt_ready + 1;   // [2] O1 and O2 of a chunk done
-  uint64_t* o_free = grp_ready + 2;     // [2] the output warps have read the accumulator pair
+  uint64_t* full2 = full + NSTAGE;      // K of a stage
+  uint64_t* full3 = full2 + NSTAGE;     // OUT: Q, P~ of a stage
+  // A wait on a parity cannot tell a phase from the one two later, so every barrier that a warp off the chain waits for is
+  // one of a set that is re-used only after that warp has moved on: per stage (a stage is refilled only when all its readers
+  // are done) or per buffer of a double-buffered tile.
+  uint64_t* empty = full3 + NSTAGE;     // OUT: the output's products and warps are done with Q, P~ and the gate vector
+  uint64_t* v_done = empty + NSTAGE;    // V_acc done (MMA 1)
+  uint64_t* s_done = v_done + NSTAGE;   // S accumulated (MMA 2): the stage's W, K, U tiles are free
+  uint64_t* sb_ready = s_done + NSTAGE; // bf16 snapshot in shared memory
+  uint64_t* vt_ready = sb_ready + 1;    // V~ tile written, decayed S back in TMEM
+  uint64_t* vn_ready = vt_ready + 1;    // [2] v_new tile written
+  uint64_t* st_free = vn_ready + 2;     // [2] the TMA stores have read the snapshot and the v_new tile
+  uint64_t* grp_ready = st_free + 2;    // [2] OUT: O1 and O2 of a chunk done (and the tiles they read free)
+  uint64_t* o_free = grp_ready + 2;     // [2] OUT: the output warps have read the accumulator pair
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_free + 2);
 
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   // CTAs past the DV / 64 value slices (launched only when cp_M is given) scan the transition matrix of the sequence
   // instead: zero u, identity start state, V := K, nothing stored but the final "state" M
   const bool m_mode = !OUT && (int)blockIdx.x >= DV / BV;
@@ -106,17 +114,19 @@ __global__ void __launch_bounds__(NEPI + 64 + (OUT ? NOUT * 32 : 0))
     for (int s = 0; s < NSTAGE; ++s) {
       tc5::mbar_init(&full[s], 1);    // producer's expect_tx arrive; the copies complete the transaction count
       tc5::mbar_init(&full2[s], 1);
-      // tcgen05.commit of the step's last MMA (+ OUT: the output warps are done with the stage's gate vector)
-      tc5::mbar_init(&empty[s], OUT ? 1 + NOUT : 1);
+      tc5::mbar_init(&full3[s], 1);
+      tc5::mbar_init(&empty[s], 1 + NOUT);   // the commit of O2 and the output warps (done with the gate vector)
+      tc5::mbar_init(&v_done[s], 1);
+      tc5::mbar_init(&s_done[s], 1);
     }
-    tc5::mbar_init(s_ready, 1);
     tc5::mbar_init(sb_ready, NEPI / 32);
-    tc5::mbar_init(v_ready, 1);
     tc5::mbar_init(vt_ready, NEPI / 32);
-    tc5::mbar_init(&grp_ready[0], 1);
-    tc5::mbar_init(&grp_ready[1], 1);
-    tc5::mbar_init(&o_free[0], NOUT);
-    tc5::mbar_init(&o_free[1], NOUT);
+    for (int i = 0; i < 2; ++i) {
+      tc5::mbar_init(&vn_ready[i], NEPI / 32);
+      tc5::mbar_init(&st_free[i], 1);
+      tc5::mbar_init(&grp_ready[i], 1);
+      tc5::mbar_init(&o_free[i], NOUT);
+    }
     tc5::fence_mbar_init();
   }
   tc5::fence_before_sync();
@@ -136,7 +146,6 @@ __global__ void __launch_bounds__(NEPI + 64 + (OUT ? NOUT * 32 : 0))
       if (OUT) tma::prefetch_map(&maps.q);
     }
     const uint32_t tx1 = (uint32_t)(S::w_bytes + (has_u ? S::u_bytes : 0) + BT * 4);
-    const uint32_t tx2 = (uint32_t)(S::w_bytes + (OUT ? S::w_bytes + S::u_bytes : 0));
     if (lane == 0) {
       int row_next = nc > 0 ? load_chunk_meta(a.chunk_meta, c_first).row : 0;
       for (int ic = 0; ic < nc; ++ic) {
@@ -153,72 +162,88 @@ __global__ void __launch_bounds__(NEPI + 64 + (OUT ? NOUT * 32 : 0))
           tma::prefetch_3d(&maps.k, row_pf, (hq * DK) / 64);
           tma::prefetch_2d(&maps.pq, hv * BT, row_pf);
         }
-        if (ic >= NSTAGE && !tc5::mbar_wait(&empty[s], ((ic / NSTAGE) - 1) & 1)) { failed = true; break; }
+        if (ic >= NSTAGE && !tc5::mbar_wait(&s_done[s], ((ic / NSTAGE) - 1) & 1)) { failed = true; break; }
         unsigned char* base = smem + (size_t)s * S::stage_bytes;
-        // in the order the step needs them, on two barriers: the first product does not wait for K, Q and P~
+        // in the order the step needs them, on barriers of their own: the first product does not wait for the tiles of the
+        // last, and the chain's tiles are refilled as soon as the chain has left them, half a step before the output's.
+        // (The gate vectors, which the output warps read late, have twice as many slots.)
         tc5::mbar_expect_tx(&full[s], tx1);
         tma::load_3d(base, &maps.w, row, (hv * DK) / 64, &full[s]);                 // W  [64 x K], all panels
         if (has_u) tma::load_2d(base + 2 * S::w_bytes, &maps.u, hv * DV + v0, row, &full[s]);
-        tma::load_1d(gam_all + s * BT, gamma_ptr(a.gamma, c_first + ic, a.HV, hv), BT * 4, &full[s]);
-        tc5::mbar_expect_tx(&full2[s], tx2);
-        if (OUT) tma::load_3d(base + S::o_qt, &maps.q, row, (hq * DK) / 64, &full2[s]);   // Q  [64 x K]
+        tma::load_1d(gam_all + (ic % (2 * NSTAGE)) * BT, gamma_ptr(a.gamma, c_first + ic, a.HV, hv), BT * 4, &full[s]);
+        tc5::mbar_expect_tx(&full2[s], (uint32_t)S::w_bytes);
         tma::load_3d(base + S::w_bytes, &maps.k, row, (hq * DK) / 64, &full2[s]);    // K  [64 x K]
-        if (OUT) tma::load_2d(base + S::o_pq, &maps.pq, hv * BT, row, &full2[s]);    // P~ [64 x 64]
+        if (OUT) {
+          if (ic >= NSTAGE && !tc5::mbar_wait(&empty[s], ((ic / NSTAGE) - 1) & 1)) { failed = true; break; }
+          tc5::mbar_expect_tx(&full3[s], (uint32_t)(S::w_bytes + S::u_bytes));
+          tma::load_3d(base + S::o_qt, &maps.q, row, (hq * DK) / 64, &full3[s]);     // Q  [64 x K]
+          tma::load_2d(base + S::o_pq, &maps.pq, hv * BT, row, &full3[s]);           // P~ [64 x 64]
+        }
       }
     }
   } else if (warp == WARP_MMA) {
-    // ================= MMA warp: one thread issues the contractions and the TMA stores =================
-    if (lane == 0) {
+    // ================= chain MMA warp: the two contractions of the recurrence and nothing else =================
+    {
       const uint32_t vt_addr = tc5::smem_addr(smem + S::o_vt);
-      const uint32_t vn_addr0 = tc5::smem_addr(smem + S::o_vn);
-      ChunkMeta cm_next = nc > 0 ? load_chunk_meta(a.chunk_meta, c_first) : ChunkMeta{0, 0, 0, 0};   // an empty sequence owns no chunk
       for (int ic = 0; ic < nc; ++ic) {
-        const int c = c_first + ic, s = ic % NSTAGE, buf = ic & 1;
-        const ChunkMeta cm = cm_next;
-        if (ic + 1 < nc) cm_next = load_chunk_meta(a.chunk_meta, c + 1);
-        const uint32_t w_addr = tc5::smem_addr(smem + (size_t)s * S::stage_bytes);
-        const uint32_t k_addr = w_addr + (uint32_t)S::w_bytes, q_addr = w_addr + (uint32_t)S::o_qt;
-        const uint32_t pq_addr = w_addr + (uint32_t)S::o_pq;
-        unsigned char* sb_ptr = smem + S::o_sb + buf * S::sb_bytes;
-        if (!tc5::mbar_wait(&full[s], (ic / NSTAGE) & 1) || !tc5::mbar_wait(sb_ready, ic & 1)) { failed = true; break; }
+        const int s = ic % NSTAGE, par = (ic / NSTAGE) & 1;
+        const uint32_t w_addr = tc5::smem_addr(smem + (size_t)s * S::stage_bytes), k_addr = w_addr + (uint32_t)S::w_bytes;
+        const uint32_t sb_addr = tc5::smem_addr(smem + S::o_sb + (ic & 1) * S::sb_bytes);
+        if (!tc5::mbar_wait_warp(&full[s], par) || !tc5::mbar_wait_warp(sb_ready, ic & 1)) { failed = true; break; }
         tc5::fence_after_sync();
         // V_acc = W S_bf16
-        issue_mma_t<DK / 16>(TM_V, Operand{w_addr, BT, 0}, Operand{tc5::smem_addr(sb_ptr), DK, 1}, 64, BV, 0);
-        tc5::mma_commit(v_ready);
-        if (!tc5::mbar_wait(&full2[s], (ic / NSTAGE) & 1)) { failed = true; break; }
-        if (OUT) {
-          // O1 = Q S_bf16, behind the first product: it runs while the epilogue warps form v_new.  The accumulator pair
-          // of this parity was last used two chunks ago; the output warps have read it.
-          if (ic >= 2 && !tc5::mbar_wait(&o_free[buf], ((ic >> 1) - 1) & 1)) { failed = true; break; }
-          tc5::fence_after_sync();
-          issue_mma_t<DK / 16>(TM_O1 + 64 * buf, Operand{q_addr, BT, 0}, Operand{tc5::smem_addr(sb_ptr), DK, 1}, 64, BV, 0);
-        }
-        if (st_h) {
-          tma::store_2d(&maps.h, v0, (c * a.HV + hv) * DK, sb_ptr);
-          tma::store_commit();
-          // every store older than this h_c has released its shared tile before the next step re-writes it;
-          // waiting here costs nothing, this thread would otherwise idle until the v_new tiles are ready
-          tma::store_wait_read<1>();
-        } else {
-          tma::store_wait_read<0>();
-        }
-        if (!tc5::mbar_wait(vt_ready, ic & 1)) { failed = true; break; }
+        issue_mma_t<DK / 16>(TM_V, Operand{w_addr, BT, 0}, Operand{sb_addr, DK, 1}, 64, BV, 0);
+        tc5::mma_commit(&v_done[s]);
+        if (!tc5::mbar_wait_warp(&full2[s], par) || !tc5::mbar_wait_warp(vt_ready, ic & 1)) { failed = true; break; }
         tc5::fence_after_sync();
         // S += K^T V~
         issue_mma_t<BT / 16>(TM_S, Operand{k_addr, BT, 1}, Operand{vt_addr, BT, 1}, DK, BV, 1);
-        tc5::mma_commit(s_ready);
-        if (OUT) {
-          // O2 = P~ v_new, behind the second product: it runs while the epilogue warps convert S
-          issue_mma_t<BT / 16>(TM_O2 + 64 * buf, Operand{pq_addr, BT, 0}, Operand{vn_addr0 + buf * (uint32_t)S::u_bytes, BT, 1}, 64, BV, 0);
-          tc5::mma_commit(&grp_ready[buf]);
+        tc5::mma_commit(&s_done[s]);
+      }
+    }
+  } else if (warp == WARP_STORE) {
+    // ================= store warp: the snapshot h_c and v_new leave by TMA =================
+    if (lane == 0 && (st_h || st_vn)) {
+      for (int ic = 0; ic < nc; ++ic) {
+        const int c = c_first + ic, s = ic % NSTAGE, par = (ic / NSTAGE) & 1, buf = ic & 1;
+        const ChunkMeta cm = load_chunk_meta(a.chunk_meta, c);
+        if (!tc5::mbar_wait(&v_done[s], par)) { failed = true; break; }   // the snapshot is complete, and the chain has read it
+        if (st_h) {
+          tma::store_2d(&maps.h, v0, (c * a.HV + hv) * DK, smem + S::o_sb + buf * S::sb_bytes);
+          tma::store_commit();
         }
-        tc5::mma_commit(&empty[s]);   // every product that reads this stage's tiles has been issued before this commit
+        if (!tc5::mbar_wait(&vn_ready[buf], (ic >> 1) & 1)) { failed = true; break; }
         if (st_vn && cm.len == BT) {
           tma::store_2d(&maps.vn, hv * DV + v0, cm.row, smem + S::o_vn + buf * S::u_bytes);
           tma::store_commit();
         }
+        tma::store_wait_read<0>();
+        tc5::mbar_arrive(&st_free[buf]);
       }
       tma::store_wait_all<0>();   // shared tiles must outlive the stores that read them
+    }
+  } else if (OUT && warp == WARP_OMMA) {
+    // ================= the output's products, in the gaps of the chain on the (in-order) tensor pipe: O1 while the epilogue
+    // warps form v_new, O2 while they convert S =================
+    {
+      const uint32_t vn_addr0 = tc5::smem_addr(smem + S::o_vn), sb_addr0 = tc5::smem_addr(smem + S::o_sb);
+      for (int ic = 0; ic < nc; ++ic) {
+        const int s = ic % NSTAGE, par = (ic / NSTAGE) & 1, buf = ic & 1;
+        const uint32_t stage = tc5::smem_addr(smem + (size_t)s * S::stage_bytes);
+        if (!tc5::mbar_wait_warp(&full3[s], par) || !tc5::mbar_wait_warp(&v_done[s], par) ||
+            (ic >= 2 && !tc5::mbar_wait_warp(&o_free[buf], ((ic >> 1) - 1) & 1))) { failed = true; break; }
+        tc5::fence_after_sync();
+        // O1 = Q S_bf16
+        issue_mma_t<DK / 16>(TM_O1 + 64 * buf, Operand{stage + (uint32_t)S::o_qt, BT, 0}, Operand{sb_addr0 + buf * (uint32_t)S::sb_bytes, DK, 1},
+                             64, BV, 0);
+        if (!tc5::mbar_wait_warp(&vn_ready[buf], (ic >> 1) & 1) || !tc5::mbar_wait_warp(&s_done[s], par)) { failed = true; break; }
+        tc5::fence_after_sync();
+        // O2 = P~ v_new
+        issue_mma_t<BT / 16>(TM_O2 + 64 * buf, Operand{stage + (uint32_t)S::o_pq, BT, 0}, Operand{vn_addr0 + buf * (uint32_t)S::u_bytes, BT, 1},
+                             64, BV, 0);
+        tc5::mma_commit(&grp_ready[buf]);
+        tc5::mma_commit(&empty[s]);
+      }
     }
   } else if (warp < WARP_PROD) {
     // ================= epilogue warps =================
@@ -250,12 +275,15 @@ __global__ void __launch_bounds__(NEPI + 64 + (OUT ? NOUT * 32 : 0))
       const int c = c_first + ic, s = ic % NSTAGE, buf = ic & 1;
       const ChunkMeta cm = load_chunk_meta(a.chunk_meta, c);   // consumed late in the step
       const uint32_t u_tile = smem_u32(smem + (size_t)s * S::stage_bytes + 2 * S::w_bytes);
-      const float* gs = gam_all + s * BT;
+      const float* gs = gam_all + (ic % (2 * NSTAGE)) * BT;
       const uint32_t sb_tile = sb_base + buf * (uint32_t)S::sb_bytes;
       const uint32_t vn_tile = vn_base + buf * (uint32_t)S::u_bytes;
 
+      // the snapshot and v_new tiles of two chunks ago are no longer read (waited for in the shadow of the last product)
+      if (ic >= 2 && ((OUT && !tc5::mbar_wait(&grp_ready[buf], ((ic >> 1) - 1) & 1)) ||
+                      ((st_h || st_vn) && !tc5::mbar_wait(&st_free[buf], ((ic >> 1) - 1) & 1)))) { failed = true; break; }
       if (ic > 0) {
-        if (!tc5::mbar_wait(s_ready, (ic - 1) & 1)) { failed = true; break; }
+        if (!tc5::mbar_wait(&s_done[(ic - 1) % NSTAGE], ((ic - 1) / NSTAGE) & 1)) { failed = true; break; }
         tc5::fence_after_sync();
 #pragma unroll
         for (int hf = 0; hf < NH; ++hf) tc5::tmem_ld_16x256b_x4(TM_S + s_lane + ((uint32_t)(16 * hf) << 16) + 32 * hc, Sr[hf]);
@@ -301,7 +329,7 @@ __global__ void __launch_bounds__(NEPI + 64 + (OUT ? NOUT * 32 : 0))
       const bool ok_lo = r_lo < cm.len, ok_hi = r_hi < cm.len;
       const float e_lo = fast_exp2(glast - gs[r_lo]), e_hi = fast_exp2(glast - gs[r_hi]);
       tc5::tmem_st_wait();
-      if (!tc5::mbar_wait(v_ready, ic & 1)) { failed = true; break; }
+      if (!tc5::mbar_wait(&v_done[s], (ic / NSTAGE) & 1)) { failed = true; break; }
       tc5::fence_after_sync();
       float acc[16];
       tc5::tmem_ld_16x256b_x4(TM_V + s_lane + 32 * hc, acc);
@@ -314,12 +342,18 @@ __global__ void __launch_bounds__(NEPI + 64 + (OUT ? NOUT * 32 : 0))
         fs_vn.set(i, v00, v01, v10, v11);
         fs_vt.set(i, v00 * e_lo, v01 * e_lo, v10 * e_hi, v11 * e_hi);
       }
-      fs_vn.store(vn_tile, BT, 16 * q, 32 * hc, lane);
+      // V~ first: it is all the chain waits for
       fs_vt.store(vt_tile, BT, 16 * q, 32 * hc, lane);
       tc5::fence_async_smem();
       tc5::fence_before_sync();
       __syncwarp();
       if (lane == 0) tc5::mbar_arrive(vt_ready);
+      if (OUT || st_vn || st_h) {
+        fs_vn.store(vn_tile, BT, 16 * q, 32 * hc, lane);
+        tc5::fence_async_smem();
+        __syncwarp();
+        if (lane == 0) tc5::mbar_arrive(&vn_ready[buf]);
+      }
 
       if (st_vn && cm.len < BT) {
         // ragged chunk: every warp writes the valid rows of its own block straight from its registers (no CTA-wide
@@ -336,7 +370,7 @@ __global__ void __launch_bounds__(NEPI + 64 + (OUT ? NOUT * 32 : 0))
 
     if (!failed && ht_out != nullptr) {
       if (nc > 0) {
-        if (tc5::mbar_wait(s_ready, (nc - 1) & 1)) {
+        if (tc5::mbar_wait(&s_done[(nc - 1) % NSTAGE], ((nc - 1) / NSTAGE) & 1)) {
           tc5::fence_after_sync();
 #pragma unroll
           for (int hf = 0; hf < NH; ++hf) tc5::tmem_ld_16x256b_x4(TM_S + s_lane + ((uint32_t)(16 * hf) << 16) + 32 * hc, Sr[hf]);
@@ -380,7 +414,7 @@ __global__ void __launch_bounds__(NEPI + 64 + (OUT ? NOUT * 32 : 0))
       tc5::tmem_ld_16x256b_x4(TM_O1 + 64 * buf + lane_off + 32, o1[1]);
       tc5::tmem_ld_16x256b_x4(TM_O2 + 64 * buf + lane_off, o2[0]);
       tc5::tmem_ld_16x256b_x4(TM_O2 + 64 * buf + lane_off + 32, o2[1]);
-      const float* gs = gam_all + s * BT;
+      const float* gs = gam_all + (j % (2 * NSTAGE)) * BT;
       const float e_lo = a.scale * fast_exp2(gs[r_lo]), e_hi = a.scale * fast_exp2(gs[r_hi]);
       tc5::tmem_ld_wait();
       tc5::fence_before_sync();
@@ -460,7 +494,7 @@ int launch(const b200gdn_chunk_args& a, cudaStream_t st) {
   }
   if (rc != 0) return set_error(B200GDN_ERR_CUDA, "scan_fwd: cuTensorMapEncodeTiled failed (%d)", rc);
   dim3 grid(DV / BV + ((!OUT && a.cp_M != nullptr) ? DK / BV : 0), a.HV, a.n_seq);
-  scan_fwd_kernel<DK, DV, NSTAGE, OUT><<<grid, NEPI + 64 + (OUT ? NOUT * 32 : 0), S::bytes, st>>>(a, m);
+  scan_fwd_kernel<DK, DV, NSTAGE, OUT><<<grid, threads_of(OUT), S::bytes, st>>>(a, m);
   return check_launch(OUT ? "scan_out_fwd" : "scan_fwd");
 }
 

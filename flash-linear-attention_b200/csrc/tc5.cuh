@@ -47,6 +47,11 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32
   return false;
 }
 
+// The same for a whole converged warp, with a result the compiler knows to be uniform.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity));
+}
+
 // generic-proxy writes to shared memory -> visible to the async proxy (tensor core / TMA reads)
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory"); }
 
@@ -86,19 +91,27 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N, int a_mn, int b_
          ((uint32_t)(M >> 4) << 24);
 }
 
-// D[tmem] (+)= A[smem] B[smem]; issued by ONE thread.
+// The tensor-core instructions are issued by ONE thread, but these functions are called by a WHOLE converged warp: the
+// elected lane executes the instruction, and because control flow stays uniform the compiler keeps descriptors and
+// addresses in uniform registers, where the instruction wants them.  (Inside `if (lane == 0)` every operand is moved there
+// through a vector register first: measured 75-80 cycles per tcgen05.mma instead of the pipe's 45.)
+// D[tmem] (+)= A[smem] B[smem]
 __device__ __forceinline__ void mma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
-      "{\n.reg .pred p;\n"
+      "{\n.reg .pred p, e;\n"
+      "elect.sync _|e, 0xffffffff;\n"
       "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),
       "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// All previously issued MMAs of this thread arrive on `bar` when they complete.
+// All previously issued MMAs of the elected lane arrive on `bar` when they complete.
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(smem_addr(bar))
-               : "memory");
+  asm volatile(
+      "{\n.reg .pred e;\n"
+      "elect.sync _|e, 0xffffffff;\n"
+      "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(smem_addr(bar))
+      : "memory");
 }
 
 // ---- TMEM -> registers -------------------------------------------------------------------------------

@@ -94,7 +94,7 @@ __device__ __forceinline__ void zero_tail_rows(unsigned char* tile, int valid, i
   }
 }
 
-// ---- MMA issue (one thread) -----------------------------------------------------------------------------
+// ---- MMA issue (one converged warp) -----------------------------------------------------------------------------
 // Operand descriptions.  A tile is stored [rows][cols]; as a K-major operand its MN index runs over rows
 // and the contraction over columns; as an MN-major operand the MN index runs over columns and the
 // contraction over rows.
@@ -135,7 +135,7 @@ __device__ __forceinline__ void acc_ld32q(uint32_t tmem_acc, int quad, int c0, f
   tc5::tmem_ld_16x256b_x4(tmem_acc + ((uint32_t)(quad * 32) << 16) + c0, r);
 }
 
-// One phase boundary: the issuing thread commits, everybody waits for the MMAs (bounded).
+// One phase boundary: the issuing warp commits, everybody waits for the MMAs (bounded).
 struct PhaseBarrier {
   uint64_t* bar;
   uint32_t parity;
