@@ -96,6 +96,8 @@ int b200gdn_chunk_fwd(const b200gdn_chunk_args* a, void* stream) {
     if (int e = launch_scan_fwd(*a, st)) return e;
   }
   if (m & B200GDN_FWD_OUT) {
+    if (a->options & B200GDN_PREP_L2NORM)
+      return set_error(B200GDN_ERR_UNSUPPORTED, "chunk_fwd: the fused L2 norm needs the scan and the output in one call");
     REQUIRE(a->q, "chunk_fwd"); REQUIRE(a->k, "chunk_fwd"); REQUIRE(a->v_new, "chunk_fwd"); REQUIRE(a->h, "chunk_fwd");
     REQUIRE(a->gamma, "chunk_fwd"); REQUIRE(a->o, "chunk_fwd");
     if (int e = launch_out_fwd(*a, st)) return e;

@@ -259,9 +259,21 @@ ChunkForward chunk_forward(const Tensor& q_in, const Tensor& k_in, const Tensor&
   s->has_h0 = initial_state.defined();
   const bool zero = !plan->covered;
   r.v = dense(v_in, at::kBFloat16);
-  if (options & B200GDN_PREP_L2NORM) {
-    // q, k L2-normalised to bf16 in one pass (fla/modules/l2norm.py:84-144); the reciprocal norms go to the backward
-    // kernels, which finish dq and dk with the norm's backward themselves
+  // q / k L2 norm (fla/modules/l2norm.py:84-144): for bf16 tensors the first forward kernel normalises the tiles it loads
+  // and writes them for the others; other types are normalised to bf16 by a pass of their own.  The reciprocal norms go to
+  // the backward kernels, which finish dq and dk with the norm's backward themselves.
+  const bool l2_fused = (options & B200GDN_PREP_L2NORM) && s->qt == at::kBFloat16 && s->kt == at::kBFloat16;
+  Tensor q_raw, k_raw;
+  if (l2_fused) {
+    q_raw = dense(q_in);
+    k_raw = dense(k_in);
+    r.q = new_tensor(q_raw.sizes(), at::kBFloat16, dev, zero);
+    r.k = new_tensor(k_raw.sizes(), at::kBFloat16, dev, zero);
+    if (need_grad) {
+      r.rstd_q = new_tensor(q_raw.sizes().slice(0, 3), at::kFloat, dev, zero);
+      r.rstd_k = new_tensor(q_raw.sizes().slice(0, 3), at::kFloat, dev, zero);
+    }
+  } else if (options & B200GDN_PREP_L2NORM) {
     const Tensor q = dense(q_in), k = dense(k_in);
     b200gdn_prep_args p{};
     p.rows = (int32_t)(q.size(0) * q.size(1));
@@ -296,8 +308,8 @@ ChunkForward chunk_forward(const Tensor& q_in, const Tensor& k_in, const Tensor&
     options &= ~B200GDN_STATE_V_FIRST;
     if (h0.defined()) h0 = h0.transpose(-1, -2).contiguous();
   }
-  s->options = options;
-  b200gdn_chunk_args a = chunk_args(r.q, r.k, r.v, scale, *plan);
+  s->options = options & ~B200GDN_PREP_L2NORM;
+  b200gdn_chunk_args a = chunk_args(l2_fused ? q_raw : r.q, l2_fused ? k_raw : r.k, r.v, scale, *plan);
   const int64_t rows = a.rows, HV = a.HV, K = a.K, V = a.V, C = a.n_chunks, N = a.n_seq;
   r.o = new_tensor(r.v.sizes(), at::kBFloat16, dev, zero);
   if (output_final_state)
@@ -334,6 +346,12 @@ ChunkForward chunk_forward(const Tensor& q_in, const Tensor& k_in, const Tensor&
   a.qk = piece(r.slab, s->off_qk);
   a.w = piece(r.slab, s->off_w);
   a.u = ptr(u);
+  if (l2_fused) {
+    a.qn = ptr(r.q);
+    a.kn = ptr(r.k);
+    a.rstd_q = fptr(r.rstd_q);
+    a.rstd_k = fptr(r.rstd_k);
+  }
   a.v_new = piece(r.slab, s->off_vnew);
   a.h = piece(r.slab, s->off_h);
   if (!plan->split) {
@@ -347,7 +365,10 @@ ChunkForward chunk_forward(const Tensor& q_in, const Tensor& k_in, const Tensor&
     float* h_pre = fptr(ws);
     float* M_pre = h_pre + P * kv;
     float* h0_v = M_pre + P * HV * K * K;
-    b200gdn_chunk_args p = chunk_args(r.q, r.k, r.v, scale, *plan);
+    b200gdn_chunk_args p = chunk_args(l2_fused ? q_raw : r.q, l2_fused ? k_raw : r.k, r.v, scale, *plan);
+    p.options = a.options;
+    p.qn = a.qn;
+    p.kn = a.kn;
     p.seq_meta = iptr(plan->pre_fwd);
     p.n_seq = plan->n_pre;
     p.gamma = a.gamma;

@@ -7,14 +7,19 @@
 // Replaces chunk_local_cumsum (fla/ops/utils/cumsum.py:33-68), the fused K K^T + triangular solve
 // (fla/ops/gated_delta_rule/chunk_fwd.py:40-328) and recompute_w_u_fwd (gated_delta_rule/wy_fast.py:43-106).
 //   * K and V tiles arrive by TMA; K K^T, W and U run on tcgen05 with TMEM accumulators (128 columns, used
-//     one product after the other); A, W, U leave through TMA stores (plain predicated stores for a ragged
-//     chunk); shared-memory regions are reused along the way so that three CTAs share an SM and hide each
-//     other's latencies;
-//   * the inverse is formed in exact fp32 on the CUDA cores: the four 16x16 diagonal blocks by
-//     right-looking forward substitution (one thread per column), then two levels of block merges
-//     A21 = -A22 (L21 A11) (16 -> 32 -> 64); the reference uses tf32 tensor-core merges;
-//   * the row scalings of the W/U right-hand sides are folded into the columns of A, so the K and V
-//     tiles are used exactly as loaded.
+//     one product after the other); W, U leave through TMA stores (plain predicated stores for a ragged
+//     chunk), A and qk from registers in 16-byte words; shared-memory regions are reused along the way so that four CTAs
+//     share an SM and hide each other's latencies;
+//   * the inverse is formed in exact fp32 on the CUDA cores: the four 16x16 diagonal blocks by forward substitution (one
+//     thread per column), then two levels of block merges A21 = -A22 (L21 A11) (16 -> 32 -> 64); the reference uses tf32
+//     tensor-core merges;
+//   * the row scalings of the W/U right-hand sides are folded into the columns of A, so the K and V tiles are used exactly as
+//     loaded (L2-norm option: as normalised in place).
+// What bounds it is the shared-memory / L1 data pipe (counters: 76 % of its wavefronts with a lane-per-output mapping of the
+// merges, 4-byte stores of qk and A and a zero fill of the inverse, 5.8 k wavefronts a CTA).  So every merge has one operand
+// at an address that is uniform over the warp (one wavefront) and 16-byte reads along rows for the other, skips what is
+// zero by triangularity, and nothing is filled with zeros first.
+// B4 T4096 H16 K=V=128: 86 us (105); with the L2 norm, gate and beta options 120 us (108 + 47 for a norm pass of its own).
 #include "tc5_tile.cuh"
 #include "tma.cuh"
 
@@ -50,37 +55,101 @@ struct IntraMaps {
   CUtensorMap k, v, w, u, q;
 };
 
-// T = L21 * A11 ;  A21 = -A22 * T   for an N x N off-diagonal block whose top-left corner is (r0, c0).
-// T is kept in a compact temporary (row stride LDT).  `nthr` threads with local index `t` cooperate
-// (one row x four columns each).
+// A21 = -A22 (L21 A11) for an N x N block below the diagonal whose corner is (r0, c0), T = L21 A11 going through a compact
+// temporary (row stride LDT).  Both A11 and A22 are lower triangular.
+// First product: a warp owns four columns of T (j0 ..), a lane a row: A11's row pieces are uniform over the warp, L21's rows
+// are read in 16-byte words; rows m < j0 of A11 have only zeros in these columns.
+// Second product: a warp owns four rows (i0 ..), a lane a column: A22's row pieces are uniform, T's rows are consecutive;
+// columns m > i0 + 3 of A22 hold only zeros in these rows.
+// N = 16: lanes 0-15 and 16-31 take halves of the contraction and add up at the end.
 template <int N>
-__device__ __forceinline__ void merge_step1(const float* Lf, const float* Af, float* T, int r0, int c0, int t, int nthr) {
-  for (int o = t; o < N * N / 4; o += nthr) {
-    const int i = o / (N / 4), j0 = (o % (N / 4)) * 4;
-    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+__device__ __forceinline__ void merge_step1(const float* Lf, const float* Af, float* T, int r0, int c0, int j0, int lane) {
+  const int i = lane & (N - 1);
+  const int m_beg = N == 32 ? j0 : (lane >> 4) * 8, m_end = N == 32 ? 32 : m_beg + 8;
+  float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 2
+  for (int m = m_beg; m < m_end; m += 4) {
+    const float4 l = *reinterpret_cast<const float4*>(&Lf[(r0 + i) * LDF + c0 + m]);
+    const float ll[4] = {l.x, l.y, l.z, l.w};
 #pragma unroll
-    for (int m = 0; m < N; ++m) {
-      const float l = Lf[(r0 + i) * LDF + c0 + m];
-      const float4 x = *reinterpret_cast<const float4*>(&Af[(c0 + m) * LDF + c0 + j0]);
-      acc[0] += l * x.x; acc[1] += l * x.y; acc[2] += l * x.z; acc[3] += l * x.w;
+    for (int e = 0; e < 4; ++e) {
+      const float4 x = *reinterpret_cast<const float4*>(&Af[(c0 + m + e) * LDF + c0 + j0]);
+      acc[0] += ll[e] * x.x; acc[1] += ll[e] * x.y; acc[2] += ll[e] * x.z; acc[3] += ll[e] * x.w;
     }
-    *reinterpret_cast<float4*>(&T[i * LDT + j0]) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+  }
+  if (N == 16) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], 16);
+    if (lane >= 16) return;
+  }
+  *reinterpret_cast<float4*>(&T[i * LDT + j0]) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+}
+template <int N>
+__device__ __forceinline__ void merge_step2(const float* T, float* Af, int r0, int c0, int i0, int lane) {
+  const int j = lane & (N - 1);
+  const int m_beg = N == 32 ? 0 : (lane >> 4) * 8, m_end = N == 32 ? i0 + 4 : m_beg + 8;
+  float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 2
+  for (int m = m_beg; m < m_end; m += 4) {
+    float t[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) t[e] = T[(m + e) * LDT + j];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const float4 x = *reinterpret_cast<const float4*>(&Af[(r0 + i0 + r) * LDF + r0 + m]);
+      acc[r] += x.x * t[0] + x.y * t[1] + x.z * t[2] + x.w * t[3];
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    if (N == 16) acc[r] += __shfl_xor_sync(0xffffffffu, acc[r], 16);
+    if (N == 32 || lane < 16) Af[(r0 + i0 + r) * LDF + c0 + j] = -acc[r];
   }
 }
-// A22 is lower triangular, so row i only needs m <= i; `m_end` is that bound rounded up to something uniform over
-// the calling warp (the rows of a warp are consecutive), which keeps the loop free of divergence.
-template <int N>
-__device__ __forceinline__ void merge_step2(const float* T, float* Af, int r0, int c0, int t, int nthr, int m_end) {
-  for (int o = t; o < N * N / 4; o += nthr) {
-    const int i = o / (N / 4), j0 = (o % (N / 4)) * 4;
-    float acc[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 4
-    for (int m = 0; m < m_end; ++m) {
-      const float a22 = Af[(r0 + i) * LDF + r0 + m];
-      const float4 tv = *reinterpret_cast<const float4*>(&T[m * LDT + j0]);
-      acc[0] += a22 * tv.x; acc[1] += a22 * tv.y; acc[2] += a22 * tv.z; acc[3] += a22 * tv.w;
+
+// Four words per lane of a quad (word i: columns 8 i + 2 t, + 1 of a row) -> the four words of column group t, so that a row's
+// 32 columns leave in 16-byte words.
+__device__ __forceinline__ uint4 quad_words(const uint32_t (&w)[4], int t) {
+  const bool odd = t & 1, hi = t & 2;
+  uint32_t a0 = w[0], a1 = w[1], a2 = w[2], a3 = w[3];
+  const uint32_t r0 = __shfl_xor_sync(0xffffffffu, odd ? a0 : a1, 1), r1 = __shfl_xor_sync(0xffffffffu, odd ? a2 : a3, 1);
+  if (odd) { a0 = r0; a2 = r1; } else { a1 = r0; a3 = r1; }
+  const uint32_t s0 = __shfl_xor_sync(0xffffffffu, hi ? a0 : a2, 2), s1 = __shfl_xor_sync(0xffffffffu, hi ? a1 : a3, 2);
+  return hi ? make_uint4(s0, s1, a2, a3) : make_uint4(a0, a1, s0, s1);
+}
+
+// L2-normalises the rows of a swizzled [64][DK] tile in place (four lanes per row), rounded to bf16; with `out` the rows also
+// go to global memory and their reciprocal norms to `rstd`
+template <int DK>
+__device__ __forceinline__ void normalise_rows(unsigned char* tile, int tid, int len, float* rstd, int64_t rstride, __nv_bfloat16* out,
+                                               int64_t ostride) {
+  const int r = tid >> 2, seg = tid & 3;
+  float2 x[DK / 32][4];
+  float ss = 0.f;
+  auto chunk = [&](int i) {   // the lane's i-th 16-byte word of the row
+    const int c = seg + 4 * i;
+    return reinterpret_cast<uint4*>(tile + (c >> 3) * (BT * 128) + r * 128 + (((c & 7) ^ (r & 7)) << 4));
+  };
+#pragma unroll
+  for (int i = 0; i < DK / 32; ++i) {
+    const uint4 w = *chunk(i);
+    const uint32_t u[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      x[i][e] = unpack_bf16(u[e]);
+      ss += x[i][e].x * x[i][e].x + x[i][e].y * x[i][e].y;
     }
-    *reinterpret_cast<float4*>(&Af[(r0 + i) * LDF + c0 + j0]) = make_float4(-acc[0], -acc[1], -acc[2], -acc[3]);
+  }
+  ss += __shfl_xor_sync(0xffffffffu, ss, 1);
+  ss += __shfl_xor_sync(0xffffffffu, ss, 2);
+  const float y = 1.f / sqrtf(ss + 1e-6f);
+  if (rstd != nullptr && seg == 0 && r < len) rstd[r * rstride] = y;
+#pragma unroll
+  for (int i = 0; i < DK / 32; ++i) {
+    const uint4 w = make_uint4(pack_bf16(x[i][0].x * y, x[i][0].y * y), pack_bf16(x[i][1].x * y, x[i][1].y * y),
+                               pack_bf16(x[i][2].x * y, x[i][2].y * y), pack_bf16(x[i][3].x * y, x[i][3].y * y));
+    *chunk(i) = w;
+    if (out != nullptr && r < len) *reinterpret_cast<uint4*>(out + r * ostride + (seg + 4 * i) * 8) = w;
   }
 }
 
@@ -142,8 +211,6 @@ __global__ void __launch_bounds__(NTHREADS, 4) intra_fwd_kernel(const b200gdn_ch
     g_raw = ld_param(a.g, (row0 + tid) * a.HV + hv, a.gb_dtype);
     b_raw = ld_param(a.beta, (row0 + tid) * a.HV + hv, a.gb_dtype);
   }
-  // zero the fp32 inverse (the merges and the final conversion read the untouched blocks as zeros)
-  for (int i = tid; i < BT * LDF / 4; i += NTHREADS) reinterpret_cast<float4*>(Af)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
   tc5::fence_before_sync();
   __syncthreads();
   tc5::fence_after_sync();
@@ -188,6 +255,16 @@ __global__ void __launch_bounds__(NTHREADS, 4) intra_fwd_kernel(const b200gdn_ch
     zero_tail_rows<BT, DK>(Ks, cm.len, tid, NTHREADS);
     tc5::fence_async_smem();
   }
+  if ((a.options & B200GDN_PREP_L2NORM) && !failed) {   // q and k are the raw tensors; the scans read the normalised ones
+    const bool lead = hv % G == 0;   // one of the value heads that share these q and k
+    const int64_t at = row0 * a.H + hq, st = (int64_t)a.H * DK;
+    if (cm.len < BT) __syncthreads();   // the zeroed tail of K
+    normalise_rows<DK>(Ks, tid, cm.len, lead && a.rstd_k ? a.rstd_k + at : nullptr, a.H,
+                       lead ? reinterpret_cast<__nv_bfloat16*>(a.kn) + at * DK : nullptr, st);
+    if (with_qk) normalise_rows<DK>(Qs, tid, cm.len, lead && a.rstd_q ? a.rstd_q + at : nullptr, a.H,
+                                    lead ? reinterpret_cast<__nv_bfloat16*>(a.qn) + at * DK : nullptr, st);
+    tc5::fence_async_smem();
+  }
   if (__syncthreads_or(failed)) {
     failed = true;
   } else {
@@ -215,67 +292,74 @@ __global__ void __launch_bounds__(NTHREADS, 4) intra_fwd_kernel(const b200gdn_ch
     //      qk = tril(<q_i,k_j> 2^(gamma_i - gamma_j)) with the same gate factors, as bf16 straight to global memory
     //      (rows past a ragged chunk's end are another sequence's rows and are not written)
     {
-      __nv_bfloat16* Pg = reinterpret_cast<__nv_bfloat16*>(a.qk) + (row0 * a.HV + hv) * BT + cs + 2 * t;
+      __nv_bfloat16* Pg = reinterpret_cast<__nv_bfloat16*>(a.qk) + (row0 * a.HV + hv) * BT + cs + 8 * t;
       const int64_t pstride = (int64_t)a.HV * BT;
       if (q * 16 + 15 >= cs) {   // a block entirely above the diagonal is never read by the solve and is zero in qk
         float r[16], pq[16];
         acc_ld32q(tm, q, cs, r);
         if (with_qk) acc_ld32q(tm + 64, q, cs, pq);
         tc5::tmem_ld_wait();
-        const float g_lo = gam[r_lo], g_hi = gam[r_hi], b_lo = bet[r_lo], b_hi = bet[r_hi];
+        const float g_lo = gam[r_lo], g_hi = gam[r_hi];
+        const float b_lo = bet[r_lo], b_hi = bet[r_hi];
+        uint32_t p_lo[4], p_hi[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const int j0 = cs + i * 8 + 2 * t;
+          const float2 gj = *reinterpret_cast<const float2*>(&gam[j0]);
           float v[4], w4[4];
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             const int ii = (e & 2) ? r_hi : r_lo, jj = j0 + (e & 1);
-            const float f = fast_exp2(((e & 2) ? g_hi : g_lo) - gam[jj]);
+            const float f = fast_exp2(((e & 2) ? g_hi : g_lo) - ((e & 1) ? gj.y : gj.x));
             v[e] = (ii > jj) ? r[4 * i + e] * ((e & 2) ? b_hi : b_lo) * f : 0.f;
             w4[e] = (with_qk && ii >= jj) ? pq[4 * i + e] * f : 0.f;
           }
           *reinterpret_cast<float2*>(&Lf[r_lo * LDF + j0]) = make_float2(v[0], v[1]);
           *reinterpret_cast<float2*>(&Lf[r_hi * LDF + j0]) = make_float2(v[2], v[3]);
-          if (with_qk) {
-            if (r_lo < cm.len) *reinterpret_cast<uint32_t*>(Pg + r_lo * pstride + i * 8) = pack_bf16(w4[0], w4[1]);
-            if (r_hi < cm.len) *reinterpret_cast<uint32_t*>(Pg + r_hi * pstride + i * 8) = pack_bf16(w4[2], w4[3]);
-          }
+          p_lo[i] = pack_bf16(w4[0], w4[1]);
+          p_hi[i] = pack_bf16(w4[2], w4[3]);
+        }
+        if (with_qk) {
+          const uint4 lo = quad_words(p_lo, t), hi = quad_words(p_hi, t);
+          if (r_lo < cm.len) *reinterpret_cast<uint4*>(Pg + r_lo * pstride) = lo;
+          if (r_hi < cm.len) *reinterpret_cast<uint4*>(Pg + r_hi * pstride) = hi;
         }
       } else if (with_qk) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          if (r_lo < cm.len) *reinterpret_cast<uint32_t*>(Pg + r_lo * pstride + i * 8) = 0u;
-          if (r_hi < cm.len) *reinterpret_cast<uint32_t*>(Pg + r_hi * pstride + i * 8) = 0u;
-        }
+        if (r_lo < cm.len) *reinterpret_cast<uint4*>(Pg + r_lo * pstride) = make_uint4(0, 0, 0, 0);
+        if (r_hi < cm.len) *reinterpret_cast<uint4*>(Pg + r_hi * pstride) = make_uint4(0, 0, 0, 0);
       }
     }
     tc5::fence_before_sync();
     __syncthreads();
 
-    // ---- four 16x16 diagonal inverses: thread (block b, column cc) solves (I + L_bb) x = e_cc right-looking,
-    //      so that the updates of one step are independent of each other
-    if (tid < BT) {
-      const int b0 = (tid >> 4) * 16, cc = tid & 15;
+    // ---- four 16x16 diagonal inverses, one per warp: lane cc (and its copy cc + 16) solves (I + L_bb) x = e_cc row by row;
+    //      the rows of L_bb are uniform over the warp and do not depend on the chain, so their loads run ahead of it
+    if (warp < 4) {
+      const int b0 = warp * 16, cc = lane & 15;
       float s[16];
 #pragma unroll
-      for (int i = 0; i < 16; ++i) s[i] = (i == cc) ? 1.f : 0.f;
+      for (int i = 0; i < 16; ++i) {
+        float x0 = (i == cc) ? 1.f : 0.f, x1 = 0.f;
 #pragma unroll
-      for (int j = 0; j < 15; ++j) {
-        const float xj = s[j];
-#pragma unroll
-        for (int i = j + 1; i < 16; ++i) s[i] -= Lf[(b0 + i) * LDF + b0 + j] * xj;
+        for (int j = 0; j < i; j += 4) {
+          const float4 l = *reinterpret_cast<const float4*>(&Lf[(b0 + i) * LDF + b0 + j]);
+          x1 -= l.x * s[j];
+          if (j + 1 < i) x0 -= l.y * s[j + 1];
+          if (j + 2 < i) x1 -= l.z * s[j + 2];
+          if (j + 3 < i) x0 -= l.w * s[j + 3];
+        }
+        s[i] = x0 + x1;
+        if (lane < 16) Af[(b0 + i) * LDF + b0 + cc] = s[i];
       }
-#pragma unroll
-      for (int i = 0; i < 16; ++i) Af[(b0 + i) * LDF + b0 + cc] = s[i];
     }
     __syncthreads();
-    // ---- 16 -> 32: blocks (16,0) and (48,32), 64 threads each
-    if (tid < 128) merge_step1<16>(Lf, Af, Tf + (tid >> 6) * 16, (tid >> 6) ? 48 : 16, (tid >> 6) ? 32 : 0, tid & 63, 64);
+    // ---- 16 -> 32: blocks (16,0) and (48,32), four warps each
+    merge_step1<16>(Lf, Af, Tf + (warp >> 2) * 16, hc ? 48 : 16, hc ? 32 : 0, 4 * q, lane);
     __syncthreads();
-    if (tid < 128) merge_step2<16>(Tf + (tid >> 6) * 16, Af, (tid >> 6) ? 48 : 16, (tid >> 6) ? 32 : 0, tid & 63, 64, 8 * (warp & 1) + 8);
+    merge_step2<16>(Tf + (warp >> 2) * 16, Af, hc ? 48 : 16, hc ? 32 : 0, 4 * q, lane);
     __syncthreads();
-    // ---- 32 -> 64: block (32,0), all threads
-    merge_step1<32>(Lf, Af, Tf, 32, 0, tid, NTHREADS);
+    // ---- 32 -> 64: block (32,0), all warps
+    merge_step1<32>(Lf, Af, Tf, 32, 0, 4 * warp, lane);
     __syncthreads();
     // L is dead: its place takes the V tile while the last merge step and the conversion run
     if (tid == 0) {
@@ -283,7 +367,7 @@ __global__ void __launch_bounds__(NTHREADS, 4) intra_fwd_kernel(const b200gdn_ch
       tc5::mbar_expect_tx(bar_v, (uint32_t)(BT * DV * 2));
       tma::load_3d(Vs, &maps.v, cm.row, (hv * DV) / 64, bar_v);
     }
-    merge_step2<32>(Tf, Af, 32, 0, tid, NTHREADS, 4 * warp + 4);
+    merge_step2<32>(Tf, Af, 32, 0, 4 * warp, lane);
     __syncthreads();
 
     // ---- bf16 operand tiles (over the fp32 inverse and the merge temporary, hence through registers):
@@ -295,6 +379,11 @@ __global__ void __launch_bounds__(NTHREADS, 4) intra_fwd_kernel(const b200gdn_ch
         const int col = cs + i * 8 + 2 * t;
         x_lo[i] = *reinterpret_cast<const float2*>(&Af[r_lo * LDF + col]);
         x_hi[i] = *reinterpret_cast<const float2*>(&Af[r_hi * LDF + col]);
+        // above the diagonal only the 16x16 diagonal blocks have been written
+        if (col > r_lo) x_lo[i].x = 0.f;
+        if (col + 1 > r_lo) x_lo[i].y = 0.f;
+        if (col > r_hi) x_hi[i].x = 0.f;
+        if (col + 1 > r_hi) x_hi[i].y = 0.f;
       }
       __syncthreads();
       FragStore fw, fu, fa;
@@ -308,14 +397,12 @@ __global__ void __launch_bounds__(NTHREADS, 4) intra_fwd_kernel(const b200gdn_ch
       }
       fw.store(Aw, BT, q * 16, cs, lane);
       fu.store(Au, BT, q * 16, cs, lane);
-      // A itself goes straight to global memory (16 contiguous bytes per lane quad and row)
-      __nv_bfloat16* Ag = reinterpret_cast<__nv_bfloat16*>(a.A) + (row0 * a.HV + hv) * BT + cs + 2 * t;
+      // A itself goes straight to global memory, 64 contiguous bytes per row and quad
+      __nv_bfloat16* Ag = reinterpret_cast<__nv_bfloat16*>(a.A) + (row0 * a.HV + hv) * BT + cs + 8 * t;
       const int64_t astride = (int64_t)a.HV * BT;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        if (r_lo < cm.len) *reinterpret_cast<uint32_t*>(Ag + r_lo * astride + i * 8) = fa.lo[i];
-        if (r_hi < cm.len) *reinterpret_cast<uint32_t*>(Ag + r_hi * astride + i * 8) = fa.hi[i];
-      }
+      const uint4 lo = quad_words(fa.lo, t), hi = quad_words(fa.hi, t);
+      if (r_lo < cm.len) *reinterpret_cast<uint4*>(Ag + r_lo * astride) = lo;
+      if (r_hi < cm.len) *reinterpret_cast<uint4*>(Ag + r_hi * astride) = hi;
     }
     tc5::fence_async_smem();
     tc5::fence_before_sync();
@@ -424,6 +511,8 @@ int launch(const b200gdn_chunk_args& a, cudaStream_t st) {
 int launch_intra_fwd(const b200gdn_chunk_args& a, cudaStream_t st) {
   if ((a.options & B200GDN_PREP_GATE) && a.A_log == nullptr)
     return set_error(B200GDN_ERR_BAD_ARGUMENT, "intra_fwd: the fused gate needs A_log");
+  if ((a.options & B200GDN_PREP_L2NORM) && (a.qn == nullptr || a.kn == nullptr))
+    return set_error(B200GDN_ERR_BAD_ARGUMENT, "intra_fwd: the fused L2 norm needs qn and kn");
   if (a.K == 128 && a.V == 128) return launch<128, 128>(a, st);
   if (a.K == 64 && a.V == 64) return launch<64, 64>(a, st);
   return set_error(B200GDN_ERR_UNSUPPORTED, "intra_fwd: K=%d V=%d not built (64/64 and 128/128 are)", a.K, a.V);

@@ -50,7 +50,8 @@ constexpr int WARP_OMMA = WARP_STORE + 1 + NOUT;
 constexpr int threads_of(bool out) { return 32 * (out ? WARP_OMMA + 1 : WARP_STORE + 1); }
 __device__ int g_scan_fwd_timeout = 0;
 
-template <int DK, int NSTAGE, bool OUT>
+// PRE: the scan of a sequence's affine map alone (nothing stored but the final state): one snapshot buffer, no v_new tile.
+template <int DK, int NSTAGE, bool OUT, bool PRE>
 struct ScanFwdSmem {
   static constexpr size_t w_bytes = BT * DK * 2;            // W tile, K tile, Q tile
   static constexpr size_t u_bytes = BT * BV * 2;            // U slice, P~ tile, v_new / o slices
@@ -59,8 +60,8 @@ struct ScanFwdSmem {
   static constexpr size_t stage_bytes = OUT ? o_pq + u_bytes : o_qt;
   static constexpr size_t o_sb = NSTAGE * stage_bytes;      // 2 x state snapshot [DK][64]
   static constexpr size_t sb_bytes = DK * BV * 2;
-  static constexpr size_t o_vn = o_sb + 2 * sb_bytes;       // 2 x v_new slice [64][64]
-  static constexpr size_t o_vt = o_vn + 2 * u_bytes;        // gated v_new slice
+  static constexpr size_t o_vn = o_sb + (PRE ? 1 : 2) * sb_bytes;   // 2 x v_new slice [64][64]
+  static constexpr size_t o_vt = o_vn + (PRE ? 0 : 2) * u_bytes;    // gated v_new slice
   static constexpr size_t o_os = o_vt + u_bytes;            // OUT: 2 x o staging [64][64]
   static constexpr size_t o_gam = o_os + (OUT ? 2 * u_bytes : 0);  // 2 NSTAGE x 64 floats
   static constexpr size_t o_bar = o_gam + 2 * NSTAGE * BT * 4;
@@ -71,10 +72,10 @@ struct ScanFwdMaps {
   CUtensorMap w, k, u, h, vn, q, o, pq;
 };
 
-template <int DK, int DV, int NSTAGE, bool OUT>
-__global__ void __launch_bounds__(threads_of(OUT))
+template <int DK, int DV, int NSTAGE, bool OUT, bool PRE>
+__global__ void __launch_bounds__(threads_of(OUT), PRE ? 2 : 1)
     scan_fwd_kernel(const b200gdn_chunk_args a, const __grid_constant__ ScanFwdMaps maps) {
-  using S = ScanFwdSmem<DK, NSTAGE, OUT>;
+  using S = ScanFwdSmem<DK, NSTAGE, OUT, PRE>;
   constexpr int NH = DK / 64;   // 16-row halves of the state per epilogue warp
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -104,7 +105,7 @@ __global__ void __launch_bounds__(threads_of(OUT))
   const int G = a.HV / a.H, hq = hv / G;
   const int c_first = a.seq_meta[2 * n], nc = a.seq_meta[2 * n + 1];
   const bool has_u = !m_mode && a.u != nullptr;
-  const bool st_h = !m_mode && a.h != nullptr, st_vn = !m_mode && a.v_new != nullptr;
+  const bool st_h = !PRE && !m_mode && a.h != nullptr, st_vn = !PRE && !m_mode && a.v_new != nullptr;
   float* const ht_out = m_mode ? a.cp_M : a.ht;
   const bool vfirst = !m_mode && (a.options & B200GDN_STATE_V_FIRST);   // h0 and ht stored [V][K]
   constexpr uint32_t TMEM_COLS = OUT ? 512 : 128;   // 384 used; the allocation is a power of two
@@ -188,7 +189,7 @@ __global__ void __launch_bounds__(threads_of(OUT))
       for (int ic = 0; ic < nc; ++ic) {
         const int s = ic % NSTAGE, par = (ic / NSTAGE) & 1;
         const uint32_t w_addr = tc5::smem_addr(smem + (size_t)s * S::stage_bytes), k_addr = w_addr + (uint32_t)S::w_bytes;
-        const uint32_t sb_addr = tc5::smem_addr(smem + S::o_sb + (ic & 1) * S::sb_bytes);
+        const uint32_t sb_addr = tc5::smem_addr(smem + S::o_sb + (PRE ? 0 : ic & 1) * S::sb_bytes);
         if (!tc5::mbar_wait_warp(&full[s], par) || !tc5::mbar_wait_warp(sb_ready, ic & 1)) { failed = true; break; }
         tc5::fence_after_sync();
         // V_acc = W S_bf16
@@ -276,7 +277,7 @@ __global__ void __launch_bounds__(threads_of(OUT))
       const ChunkMeta cm = load_chunk_meta(a.chunk_meta, c);   // consumed late in the step
       const uint32_t u_tile = smem_u32(smem + (size_t)s * S::stage_bytes + 2 * S::w_bytes);
       const float* gs = gam_all + (ic % (2 * NSTAGE)) * BT;
-      const uint32_t sb_tile = sb_base + buf * (uint32_t)S::sb_bytes;
+      const uint32_t sb_tile = sb_base + (PRE ? 0 : buf) * (uint32_t)S::sb_bytes;   // (PRE: its only reader is the chain's last product)
       const uint32_t vn_tile = vn_base + buf * (uint32_t)S::u_bytes;
 
       // the snapshot and v_new tiles of two chunks ago are no longer read (waited for in the shadow of the last product)
@@ -465,26 +466,30 @@ __global__ void __launch_bounds__(threads_of(OUT))
   if (warp == 0) tc5::tmem_dealloc(tm, TMEM_COLS);
 }
 
-template <int DK, int DV, int NSTAGE, bool OUT>
+template <int DK, int DV, int NSTAGE, bool OUT, bool PRE>
 int launch(const b200gdn_chunk_args& a, cudaStream_t st) {
-  using S = ScanFwdSmem<DK, NSTAGE, OUT>;
+  using S = ScanFwdSmem<DK, NSTAGE, OUT, PRE>;
   static_assert(DV % BV == 0, "value dimension is processed in 64-column slices");
-  static_assert(S::bytes <= 227 * 1024, "shared memory of one CTA");
+  static_assert(S::bytes <= 227 * 1024 && (!PRE || S::bytes <= 112 * 1024), "shared memory of one CTA");
   static_assert(DK == DV, "the transition-matrix slices reuse the value-slice code with V := K");
-  if (int e = ensure_smem(scan_fwd_kernel<DK, DV, NSTAGE, OUT>, S::bytes)) return e;
+  if (int e = ensure_smem(scan_fwd_kernel<DK, DV, NSTAGE, OUT, PRE>, S::bytes)) return e;
   ScanFwdMaps m;
   const uint64_t pk = (uint64_t)a.H * DK, pw = (uint64_t)a.HV * DK, pv = (uint64_t)a.HV * DV;
   int rc = 0;
   rc |= tma::encode_bf16_panels(&m.w, a.w, a.rows, pw, pw, BT, DK / 64);
-  rc |= tma::encode_bf16_panels(&m.k, a.k, a.rows, pk, pk, BT, DK / 64);
+  const bool l2 = a.options & B200GDN_PREP_L2NORM;   // q and k as passed are raw: the intra stage has left the normalised ones
+  const void* q = l2 ? a.qn : a.q;
+  const void* k = l2 ? a.kn : a.k;
+  if (k == nullptr || (OUT && q == nullptr)) return set_error(B200GDN_ERR_BAD_ARGUMENT, "scan_fwd: the fused L2 norm needs qn and kn");
+  rc |= tma::encode_bf16_panels(&m.k, k, a.rows, pk, pk, BT, DK / 64);
   CUtensorMap dummy;
-  rc |= tma::encode_bf16_2d(&dummy, a.k, a.rows, pk, pk, BT);
+  rc |= tma::encode_bf16_2d(&dummy, k, a.rows, pk, pk, BT);
   // an absent tensor gets a well-formed map over k; it is never used
   if (a.u) rc |= tma::encode_bf16_2d(&m.u, a.u, a.rows, pv, pv, BT); else m.u = dummy;
   if (a.h) rc |= tma::encode_bf16_2d(&m.h, a.h, (uint64_t)a.n_chunks * a.HV * DK, DV, DV, DK); else m.h = dummy;
   if (a.v_new) rc |= tma::encode_bf16_2d(&m.vn, a.v_new, a.rows, pv, pv, BT); else m.vn = dummy;
   if (OUT) {
-    rc |= tma::encode_bf16_panels(&m.q, a.q, a.rows, pk, pk, BT, DK / 64);
+    rc |= tma::encode_bf16_panels(&m.q, q, a.rows, pk, pk, BT, DK / 64);
     rc |= tma::encode_bf16_2d(&m.o, a.o, a.rows, pv, pv, 16);   // one output warp stores 16 rows
     rc |= tma::encode_bf16_2d(&m.pq, a.qk, a.rows, (uint64_t)a.HV * BT, (uint64_t)a.HV * BT, BT);
   } else {
@@ -494,23 +499,27 @@ int launch(const b200gdn_chunk_args& a, cudaStream_t st) {
   }
   if (rc != 0) return set_error(B200GDN_ERR_CUDA, "scan_fwd: cuTensorMapEncodeTiled failed (%d)", rc);
   dim3 grid(DV / BV + ((!OUT && a.cp_M != nullptr) ? DK / BV : 0), a.HV, a.n_seq);
-  scan_fwd_kernel<DK, DV, NSTAGE, OUT><<<grid, threads_of(OUT), S::bytes, st>>>(a, m);
+  scan_fwd_kernel<DK, DV, NSTAGE, OUT, PRE><<<grid, threads_of(OUT), S::bytes, st>>>(a, m);
   return check_launch(OUT ? "scan_out_fwd" : "scan_fwd");
 }
 
 }  // namespace
 
 int launch_scan_fwd(const b200gdn_chunk_args& a, cudaStream_t st) {
-  if (a.K == 128 && a.V == 128) return launch<128, 128, 3, false>(a, st);
-  if (a.K == 64 && a.V == 64) return launch<64, 64, 3, false>(a, st);
+  // Nothing stored on the way (a pre-scan): 108 KiB at K = V = 128, so that two CTAs share an SM.  A pre-scan has twice the
+  // slices of a scan (values and transition matrix), so one CTA per SM would often need a second wave: 3 pieces x 16 heads x
+  // 4 slices of 256 chunks took 523 us, 376 now.
+  const bool pre = a.h == nullptr && a.v_new == nullptr;
+  if (a.K == 128 && a.V == 128) return pre ? launch<128, 128, 2, false, true>(a, st) : launch<128, 128, 3, false, false>(a, st);
+  if (a.K == 64 && a.V == 64) return pre ? launch<64, 64, 3, false, true>(a, st) : launch<64, 64, 3, false, false>(a, st);
   return set_error(B200GDN_ERR_UNSUPPORTED, "scan_fwd: K=%d V=%d not built (64/64 and 128/128 are)", a.K, a.V);
 }
 
 // The scan and the chunk output in one kernel (needs q, qk and o in addition to the scan's arguments).
 int launch_scan_out_fwd(const b200gdn_chunk_args& a, cudaStream_t st) {
   if (a.qk == nullptr) return set_error(B200GDN_ERR_BAD_ARGUMENT, "scan_out_fwd: qk (written by the intra stage) is NULL");
-  if (a.K == 128 && a.V == 128) return launch<128, 128, 2, true>(a, st);
-  if (a.K == 64 && a.V == 64) return launch<64, 64, 3, true>(a, st);
+  if (a.K == 128 && a.V == 128) return launch<128, 128, 2, true, false>(a, st);
+  if (a.K == 64 && a.V == 64) return launch<64, 64, 3, true, false>(a, st);
   return set_error(B200GDN_ERR_UNSUPPORTED, "scan_out_fwd: K=%d V=%d not built (64/64 and 128/128 are)", a.K, a.V);
 }
 

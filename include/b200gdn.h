@@ -131,13 +131,18 @@ typedef struct b200gdn_chunk_args {
   /* written by the forward pass (intra stage, needs q), read by the fused scan stages of both passes:
    * bf16 [rows,HV,64], row i of a chunk holds <q_i,k_j> 2^(gamma_i - gamma_j) for j <= i, zero for j > i */
   void* qk;
-  /* Backward only.  q / k as passed are the L2-normalised tensors b200gdn_prep_fwd produced
-   * (fla/modules/l2norm.py:84-144); with their reciprocal norms given here (fp32 [rows,H]) the backward pass returns
-   * dq / dk w.r.t. the un-normalised tensors, dx = (dy - y <dy,y>) rstd, applied where dq and dk are completed
-   * (replaces l2norm_bwd, fla/modules/l2norm.py:200-251).  NULL: dq / dk are gradients w.r.t. q / k as passed. */
-  const float* rstd_q;
-  const float* rstd_k;
+  /* The layer's q / k L2 norm (fla/modules/l2norm.py:84-144), y = x rsqrt(sum x^2 + 1e-6), y rounded to bf16.
+   * Forward, with B200GDN_PREP_L2NORM in `options`: q and k are the raw tensors; the intra stage normalises the tiles it
+   * loads, writes them to qn / kn (bf16 [rows,H,K], required), which the scans then read, and leaves the reciprocal norms in
+   * rstd_q / rstd_k (fp32 [rows,H], either may be NULL).
+   * Backward: q / k as passed are the normalised tensors; with rstd_q / rstd_k given it returns dq / dk w.r.t. the
+   * un-normalised ones, dx = (dy - y <dy,y>) rstd, applied where dq and dk are completed (replaces l2norm_bwd,
+   * fla/modules/l2norm.py:200-251).  NULL: dq / dk are gradients w.r.t. q / k as passed. */
+  float* rstd_q;
+  float* rstd_k;
   int32_t gb_dtype;              /* B200GDN_F32 / BF16 / F16: element type of g, beta, dg and dbeta */
+  void* qn;
+  void* kn;
 } b200gdn_chunk_args;
 
 /* Replaces chunk_gated_delta_rule_fwd (fla/ops/gated_delta_rule/chunk.py:33-123):

@@ -202,3 +202,40 @@ def test_context_parallel_convolution_matches_single_gpu(world):
     for rank, errs in res:
         assert not isinstance(errs, str), f'rank {rank}: {errs}'
         assert errs['y'] < 1e-5 and errs['dx'] < 1e-5 and errs['dw'] < 1e-5 and errs['db'] < 1e-5, (rank, errs)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('K,V', [(64, 64), (128, 128), (128, 32), (256, 64)])
+@pytest.mark.parametrize('reverse', [False, True])
+def test_prefix_chains_against_torch(K, V, reverse):
+    """b200gdn_cp_prefix on chains of one to four pieces, with and without a start state: every piece's start (reverse: end)
+    value and the chain's final value against the recurrence written out in fp64."""
+    from b200gdn import _lib
+    dev = 'cuda'
+    gen = torch.Generator(device=dev).manual_seed(K + V)
+    HV, counts = 2, [1, 3, 4, 2]
+    n_out, n_pre = sum(counts), sum(c - 1 for c in counts)
+    M = torch.randn(n_pre, HV, K, K, device=dev, generator=gen) * K ** -0.5
+    h = torch.randn(n_pre, HV, K, V, device=dev, generator=gen)
+    x0 = torch.randn(len(counts), HV, K, V, device=dev, generator=gen)
+    table, o, p = [], 0, 0
+    for c in counts:
+        table.append([o, c, p])
+        o, p = o + c, p + c - 1
+    table = torch.tensor(table, dtype=torch.int32, device=dev)
+    for start in (None, x0):
+        out, last = torch.full((n_out, HV, K, V), float('nan'), device=dev), torch.empty_like(x0)
+        a = _lib.PrefixArgs()
+        a.HV, a.K, a.V, a.n_chains, a.reverse = HV, K, V, len(counts), int(reverse)
+        a.table, a.M, a.h, a.x0, a.out, a.last = table.data_ptr(), M.data_ptr(), h.data_ptr(), _lib.ptr(start), out.data_ptr(), last.data_ptr()
+        _lib.call('b200gdn_cp_prefix', a, torch.cuda.current_stream().cuda_stream)
+        for c, (fo, cnt, fp) in enumerate(table.tolist()):
+            x = torch.zeros(HV, K, V, dtype=torch.float64, device=dev) if start is None else start[c].double()
+            steps = range(cnt - 1)
+            pieces = [fo + cnt - 1 - t if reverse else fo + t for t in range(cnt)]
+            assert torch.allclose(out[pieces[0]].double(), x, atol=1e-6)
+            for t in steps:
+                j = fp + cnt - 2 - t if reverse else fp + t
+                x = M[j].double() @ x + h[j].double()
+                assert torch.allclose(out[pieces[t + 1]].double(), x, rtol=1e-4, atol=1e-4), (c, t)
+            assert torch.allclose(last[c].double(), x, rtol=1e-4, atol=1e-4)
