@@ -129,6 +129,14 @@ int b200gdn_chunk_bwd(const b200gdn_chunk_args* a, void* stream) {
       if (int e = launch_scan_bwd(*a, st)) return e;
     }
   }
+  if ((m & B200GDN_BWD_DQKWG) && (m & B200GDN_BWD_WY) && bwd_local_serves(*a)) {
+    // both chunk-local stages in one kernel: neither the chunk-local part of dk nor dG leaves the chip
+    REQUIRE(a->q, "chunk_bwd"); REQUIRE(a->k, "chunk_bwd"); REQUIRE(a->v, "chunk_bwd"); REQUIRE(a->v_new, "chunk_bwd");
+    REQUIRE(a->beta, "chunk_bwd"); REQUIRE(a->gamma, "chunk_bwd"); REQUIRE(a->A, "chunk_bwd"); REQUIRE(a->h, "chunk_bwd");
+    REQUIRE(a->dh, "chunk_bwd"); REQUIRE(a->dv2, "chunk_bwd"); REQUIRE(a->d_o, "chunk_bwd"); REQUIRE(a->dq, "chunk_bwd");
+    REQUIRE(a->dk, "chunk_bwd"); REQUIRE(a->dv, "chunk_bwd"); REQUIRE(a->dg, "chunk_bwd"); REQUIRE(a->dbeta, "chunk_bwd");
+    return launch_bwd_local(*a, st);
+  }
   if (m & B200GDN_BWD_DQKWG) {
     REQUIRE(a->q, "chunk_bwd"); REQUIRE(a->k, "chunk_bwd"); REQUIRE(a->v_new, "chunk_bwd"); REQUIRE(a->gamma, "chunk_bwd");
     REQUIRE(a->h, "chunk_bwd"); REQUIRE(a->dh, "chunk_bwd"); REQUIRE(a->dv2, "chunk_bwd"); REQUIRE(a->d_o, "chunk_bwd");
@@ -339,7 +347,8 @@ int b200gdn_device_status(void) {
   struct { const char* name; int (*flag)(); } k[] = {
       {"intra_fwd", gdn::intra_fwd_timeout_flag}, {"scan_fwd", gdn::scan_fwd_timeout_flag}, {"out_fwd", gdn::out_fwd_timeout_flag},
       {"dv_local", gdn::dv_local_timeout_flag},   {"scan_bwd", gdn::scan_bwd_timeout_flag}, {"bwd_dqk", gdn::bwd_dqk_timeout_flag},
-      {"bwd_wy", gdn::bwd_wy_timeout_flag},       {"selftest", gdn::selftest_timeout_flag},
+      {"bwd_wy", gdn::bwd_wy_timeout_flag},       {"bwd_local", gdn::bwd_local_timeout_flag},
+            {"selftest", gdn::selftest_timeout_flag},
       {"decode_stream", gdn::decode_timeout_flag}};
   cudaError_t e = cudaDeviceSynchronize();
   if (e != cudaSuccess) return gdn::set_error(B200GDN_ERR_CUDA, "device_status: %s", cudaGetErrorString(e));

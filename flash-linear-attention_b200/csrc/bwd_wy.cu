@@ -625,18 +625,26 @@ int launch(const b200gdn_chunk_args& a, cudaStream_t st) {
   dim3 grid(a.n_chunks, a.H);
   bwd_wy_kernel<DK, DV, GROUPED><<<grid, NTHREADS, S::bytes, st>>>(a, m);
   if (int e = check_launch("bwd_wy")) return e;
-  if (a.options & B200GDN_PREP_GATE) {
-    gate_param_reduce_kernel<<<a.HV, 256, 0, st>>>(a);
-    return check_launch("gate_param_reduce");
-  }
-  return 0;
+  return launch_gate_reduce(a, st);
 }
 
 }  // namespace
 
-int launch_bwd_wy(const b200gdn_chunk_args& a, cudaStream_t st) {
+int check_gate_args(const b200gdn_chunk_args& a, const char* who) {
   if ((a.options & B200GDN_PREP_GATE) && (a.g == nullptr || a.A_log == nullptr || a.gate_partials == nullptr || a.dA_log == nullptr))
-    return set_error(B200GDN_ERR_BAD_ARGUMENT, "bwd_wy: the fused gate needs g (raw), A_log, gate_partials and dA_log");
+    return set_error(B200GDN_ERR_BAD_ARGUMENT, "%s: the fused gate needs g (raw), A_log, gate_partials and dA_log", who);
+  return 0;
+}
+
+// the parameter gradients of the fused gate from the per-chunk sums the kernels leave (nothing without that option)
+int launch_gate_reduce(const b200gdn_chunk_args& a, cudaStream_t st) {
+  if (!(a.options & B200GDN_PREP_GATE)) return 0;
+  gate_param_reduce_kernel<<<a.HV, 256, 0, st>>>(a);
+  return check_launch("gate_param_reduce");
+}
+
+int launch_bwd_wy(const b200gdn_chunk_args& a, cudaStream_t st) {
+  if (int e = check_gate_args(a, "bwd_wy")) return e;
   if (a.HV > a.H && a.dk_part == nullptr) return set_error(B200GDN_ERR_BAD_ARGUMENT, "bwd_wy: dk_part is required when HV > H");
   const bool grouped = a.HV > a.H;
   if (a.K == 128 && a.V == 128) return grouped ? launch<128, 128, true>(a, st) : launch<128, 128, false>(a, st);

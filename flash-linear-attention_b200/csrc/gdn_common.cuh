@@ -96,6 +96,10 @@ int launch_scan_bwd(const b200gdn_chunk_args& a, cudaStream_t st);
 int launch_scan_dvl_bwd(const b200gdn_chunk_args& a, cudaStream_t st);
 int launch_bwd_dqk(const b200gdn_chunk_args& a, cudaStream_t st);
 int launch_bwd_wy(const b200gdn_chunk_args& a, cudaStream_t st);
+int launch_bwd_local(const b200gdn_chunk_args& a, cudaStream_t st);
+bool bwd_local_serves(const b200gdn_chunk_args& a);
+int launch_gate_reduce(const b200gdn_chunk_args& a, cudaStream_t st);
+int check_gate_args(const b200gdn_chunk_args& a, const char* who);
 int launch_recurrent(const b200gdn_recurrent_args& a, cudaStream_t st);
 int launch_affine(const b200gdn_affine_args& a, cudaStream_t st);
 int launch_cp_fold(const b200gdn_fold_args& a, cudaStream_t st);
@@ -112,6 +116,7 @@ int dv_local_timeout_flag();
 int scan_bwd_timeout_flag();
 int bwd_dqk_timeout_flag();
 int bwd_wy_timeout_flag();
+int bwd_local_timeout_flag();
 int set_error(int code, const char* fmt, ...);
 int check_launch(const char* what);
 void reset_launch_count();

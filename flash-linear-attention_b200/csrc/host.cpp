@@ -417,7 +417,8 @@ class ChunkFunction : public torch::autograd::Function<ChunkFunction> {
     const bool zero = !plan.covered, gate = s.options & B200GDN_PREP_GATE;
     b200gdn_chunk_args a = chunk_args(q, k, v, s.scale, plan);
     const int64_t rows = a.rows, H = a.H, HV = a.HV, K = a.K, V = a.V, C = a.n_chunks, N = a.n_seq;
-    const bool grouped = HV > H;
+    const int64_t G = HV / H;
+    const bool grouped = G > 1 && G != 2 && G != 4 && G != 8;   // group sums through HBM (other sizes stay on the chip)
     const Tensor d_o = grads[0].defined() ? dense(grads[0], at::kBFloat16) : new_tensor(v.sizes(), at::kBFloat16, dev, true);
     Tensor dht = grads.size() > 1 ? dense(grads[1], at::kFloat) : Tensor();
     if (s.transpose_states && dht.defined()) dht = dht.transpose(-1, -2).contiguous();

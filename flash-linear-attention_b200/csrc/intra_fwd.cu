@@ -107,17 +107,6 @@ __device__ __forceinline__ void merge_step2(const float* T, float* Af, int r0, i
   }
 }
 
-// Four words per lane of a quad (word i: columns 8 i + 2 t, + 1 of a row) -> the four words of column group t, so that a row's
-// 32 columns leave in 16-byte words.
-__device__ __forceinline__ uint4 quad_words(const uint32_t (&w)[4], int t) {
-  const bool odd = t & 1, hi = t & 2;
-  uint32_t a0 = w[0], a1 = w[1], a2 = w[2], a3 = w[3];
-  const uint32_t r0 = __shfl_xor_sync(0xffffffffu, odd ? a0 : a1, 1), r1 = __shfl_xor_sync(0xffffffffu, odd ? a2 : a3, 1);
-  if (odd) { a0 = r0; a2 = r1; } else { a1 = r0; a3 = r1; }
-  const uint32_t s0 = __shfl_xor_sync(0xffffffffu, hi ? a0 : a2, 2), s1 = __shfl_xor_sync(0xffffffffu, hi ? a1 : a3, 2);
-  return hi ? make_uint4(s0, s1, a2, a3) : make_uint4(a0, a1, s0, s1);
-}
-
 // L2-normalises the rows of a swizzled [64][DK] tile in place (four lanes per row), rounded to bf16; with `out` the rows also
 // go to global memory and their reciprocal norms to `rstd`
 template <int DK>

@@ -82,6 +82,43 @@ struct FragLoad {
   __device__ __forceinline__ float2 hi2(int i) const { return unpack_bf16(hi[i]); }
 };
 
+// Four words per lane of a quad (lanes t = 0..3; word i: columns 8 i + 2 t, + 1 of a row) -> the four words of column group t, so that a row's
+// 32 columns leave in 16-byte words.
+__device__ __forceinline__ uint4 quad_words(const uint32_t (&w)[4], int t) {
+  const bool odd = t & 1, hi = t & 2;
+  uint32_t a0 = w[0], a1 = w[1], a2 = w[2], a3 = w[3];
+  const uint32_t r0 = __shfl_xor_sync(0xffffffffu, odd ? a0 : a1, 1), r1 = __shfl_xor_sync(0xffffffffu, odd ? a2 : a3, 1);
+  if (odd) { a0 = r0; a2 = r1; } else { a1 = r0; a3 = r1; }
+  const uint32_t s0 = __shfl_xor_sync(0xffffffffu, hi ? a0 : a2, 2), s1 = __shfl_xor_sync(0xffffffffu, hi ? a1 : a3, 2);
+  return hi ? make_uint4(s0, s1, a2, a3) : make_uint4(a0, a1, s0, s1);
+}
+
+// A 16 x 32 block of the TRANSPOSE of a swizzled bf16 tile [token][column] in the accumulator-fragment layout: lo[i] / hi[i] hold
+// (column col0 + g / col0 + 8 + g) x (tokens tok0 + 8 i + 2 t, + 1).
+struct FragLoadT {
+  uint32_t lo[4], hi[4];
+  __device__ __forceinline__ void load(const unsigned char* tile, int rows, int tok0, int col0, int lane) {
+    const uint32_t base = tc5::smem_addr(tile);
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];\n"
+                 : "=r"(lo[0]), "=r"(lo[1]), "=r"(lo[2]), "=r"(lo[3])
+                 : "r"(base + tc5::swz_offset(tok0 + lane, col0, rows))
+                 : "memory");
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];\n"
+                 : "=r"(hi[0]), "=r"(hi[1]), "=r"(hi[2]), "=r"(hi[3])
+                 : "r"(base + tc5::swz_offset(tok0 + lane, col0 + 8, rows))
+                 : "memory");
+  }
+  __device__ __forceinline__ float2 lo2(int i) const { return unpack_bf16(lo[i]); }
+  __device__ __forceinline__ float2 hi2(int i) const { return unpack_bf16(hi[i]); }
+};
+
+// transpose of an 8 x 8 matrix of 16-bit elements held one 32-bit word (two elements of a row) per lane
+__device__ __forceinline__ uint32_t transpose8(uint32_t x) {
+  uint32_t y;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;\n" : "=r"(y) : "r"(x));
+  return y;
+}
+
 // Zero rows [valid, ROWS) of a swizzled [ROWS][COLS] tile (a ragged last chunk arrives by TMA as a full box
 // whose extra rows belong to the next sequence).  The caller fences and synchronises afterwards.
 template <int ROWS, int COLS>
