@@ -45,7 +45,7 @@ struct LocalSmem {
   static constexpr size_t o_vec = o_ab + BT * 128;
   static constexpr int LDS = DK + 4;                                // fp32 row stride of the group-sum staging
   static constexpr size_t stage = (size_t)BT * LDS * 4;             // dq, then dk, from R2 on
-  static constexpr size_t bytes = o_vec + 27 * BT * 4 + 160 + 1024; // + vectors, barriers, alignment slack
+  static constexpr size_t bytes = o_vec + 28 * BT * 4 + 160 + 1024; // + vectors, barriers, alignment slack
   static_assert(o_do + 2 * stage <= o_vec, "the group-sum staging fits over the dead tiles");
 };
 
@@ -167,7 +167,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
   unsigned char *H1 = smem + S::o_h1, *Vs = H1, *dAs = H1, *M2s = H1, *Ys = H1 + BT * 128;
   unsigned char *As = smem + S::o_a, *Ps = smem + S::o_ps, *Abs = smem + S::o_ab;
   float* gs = reinterpret_cast<float*>(smem + S::o_vec);
-  float *bet = gs + BT, *bge = bet + BT, *eg = bge + BT, *sgm = eg + BT, *gx = sgm + BT, *dGs = gx + BT, *rsq = dGs + BT, *rsk = rsq + BT;
+  float *bet = gs + BT, *bge = bet + BT, *eg = bge + BT, *sgm = eg + BT, *gx = sgm + BT, *gv = gx + BT, *dGs = gv + BT, *rsq = dGs + BT, *rsk = rsq + BT;
   // sums over rows: each of the four row-quadrant warps leaves its partial in its own slot and the consumer adds the four in
   // a fixed order (no atomics: results are bit-reproducible)
   float* c_rq = rsk + BT;        // [4][64] <dq_i, q_i>
@@ -217,8 +217,14 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
       b = ok ? ((a.options & B200GDN_PREP_NEG_EIGVAL) ? 2.f : 1.f) * sg : 0.f;
     }
     bet[tid] = b;
-    if (a.options & B200GDN_PREP_GATE)
-      gx[tid] = (ok ? ld_param(a.g, (row0 + tid) * a.HV + hv, a.gb_dtype) : 0.f) + (a.dt_bias ? a.dt_bias[hv] : 0.f);
+  }
+  if ((a.options & B200GDN_PREP_GATE) && tid >= 2 * BT && tid < 3 * BT) {
+    // fused gate: g = -exp(A_log) softplus(x), x = g_raw + dt_bias; its value and derivative, while the tiles are on their way
+    const int r = tid - 2 * BT;
+    const float x = (r < cm.len ? ld_param(a.g, (row0 + r) * a.HV + hv, a.gb_dtype) : 0.f) + (a.dt_bias ? a.dt_bias[hv] : 0.f);
+    const float negA = -expf(a.A_log[hv]);
+    gx[r] = negA / (1.f + expf(-x));
+    gv[r] = negA * (x > 20.f ? x : log1pf(expf(x)));
   }
   if (!GROUPED && tid >= BT && tid < 2 * BT) {   // L2-norm option: reciprocal norms of the rows
     const int r = tid - BT;
@@ -629,16 +635,15 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
     if (!(a.options & B200GDN_PREP_GATE)) {
       if (tid < cm.len) st_param(a.dg, (row0 + tid) * a.HV + hv, a.gb_dtype, dGs[tid] + (tid < 32 ? dGs[32] : 0.f));
     } else {
-      // fused gate: g = -exp(A_log) softplus(x), x = g_raw + dt_bias.  dg_raw = dg (-exp(A_log)) sigmoid(x);
-      // dA_log += dg g and ddt_bias += dg_raw, summed over the chunk here and over the chunks by a second kernel
+      // dg_raw = dg dg/dg_raw; dA_log += dg g and ddt_bias += dg_raw, summed over the chunk here and over the chunks by a second
+      // kernel
       if (tid < BT) {
         float sA = 0.f, sB = 0.f;
         if (tid < cm.len) {
           const float dgi = dGs[tid] + (tid < 32 ? dGs[32] : 0.f);
-          const float x = gx[tid], negA = -expf(a.A_log[hv]);
-          const float draw = dgi * negA / (1.f + expf(-x));
+          const float draw = dgi * gx[tid];
           st_param(a.dg, (row0 + tid) * a.HV + hv, a.gb_dtype, draw);
-          sA = dgi * negA * (x > 20.f ? x : log1pf(expf(x)));
+          sA = dgi * gv[tid];
           sB = draw;
         }
         sA = warp_sum(sA);
