@@ -50,11 +50,11 @@ STAGE_FLOPS = {
     'intra_fwd': 2 * BT * (3 * K + V),                                 # K K^T, W, U | Q K^T
     'scan_out_fwd': 4 * K * V + 2 * K * V + 2 * BT * V,                # W S, K^T V~ | Q S, P V
     'scan_dvl_bwd': 6 * K * V + 2 * BT * (K + V),                      # K dS, Q^T do, W^T dv2 | P^T do (+ the Q K^T it does not redo)
-    'bwd_dqk': 4 * K * V + 2 * BT * (V + 2 * K),                       # dP, do h^T, v dh^T, dP k, dP^T q
-    'bwd_wy': 2 * K * V + 2 * BT * (5 * K + 2 * V + 2 * BT),           # dv2 h^T + WY backward
+    # dP, do h^T, v dh^T, dP k, dP^T q | dv2 h^T + WY backward
+    'bwd_local': 6 * K * V + 2 * BT * (V + 2 * K) + 2 * BT * (5 * K + 2 * V + 2 * BT),
 }
 F_FWD = STAGE_FLOPS['intra_fwd'] + STAGE_FLOPS['scan_out_fwd']
-F_BWD = STAGE_FLOPS['scan_dvl_bwd'] + STAGE_FLOPS['bwd_dqk'] + STAGE_FLOPS['bwd_wy']
+F_BWD = STAGE_FLOPS['scan_dvl_bwd'] + STAGE_FLOPS['bwd_local']
 assert F_FWD == 180224 and F_BWD == 409600
 
 
@@ -77,13 +77,12 @@ def staged_bytes(R, C, NS):
     snap = C * HV * K * V * 2                         # h or dh snapshots
     st32 = NS * HV * K * V * 4                        # h0, ht, dht, dh0
     gam, vec = C * HV * BT * 4, R * HV * 4
-    dkp = R * H * K * 2                               # chunk-local part of dk, bf16, passed through the dk buffer
     return {
         'intra_fwd': 2 * qk + wv + 2 * vec + 2 * a_ + w + wv + gam,                          # k q v -> A qk w u
         'scan_out_fwd': w + 2 * qk + wv + a_ + gam + st32 + snap + wv + st32 + wv,     # w k q u qk -> h v_new o
         'scan_dvl_bwd': 2 * qk + w + wv + a_ + gam + st32 + wv + snap + st32,          # q k w do qk -> dv2 dh dh0
-        'bwd_dqk': 2 * qk + 2 * wv + 2 * snap + gam + qk + dkp + vec,
-        'bwd_wy': qk + 2 * wv + a_ + snap + gam + 2 * vec + dkp + qk + wv + 2 * vec,
+        # q k v do v_new dv2 A h dh -> dq dk dv dbeta dg
+        'bwd_local': 2 * qk + 4 * wv + a_ + 2 * snap + gam + vec + 2 * qk + wv + 2 * vec,
     }
 
 
@@ -254,8 +253,8 @@ def time_stages(batch, steps):
         setattr(a, n, x.data_ptr())
     stream = torch.cuda.current_stream(dev)
     plan = [('intra_fwd', 'b200gdn_chunk_fwd', _lib.FWD_INTRA), ('scan_out_fwd', 'b200gdn_chunk_fwd', _lib.FWD_SCAN | _lib.FWD_OUT),
-            ('scan_dvl_bwd', 'b200gdn_chunk_bwd', _lib.BWD_DVLOCAL | _lib.BWD_SCAN), ('bwd_dqk', 'b200gdn_chunk_bwd', _lib.BWD_DQKWG),
-            ('bwd_wy', 'b200gdn_chunk_bwd', _lib.BWD_WY)]
+            ('scan_dvl_bwd', 'b200gdn_chunk_bwd', _lib.BWD_DVLOCAL | _lib.BWD_SCAN),
+            ('bwd_local', 'b200gdn_chunk_bwd', _lib.BWD_DQKWG | _lib.BWD_WY)]
     total = {n: 0.0 for n, _, _ in plan}
     for it in range(steps + 1):
         evs = []

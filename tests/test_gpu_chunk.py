@@ -631,6 +631,41 @@ def test_trailing_empty_sequence():
     b200gdn.device_status()
 
 
+@pytest.mark.parametrize('K,H,HV', [(64, 2, 2), (64, 1, 8), (128, 1, 3), (128, 2, 4), (128, 2, 8), (128, 1, 8)])
+def test_chunk_local_backward_by_group_size(K, H, HV):
+    """One to eight value heads per key head sum their dq and dk in a cluster, other group sizes take the separate
+    kernels; sequences of one token up to one past a tile, with and without the layer's options."""
+    cu = [0, 1, 64, 129, 192, 255, 300]
+    d = O.make_inputs(1, 300, H, HV, K, K, seed=17, cu_seqlens=cu)
+    bf = {n: d[n].to(torch.bfloat16) for n in ('q', 'k', 'v', 'do')}
+    cu_t = torch.tensor(cu, dtype=torch.int32, device='cuda')
+    _, _, ref = O.naive_with_grads(*(bf[n].float() for n in ('q', 'k', 'v')), d['g'], d['beta'], K ** -0.5, d['h0'],
+                                   bf['do'].float(), torch.zeros_like(d['h0']), cu_seqlens=cu)
+    from b200gdn import chunk_gated_delta_rule
+    for options in (False, True):
+        ins = [bf['q'], bf['k'], bf['v'], d['g'], d['beta']]
+        kw, extra = {}, []
+        if options:   # the same q, k, g and beta through the in-kernel steps
+            log_a, dt = torch.zeros(HV, device='cuda', requires_grad=True), torch.zeros(HV, device='cuda', requires_grad=True)
+            ins[3] = torch.log(torch.expm1(-d['g'].double()).clamp_min(1e-12)).float()   # g = -softplus(raw)
+            ins[4] = torch.logit(d['beta'].double()).float()
+            kw = dict(use_qk_l2norm_in_kernel=True, use_gate_in_kernel=True, A_log=log_a, dt_bias=dt, use_beta_sigmoid_in_kernel=True)
+            extra = [log_a, dt]
+        leaves = [x.cuda().requires_grad_(True) for x in ins]
+        o, _ = chunk_gated_delta_rule(*leaves, initial_state=d['h0'].cuda(), cu_seqlens=cu_t, **kw)
+        got = torch.autograd.grad(o, leaves + extra, bf['do'].cuda())
+        want = [ref[n].float() for n in ('dq', 'dk', 'dv', 'dg', 'dbeta')]
+        if options:
+            for i, x in ((0, bf['q']), (1, bf['k'])):   # backward of x / |x|
+                x = x.float().requires_grad_(True)
+                want[i], = torch.autograd.grad(torch.nn.functional.normalize(x, dim=-1), x, want[i])
+            want[4] = want[4] * d['beta'] * (1 - d['beta'])
+            dg, want[3] = want[3], want[3] * -torch.sigmoid(ins[3])
+            want += [(dg * d['g']).sum((0, 1)), want[3].sum((0, 1))]
+        for n, w, x, tol in zip(('dq', 'dk', 'dv', 'dg', 'dbeta', 'dA_log', 'ddt_bias'), want, got, (0.008,) * 3 + (0.02,) * 4):
+            O.assert_close(f'{n} options={options}', w, x.float().cpu(), tol)
+
+
 def test_fp32_and_fp16_inputs_are_rounded_to_bf16_and_keep_their_dtype():
     """q, k, v in fp32 / fp16: the result is the bf16 computation on the rounded inputs (documented), returned in
     the caller's dtype, gradients in each input's dtype."""
