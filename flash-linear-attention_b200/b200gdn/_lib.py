@@ -37,7 +37,7 @@ class ChunkArgs(C.Structure):
         ('dh', _p), ('dv2', _p), ('dw', _p), ('dk_part', _p), ('dG', _p), ('dq_acc', _p),
         ('options', C.c_uint32), ('A_log', _p), ('dt_bias', _p), ('gate_partials', _p), ('dA_log', _p), ('ddt_bias', _p),
         ('cp_M', _p), ('cp_dM', _p), ('qk', _p), ('rstd_q', _p), ('rstd_k', _p), ('gb_dtype', C.c_int32),
-        ('qn', _p), ('kn', _p),
+        ('qn', _p), ('kn', _p), ('seq_order', _p),
     ]
 
 

@@ -18,11 +18,12 @@ class Tables(tuple):
     the last sequence belong to no sequence (a padded packed buffer).  The kernels never write such rows, so the
     caller zero-fills its intermediates then.  ``native()`` is the same as one handle for the native host path."""
     covered = True
+    order = None      # int32 [n_seq]: sequences by falling length, None when all are of one length
     _native = None
 
     def native(self):
         if self._native is None:
-            self._native = _lib.host().plan(self[0], self[1], self[2][0], self[2][1], self.covered)
+            self._native = _lib.host().plan(self[0], self[1], self[2][0], self[2][1], self.covered, self.order)
         return self._native
 
 
@@ -46,6 +47,16 @@ def build_tables(bounds: Sequence[Tuple[int, int]]):
     return chunk_meta, seq_meta
 
 
+def device_tables(bounds, device) -> Tables:
+    """build_tables on the device, with the order in which the scans take the sequences: a scan CTA walks one sequence,
+    so with more CTAs than SMs a long sequence that starts late is what everything else waits for."""
+    cm, sm = build_tables(bounds)
+    out = Tables((torch.from_numpy(cm).to(device), torch.from_numpy(sm).to(device), (cm.shape[0], sm.shape[0])))
+    if len(sm) > 1 and (sm[:, 1] != sm[0, 1]).any():
+        out.order = torch.from_numpy(np.argsort(-sm[:, 1], kind='stable').astype(np.int32)).to(device)
+    return out
+
+
 def tables_for(B: int, T: int, cu_seqlens: Optional[torch.Tensor], cu_seqlens_cpu: Optional[torch.Tensor],
                device: torch.device) -> Tables:
     """Device tables for a dense [B,T] batch or a packed batch; memoised by shape / by the identity of
@@ -67,8 +78,7 @@ def tables_for(B: int, T: int, cu_seqlens: Optional[torch.Tensor], cu_seqlens_cp
         bounds = [(cu[i], cu[i + 1]) for i in range(len(cu) - 1)]
         if cu and (cu[0] < 0 or cu[-1] > B * T):
             raise ValueError(f'cu_seqlens [{cu[0]}, {cu[-1]}] reaches outside the {B * T} token rows')
-    cm, sm = build_tables(bounds)
-    out = Tables((torch.from_numpy(cm).to(device), torch.from_numpy(sm).to(device), (cm.shape[0], sm.shape[0])))
+    out = device_tables(bounds, device)
     out.covered = bool(bounds) and bounds[0][0] == 0 and bounds[-1][1] == B * T
     if len(_cache) > 64:
         _cache.clear()
@@ -98,7 +108,7 @@ class SplitPlan:
         """The plan as one handle for the native host path."""
         if self._native is None:
             t = self.tables
-            self._native = _lib.host().plan(t[0], t[1], t[2][0], t[2][1], t.covered, self.chains, self.pre_fwd, self.pre_bwd,
+            self._native = _lib.host().plan(t[0], t[1], t[2][0], t[2][1], t.covered, t.order, self.chains, self.pre_fwd, self.pre_bwd,
                                             self.first_piece, self.last_piece, self.n_chains, self.n_pre)
         return self._native
 
@@ -139,9 +149,9 @@ def split_plan(bounds, HV: int, slices: int, device, rows: int) -> Optional[Spli
         n_pre += P - 1
         first_piece.append(first)
         last_piece.append(first + P - 1)
-    cm, sm = build_tables(vbounds)
     plan = SplitPlan()
-    tables = Tables((torch.from_numpy(cm).to(device), torch.from_numpy(sm).to(device), (cm.shape[0], sm.shape[0])))
+    tables = device_tables(vbounds, device)
+    sm = build_tables(vbounds)[1]
     tables.covered = bool(bounds) and bounds[0][0] == 0 and bounds[-1][1] == rows
     plan.tables, plan.n_pieces, plan.n_pre, plan.n_chains = tables, len(vbounds), n_pre, len(bounds)
     plan.chains = torch.tensor(chains, dtype=torch.int32).to(device)

@@ -115,7 +115,7 @@ void* piece(const Tensor& buf, int64_t off) { return off < 0 ? nullptr : static_
 
 // ---- chunk tables and the split plan of a shape, built once by b200gdn/index.py ----------------------------------
 struct Plan : torch::CustomClassHolder {
-  Tensor chunk_meta, seq_meta;
+  Tensor chunk_meta, seq_meta, seq_order;
   int32_t n_chunks = 0, n_seq = 0;   // n_seq counts pieces under a split
   bool covered = true, split = false;
   Tensor chains, pre_fwd, pre_bwd, first_piece, last_piece;
@@ -213,6 +213,7 @@ b200gdn_chunk_args chunk_args(const Tensor& q, const Tensor& k, const Tensor& v,
   a.scale = (float)scale;
   a.chunk_meta = iptr(plan.chunk_meta);
   a.seq_meta = iptr(plan.seq_meta);
+  a.seq_order = iptr(plan.seq_order);
   a.q = ptr(q);
   a.k = ptr(k);
   a.v = ptr(v);
@@ -370,6 +371,7 @@ ChunkForward chunk_forward(const Tensor& q_in, const Tensor& k_in, const Tensor&
     p.qn = a.qn;
     p.kn = a.kn;
     p.seq_meta = iptr(plan->pre_fwd);
+    p.seq_order = nullptr;
     p.n_seq = plan->n_pre;
     p.gamma = a.gamma;
     p.w = a.w;
@@ -483,6 +485,7 @@ class ChunkFunction : public torch::autograd::Function<ChunkFunction> {
       float* dht_v = dM_pre + P * HV * K * K;
       b200gdn_chunk_args p = chunk_args(q, k, v, s.scale, plan);
       p.seq_meta = iptr(plan.pre_bwd);
+      p.seq_order = nullptr;
       p.n_seq = plan.n_pre;
       p.gamma = a.gamma;
       p.w = a.w;
@@ -882,21 +885,21 @@ PyObject* py_norm_gate(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   END_HANDLE_TH_ERRORS
 }
 
-// plan(chunk_meta, seq_meta, n_chunks, n_seq, covered[, chains, pre_fwd, pre_bwd, first_piece, last_piece, n_chains, n_pre])
+// plan(chunk_meta, seq_meta, n_chunks, n_seq, covered, seq_order or None[, chains, pre_fwd, pre_bwd, first_piece, last_piece, n_chains, n_pre])
 PyObject* py_plan(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
-  if (nargs != 5) NEED_ARGS(12);
+  if (nargs != 6) NEED_ARGS(13);
   auto p = c10::make_intrusive<Plan>();
-  bool ok = get(args[0], p->chunk_meta) && get(args[1], p->seq_meta);
+  bool ok = get(args[0], p->chunk_meta) && get(args[1], p->seq_meta) && get(args[5], p->seq_order);
   p->n_chunks = (int32_t)PyLong_AsLong(args[2]);
   p->n_seq = (int32_t)PyLong_AsLong(args[3]);
   p->covered = truth(args[4]);
-  if (nargs == 12) {
+  if (nargs == 13) {
     p->split = true;
-    ok = ok && get(args[5], p->chains) && get(args[6], p->pre_fwd) && get(args[7], p->pre_bwd) && get(args[8], p->first_piece) &&
-         get(args[9], p->last_piece);
-    p->n_chains = (int32_t)PyLong_AsLong(args[10]);
-    p->n_pre = (int32_t)PyLong_AsLong(args[11]);
+    ok = ok && get(args[6], p->chains) && get(args[7], p->pre_fwd) && get(args[8], p->pre_bwd) && get(args[9], p->first_piece) &&
+         get(args[10], p->last_piece);
+    p->n_chains = (int32_t)PyLong_AsLong(args[11]);
+    p->n_pre = (int32_t)PyLong_AsLong(args[12]);
   }
   if (!ok && !PyErr_Occurred()) PyErr_SetString(PyExc_TypeError, "plan: tensors expected");
   if (PyErr_Occurred()) return nullptr;

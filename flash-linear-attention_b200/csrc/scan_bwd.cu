@@ -77,7 +77,8 @@ __global__ void __launch_bounds__(NTHREADS)
   // sequence instead: zero do and dv_local, identity end gradient, V := K, nothing stored but the final "gradient" dM
   const bool m_mode = (int)blockIdx.x >= DV / BV;
   const bool dvl = DVL && !m_mode;
-  const int v0 = (m_mode ? (int)blockIdx.x - DV / BV : (int)blockIdx.x) * BV, hv = blockIdx.y, n = blockIdx.z;
+  const int v0 = (m_mode ? (int)blockIdx.x - DV / BV : (int)blockIdx.x) * BV, hv = blockIdx.y;
+  const int n = a.seq_order != nullptr ? a.seq_order[blockIdx.z] : (int)blockIdx.z;   // longest sequences first
   const int G = a.HV / a.H, hq = hv / G;
   const int c_first = a.seq_meta[2 * n], nc = a.seq_meta[2 * n + 1];
   const int c_last = c_first + nc - 1;

@@ -101,7 +101,8 @@ __global__ void __launch_bounds__(threads_of(OUT), PRE ? 2 : 1)
   // CTAs past the DV / 64 value slices (launched only when cp_M is given) scan the transition matrix of the sequence
   // instead: zero u, identity start state, V := K, nothing stored but the final "state" M
   const bool m_mode = !OUT && (int)blockIdx.x >= DV / BV;
-  const int v0 = (m_mode ? (int)blockIdx.x - DV / BV : (int)blockIdx.x) * BV, hv = blockIdx.y, n = blockIdx.z;
+  const int v0 = (m_mode ? (int)blockIdx.x - DV / BV : (int)blockIdx.x) * BV, hv = blockIdx.y;
+  const int n = a.seq_order != nullptr ? a.seq_order[blockIdx.z] : (int)blockIdx.z;   // longest sequences first
   const int G = a.HV / a.H, hq = hv / G;
   const int c_first = a.seq_meta[2 * n], nc = a.seq_meta[2 * n + 1];
   const bool has_u = !m_mode && a.u != nullptr;

@@ -143,6 +143,7 @@ typedef struct b200gdn_chunk_args {
   int32_t gb_dtype;              /* B200GDN_F32 / BF16 / F16: element type of g, beta, dg and dbeta */
   void* qn;
   void* kn;
+  const int32_t* seq_order;      /* device [n_seq]: the order in which the scans start the sequences, or NULL (as numbered) */
 } b200gdn_chunk_args;
 
 /* Replaces chunk_gated_delta_rule_fwd (fla/ops/gated_delta_rule/chunk.py:33-123):
