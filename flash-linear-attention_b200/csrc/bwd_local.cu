@@ -283,6 +283,8 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
       const int idx = tid + n * NTHREADS;   // 16-byte words of both panels; the same positions are read in h
       dhr[n] = *reinterpret_cast<const uint4*>((idx < DK * 8 ? H0 : H1 - DK * 128) + idx * 16);
     }
+    // the reads above are only issued: without this fence the copy of h can overtake those still queued
+    tc5::fence_async_smem();
     __syncthreads();
     if (tid == 0) {
       tc5::mbar_expect_tx(bar_b, (uint32_t)(NP * DK * 128 + S::tile));
