@@ -17,16 +17,6 @@ namespace {
 constexpr int NTHREADS = 128;
 constexpr int VS = 32;  // value channels per CTA
 
-__device__ __forceinline__ float ld_elem(const void* p, int64_t i, int dtype) {
-  if (dtype == 0) return __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p)[i]);
-  if (dtype == 1) return __half2float(reinterpret_cast<const __half*>(p)[i]);
-  return reinterpret_cast<const float*>(p)[i];
-}
-__device__ __forceinline__ void st_elem(void* p, int64_t i, int dtype, float x) {
-  if (dtype == 0) reinterpret_cast<__nv_bfloat16*>(p)[i] = __float2bfloat16(x);
-  else if (dtype == 1) reinterpret_cast<__half*>(p)[i] = __float2half(x);
-  else reinterpret_cast<float*>(p)[i] = x;
-}
 __device__ __forceinline__ float softplus_f(float x) { return x > 20.f ? x : log1pf(expf(x)); }
 
 // Slot of the state pool that sequence n uses.  With a pool (state_indices) and a known pool size, an index outside
@@ -399,113 +389,195 @@ __global__ void __launch_bounds__(NTHREADS) recurrent_kernel(const b200gdn_recur
   if (a.ht != nullptr && writeback) w.store(a.ht + (slot * a.HV + hv) * DK * DV, r0, c0, DV);
 }
 
-// Single-token decode at large batch as a stream: the kernels above load a state, compute and store it, so the
-// memory pipe of an SM idles while its CTAs compute.  Here one persistent CTA per SM walks its (sequence, head) items
-// through a three-stage ring in shared memory: a producer warp brings each 64 KiB state (one contiguous bulk copy), the
-// token's q, k, v rows and the activated gate scalars two items ahead and writes finished states back (one bulk copy);
-// eight consumer warps only compute, shared memory to shared memory.  Every wait is bounded.
+// Single-token decode at large batch as a stream: the step kernel loads a state, computes and stores it, so the memory pipe
+// of an SM idles while its CTAs compute.  Here one persistent CTA per SM walks its (sequence, head) items through a ring of
+// states in shared memory: a mover thread brings and takes away each 64 KiB state (one contiguous bulk copy each way), two
+// warps prepare the tokens (q and k as fp32 with their norms' factors, v, the activated gate scalars) for the same ring, and
+// eight consumer warps only compute, shared memory to shared memory.  Bound by HBM (one read and one write of every state).
+// 256 sequences x 16 heads, K = V = 128: 91 us, 5.9 TB/s (100 with the tokens fetched and the gates activated by the thread that
+// moves the states).  New states stored from registers instead, which leaves the ring to the reads: 92.  Every wait is bounded.
 __device__ int g_decode_timeout = 0;
 
-template <int DK>
+constexpr int kTokenWarps = 3;
+template <int DK, int DV>
 struct DecodeSmem {
-  static constexpr int NS = 3;
-  static constexpr size_t state_bytes = (size_t)DK * 128 * 4;
-  static constexpr size_t o_q = state_bytes, o_k = o_q + 512, o_v = o_k + 512, o_sc = o_v + 512;
+  static constexpr size_t state_bytes = (size_t)DK * DV * 4;
+  static constexpr int NS = (int)(192 * 1024 / state_bytes);   // 3 (128 x 128) to 12 (64 x 64) states in the ring
+  static constexpr size_t o_k = state_bytes, o_q = o_k + DK * 4, o_v = o_q + DK * 4, o_sc = o_v + DV * 4;
   static constexpr size_t stage = o_sc + 128;
   static constexpr size_t o_red = NS * stage;
-  static constexpr size_t o_bar = o_red + 8 * 128 * 4;
-  static constexpr size_t bytes = o_bar + 128;
+  static constexpr size_t red_bytes = 8 * 2 * DV * 4;   // one item's partial sums
+  static constexpr size_t o_bar = o_red + 2 * red_bytes;
+  static constexpr size_t bytes = o_bar + 2 * NS * 8;
+  static_assert(NS < 32 && bytes <= 227 * 1024, "the ring fits, and the mover's block of slots covers it");
+  // a token warp's next item is at most one turn of the ring on: its wait for the stage then never sees a phase two back
+  static_assert(kTokenWarps <= NS, "one phase of `freed` at a time");
 };
+constexpr int kStreamThreads = 32 * (8 + 1 + kTokenWarps);   // consumers, mover, token warps
 
-template <int DK>
-__global__ void __launch_bounds__(288, 1) decode_stream_kernel(const b200gdn_recurrent_args a, const int n_items) {
-  using S = DecodeSmem<DK>;
-  constexpr int NS = S::NS, DV = 128, RW = DK / 8;
+template <int DK, int DV, typename T>
+__global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const b200gdn_recurrent_args a, const int n_items) {
+  using S = DecodeSmem<DK, DV>;
+  constexpr int NS = S::NS;
+  constexpr int LPR = DV / 4, RPI = 32 / LPR, RW = DK / 8 / RPI;   // lanes to a row, rows to a warp instruction, rows per lane
   extern __shared__ __align__(128) unsigned char dsm[];
-  float (*red)[DV] = reinterpret_cast<float (*)[DV]>(dsm + S::o_red);
   uint64_t* full = reinterpret_cast<uint64_t*>(dsm + S::o_bar);
-  uint64_t* done = full + NS;
+  uint64_t* freed = full + NS;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int esz = a.qkv_dtype == 2 ? 4 : 2;
   const int n_local = (n_items - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
   const int G = a.HV / a.H;
 
   if (tid == 0) {
     for (int s = 0; s < NS; ++s) {
-      tc5::mbar_init(&full[s], 1);
-      tc5::mbar_init(&done[s], 256);
+      tc5::mbar_init(&full[s], 2);    // the state and the token
+      tc5::mbar_init(&freed[s], 8);   // the consumer warps
     }
     tc5::fence_mbar_init();
   }
   __syncthreads();
 
   if (warp == 8) {
-    // ---- producer: write-back of the item that used the stage last, then the load of the item NS further on
-    if (lane == 0) {
-      bool failed = false;
-      for (int jj = 0; jj < n_local + NS && !failed; ++jj) {
-        const int s = jj % NS;
-        unsigned char* stg = dsm + (size_t)s * S::stage;
-        if (jj >= NS) {
-          const int item = (int)blockIdx.x + (jj - NS) * (int)gridDim.x;
-          if (!tc5::mbar_wait(&done[s], ((jj - NS) / NS) & 1)) { failed = true; break; }
-          bool writeback;
-          const int64_t slot = state_slot(a, item / a.HV, &writeback);
-          if (writeback) {
-            float* ht = a.ht + (slot * a.HV + item % a.HV) * DK * DV;
-            asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n" ::"l"(ht), "r"(tc5::smem_addr(stg)),
-                         "r"((uint32_t)S::state_bytes)
-                         : "memory");
-            tma::store_commit();
-            tma::store_wait_read<0>();   // the stage may be refilled once the copy has read it
+    // ---- mover: write-back of the item that used the stage last, then the load of the next one.  The states' places are
+    // looked up 32 items at a time (a look-up per item would be a memory latency in this thread's chain).
+    int64_t cur = 0, prev = 0;
+    bool cur_wb = false, prev_wb = false;
+    for (int j = 0; j < n_local + NS; ++j) {
+      const int s = j % NS, i = j - NS;
+      if (j % 32 == 0) {
+        prev = cur;
+        prev_wb = cur_wb;
+        const int item = (int)blockIdx.x + (j + lane) * (int)gridDim.x;
+        if (j + lane < n_local) cur = (state_slot(a, item / a.HV, &cur_wb) * a.HV + item % a.HV) * DK * DV;
+      }
+      const bool same = i / 32 == j / 32;
+      const int64_t at_out = __shfl_sync(0xffffffffu, same ? cur : prev, i & 31), at_in = __shfl_sync(0xffffffffu, cur, j & 31);
+      const bool writeback = __shfl_sync(0xffffffffu, (int)(same ? cur_wb : prev_wb), i & 31);
+      if (i >= 0 && i < n_local) {
+        if (!tc5::mbar_wait_warp(&freed[s], (i / NS) & 1)) {
+          if (lane == 0) {
+            atomicExch(&g_decode_timeout, 1);
+            for (int l = i; l < min(j, n_local); ++l) tc5::mbar_wait(&full[l % NS], (l / NS) & 1);   // copies on their way land first
           }
+          break;
         }
-        if (jj < n_local) {
-          const int item = (int)blockIdx.x + jj * (int)gridDim.x;
-          const int n = item / a.HV, hv = item % a.HV, hq = hv / G;
-          const int64_t row = n;   // one token per sequence
-          float gg = a.g ? ld_param(a.g, row * a.HV + hv, a.gb_dtype) : 0.f;
-          if (a.flags & B200GDN_REC_GATE) {
-            if (a.dt_bias) gg += a.dt_bias[hv];
-            gg = -expf(a.A_log[hv]) * softplus_f(gg);
-          }
-          float bb = ld_param(a.beta, row * a.HV + hv, a.gb_dtype);
-          if (a.flags & B200GDN_REC_BETA_SIGMOID) {
-            bb = 1.f / (1.f + expf(-bb));
-            if (a.flags & B200GDN_REC_NEG_EIGVAL) bb *= 2.f;
-          }
-          float* sc = reinterpret_cast<float*>(stg + S::o_sc);
-          sc[0] = expf(gg);
-          sc[1] = bb;
-          const uint32_t qk_bytes = (uint32_t)(DK * esz), v_bytes = (uint32_t)(DV * esz);
-          tc5::mbar_expect_tx(&full[s], (uint32_t)S::state_bytes + 2 * qk_bytes + v_bytes);
-          bool writeback_unused;
-          const int64_t slot = state_slot(a, n, &writeback_unused);
-          tma::load_1d(stg, a.h0 + (slot * a.HV + hv) * DK * DV, (uint32_t)S::state_bytes, &full[s]);
-          tma::load_1d(stg + S::o_q, static_cast<const char*>(a.q) + (row * a.H + hq) * DK * esz, qk_bytes, &full[s]);
-          tma::load_1d(stg + S::o_k, static_cast<const char*>(a.k) + (row * a.H + hq) * DK * esz, qk_bytes, &full[s]);
-          tma::load_1d(stg + S::o_v, static_cast<const char*>(a.v) + (row * a.HV + hv) * DV * esz, v_bytes, &full[s]);
+        if (writeback && lane == 0) {
+          asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n" ::"l"(a.ht + at_out),
+                       "r"(tc5::smem_addr(dsm + (size_t)s * S::stage)), "r"((uint32_t)S::state_bytes)
+                       : "memory");
+          tma::store_commit();
         }
       }
-      tma::store_wait_all<0>();
-      if (failed) atomicExch(&g_decode_timeout, 1);
+      if (j < n_local && lane == 0) {
+        tma::store_wait_read<0>();   // the stage may be refilled once the copy has read it
+        tc5::mbar_expect_tx(&full[s], (uint32_t)S::state_bytes);
+        tma::load_1d(dsm + (size_t)s * S::stage, a.h0 + at_in, (uint32_t)S::state_bytes, &full[s]);
+      }
+    }
+    if (lane == 0) tma::store_wait_all<0>();
+    return;
+  }
+  if (warp > 8) {
+    // ---- token warps, in turn: k, scale q (with the L2-norm factors), v, decay, beta, <k, q>
+    for (int j = warp - 9; j < n_local; j += kTokenWarps) {
+      const int s = j % NS, item = (int)blockIdx.x + j * (int)gridDim.x;
+      const int n = item / a.HV, hv = item % a.HV, hq = hv / G;
+      float k[DK / 32], q[DK / 32], v[DV / 32], dec, beta;
+      const int64_t qk_at = ((int64_t)n * a.H + hq) * DK + lane, v_at = ((int64_t)n * a.HV + hv) * DV + lane;
+#pragma unroll
+      for (int i = 0; i < DK / 32; ++i) {
+        k[i] = Io<T>::ld(a.k, qk_at + 32 * i);
+        q[i] = Io<T>::ld(a.q, qk_at + 32 * i);
+      }
+#pragma unroll
+      for (int i = 0; i < DV / 32; ++i) v[i] = Io<T>::ld(a.v, v_at + 32 * i);
+      gate_beta(a, n, hv, dec, beta);
+      float kk = 0.f, qq = 0.f, kq = 0.f;
+#pragma unroll
+      for (int i = 0; i < DK / 32; ++i) {
+        kk += k[i] * k[i];
+        qq += q[i] * q[i];
+        kq += k[i] * q[i];
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        kk += __shfl_xor_sync(0xffffffffu, kk, o);
+        qq += __shfl_xor_sync(0xffffffffu, qq, o);
+        kq += __shfl_xor_sync(0xffffffffu, kq, o);
+      }
+      float kn = 1.f, qn = a.scale;
+      if (a.flags & B200GDN_REC_L2NORM) {
+        kn = rsqrtf(kk + 1e-6f);
+        qn *= rsqrtf(qq + 1e-6f);
+      }
+      if (j >= NS && !tc5::mbar_wait(&freed[s], ((j / NS) - 1) & 1)) {
+        atomicExch(&g_decode_timeout, 1);
+        return;
+      }
+      unsigned char* stg = dsm + (size_t)s * S::stage;
+      float *sk = reinterpret_cast<float*>(stg + S::o_k), *sq = reinterpret_cast<float*>(stg + S::o_q);
+      float *sv = reinterpret_cast<float*>(stg + S::o_v), *sc = reinterpret_cast<float*>(stg + S::o_sc);
+#pragma unroll
+      for (int i = 0; i < DK / 32; ++i) {
+        sk[lane + 32 * i] = k[i] * kn;
+        sq[lane + 32 * i] = q[i] * qn;
+      }
+#pragma unroll
+      for (int i = 0; i < DV / 32; ++i) sv[lane + 32 * i] = v[i];
+      if (lane == 0) *reinterpret_cast<float4*>(sc) = make_float4(dec, beta, kq * kn * qn, 0.f);
+      __syncwarp();
+      if (lane == 0) tc5::mbar_arrive(&full[s]);
     }
     return;
   }
 
-  // ---- consumers (8 warps): warp w keeps rows [w RW, (w+1) RW), lane l the columns 4 l .. 4 l + 3
-  const int col = 4 * lane, r0 = warp * RW;
-  auto sync_consumers = [] { asm volatile("bar.sync 1, 256;\n" ::: "memory"); };
+  // ---- consumers: warp w keeps rows [w DK/8, (w+1) DK/8), a lane four columns of every row (128 columns) or of every other
+  // one.  As in the step kernel both row reductions are taken from the state before its update, so that one barrier per item
+  // serves both.
+  const int col = 4 * (lane % LPR), r0 = warp * (DK / 8) + (lane / LPR) * RW;
   for (int j = 0; j < n_local; ++j) {
-    const int s = j % NS;
+    const int s = j % NS, item = (int)blockIdx.x + j * (int)gridDim.x;
     unsigned char* stg = dsm + (size_t)s * S::stage;
-    float* St = reinterpret_cast<float*>(stg);
-    const int item = (int)blockIdx.x + j * (int)gridDim.x;
-    const int hv = item % a.HV;
+    float* St = reinterpret_cast<float*>(stg) + r0 * DV + col;
+    float (*red)[2][DV] = reinterpret_cast<float (*)[2][DV]>(dsm + S::o_red + (j & 1) * S::red_bytes);
+    const uint32_t bad = tc5::mbar_wait(&full[s], (j / NS) & 1) ? 0u : 1u;
+    uint64_t st[RW][2], k2[RW], d[2] = {0ull, 0ull}, e[2] = {0ull, 0ull};
+#pragma unroll
+    for (int i = 0; i < RW; i += 4) {
+      const float4 kf = *reinterpret_cast<const float4*>(stg + S::o_k + (r0 + i) * 4);
+      const float4 qf = *reinterpret_cast<const float4*>(stg + S::o_q + (r0 + i) * 4);
+      const float kv[4] = {kf.x, kf.y, kf.z, kf.w}, qv[4] = {qf.x, qf.y, qf.z, qf.w};
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const float4 x = *reinterpret_cast<const float4*>(St + (i + u) * DV);
+        st[i + u][0] = pack2(x.x, x.y);
+        st[i + u][1] = pack2(x.z, x.w);
+        k2[i + u] = pack2(kv[u], kv[u]);
+        const uint64_t q2 = pack2(qv[u], qv[u]);
+        d[0] = fma2(st[i + u][0], k2[i + u], d[0]);
+        d[1] = fma2(st[i + u][1], k2[i + u], d[1]);
+        e[0] = fma2(st[i + u][0], q2, e[0]);
+        e[1] = fma2(st[i + u][1], q2, e[1]);
+      }
+    }
+    const float4 v = *reinterpret_cast<const float4*>(stg + S::o_v + col * 4);
+    const float4 sc = *reinterpret_cast<const float4*>(stg + S::o_sc);   // decay, beta, <k, q>
     {
-      // the consumers agree on the outcome of the bounded wait (a barrier-wide OR), so that they leave together;
-      // the producer then gives up on its own bounded wait
-      const uint32_t bad = tc5::mbar_wait(&full[s], (j / NS) & 1) ? 0u : 1u;
+      const float2 d0 = unpack2(d[0]), d1 = unpack2(d[1]), e0 = unpack2(e[0]), e1 = unpack2(e[1]);
+      float4 dv = make_float4(d0.x, d0.y, d1.x, d1.y), ev = make_float4(e0.x, e0.y, e1.x, e1.y);
+      if constexpr (RPI == 2) {   // the warp's two rows
+        dv.x += __shfl_xor_sync(0xffffffffu, dv.x, 16); dv.y += __shfl_xor_sync(0xffffffffu, dv.y, 16);
+        dv.z += __shfl_xor_sync(0xffffffffu, dv.z, 16); dv.w += __shfl_xor_sync(0xffffffffu, dv.w, 16);
+        ev.x += __shfl_xor_sync(0xffffffffu, ev.x, 16); ev.y += __shfl_xor_sync(0xffffffffu, ev.y, 16);
+        ev.z += __shfl_xor_sync(0xffffffffu, ev.z, 16); ev.w += __shfl_xor_sync(0xffffffffu, ev.w, 16);
+      }
+      if (lane < LPR) {
+        *reinterpret_cast<float4*>(&red[warp][0][col]) = dv;
+        *reinterpret_cast<float4*>(&red[warp][1][col]) = ev;
+      }
+    }
+    {
+      // the partial sums are complete; the same barrier carries the outcome of the bounded wait, so that all leave together
+      // (the loader and the token warps then give up on their own bounded waits)
       uint32_t any_bad;
       asm volatile(
           "{\n.reg .pred p, q;\nsetp.ne.b32 q, %1, 0;\nbar.red.or.pred p, 1, 256, q;\nselp.u32 %0, 1, 0, p;\n}\n"
@@ -517,91 +589,70 @@ __global__ void __launch_bounds__(288, 1) decode_stream_kernel(const b200gdn_rec
         return;
       }
     }
-    const float* sc = reinterpret_cast<const float*>(stg + S::o_sc);
-    const float decay = sc[0], beta = sc[1];
-    float qn = a.scale, kn = 1.f;
-    if (a.flags & B200GDN_REC_L2NORM) {
-      float sq = 0.f, sk = 0.f;
-      for (int i = lane; i < DK; i += 32) {
-        const float x = ld_elem(stg + S::o_q, i, a.qkv_dtype), y = ld_elem(stg + S::o_k, i, a.qkv_dtype);
-        sq += x * x;
-        sk += y * y;
-      }
+    float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        sq += __shfl_xor_sync(0xffffffffu, sq, o);
-        sk += __shfl_xor_sync(0xffffffffu, sk, o);
-      }
-      qn = a.scale * rsqrtf(sq + 1e-6f);
-      kn = rsqrtf(sk + 1e-6f);
+    for (int w = 0; w < 8; ++w) {
+      const float4 x = *reinterpret_cast<const float4*>(&red[w][0][col]);
+      r.x += x.x; r.y += x.y; r.z += x.z; r.w += x.w;
     }
-    float4 st[RW];
-    float kr[RW];
-    float4 d = make_float4(0.f, 0.f, 0.f, 0.f);
+    r.x = sc.y * (v.x - sc.x * r.x); r.y = sc.y * (v.y - sc.x * r.y);
+    r.z = sc.y * (v.z - sc.x * r.z); r.w = sc.y * (v.w - sc.x * r.w);
+    const uint64_t dec2 = pack2(sc.x, sc.x), rl = pack2(r.x, r.y), rh = pack2(r.z, r.w);
 #pragma unroll
     for (int i = 0; i < RW; ++i) {
-      st[i] = *reinterpret_cast<const float4*>(St + (r0 + i) * DV + col);
-      kr[i] = ld_elem(stg + S::o_k, r0 + i, a.qkv_dtype) * kn;
-      st[i].x *= decay; st[i].y *= decay; st[i].z *= decay; st[i].w *= decay;
-      d.x += st[i].x * kr[i]; d.y += st[i].y * kr[i]; d.z += st[i].z * kr[i]; d.w += st[i].w * kr[i];
+      const float2 lo = unpack2(fma2(k2[i], rl, mul2(st[i][0], dec2))), hi = unpack2(fma2(k2[i], rh, mul2(st[i][1], dec2)));
+      *reinterpret_cast<float4*>(St + i * DV) = make_float4(lo.x, lo.y, hi.x, hi.y);
     }
-    *reinterpret_cast<float4*>(&red[warp][col]) = d;
-    sync_consumers();
-    float4 r;
-    {
-      float4 sum = *reinterpret_cast<const float4*>(&red[0][col]);
+    tc5::fence_async_smem();   // the new state is read by the mover's bulk copy
+    __syncwarp();
+    if (lane == 0) tc5::mbar_arrive(&freed[s]);
+    if (warp == (j & 7) && lane < LPR) {   // the output row, by the warps in turn
+      float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-      for (int w = 1; w < 8; ++w) {
-        const float4 x = *reinterpret_cast<const float4*>(&red[w][col]);
-        sum.x += x.x; sum.y += x.y; sum.z += x.z; sum.w += x.w;
+      for (int w = 0; w < 8; ++w) {
+        const float4 x = *reinterpret_cast<const float4*>(&red[w][1][col]);
+        o.x += x.x; o.y += x.y; o.z += x.z; o.w += x.w;
       }
-      const float v0 = ld_elem(stg + S::o_v, col, a.qkv_dtype), v1 = ld_elem(stg + S::o_v, col + 1, a.qkv_dtype);
-      const float v2 = ld_elem(stg + S::o_v, col + 2, a.qkv_dtype), v3 = ld_elem(stg + S::o_v, col + 3, a.qkv_dtype);
-      r.x = beta * (v0 - sum.x); r.y = beta * (v1 - sum.y); r.z = beta * (v2 - sum.z); r.w = beta * (v3 - sum.w);
+      const int64_t at = (int64_t)item * DV + col;   // [sequence][head][V]
+      Io<T>::st(a.o, at, sc.x * o.x + sc.z * r.x);
+      Io<T>::st(a.o, at + 1, sc.x * o.y + sc.z * r.y);
+      Io<T>::st(a.o, at + 2, sc.x * o.z + sc.z * r.z);
+      Io<T>::st(a.o, at + 3, sc.x * o.w + sc.z * r.w);
     }
-    sync_consumers();   // the partial sums have been read by everybody before they are overwritten
-    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-    for (int i = 0; i < RW; ++i) {
-      const float qq = ld_elem(stg + S::o_q, r0 + i, a.qkv_dtype) * qn;
-      st[i].x += kr[i] * r.x; st[i].y += kr[i] * r.y; st[i].z += kr[i] * r.z; st[i].w += kr[i] * r.w;
-      o.x += st[i].x * qq; o.y += st[i].y * qq; o.z += st[i].z * qq; o.w += st[i].w * qq;
-      *reinterpret_cast<float4*>(St + (r0 + i) * DV + col) = st[i];
-    }
-    *reinterpret_cast<float4*>(&red[warp][col]) = o;
-    tc5::fence_async_smem();       // the new state is read by the producer's bulk copy
-    sync_consumers();
-    if (tid < DV) {
-      float sum = 0.f;
-#pragma unroll
-      for (int w = 0; w < 8; ++w) sum += red[w][tid];
-      st_elem(a.o, ((int64_t)(item / a.HV) * a.HV + hv) * DV + tid, a.qkv_dtype, sum);
-    }
-    tc5::mbar_arrive(&done[s]);
-    sync_consumers();   // red is free again for the next item
   }
 }
 
-// (sequence, head) pairs from which a single-token step streams its states: measured at K = V = 128, 512 pairs 12.4 us
-// for the step kernel against 14.0, 1024 pairs 30.4 against 28.1, 4096 pairs 104 against 97.
-constexpr int kStreamPairs = 768;
+// Elements of all states together (16 MiB) from which a single-token step streams them.  Measured, step kernel against stream:
+// K = V = 128, 256 pairs 10.8 / 10.0 us, 512 pairs 18.0 / 15.8, 4096 pairs 106 / 91; K = V = 64, 512 pairs 7.2 / 8.2, 1024 pairs
+// 12.0 / 11.7, 4096 pairs 37 / 32.
+constexpr int64_t kStreamElements = 256 * 128 * 128;
 
 template <int DK>
 int launch(const b200gdn_recurrent_args& a, cudaStream_t st) {
   if constexpr (DK == 64 || DK == 128) {
-    // one token per sequence at large batch: the streaming kernel (state and token rows by bulk copies, ring of three;
-    // it needs 16-byte boundaries, [K,V] states and V = 128)
-    if (!(a.flags & B200GDN_REC_STATE_V_FIRST) && a.V == 128 && a.T == 1 && a.cu_seqlens == nullptr && a.h0 != nullptr &&
-        a.ht != nullptr && (int64_t)a.n_seq * a.HV >= kStreamPairs && (reinterpret_cast<uintptr_t>(a.q) & 15) == 0 &&
-        (reinterpret_cast<uintptr_t>(a.k) & 15) == 0 && (reinterpret_cast<uintptr_t>(a.v) & 15) == 0 &&
+    // one token per sequence at large batch: the streaming kernel (16-byte boundaries, [K,V] states, V = 64 or 128)
+    if (!(a.flags & B200GDN_REC_STATE_V_FIRST) && (a.V == 64 || a.V == 128) && a.T == 1 && a.cu_seqlens == nullptr &&
+        a.h0 != nullptr && a.ht != nullptr && (int64_t)a.n_seq * a.HV * DK * a.V >= kStreamElements &&
         (reinterpret_cast<uintptr_t>(a.h0) & 15) == 0 && (reinterpret_cast<uintptr_t>(a.ht) & 15) == 0) {
-      using S = DecodeSmem<DK>;
-      if (int e = ensure_smem(decode_stream_kernel<DK>, S::bytes)) return e;
       int dev = 0, sms = 148;
       cudaGetDevice(&dev);
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
       const int n_items = a.n_seq * a.HV;
-      decode_stream_kernel<DK><<<n_items < sms ? n_items : sms, 288, S::bytes, st>>>(a, n_items);
+      auto stream = [&](auto* kernel, size_t bytes) -> int {
+        if (int e = ensure_smem(kernel, bytes)) return e;
+        kernel<<<n_items < sms ? n_items : sms, kStreamThreads, bytes, st>>>(a, n_items);
+        return 0;
+      };
+      int e;
+#define STREAM(TY) e = a.V == 64 ? stream(decode_stream_kernel<DK, 64, TY>, DecodeSmem<DK, 64>::bytes) \
+                                 : stream(decode_stream_kernel<DK, 128, TY>, DecodeSmem<DK, 128>::bytes)
+      switch (a.qkv_dtype) {
+        case 0: STREAM(__nv_bfloat16); break;
+        case 1: STREAM(__half); break;
+        default: STREAM(float); break;
+      }
+#undef STREAM
+      if (e) return e;
       return check_launch("decode_stream");
     }
   }

@@ -237,3 +237,33 @@ def test_token_blocks_and_unaligned_rows(K, V, T, misaligned):
         use_beta_sigmoid_in_kernel=True, allow_neg_eigval=True)
     O.assert_close('o', ref_o, o.float().cpu(), 0.004)
     O.assert_close('ht', ref_ht, ht.cpu(), 1e-5)
+
+
+@pytest.mark.parametrize('K,V,N,HV', [(128, 128, 32, 8), (128, 128, 31, 8), (64, 64, 65, 16), (64, 64, 305, 16), (128, 64, 43, 12), (64, 128, 150, 4)])
+def test_single_token_steps_around_the_streaming_size(K, V, N, HV):
+    """One token per sequence on a pool of states, either side of the size from which the states are streamed, with a
+    sequence that is padding (index -1); the largest case gives every CTA more than 32 states."""
+    from b200gdn import fused_recurrent_gated_delta_rule
+    H, slots = HV // 2, N + 3
+    gen = torch.Generator(device='cuda').manual_seed(N)
+    mk = lambda *s: torch.randn(*s, device='cuda', generator=gen)   # noqa: E731
+    q, k, v = (mk(N, 1, h, d).to(torch.bfloat16) for h, d in ((H, K), (H, K), (HV, V)))
+    g, beta, pool = mk(N, 1, HV), mk(N, 1, HV), mk(slots, HV, K, V) * 0.1
+    a_log, dt_bias = mk(HV) * 0.3, mk(HV) * 0.3
+    at = torch.randperm(slots, device='cuda', generator=gen)[:N].to(torch.int32)
+    at[N // 2] = -1
+    before = pool.clone()
+    o, _ = fused_recurrent_gated_delta_rule(q, k, v, g, beta=beta, initial_state=pool, output_final_state=True, state_indices=at,
+                                            inplace_state=True, use_qk_l2norm_in_kernel=True, use_gate_in_kernel=True,
+                                            A_log=a_log, dt_bias=dt_bias, use_beta_sigmoid_in_kernel=True)
+    used = at >= 0
+    qf, kf = (torch.nn.functional.normalize(x[:, 0].double(), dim=-1).repeat_interleave(2, 1)[used] for x in (q, k))
+    dec = (-a_log.double().exp() * torch.nn.functional.softplus(g[used, 0].double() + dt_bias)).exp()
+    S = before[at[used].long()].double() * dec[..., None, None]
+    r = (v[used, 0].double() - torch.einsum('nhkv,nhk->nhv', S, kf)) * torch.sigmoid(beta[used, 0].double())[..., None]
+    S = S + torch.einsum('nhk,nhv->nhkv', kf, r)
+    O.assert_close('o', torch.einsum('nhkv,nhk->nhv', S, qf) * K ** -0.5, o[used, 0].double(), 0.004)
+    O.assert_close('states', S, pool[at[used].long()].double(), 1e-5)
+    rest = torch.ones(slots, dtype=torch.bool, device='cuda')
+    rest[at[used].long()] = False
+    assert torch.equal(pool[rest], before[rest]), 'a slot that no sequence uses was written'
