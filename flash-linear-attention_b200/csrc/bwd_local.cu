@@ -21,12 +21,14 @@
 // K- or V-wide result are formed TRANSPOSED ([K x 64 tokens], M = 128): the same tcgen05 instruction then does twice the
 // work of an M = 64 one, an accumulator takes 64 TMEM columns instead of 128, and every lane of a TMEM load carries data.
 // Tiles leave token-major straight from registers (movmatrix, then 16-byte words).
-// One CTA of eight warps; 256 TMEM columns (C0: dP, dq^T; C1: dU V^T, K K^T; C2: dW^T, dW K^T, Y, X, dv^T; C3: dk^T) and
-// ~111 KiB of shared memory whose regions change hands, so two CTAs per SM overlap each other's phases:
+// One CTA of eight warps; 256 TMEM columns (C0: dP, dq^T, dU V^T, K K^T; C1: the sum of dq over a group; C2: dW^T, dW K^T, Y, X,
+// dv^T; C3: dk^T) and ~111 KiB of shared memory whose regions change hands, so two CTAs per SM overlap each other's phases:
 //   R1: K      R2: do -> q      R3: v_new -> dU      R4: dh panel 0 -> h panel 0 -> dW^T
 //   R5: dh panel 1 -> h panel 1 -> V -> dA | Y -> M2 | Y
-// Grouped value heads: the CTAs of a group form a cluster; each leaves its fp32 dq and dk in shared memory and adds up a
-// share of the rows over distributed shared memory in head order (no atomics, no fp32 tensors in HBM).
+// Grouped value heads, many chunks: a CTA takes the heads of a group in turn, K stays, the tiles of the next head are fetched
+// under the last epilogue; the sum of dq waits in C1, that of dk in local memory (TMEM is full; 32 KiB per CTA that stay in L2).
+// Few chunks: a CTA per head, the CTAs of a group form a cluster; each leaves its fp32 dq and dk in shared memory and adds up
+// a share of the rows over distributed shared memory.  Both add in head order (no atomics, no fp32 tensors in HBM).
 #include "tc5_tile.cuh"
 #include "tma.cuh"
 
@@ -45,7 +47,7 @@ struct LocalSmem {
   static constexpr size_t o_vec = o_ab + BT * 128;
   static constexpr int LDS = DK + 4;                                // fp32 row stride of the group-sum staging
   static constexpr size_t stage = (size_t)BT * LDS * 4;             // dq, then dk, from R2 on
-  static constexpr size_t bytes = o_vec + 28 * BT * 4 + 160 + 1024; // + vectors, barriers, alignment slack
+  static constexpr size_t bytes = o_vec + 29 * BT * 4 + 160 + 1024; // + vectors, barriers, alignment slack
   static_assert(o_do + 2 * stage <= o_vec, "the group-sum staging fits over the dead tiles");
 };
 
@@ -80,6 +82,13 @@ template <int NH>
 __device__ __forceinline__ void acc_ld_t(uint32_t tm, int q, int cs, float (&r)[NH][16]) {
 #pragma unroll
   for (int hf = 0; hf < NH; ++hf) tc5::tmem_ld_16x256b_x4(tm + ((uint32_t)(32 * q + 16 * hf) << 16) + cs, r[hf]);
+}
+template <int NH>
+__device__ __forceinline__ void add_t(float (&r)[NH][16], const float (&before)[NH][16]) {
+#pragma unroll
+  for (int hf = 0; hf < NH; ++hf)
+#pragma unroll
+    for (int e = 0; e < 16; ++e) r[hf][e] = before[hf][e] + r[hf][e];
 }
 // ... its dot products with the same block of a [token][column] tile, added over the rows: value 2 i + p of the result
 // belongs to token 8 i + 2 t + p and still has to be summed over g
@@ -156,8 +165,12 @@ __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
 }
 
-template <int DK, bool GROUPED>
+// How the value heads of a q/k head meet: there is one; each has a CTA and the CTAs form a cluster; one CTA takes them in turn
+enum Heads { kOne, kCluster, kTurns };
+
+template <int DK, Heads MODE>
 __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_chunk_args a, const __grid_constant__ LocalMaps maps) {
+  constexpr bool GROUPED = MODE == kCluster;
   using S = LocalSmem<DK>;
   constexpr int NP = DK / 64;   // 64-column panels of a V-wide tile (V = K)
   constexpr int NH = DK / 64;   // 16-row halves of a transposed accumulator per warp
@@ -166,8 +179,8 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
   unsigned char *Ks = smem + S::o_k, *Do = smem + S::o_do, *Qs = Do, *Vn = smem + S::o_vn, *dUs = Vn, *H0 = smem + S::o_h0, *dWt = H0;
   unsigned char *H1 = smem + S::o_h1, *Vs = H1, *dAs = H1, *M2s = H1, *Ys = H1 + BT * 128;
   unsigned char *As = smem + S::o_a, *Ps = smem + S::o_ps, *Abs = smem + S::o_ab;
-  float* gs = reinterpret_cast<float*>(smem + S::o_vec);
-  float *bet = gs + BT, *bge = bet + BT, *eg = bge + BT, *sgm = eg + BT, *gx = sgm + BT, *gv = gx + BT, *dGs = gv + BT, *rsq = dGs + BT, *rsk = rsq + BT;
+  float* const gs2 = reinterpret_cast<float*>(smem + S::o_vec);   // [2][64]: a head's and the next one's
+  float *bet = gs2 + 2 * BT, *bge = bet + BT, *eg = bge + BT, *sgm = eg + BT, *gx = sgm + BT, *gv = gx + BT, *dGs = gv + BT, *rsq = dGs + BT, *rsk = rsq + BT;
   // sums over rows: each of the four row-quadrant warps leaves its partial in its own slot and the consumer adds the four in
   // a fixed order (no atomics: results are bit-reproducible)
   float* c_rq = rsk + BT;        // [4][64] <dq_i, q_i>
@@ -182,50 +195,57 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
 
   const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int q = warp & 3, hc = warp >> 2, g = lane >> 2, t = lane & 3;
-  const int c = blockIdx.x, hv = blockIdx.y, G = a.HV / a.H, hq = hv / G;
+  const int c = blockIdx.x, G = a.HV / a.H, hq = MODE == kTurns ? blockIdx.y : blockIdx.y / G;
+  const int hv0 = MODE == kTurns ? hq * G : blockIdx.y, n_heads = MODE == kTurns ? G : 1;
   const ChunkMeta cm = load_chunk_meta(a.chunk_meta, c);
   const int64_t row0 = cm.row;
   const int r_lo = q * 16 + g, r_hi = r_lo + 8, cs = hc * 32;   // this warp's block of a [64][64] tile
   const int kr = (DK / 4) * q;                                  // ... and its first row of a transposed accumulator
   const int gcol = cs + 8 * (g >> 1) + 2 * t + (g & 1);         // the column whose sum sum8_over_g leaves in this lane
-  const int hrow = (c * a.HV + hv) * DK;                        // this head's state snapshot in the [.., V] view
 
-  if (tid == 0) {
-    for (int i = 0; i < 5; ++i) tc5::mbar_init(bar + i, 1);
-    tc5::fence_mbar_init();
+  // one thread: what a head's first phases need, and the rest into L2
+  auto load_head = [&](int hv, bool first) {
+    const int hrow = (c * a.HV + hv) * DK;   // the head's state snapshot in the [.., V] view
     tc5::mbar_expect_tx(bar_a, (uint32_t)(2 * S::tile + NP * DK * 128 + BT * 4));
     tma::load_3d(Do, &maps.d_o, cm.row, (hv * DK) / 64, bar_a);
     tma::load_3d(Vn, &maps.vn, cm.row, (hv * DK) / 64, bar_a);
-    tma::load_1d(gs, gamma_ptr(a.gamma, c, a.HV, hv), BT * 4, bar_a);
+    tma::load_1d(gs2 + ((hv - hv0) & 1) * BT, gamma_ptr(a.gamma, c, a.HV, hv), BT * 4, bar_a);
     for (int p = 0; p < NP; ++p) tma::load_2d(p ? H1 : H0, &maps.dh, p * 64, hrow, bar_a);
-    tc5::mbar_expect_tx(bar_k, (uint32_t)(S::tile + BT * 128));
-    tma::load_3d(Ks, &maps.k, cm.row, (hq * DK) / 64, bar_k);
+    tc5::mbar_expect_tx(bar_k, (uint32_t)((first ? S::tile : 0) + BT * 128));
+    if (first) tma::load_3d(Ks, &maps.k, cm.row, (hq * DK) / 64, bar_k);
     tma::load_2d(As, &maps.a, hv * BT, cm.row, bar_k);
-    // what the later phases load: in L2 by then
     for (int p = 0; p < NP; ++p) tma::prefetch_2d(&maps.h, p * 64, hrow);
     tma::prefetch_3d(&maps.du, cm.row, (hv * DK) / 64);
-    tma::prefetch_3d(&maps.q, cm.row, (hq * DK) / 64);
+    if (first) tma::prefetch_3d(&maps.q, cm.row, (hq * DK) / 64);
     tma::prefetch_3d(&maps.v, cm.row, (hv * DK) / 64);
+  };
+  if (tid == 0) {
+    for (int i = 0; i < 5; ++i) tc5::mbar_init(bar + i, 1);
+    tc5::fence_mbar_init();
+    load_head(hv0, true);
   }
   if (warp == 1) tc5::tmem_alloc(tmem_slot, 256);
-  if (tid < BT) {
-    const bool ok = tid < cm.len;
-    float b = ok ? ld_param(a.beta, (row0 + tid) * a.HV + hv, a.gb_dtype) : 0.f;
-    if (a.options & B200GDN_PREP_BETA_SIGMOID) {   // raw beta: the kernels work with (1|2) sigmoid(beta)
-      const float sg = 1.f / (1.f + expf(-b));
-      sgm[tid] = sg;
-      b = ok ? ((a.options & B200GDN_PREP_NEG_EIGVAL) ? 2.f : 1.f) * sg : 0.f;
+  auto head_vectors = [&](int hv) {   // beta and, with the gate option, the gate's value and derivative
+    if (tid < BT) {
+      const bool ok = tid < cm.len;
+      float b = ok ? ld_param(a.beta, (row0 + tid) * a.HV + hv, a.gb_dtype) : 0.f;
+      if (a.options & B200GDN_PREP_BETA_SIGMOID) {   // raw beta: the kernels work with (1|2) sigmoid(beta)
+        const float sg = 1.f / (1.f + expf(-b));
+        sgm[tid] = sg;
+        b = ok ? ((a.options & B200GDN_PREP_NEG_EIGVAL) ? 2.f : 1.f) * sg : 0.f;
+      }
+      bet[tid] = b;
     }
-    bet[tid] = b;
-  }
-  if ((a.options & B200GDN_PREP_GATE) && tid >= 2 * BT && tid < 3 * BT) {
-    // fused gate: g = -exp(A_log) softplus(x), x = g_raw + dt_bias; its value and derivative, while the tiles are on their way
-    const int r = tid - 2 * BT;
-    const float x = (r < cm.len ? ld_param(a.g, (row0 + r) * a.HV + hv, a.gb_dtype) : 0.f) + (a.dt_bias ? a.dt_bias[hv] : 0.f);
-    const float negA = -expf(a.A_log[hv]);
-    gx[r] = negA / (1.f + expf(-x));
-    gv[r] = negA * (x > 20.f ? x : log1pf(expf(x)));
-  }
+    if ((a.options & B200GDN_PREP_GATE) && tid >= 2 * BT && tid < 3 * BT) {
+      // fused gate: g = -exp(A_log) softplus(x), x = g_raw + dt_bias; its value and derivative, while the tiles are on their way
+      const int r = tid - 2 * BT;
+      const float x = (r < cm.len ? ld_param(a.g, (row0 + r) * a.HV + hv, a.gb_dtype) : 0.f) + (a.dt_bias ? a.dt_bias[hv] : 0.f);
+      const float negA = -expf(a.A_log[hv]);
+      gx[r] = negA / (1.f + expf(-x));
+      gv[r] = negA * (x > 20.f ? x : log1pf(expf(x)));
+    }
+  };
+  head_vectors(hv0);
   if (!GROUPED && tid >= BT && tid < 2 * BT) {   // L2-norm option: reciprocal norms of the rows
     const int r = tid - BT;
     if (a.rstd_q != nullptr) rsq[r] = r < cm.len ? a.rstd_q[(row0 + r) * a.H + hq] : 0.f;
@@ -242,9 +262,16 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
   const Operand opK_k{sK, BT, 0}, opK_mn{sK, BT, 1};      // K as (rows = token, contraction = key dim), and the reverse
   const Operand opA_k{sA, BT, 0}, opA_mn{sA, BT, 1};
   bool failed = false;
+  // turns: this thread's part of the sum of dk over the heads, in local memory between them
+  __align__(16) float dk_local[MODE == kTurns ? 16 * NH : 4];
+  const uint64_t dk_sum = __cvta_generic_to_local(dk_local);
 
-  do {
-    if (!tc5::mbar_wait(bar_a, 0)) failed = true;
+  for (int hh = 0; hh < n_heads; ++hh) {
+    const int hv = hv0 + hh, hrow = (c * a.HV + hv) * DK;
+    const uint32_t par = hh & 1;
+    const bool first = MODE != kTurns || hh == 0, last = MODE != kTurns || hh + 1 == n_heads;
+    const float* gs = gs2 + par * BT;
+    if (!tc5::mbar_wait(bar_a, par)) failed = true;
     if (cm.len < BT) {   // ragged chunk: the extra rows of the boxes belong to the next sequence
       zero_tail_rows<BT, DK>(Do, cm.len, tid, NTHREADS);
       zero_tail_rows<BT, DK>(Vn, cm.len, tid, NTHREADS);
@@ -267,9 +294,9 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
       eg[tid] = e;
       bge[tid] = bet[tid] * e;
     }
-    if (!tc5::mbar_wait(bar_k, 0)) failed = true;
+    if (!tc5::mbar_wait(bar_k, par)) failed = true;
     if (cm.len < BT) {
-      zero_tail_rows<BT, DK>(Ks, cm.len, tid, NTHREADS);
+      if (first) zero_tail_rows<BT, DK>(Ks, cm.len, tid, NTHREADS);
       zero_tail_rows<BT, BT>(As, cm.len, tid, NTHREADS);
       tc5::fence_async_smem();
     }
@@ -345,7 +372,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
       if (lane == 0) red[8 + warp] = rs;
       tc5::tmem_st_wait();
     }
-    if (!tc5::mbar_wait(bar_b, 0)) failed = true;
+    if (!tc5::mbar_wait(bar_b, par)) failed = true;
     if (cm.len < BT) zero_tail_rows<BT, DK>(dUs, cm.len, tid, NTHREADS);
     {
       float hd = 0.f;
@@ -410,11 +437,14 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
         fs.store(dWt, DK, kr + 16 * hf, cs, lane);
       }
     }
-    if (!tc5::mbar_wait(bar_c, 0)) failed = true;
+    float rq[NH][16];   // dq: C0 is phase 3's
+    acc_ld_t<NH>(C0, q, cs, rq);
+    if (!tc5::mbar_wait(bar_c, par)) failed = true;
     if (cm.len < BT) {
       zero_tail_rows<BT, DK>(Qs, cm.len, tid, NTHREADS);
       zero_tail_rows<BT, DK>(Vs, cm.len, tid, NTHREADS);
     }
+    tc5::tmem_ld_wait();
     tc5::fence_async_smem();
     tc5::fence_before_sync();
     if (__syncthreads_or(failed)) { failed = true; break; }
@@ -423,21 +453,35 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
     if (warp == 0) {
       tc5::fence_after_sync();
       issue_mma_t<DK / 16>(C2, Operand{sH0, DK, 1}, opK_k, 64, 64, 0);
-      issue_mma_t<DK / 16>(C1, Operand{sVn, BT, 0}, Operand{sH1, BT, 0}, 64, 64, 0);
+      issue_mma_t<DK / 16>(C0, Operand{sVn, BT, 0}, Operand{sH1, BT, 0}, 64, 64, 0);
       ph.commit();
     }
-    {   // dq: its dots with q; ungrouped heads: it leaves
-      float r[NH][16], pv[8];
-      acc_ld_t<NH>(C0, q, cs, r);
-      tc5::tmem_ld_wait();
-      dots_t<NH>(r, Qs, kr, cs, lane, pv);
+    {   // dq: its dots with q, the sum over the heads (C1); ungrouped heads, and the last one in turn: it leaves
+      float pv[8];
+      dots_t<NH>(rq, Qs, kr, cs, lane, pv);
       c_rq[q * BT + gcol] = sum8_over_g(pv, g);
-      if (!GROUPED) {
+      if (!first) {
+        float acc[NH][16];
+        acc_ld_t<NH>(C1, q, cs, acc);
+        tc5::tmem_ld_wait();
+        add_t<NH>(rq, acc);
+      }
+      if (GROUPED || !last) {
+#pragma unroll
+        for (int hf = 0; hf < NH; ++hf) tc5::tmem_st_16x256b_x4(C1 + ((uint32_t)(32 * q + 16 * hf) << 16) + cs, rq[hf]);
+        tc5::tmem_st_wait();
+      } else {
         if (a.rstd_q != nullptr) {
+          float* dots = c_rq;
+          if (MODE == kTurns) {   // of the sum; c_kbg is free until epilogue 3
+            dots = c_kbg;
+            dots_t<NH>(rq, Qs, kr, cs, lane, pv);
+            dots[q * BT + gcol] = sum8_over_g(pv, g);
+          }
           __syncthreads();
-          l2_backward_t<NH>(r, Qs, c_rq, rsq, kr, cs, lane);
+          l2_backward_t<NH>(rq, Qs, dots, rsq, kr, cs, lane);
         }
-        store_t<NH>(r, reinterpret_cast<__nv_bfloat16*>(a.dq) + (row0 * a.H + hq) * DK + kr, (int64_t)a.H * DK, cs, cm.len, g, t);
+        store_t<NH>(rq, reinterpret_cast<__nv_bfloat16*>(a.dq) + (row0 * a.H + hq) * DK + kr, (int64_t)a.H * DK, cs, cm.len, g, t);
       }
     }
     if (__syncthreads_or(!ph.wait())) { failed = true; break; }
@@ -446,7 +490,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
     {
       float r[16], dA2[16];
       acc_ld32q(C2, q, cs, r);
-      acc_ld32q(C1, q, cs, dA2);
+      acc_ld32q(C0, q, cs, dA2);
       tc5::tmem_ld_wait();
       FragStore fs;
 #pragma unroll
@@ -470,7 +514,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
         tc5::fence_after_sync();
         issue_mma_t<BT / 16>(C2, Operand{sH1, BT, 0}, opA_k, 64, 64, 0);
         ph.commit();
-        issue_mma_t<DK / 16>(C1, opK_k, opK_k, 64, 64, 0);
+        issue_mma_t<DK / 16>(C0, opK_k, opK_k, 64, 64, 0);
       }
       FragLoad fa;
       fa.load(As, BT, q * 16, cs, lane);
@@ -517,7 +561,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
       const float b_lo = bet[r_lo], b_hi = bet[r_hi];
       float m[16], kk[16];
       acc_ld32q(C2, q, cs, m);
-      acc_ld32q(C1, q, cs, kk);
+      acc_ld32q(C0, q, cs, kk);
       tc5::tmem_ld_wait();
       FragStore fs;
       float rmk_lo = 0.f, rmk_hi = 0.f;
@@ -571,6 +615,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
       store_t<NH>(r, reinterpret_cast<__nv_bfloat16*>(a.dv) + (row0 * a.HV + hv) * DK + kr, (int64_t)a.HV * DK, cs, cm.len, g, t);
     }
     if (__syncthreads_or(!ph.wait())) { failed = true; break; }
+    if (!last && tid == 0) load_head(hv + 1, false);   // every tile but K is dead
 
     // ---- epilogue 6: dk, and with its dots with k the gate and beta gradients
     float rk[NH][16];
@@ -580,6 +625,29 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
       tc5::tmem_ld_wait();
       dots_t<NH>(rk, Ks, kr, cs, lane, pv);
       c_rk[q * BT + gcol] = sum8_over_g(pv, g);
+      if (MODE == kTurns) {
+        if (!first) {
+          float acc[NH][16];
+#pragma unroll
+          for (int e = 0; e < NH * 4; ++e)
+            asm volatile("ld.local.v4.f32 {%0, %1, %2, %3}, [%4];\n"
+                         : "=f"(acc[e / 4][4 * (e % 4)]), "=f"(acc[e / 4][4 * (e % 4) + 1]), "=f"(acc[e / 4][4 * (e % 4) + 2]),
+                           "=f"(acc[e / 4][4 * (e % 4) + 3])
+                         : "l"(dk_sum + 16 * e)
+                         : "memory");
+          add_t<NH>(rk, acc);
+        }
+        if (!last) {
+#pragma unroll
+          for (int e = 0; e < NH * 4; ++e)
+            asm volatile("st.local.v4.f32 [%0], {%1, %2, %3, %4};\n" ::"l"(dk_sum + 16 * e), "f"(rk[e / 4][4 * (e % 4)]),
+                         "f"(rk[e / 4][4 * (e % 4) + 1]), "f"(rk[e / 4][4 * (e % 4) + 2]), "f"(rk[e / 4][4 * (e % 4) + 3])
+                         : "memory");
+        } else if (a.rstd_k != nullptr) {   // the sum's dots, over a tile that a last head needs no more
+          dots_t<NH>(rk, Ks, kr, cs, lane, pv);
+          reinterpret_cast<float*>(Do)[q * BT + gcol] = sum8_over_g(pv, g);
+        }
+      }
     }
     __syncthreads();
     if (tid < BT) {
@@ -612,15 +680,15 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
       }
       dGs[i] = x;
     }
-    if (!GROUPED) {
-      if (a.rstd_k != nullptr) l2_backward_t<NH>(rk, Ks, c_rk, rsk, kr, cs, lane);
+    if (!GROUPED && last) {
+      if (a.rstd_k != nullptr) l2_backward_t<NH>(rk, Ks, MODE == kTurns ? reinterpret_cast<float*>(Do) : c_rk, rsk, kr, cs, lane);
       store_t<NH>(rk, reinterpret_cast<__nv_bfloat16*>(a.dk) + (row0 * a.H + hq) * DK + kr, (int64_t)a.H * DK, cs, cm.len, g, t);
-    } else {
+    } else if (GROUPED) {
       // this head's dq and dk in fp32, token-major, over the dead tiles
       float* sq = reinterpret_cast<float*>(smem + S::o_do);
       float* sk = reinterpret_cast<float*>(smem + S::o_do + S::stage);
       float r[NH][16];
-      acc_ld_t<NH>(C0, q, cs, r);
+      acc_ld_t<NH>(C1, q, cs, r);
       tc5::tmem_ld_wait();
 #pragma unroll
       for (int hf = 0; hf < NH; ++hf)
@@ -661,14 +729,18 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
         a.gate_partials[((int64_t)c * a.HV + hv) * 2 + 1] = red[17] + red[19];
       }
     }
-  } while (false);
+    if (!last) {
+      __syncthreads();   // the vectors have been read
+      head_vectors(hv + 1);
+    }
+  }
 
   if (GROUPED) {
     // every CTA of the group takes 64 / G of the rows; all of them come here, whatever happened above
     cluster_sync();
     if (!failed) {
       constexpr int LPT = DK / 4, TPR = NTHREADS / LPT;   // lanes per token (four columns each), tokens per round
-      const int rank = hv % G, per = BT / G, col = (tid % LPT) * 4;
+      const int rank = hv0 % G, per = BT / G, col = (tid % LPT) * 4;
       for (int j = tid / LPT; j < per; j += TPR) {
         const int tok = rank * per + j;
 #pragma unroll
@@ -711,11 +783,11 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
   if (warp == 1) tc5::tmem_dealloc(tm, 256);
 }
 
-template <int DK, bool GROUPED>
+template <int DK, Heads MODE>
 int launch(const b200gdn_chunk_args& a, cudaStream_t st) {
   using S = LocalSmem<DK>;
   static_assert(S::bytes <= 113 * 1024, "two CTAs per SM");
-  if (int e = ensure_smem(bwd_local_kernel<DK, GROUPED>, S::bytes)) return e;
+  if (int e = ensure_smem(bwd_local_kernel<DK, MODE>, S::bytes)) return e;
   LocalMaps m;
   const uint64_t pk = (uint64_t)a.H * DK, pv = (uint64_t)a.HV * DK, hrows = (uint64_t)a.n_chunks * a.HV * DK;
   int rc = 0;
@@ -730,12 +802,12 @@ int launch(const b200gdn_chunk_args& a, cudaStream_t st) {
   rc |= tma::encode_bf16_2d(&m.dh, a.dh, hrows, DK, DK, DK);
   if (rc != 0) return set_error(B200GDN_ERR_CUDA, "bwd_local: cuTensorMapEncodeTiled failed (%d)", rc);
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(a.n_chunks, a.HV);
+  cfg.gridDim = dim3(a.n_chunks, MODE == kTurns ? a.H : a.HV);
   cfg.blockDim = dim3(NTHREADS);
   cfg.dynamicSmemBytes = S::bytes;
   cfg.stream = st;
   cudaLaunchAttribute attr;
-  if (GROUPED) {
+  if (MODE == kCluster) {
     attr.id = cudaLaunchAttributeClusterDimension;
     attr.val.clusterDim.x = 1;
     attr.val.clusterDim.y = a.HV / a.H;
@@ -743,24 +815,39 @@ int launch(const b200gdn_chunk_args& a, cudaStream_t st) {
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
   }
-  cudaLaunchKernelEx(&cfg, bwd_local_kernel<DK, GROUPED>, a, m);
+  cudaLaunchKernelEx(&cfg, bwd_local_kernel<DK, MODE>, a, m);
   if (int e = check_launch("bwd_local")) return e;
   return launch_gate_reduce(a, st);
 }
 
+// Several value heads per q/k head: in turn in one CTA, or a CTA each and the sums of dq and dk through a cluster.  A cluster
+// costs about a quarter more per head (it holds its CTAs until the slowest has arrived and its sums have been read: 272 us
+// against 242 at B4 T4096 8/16 heads of 128), but has G times as many CTAs, so it stays where turns would leave
+// the device to a few: two fit on an SM, and the rounds of CTAs decide.  Both add the heads in the same order and precision.
+bool in_turns(const b200gdn_chunk_args& a) {
+  constexpr int64_t slots = 2 * 148;
+  const int64_t G = a.HV / a.H, turns = G * ((a.n_chunks * (int64_t)a.H + slots - 1) / slots),
+                cluster = (a.n_chunks * (int64_t)a.HV + slots - 1) / slots;
+  return 4 * turns <= 5 * cluster;
+}
+
+template <int DK>
+int launch_heads(const b200gdn_chunk_args& a, cudaStream_t st) {
+  if (a.HV == a.H) return launch<DK, kOne>(a, st);
+  return in_turns(a) ? launch<DK, kTurns>(a, st) : launch<DK, kCluster>(a, st);
+}
+
 }  // namespace
 
-// A group's heads meet in a thread-block cluster, so it serves group sizes that are legal cluster sizes.
+// (group sizes beyond those that are legal cluster sizes are served in turns only)
 bool bwd_local_serves(const b200gdn_chunk_args& a) {
   const int G = a.HV / a.H;
-  return a.K == a.V && (a.K == 64 || a.K == 128) && (G == 1 || G == 2 || G == 4 || G == 8);
+  return a.K == a.V && (a.K == 64 || a.K == 128) && (G == 1 || G == 2 || G == 4 || G == 8 || in_turns(a));
 }
 
 int launch_bwd_local(const b200gdn_chunk_args& a, cudaStream_t st) {
   if (int e = check_gate_args(a, "bwd_local")) return e;
-  const bool grouped = a.HV > a.H;
-  if (a.K == 128) return grouped ? launch<128, true>(a, st) : launch<128, false>(a, st);
-  return grouped ? launch<64, true>(a, st) : launch<64, false>(a, st);
+  return a.K == 128 ? launch_heads<128>(a, st) : launch_heads<64>(a, st);
 }
 
 // Reads and clears the flag a bounded device wait raises when it expires (synchronises with the device).
