@@ -109,94 +109,104 @@ __global__ void cp_fold_kernel(const b200gdn_fold_args a) {
 //   forward:  j_t = first_pre + t,              o_t = first_out + t + 1
 //   reverse:  j_t = first_pre + count - 2 - t,  o_t = first_out + count - 2 - t   (out[first_out + count - 1] = x0 first)
 // and, when `last` is given, last[c] = the chain's final x.
-// A CTA owns one head and CP = 8 value columns of a chain (columns are independent), two threads per row.  The chain is
-// serial, so its step is what counts: M_j streams through shared memory in chunks of MC columns, double-buffered by
-// asynchronous 16-byte copies, while the row products are formed two columns at a time (f32x2).  Every thread reading its
-// row of M from global memory, 32 columns per CTA, took 13 us a step at K = V = 128; 3.6 us now.
+// A CTA owns one head and CP = 8 value columns of a chain (columns are independent).  The chain is serial, so its step is what
+// counts.  A thread forms four rows x all eight columns over an eighth of the contraction: every element of M_j then belongs
+// to one thread and comes straight from global memory into registers, a step ahead of its use (the maps do not depend on
+// the chain), only x is shared, and the eight partial sums meet by recursive halving (28 shuffles).  Bound by the
+// shared-memory reads of x and fp32 issue.  K = V = 128: 1.5 us a step with
+// one CTA per SM (2.3 with M through shared memory, 13 with one row per thread and 32 columns per CTA); 64: 0.65.
 constexpr int CP = 8;
 template <int DK>
-struct PrefixTile {
-  static constexpr int MC = DK == 256 ? 32 : DK / 2, NCH = DK / MC, LD = MC + 4;   // row stride: 16-byte reads of rows do not collide
-  static constexpr size_t bytes = (size_t)(2 * DK * LD + 2 * DK * CP) * sizeof(float);
-};
-
-template <int DK>
-__global__ void __launch_bounds__(2 * DK) cp_prefix_kernel(const b200gdn_prefix_args a) {
-  using P = PrefixTile<DK>;
-  extern __shared__ __align__(16) float sm[];   // M chunks [2][DK][LD], x [2][DK][CP]
-  float* const xs = sm + 2 * DK * P::LD;
+__global__ void __launch_bounds__(2 * DK, 256 / DK) cp_prefix_kernel(const b200gdn_prefix_args a) {
+  constexpr int NB = DK / 32, RB = NB < 4 ? NB : 4;          // blocks of 32 columns of M; blocks held in registers
+  constexpr int XS = DK * CP + (DK / 4) * 4;                 // x rows; four floats of padding after every four rows (banks)
+  __shared__ __align__(16) float xs[2][XS];
   const int V = a.V, hv = blockIdx.y, c0 = blockIdx.x * CP, chain = blockIdx.z;
-  const int tid = threadIdx.x, r = tid >> 1, ch = (tid & 1) * (CP / 2);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int mg = lane & 7, r0 = (warp * 4 + (lane >> 3)) * 4;                      // columns 32 b + 4 mg + e of rows r0 .. r0 + 3
+  const int r = r0 + ((mg >> 1) & 2) + ((mg >> 1) & 1), ch = (mg & 1) * 4;          // the part of x that the halving leaves here
   const int first_out = a.table[3 * chain], count = a.table[3 * chain + 1], first_pre = a.table[3 * chain + 2];
-  const int n_chunks = (count - 1) * P::NCH;
   auto pair_of = [&](int t) { return a.reverse ? first_pre + count - 2 - t : first_pre + t; };
-  auto fetch = [&](int i) {   // chunk i of the walk into buffer i & 1 (an empty group past the end)
-    if (i < n_chunks) {
-      const float* M = a.M + ((int64_t)pair_of(i / P::NCH) * a.HV + hv) * DK * DK + (i % P::NCH) * P::MC;
-      float* dst = sm + (i & 1) * DK * P::LD;
-      for (int e = tid; e < DK * P::MC / 4; e += 2 * DK) {
-        const int row = e / (P::MC / 4), c = (e % (P::MC / 4)) * 4;
-        cp_async16(dst + row * P::LD + c, M + (int64_t)row * DK + c);
-      }
-    }
-    cp_async_commit();
-  };
-  fetch(0);
-  fetch(1);
-  float x[CP / 2];
+  float4 mreg[RB][4];
+  auto fetch = [&](int t, int blk, float4 (&m)[4]) {
+    if (t + 1 < count) {
+      const float* M = a.M + (((int64_t)pair_of(t) * a.HV + hv) * DK + r0) * DK + 32 * blk + 4 * mg;
 #pragma unroll
-  for (int c = 0; c < CP / 2; ++c) {
-    const int col = c0 + ch + c;
-    x[c] = a.x0 ? a.x0[(((int64_t)chain * a.HV + hv) * DK + r) * V + col] : ((a.identity && r == col) ? 1.f : 0.f);
+      for (int i = 0; i < 4; ++i) m[i] = *reinterpret_cast<const float4*>(M + i * DK);
+    }
+  };
+  auto h_of = [&](int t) {
+    return a.h != nullptr && t + 1 < count
+               ? *reinterpret_cast<const float4*>(&a.h[(((int64_t)pair_of(t) * a.HV + hv) * DK + r) * V + c0 + ch])
+               : make_float4(0.f, 0.f, 0.f, 0.f);
+  };
+#pragma unroll
+  for (int i = 0; i < RB; ++i) fetch(0, i, mreg[i]);
+  float4 x = make_float4(0.f, 0.f, 0.f, 0.f), h = h_of(0);
+  if (a.x0 != nullptr) {
+    const float* x0 = &a.x0[(((int64_t)chain * a.HV + hv) * DK + r) * V + c0 + ch];   // a caller's tensor, on any boundary
+    x = make_float4(x0[0], x0[1], x0[2], x0[3]);
+  } else if (a.identity) {
+    const int d = r - c0 - ch;
+    x = make_float4(d == 0, d == 1, d == 2, d == 3);
   }
   auto keep = [&](int cur, int piece) {
-    const float4 v = make_float4(x[0], x[1], x[2], x[3]);
-    *reinterpret_cast<float4*>(&xs[(cur * DK + r) * CP + ch]) = v;
-    if (a.out != nullptr && piece >= 0) *reinterpret_cast<float4*>(&a.out[(((int64_t)piece * a.HV + hv) * DK + r) * V + c0 + ch]) = v;
+    *reinterpret_cast<float4*>(&xs[cur][r * CP + (r >> 2) * 4 + ch]) = x;
+    if (a.out != nullptr && piece >= 0) *reinterpret_cast<float4*>(&a.out[(((int64_t)piece * a.HV + hv) * DK + r) * V + c0 + ch]) = x;
   };
   keep(0, a.reverse ? first_out + count - 1 : first_out);
-  int cur = 0, i = 0;
+  int cur = 0;
   for (int t = 0; t + 1 < count; ++t) {
-    uint64_t acc[2] = {0ull, 0ull};
-    if (a.h) {
-      const float4 h = *reinterpret_cast<const float4*>(&a.h[(((int64_t)pair_of(t) * a.HV + hv) * DK + r) * V + c0 + ch]);
-      acc[0] = pack2(h.x, h.y);
-      acc[1] = pack2(h.z, h.w);
-    }
-    for (int k = 0; k < P::NCH; ++k, ++i) {
-      cp_async_wait<1>();
-      __syncthreads();   // the chunk has landed for everybody (and x of this step is complete)
-      const float* Mr = sm + (i & 1) * DK * P::LD + r * P::LD;
-      const float* xr = xs + (cur * DK + k * P::MC) * CP + ch;
-#pragma unroll 4
-      for (int m = 0; m < P::MC; m += 4) {
-        const float4 mv = *reinterpret_cast<const float4*>(Mr + m);
-        const float mm[4] = {mv.x, mv.y, mv.z, mv.w};
+    __syncthreads();   // x of this step is complete (and that of the step before has been read)
+    const float4 h_next = h_of(t + 1);
+    uint64_t acc[4][4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const uint64_t* y = reinterpret_cast<const uint64_t*>(xr + (m + e) * CP);
-          const uint64_t w = pack2(mm[e], mm[e]);
-          acc[0] = fma2(w, y[0], acc[0]);
-          acc[1] = fma2(w, y[1], acc[1]);
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) acc[i][c] = 0ull;
+#pragma unroll
+    for (int blk = 0; blk < NB; ++blk) {
+      float4 (&m)[4] = mreg[blk % RB];
+      const float* xr = &xs[cur][(32 * blk + 4 * mg) * CP + (8 * blk + mg) * 4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const ulonglong2 lo = *reinterpret_cast<const ulonglong2*>(xr + e * CP), hi = *reinterpret_cast<const ulonglong2*>(xr + e * CP + 4);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float f = e == 0 ? m[i].x : e == 1 ? m[i].y : e == 2 ? m[i].z : m[i].w;
+          const uint64_t w = pack2(f, f);
+          acc[i][0] = fma2(w, lo.x, acc[i][0]);
+          acc[i][1] = fma2(w, lo.y, acc[i][1]);
+          acc[i][2] = fma2(w, hi.x, acc[i][2]);
+          acc[i][3] = fma2(w, hi.y, acc[i][3]);
         }
       }
-      __syncthreads();   // everybody has read the chunk before the next one takes its place
-      fetch(i + 2);
+      // the block RB further on takes this one's registers
+      if (blk + RB < NB) fetch(t, blk + RB, m); else fetch(t + 1, blk + RB - NB, m);
     }
-    const float2 p = unpack2(acc[0]), q = unpack2(acc[1]);
-    x[0] = p.x; x[1] = p.y; x[2] = q.x; x[3] = q.y;
+    // recursive halving over the eight lanes of a row group: rows, rows, columns; a lane hands over what its partner keeps
+    uint64_t s2[2][4], s1[4], s0[2];
+    const bool b2 = mg & 4, b1 = mg & 2, b0 = mg & 1;
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) s2[i][c] = add2(b2 ? acc[2 + i][c] : acc[i][c], __shfl_xor_sync(0xffffffffu, (unsigned long long)(b2 ? acc[i][c] : acc[2 + i][c]), 4));
+#pragma unroll
+    for (int c = 0; c < 4; ++c) s1[c] = add2(b1 ? s2[1][c] : s2[0][c], __shfl_xor_sync(0xffffffffu, (unsigned long long)(b1 ? s2[0][c] : s2[1][c]), 2));
+#pragma unroll
+    for (int c = 0; c < 2; ++c) s0[c] = add2(b0 ? s1[2 + c] : s1[c], __shfl_xor_sync(0xffffffffu, (unsigned long long)(b0 ? s1[c] : s1[2 + c]), 1));
+    const float2 lo = unpack2(s0[0]), hi = unpack2(s0[1]);
+    x = make_float4(lo.x + h.x, lo.y + h.y, hi.x + h.z, hi.y + h.w);
+    h = h_next;
     cur ^= 1;
     keep(cur, a.reverse ? first_out + count - 2 - t : first_out + t + 1);
   }
-  cp_async_wait<0>();
-  if (a.last != nullptr)
-    *reinterpret_cast<float4*>(&a.last[(((int64_t)chain * a.HV + hv) * DK + r) * V + c0 + ch]) = make_float4(x[0], x[1], x[2], x[3]);
+  if (a.last != nullptr) *reinterpret_cast<float4*>(&a.last[(((int64_t)chain * a.HV + hv) * DK + r) * V + c0 + ch]) = x;
 }
 
 template <int DK>
 int launch_prefix(const b200gdn_prefix_args& a, cudaStream_t st) {
-  if (int e = ensure_smem(cp_prefix_kernel<DK>, PrefixTile<DK>::bytes)) return e;
-  cp_prefix_kernel<DK><<<dim3(a.V / CP, a.HV, a.n_chains), 2 * DK, PrefixTile<DK>::bytes, st>>>(a);
+  cp_prefix_kernel<DK><<<dim3(a.V / CP, a.HV, a.n_chains), 2 * DK, 0, st>>>(a);
   return check_launch("cp_prefix");
 }
 
