@@ -94,7 +94,6 @@ def tables_for(B: int, T: int, cu_seqlens: Optional[torch.Tensor], cu_seqlens_cp
 # over all pieces at once.  Pieces are whole numbers of chunks, so the chunking (and every chunk-local kernel) is
 # unchanged.
 SM_COUNT = 148
-MIN_PIECE_CHUNKS = 16        # a piece shorter than this does not pay for its pre-scan
 FORCE_PIECES = None          # tests: cut every sequence into (up to) this many pieces regardless of the heuristic
 _split_cache: dict = {}
 
@@ -114,15 +113,33 @@ class SplitPlan:
 
 
 def piece_counts(chunks_per_seq, HV: int, slices: int):
-    """How many pieces each sequence is cut into: as many as fill the SMs once, in proportion to the sequence lengths."""
+    """How many pieces each sequence is cut into (equal pieces, so the longest sequences into the most): the cut with the
+    least time by the model below, in microseconds as measured on a B200 with heads of 128 and 64; none unless it saves
+    a twentieth.  A scan CTA takes `step` per chunk and the pre-scan, which runs beside twice as many transition-matrix
+    CTAs (two per SM forward, one backward), nearly as long; the prefix chain takes a step per piece.  Two pieces never
+    pay: pre-scan and scan together then walk as far as the uncut scan."""
     if FORCE_PIECES is not None:
         return [max(1, min(int(FORCE_PIECES), int(c))) for c in chunks_per_seq]
-    slots = SM_COUNT // max(1, slices * HV)          # sequences' worth of scan CTAs that fit the device at once
-    n_real = sum(1 for c in chunks_per_seq if c > 0)
-    if slots < 2 or n_real >= slots:
-        return [1] * len(chunks_per_seq)
-    target = max(MIN_PIECE_CHUNKS, -(-sum(chunks_per_seq) // slots))   # chunks per piece
-    return [max(1, min(int(c) // MIN_PIECE_CHUNKS, int(round(c / target)))) if c > 0 else 1 for c in chunks_per_seq]
+    uncut = [1] * len(chunks_per_seq)
+    lens = [int(c) for c in chunks_per_seq if c > 0]
+    per_seq = max(1, slices * HV)                    # scan CTAs of a piece
+    if not lens or per_seq * (len(lens) + 2) > SM_COUNT:
+        return uncut
+    longest, step, chain = max(lens), 1.27 if slices > 1 else 1.06, 1.5 if slices > 1 else 0.65
+    if 8 * slices * HV * len(lens) > SM_COUNT:       # the chains' CTAs, eight columns each, share SMs
+        chain *= 1.8
+    best, length = 0.95 * (3.5 + step * longest), None
+    for pieces in range(3, min(longest, SM_COUNT // per_seq - len(lens) + 1) + 1):
+        n = -(-longest // pieces)
+        total = sum(-(-c // n) for c in lens)
+        pre = (total - len(lens)) * 2 * per_seq      # pre-scan CTAs
+        if total * per_seq > SM_COUNT:
+            continue
+        rounds = (-(-pre // SM_COUNT) - (-pre // (2 * SM_COUNT))) / 2
+        cost = 12. + step * n * (1 + 0.92 * rounds) + chain * (-(-longest // n) - 1)
+        if cost < best:
+            best, length = cost, n
+    return uncut if length is None else [max(1, -(-int(c) // length)) for c in chunks_per_seq]
 
 
 def split_plan(bounds, HV: int, slices: int, device, rows: int) -> Optional[SplitPlan]:

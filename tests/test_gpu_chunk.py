@@ -789,3 +789,30 @@ def test_sequence_split_heuristic_on_one_long_sequence():
     o_r, ht_r = fused_recurrent_gated_delta_rule(q, k, v, g, beta=beta, output_final_state=True)
     O.assert_close('o chunk (split) vs recurrent', o_r.float().cpu(), o.float().cpu(), 0.005)
     O.assert_close('ht chunk (split) vs recurrent', ht_r.cpu(), ht.cpu(), 0.005)
+
+
+@pytest.mark.parametrize('D,HV,lens', [(128, 4, [2048]), (64, 4, [4100]), (64, 2, [700, 1300, 5000, 1]), (128, 16, [4095])])
+def test_planned_cuts_equal_the_uncut_scan(D, HV, lens):
+    """Shapes that the planner cuts into from three pieces to many: outputs, final states and gradients against the uncut
+    run, and the outputs against the token-by-token kernel."""
+    from b200gdn import fused_recurrent_gated_delta_rule, index
+    cu = [0] + list(np.cumsum(lens))
+    chunks = [-(-n // 64) for n in lens]
+    assert max(index.piece_counts(chunks, HV, D // 64)) >= 3
+    q, k, v, g, beta, do = _inputs(1, cu[-1], HV, HV, D, D, seed=37)
+    cu_t = torch.tensor(cu, dtype=torch.int32, device='cuda')
+    h0 = torch.randn(len(lens), HV, D, D, device='cuda') * 0.1
+    out = {}
+    for force in (None, 1):
+        index.FORCE_PIECES = force
+        try:
+            index._split_cache.clear()
+            out[force] = _fwd_bwd(q, k, v, g, beta, do, cu_seqlens=cu_t, initial_state=h0)
+        finally:
+            index.FORCE_PIECES = None
+            index._split_cache.clear()
+    for n, cut, whole in zip(('o', 'ht', 'dq', 'dk', 'dv', 'dg', 'dbeta'), out[None], out[1]):
+        O.assert_close(f'{n} cut vs uncut', whole.float().cpu(), cut.float().cpu(), 0.004)
+    o_r, ht_r = fused_recurrent_gated_delta_rule(q, k, v, g, beta=beta, initial_state=h0, output_final_state=True, cu_seqlens=cu_t)
+    O.assert_close('o vs recurrent', o_r.float().cpu(), out[None][0].float().cpu(), 0.005)
+    O.assert_close('ht vs recurrent', ht_r.cpu(), out[None][1].cpu(), 0.005)
