@@ -155,3 +155,20 @@ def test_conv_single_token_step(W, misaligned):
     assert new.data_ptr() == cache.data_ptr()
     O.assert_close('y', want.cpu(), y[:, 0].float().cpu(), 4e-3)
     assert torch.equal(new, torch.cat([c[..., 1:], x[:, 0, :, None]], -1))
+
+
+@pytest.mark.parametrize('rows,D', [(1, 128), (14209, 128), (2 * 444 * 32 - 3, 64), (9473, 256), (2369, 512)])
+@pytest.mark.parametrize('bias', [False, True])
+def test_rms_norm_gated_rows_around_a_wave(rows, D, bias):
+    """A single row and row counts at and past what one wave of CTAs takes per turn, with and without a bias."""
+    from b200gdn.modules import rms_norm_gated
+    gen = torch.Generator(device='cuda').manual_seed(rows)
+    x, g, dy = (torch.randn(1, rows, 1, D, device='cuda', generator=gen).to(torch.bfloat16) for _ in range(3))
+    leaves = [x, g, torch.randn(D, device='cuda', generator=gen)] + ([torch.randn(D, device='cuda', generator=gen)] if bias else [])
+    leaves = [t.requires_grad_(True) for t in leaves]
+    wide = [t.detach().double().requires_grad_(True) for t in leaves]
+    ry = O.rms_norm_gated_ref(wide[0], wide[1], wide[2], wide[3] if bias else None)
+    y = rms_norm_gated(*leaves[:3], leaves[3] if bias else None)
+    O.assert_close('y', ry, y.double(), 5e-3)
+    for n, w, t in zip(('dx', 'dg', 'dweight', 'dbias'), torch.autograd.grad(ry, wide, dy.double()), torch.autograd.grad(y, leaves, dy)):
+        O.assert_close(n, w, t.double(), 1e-2)
