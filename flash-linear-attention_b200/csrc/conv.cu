@@ -14,10 +14,11 @@
 // gradient of the cache for a sequence's first share, and leaves per-share sums of dweight / dbias that a second kernel
 // adds in a fixed order (no atomics: results are bit-reproducible).
 // One token per sequence (a decoding step) has a kernel of its own: no walk, the cache as whole words.
-// bf16, W = 4, SiLU, [4, 4096, 2048]: forward 32.7 us (4.1 TB/s of x and y; 35.3 with scalar instructions behind a ring of
-// asynchronous copies), backward 61.8 us (80.9) + 4.6 (6.7) for the parameter sums; what is left to the copy rate is the
-// loads in flight per SM (an eighth forward CTA spills: 40.6 us; 16-byte accesses with eight channels a thread: 40.9).
-// A decoding step of 32 users: 2.3 us (4.9).
+// bf16, W = 4, SiLU, [4, 4096, 2048]: forward 27.9 us (4.8 TB/s of x and y; 35.3 with scalar instructions behind a ring of
+// asynchronous copies, 32.1 with the activation, the residual and every token's place decided at run time), backward 55.8 us
+// (80.9, 61.4) + 4.2 (6.7) for the parameter sums.  What is left to the copy rate is instruction issue (half of the cycles)
+// and latency at the warps that the registers allow (an eighth forward or a fifth backward CTA spills: 28.1 and 80.6 us;
+// 16-byte accesses with eight channels a thread: 40.9).  A decoding step of 32 users: 2.3 us (4.9).
 #include <type_traits>
 
 #include "gdn_common.cuh"
@@ -131,19 +132,26 @@ struct Taps {
   }
 };
 
-template <typename T, int W>
+template <typename T, int W, bool ACT, bool RES>
 __global__ void __launch_bounds__(CT, sizeof(T) == 4 ? 5 : 7) conv_fwd_kernel(const b200gdn_conv_args a, const int tokens) {
   const int d0 = (blockIdx.y * CT + threadIdx.x) * C;
   if (d0 >= a.D) return;
   const Share s = load_share(a, blockIdx.x, blockIdx.z, tokens);
   if (s.len <= 0) return;
-  const bool act = a.flags & B200GDN_CONV_SILU;
   const int64_t base = (int64_t)s.row * a.D + d0;
+  const T* const x = static_cast<const T*>(a.x) + base;
+  T* const y_out = static_cast<T*>(a.y) + base;
   Raw<T> buf[2][GRP];
   auto fetch = [&](int t0, Raw<T> (&r)[GRP]) {
+    const T* p = x + (int64_t)t0 * a.D;
+    if (t0 + GRP <= s.len) {
 #pragma unroll
-    for (int u = 0; u < GRP; ++u)
-      if (t0 + u < s.len) r[u].load(a.x, base + (int64_t)(t0 + u) * a.D);
+      for (int u = 0; u < GRP; ++u, p += a.D) r[u].load(p, 0);
+    } else {
+#pragma unroll
+      for (int u = 0; u < GRP; ++u, p += a.D)
+        if (t0 + u < s.len) r[u].load(p, 0);
+    }
   };
   fetch(0, buf[0]);
   fetch(GRP, buf[1]);
@@ -153,26 +161,26 @@ __global__ void __launch_bounds__(CT, sizeof(T) == 4 ? 5 : 7) conv_fwd_kernel(co
 #pragma unroll
   for (int j = 0; j < W - 1; ++j) input_at<T, W>(a, s.n, s.row - s.pos, s.pos - (W - 1) + j, d0, hist[j]);
   auto group = [&](int t0, Raw<T> (&r)[GRP], auto full) {
+    T* p = y_out + (int64_t)t0 * a.D;
 #pragma unroll
-    for (int u = 0; u < GRP; ++u) {
+    for (int u = 0; u < GRP; ++u, p += a.D) {
       if (!decltype(full)::value && t0 + u >= s.len) return;
       uint64_t cur[C / 2], y[C / 2];
       r[u].get(cur);
 #pragma unroll
       for (int i = 0; i < C / 2; ++i) {
         y[i] = k.pre(hist, cur, i);
-        if (act) y[i] = mul2(y[i], fast_sigmoid2(y[i]));
+        if (ACT) y[i] = mul2(y[i], fast_sigmoid2(y[i]));
       }
-      const int64_t off = base + (int64_t)(t0 + u) * a.D;
-      if (a.residual) {
+      if (RES) {
         Raw<T> q;
         uint64_t res[C / 2];
-        q.load(a.residual, off);
+        q.load(a.residual, base + (int64_t)(t0 + u) * a.D);
         q.get(res);
 #pragma unroll
         for (int i = 0; i < C / 2; ++i) y[i] = add2(y[i], res[i]);
       }
-      store_pairs<T>(a.y, off, y);
+      store_pairs<T>(p, 0, y);
 #pragma unroll
       for (int j = 0; j < W - 2; ++j)
 #pragma unroll
@@ -276,12 +284,11 @@ __global__ void __launch_bounds__(CT) conv_step_kernel(const b200gdn_conv_args a
   }
 }
 
-template <typename T, int W>
+template <typename T, int W, bool ACT, bool BIAS>
 __global__ void __launch_bounds__(CT, sizeof(T) == 4 ? 3 : 4) conv_bwd_kernel(const b200gdn_conv_args a, const int tokens) {
   const int d0 = (blockIdx.y * CT + threadIdx.x) * C;
   if (d0 >= a.D) return;
   const Share s = load_share(a, blockIdx.x, blockIdx.z, tokens);
-  const bool act = a.flags & B200GDN_CONV_SILU;
   // sums of this share: [W + 1][D], taps then bias
   float* const part = a.partials ? a.partials + ((int64_t)blockIdx.x * gridDim.z + blockIdx.z) * (W + 1) * a.D + d0 : nullptr;
   auto put = [&](int j, const uint64_t (&x)[C / 2]) {
@@ -299,12 +306,21 @@ __global__ void __launch_bounds__(CT, sizeof(T) == 4 ? 3 : 4) conv_bwd_kernel(co
   const int64_t base = (int64_t)s.row * a.D + d0;
   Raw<T> bx[2][GRP], by[2][GRP];
   auto fetch = [&](int t0, Raw<T> (&rx)[GRP], Raw<T> (&ry)[GRP]) {
+    int64_t at = base + (int64_t)t0 * a.D;
+    if (t0 + GRP <= n_tok) {
 #pragma unroll
-    for (int u = 0; u < GRP; ++u)
-      if (t0 + u < n_tok) {
-        rx[u].load(a.x, base + (int64_t)(t0 + u) * a.D);
-        ry[u].load(a.dy, base + (int64_t)(t0 + u) * a.D);
+      for (int u = 0; u < GRP; ++u, at += a.D) {
+        rx[u].load(a.x, at);
+        ry[u].load(a.dy, at);
       }
+    } else {
+#pragma unroll
+      for (int u = 0; u < GRP; ++u, at += a.D)
+        if (t0 + u < n_tok) {
+          rx[u].load(a.x, at);
+          ry[u].load(a.dy, at);
+        }
+    }
   };
   fetch(0, bx[0], by[0]);
   fetch(GRP, bx[1], by[1]);
@@ -326,8 +342,8 @@ __global__ void __launch_bounds__(CT, sizeof(T) == 4 ? 3 : 4) conv_bwd_kernel(co
   const bool to_cache = s.pos == 0 && a.dinitial_state != nullptr;
   const int last = n_tok - 1 + (W - 1);   // the extra steps only flush the ring
   const uint64_t one = pack2(1.f, 1.f), mone = pack2(-1.f, -1.f);
-  // one step; FULL: the token is known to lie inside the share (it is loaded and counted for the parameters), so only the
-  // store is conditional and the compiler renames the history and ring registers across the unrolled steps of a group
+  // one step; FULL: the token is known to lie inside the share (it is loaded and counted for the parameters) and not in its
+  // first group, so nothing is conditional and the compiler renames the history and ring registers across the unrolled steps of a group
   auto step = [&](int u, const Raw<T>& rx, const Raw<T>& ry, auto full) {
     constexpr bool FULL = decltype(full)::value;
     if (!FULL && u > last) return;
@@ -338,12 +354,12 @@ __global__ void __launch_bounds__(CT, sizeof(T) == 4 ? 3 : 4) conv_bwd_kernel(co
       ry.get(dpre);
 #pragma unroll
       for (int i = 0; i < C / 2; ++i) {
-        if (act) {   // d silu(p) = s (1 + p (1 - s))
+        if (ACT) {   // d silu(p) = s (1 + p (1 - s))
           const uint64_t p = k.pre(hist, cur, i), sg = fast_sigmoid2(p);
           dpre[i] = mul2(dpre[i], mul2(sg, fma2(p, fma2(sg, mone, one), one)));
         }
         if (FULL || u < s.len) {   // the parameters' gradients: every token is counted by the share that owns it
-          db[i] = add2(db[i], dpre[i]);
+          if (BIAS) db[i] = add2(db[i], dpre[i]);
           dw[W - 1][i] = fma2(dpre[i], cur[i], dw[W - 1][i]);
 #pragma unroll
           for (int j = 0; j < W - 1; ++j) dw[j][i] = fma2(dpre[i], hist[j][i], dw[j][i]);
@@ -366,7 +382,9 @@ __global__ void __launch_bounds__(CT, sizeof(T) == 4 ? 3 : 4) conv_bwd_kernel(co
       ring[0][i] = mul2(k.w[W - 1][i], dpre[i]);
     }
     const int e = u - (W - 1);
-    if (e >= 0) {
+    if (FULL) {
+      store_pairs<T>(a.dx, base + (int64_t)e * a.D, done);
+    } else if (e >= 0) {
       if (e < s.len) store_pairs<T>(a.dx, base + (int64_t)e * a.D, done);
     } else if (to_cache) {   // an input before the sequence start: gradient of the cache entry x[e] = initial_state[n, d, W + e]
 #pragma unroll
@@ -381,7 +399,7 @@ __global__ void __launch_bounds__(CT, sizeof(T) == 4 ? 3 : 4) conv_bwd_kernel(co
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       const int t = t0 + h * GRP;
-      if (t + GRP <= s.len) {
+      if (t >= GRP && t + GRP <= s.len) {
 #pragma unroll
         for (int v = 0; v < GRP; ++v) step(t + v, bx[h][v], by[h][v], std::true_type{});
       } else {
@@ -398,7 +416,7 @@ __global__ void __launch_bounds__(CT, sizeof(T) == 4 ? 3 : 4) conv_bwd_kernel(co
   if (part != nullptr) {
 #pragma unroll
     for (int j = 0; j < W; ++j) put(j, dw[j]);
-    put(W, db);
+    if (BIAS) put(W, db);
   }
 }
 
@@ -409,10 +427,10 @@ constexpr int RW = 16;
 __global__ void __launch_bounds__(32 * RW) conv_param_reduce_kernel(const b200gdn_conv_args a, const int n) {
   __shared__ float part[RW][32];
   const int lane = threadIdx.x & 31, q = threadIdx.x >> 5;
-  const int64_t per_share = (int64_t)a.D * (a.W + 1);
+  const int64_t per_share = (int64_t)a.D * (a.W + 1), n_out = (int64_t)a.D * (a.W + (a.dbias != nullptr));
   const int64_t i = (int64_t)blockIdx.x * 32 + lane;
   float s4[4] = {0.f, 0.f, 0.f, 0.f};
-  if (i < per_share) {
+  if (i < n_out) {
     int t = q;
     for (; t + 3 * RW < n; t += 4 * RW) {
 #pragma unroll
@@ -423,12 +441,12 @@ __global__ void __launch_bounds__(32 * RW) conv_param_reduce_kernel(const b200gd
   float s = (s4[0] + s4[1]) + (s4[2] + s4[3]);
   part[q][lane] = s;
   __syncthreads();
-  if (q != 0 || i >= per_share) return;
+  if (q != 0 || i >= n_out) return;
 #pragma unroll
   for (int r = 1; r < RW; ++r) s += part[r][lane];
   const int j = (int)(i / a.D), d = (int)(i % a.D);
   if (j < a.W) st_param(a.dweight, (int64_t)d * a.W + j, a.param_dtype, s);
-  else if (a.dbias != nullptr) st_param(a.dbias, d, a.param_dtype, s);
+  else st_param(a.dbias, d, a.param_dtype, s);
 }
 
 // Tokens per share: a whole tile of 64 while that still gives the SMs twelve warps each, else 32 (and 16 forward; a
@@ -449,14 +467,30 @@ int launch_t(const b200gdn_conv_args& a, cudaStream_t st, bool bwd) {
       return check_launch("conv_step");
     }
     const int tokens = share_tokens(a, 16);
-    conv_fwd_kernel<T, W><<<dim3(a.n_tiles, y, 64 / tokens), CT, 0, st>>>(a, tokens);
+    const dim3 grid(a.n_tiles, y, 64 / tokens);
+    const bool act = a.flags & B200GDN_CONV_SILU;
+    if (a.residual != nullptr) {
+      if (act) conv_fwd_kernel<T, W, true, true><<<grid, CT, 0, st>>>(a, tokens);
+      else conv_fwd_kernel<T, W, false, true><<<grid, CT, 0, st>>>(a, tokens);
+    } else {
+      if (act) conv_fwd_kernel<T, W, true, false><<<grid, CT, 0, st>>>(a, tokens);
+      else conv_fwd_kernel<T, W, false, false><<<grid, CT, 0, st>>>(a, tokens);
+    }
     return check_launch("conv_fwd");
   }
   const int tokens = share_tokens(a, 32);
-  conv_bwd_kernel<T, W><<<dim3(a.n_tiles, y, 64 / tokens), CT, 0, st>>>(a, tokens);
+  const dim3 grid(a.n_tiles, y, 64 / tokens);
+  const bool act = a.flags & B200GDN_CONV_SILU;
+  if (a.dbias != nullptr) {
+    if (act) conv_bwd_kernel<T, W, true, true><<<grid, CT, 0, st>>>(a, tokens);
+    else conv_bwd_kernel<T, W, false, true><<<grid, CT, 0, st>>>(a, tokens);
+  } else {
+    if (act) conv_bwd_kernel<T, W, true, false><<<grid, CT, 0, st>>>(a, tokens);
+    else conv_bwd_kernel<T, W, false, false><<<grid, CT, 0, st>>>(a, tokens);
+  }
   if (int e = check_launch("conv_bwd")) return e;
   if (a.partials != nullptr && a.dweight != nullptr) {
-    const int64_t n = (int64_t)a.D * (a.W + 1);
+    const int64_t n = (int64_t)a.D * (a.W + (a.dbias != nullptr));
     conv_param_reduce_kernel<<<(unsigned)((n + 31) / 32), 32 * RW, 0, st>>>(a, a.n_tiles * (64 / tokens));
     return check_launch("conv_param_reduce");
   }

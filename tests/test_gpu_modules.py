@@ -172,3 +172,31 @@ def test_rms_norm_gated_rows_around_a_wave(rows, D, bias):
     O.assert_close('y', ry, y.double(), 5e-3)
     for n, w, t in zip(('dx', 'dg', 'dweight', 'dbias'), torch.autograd.grad(ry, wide, dy.double()), torch.autograd.grad(y, leaves, dy)):
         O.assert_close(n, w, t.double(), 1e-2)
+
+
+@pytest.mark.parametrize('act', [None, 'silu'])
+@pytest.mark.parametrize('with_residual', [False, True])
+@pytest.mark.parametrize('with_bias', [False, True])
+def test_conv_forms_at_group_and_share_edges(act, with_residual, with_bias):
+    """Every compiled form (activation, residual, bias) on sequences of 1 .. 131 tokens: either side of the groups of four
+    tokens, of the shares and of the tiles."""
+    from b200gdn.modules import causal_conv1d
+    lens, D = [1, 3, 4, 5, 8, 31, 33, 63, 64, 65, 131], 72
+    cu = torch.tensor([0] + list(np.cumsum(lens)), dtype=torch.int32, device='cuda')
+    gen = torch.Generator(device='cuda').manual_seed(5)
+    mk = lambda *s: torch.randn(*s, device='cuda', generator=gen)   # noqa: E731
+    x, w, dy = mk(1, sum(lens), D).requires_grad_(True), mk(D, 4).requires_grad_(True), mk(1, sum(lens), D)
+    b = mk(D).requires_grad_(True) if with_bias else None
+    res = mk(1, sum(lens), D).requires_grad_(True) if with_residual else None
+    leaves = [t for t in (x, w, b, res) if t is not None]
+    y, _ = causal_conv1d(x, w, b, residual=res, activation=act, cu_seqlens=cu)
+    got = torch.autograd.grad(y, leaves, dy)
+    parts = []
+    for s, e in zip(cu.tolist()[:-1], cu.tolist()[1:]):
+        z = torch.nn.functional.conv1d(torch.nn.functional.pad(x[:, s:e].double().transpose(1, 2), (3, 0)), w.double()[:, None],
+                                       None if b is None else b.double(), groups=D).transpose(1, 2)
+        parts.append(torch.nn.functional.silu(z) if act else z)
+    ref = torch.cat(parts, 1) + (0 if res is None else res.double())
+    O.assert_close('y', ref, y.double(), 1e-5)
+    for i, (r, t) in enumerate(zip(torch.autograd.grad(ref, leaves, dy.double()), got)):
+        O.assert_close(f'grad {i}', r.double(), t.double(), 1e-5)
