@@ -10,18 +10,19 @@
 //     dk^T = (dh v_new^T) 2^(gamma_last - gamma_j) + q^T dP + dW^T A_b + K^T M2^T + K^T M2,   A_b = A (beta 2^gamma)_col
 //     dv^T = (dU^T A) beta_j
 //     dbeta= c_kbg 2^gamma + c_vb + r_mk,   c_kbg = colsum(A . dW K^T), c_vb = colsum(A . dU V^T), r_mk = rowsum(M . K K^T)
-//     dG_i = <dq_i,q_i> - <dk_i,k_i> + 2 (c_kbg beta 2^gamma + beta r_mk)
+//     dG_i = <dq_i,q_i> - <dk_loc_i,k_i> + c_kbg beta 2^gamma + beta r_mk - c_mk
 //            (+ at the last valid row: 2^gamma_last <h,dh> + sum_j <dk_state_j, k_j>);     dg = reverse cumsum of dG
-// (the WY terms of dk contribute c_kbg beta 2^gamma + beta r_mk + colsum(M2 . K K^T) to <dk_i,k_i> and the first two minus the
-// last to dG_i, which is why the column sum of M2 . K K^T drops out and no separate row dot of the chunk-local part of dk
-// is needed).
+// with dk_loc the first two terms of dk, <dk_loc_j,k_j> = <dk_state_j,k_j> + colsum(dP . Q K^T)_j, c_mk = colsum(M2 . K K^T).
+// (The WY terms of dk contribute c_kbg beta 2^gamma + beta r_mk + c_mk to <dk_i,k_i>, so dG could be had from the finished dk
+// without Q K^T and c_mk; but then the bf16 operands of those terms do not cancel against the fp32 sums, and the sums of dg
+// over a sequence, dA_log and ddt_bias, were twice as far from fp64 as with the terms kept apart: 0.016 against 0.008.)
 //
 // As two kernels (dq and the chunk-local part of dk; the WY backward) k, h and that part of dk went through HBM twice:
 // 296 KiB per chunk and head at K = V = 128, 216 now, and nine dependent tensor-core phases are six.  Products with a
 // K- or V-wide result are formed TRANSPOSED ([K x 64 tokens], M = 128): the same tcgen05 instruction then does twice the
 // work of an M = 64 one, an accumulator takes 64 TMEM columns instead of 128, and every lane of a TMEM load carries data.
 // Tiles leave token-major straight from registers (movmatrix, then 16-byte words).
-// One CTA of eight warps; 256 TMEM columns (C0: dP, dq^T, dU V^T, K K^T; C1: the sum of dq over a group; C2: dW^T, dW K^T, Y, X,
+// One CTA of eight warps; 256 TMEM columns (C0: dP, dq^T, dU V^T, K K^T, Q K^T; C1: the sum of dq over a group; C2: dW^T, dW K^T, Y, X,
 // dv^T; C3: dk^T) and ~111 KiB of shared memory whose regions change hands, so two CTAs per SM overlap each other's phases:
 //   R1: K      R2: do -> q      R3: v_new -> dU      R4: dh panel 0 -> h panel 0 -> dW^T
 //   R5: dh panel 1 -> h panel 1 -> V -> dA | Y -> M2 | Y
@@ -184,7 +185,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
   // sums over rows: each of the four row-quadrant warps leaves its partial in its own slot and the consumer adds the four in
   // a fixed order (no atomics: results are bit-reproducible)
   float* c_rq = rsk + BT;        // [4][64] <dq_i, q_i>
-  float* c_rk = c_rq + 4 * BT;   // [4][64] <dk_i, k_i>
+  float* c_rk = c_rq + 4 * BT;   // [4][64] <dk_loc_i, k_i> + c_mk
   float* c_kbg = c_rk + 4 * BT;  // [4][64] colsum(A . dW K^T)
   float* c_vb = c_kbg + 4 * BT;  // [4][64] colsum(A . dU V^T)
   float* r_mk = c_vb + 4 * BT;   // [2][64] rowsum(M . K K^T), two column halves
@@ -351,6 +352,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
       }
       *po = x;
     }
+    float dk_dot;   // this lane's part of c_rk
     {   // dk_state^T: column factors, the sum of its dots with k, back to TMEM where the other terms of dk accumulate
       float r[NH][16];
       acc_ld_t<NH>(C3, q, cs, r);
@@ -368,7 +370,8 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
       for (int hf = 0; hf < NH; ++hf) tc5::tmem_st_16x256b_x4(C3 + ((uint32_t)(32 * q + 16 * hf) << 16) + cs, r[hf]);
       float pv[8];
       dots_t<NH>(r, Ks, kr, cs, lane, pv);
-      const float rs = warp_sum(((pv[0] + pv[1]) + (pv[2] + pv[3])) + ((pv[4] + pv[5]) + (pv[6] + pv[7])));
+      dk_dot = sum8_over_g(pv, g);
+      const float rs = warp_sum(dk_dot);
       if (lane == 0) red[8 + warp] = rs;
       tc5::tmem_st_wait();
     }
@@ -564,7 +567,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
       acc_ld32q(C0, q, cs, kk);
       tc5::tmem_ld_wait();
       FragStore fs;
-      float rmk_lo = 0.f, rmk_hi = 0.f;
+      float rmk_lo = 0.f, rmk_hi = 0.f, pv[8];
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int col = cs + i * 8 + 2 * t;
@@ -576,8 +579,12 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
         }
         rmk_lo += m[4 * i] * kk[4 * i] + m[4 * i + 1] * kk[4 * i + 1];
         rmk_hi += m[4 * i + 2] * kk[4 * i + 2] + m[4 * i + 3] * kk[4 * i + 3];
-        fs.set(i, m[4 * i] * b_lo, m[4 * i + 1] * b_lo, m[4 * i + 2] * b_hi, m[4 * i + 3] * b_hi);
+        m[4 * i] *= b_lo; m[4 * i + 1] *= b_lo; m[4 * i + 2] *= b_hi; m[4 * i + 3] *= b_hi;
+        pv[2 * i] = m[4 * i] * kk[4 * i] + m[4 * i + 2] * kk[4 * i + 2];
+        pv[2 * i + 1] = m[4 * i + 1] * kk[4 * i + 1] + m[4 * i + 3] * kk[4 * i + 3];
+        fs.set(i, m[4 * i], m[4 * i + 1], m[4 * i + 2], m[4 * i + 3]);
       }
+      dk_dot += sum8_over_g(pv, g);
       fs.store(M2s, BT, q * 16, cs, lane);
       rmk_lo = sum_over_t(rmk_lo);
       rmk_hi = sum_over_t(rmk_hi);
@@ -590,16 +597,17 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
     tc5::fence_before_sync();
     __syncthreads();
 
-    // ---- phase 6: dv^T = dU^T A | dk^T += K^T M2^T + K^T M2
+    // ---- phase 6: dv^T = dU^T A | dk^T += K^T M2^T + K^T M2 | QK = Q K^T
     if (warp == 0) {
       tc5::fence_after_sync();
       issue_mma_t<BT / 16>(C2, Operand{sVn, BT, 1}, opA_mn, DK, 64, 0);
       ph.commit();
       issue_mma_t<BT / 16>(C3, opK_mn, Operand{sH1, BT, 0}, DK, 64, 1);
       issue_mma_t<BT / 16>(C3, opK_mn, Operand{sH1, BT, 1}, DK, 64, 1);
+      issue_mma_t<DK / 16>(C0, Operand{sDo, BT, 0}, opK_k, 64, 64, 0);
     }
     if (__syncthreads_or(!ph.wait())) { failed = true; break; }
-    if (warp == 0) ph.commit();   // ... of the dk terms
+    if (warp == 0) ph.commit();   // ... of the rest
     {
       float r[NH][16];
       acc_ld_t<NH>(C2, q, cs, r);
@@ -617,14 +625,22 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
     if (__syncthreads_or(!ph.wait())) { failed = true; break; }
     if (!last && tid == 0) load_head(hv + 1, false);   // every tile but K is dead
 
-    // ---- epilogue 6: dk, and with its dots with k the gate and beta gradients
+    // ---- epilogue 6: dk and the gate and beta gradients
     float rk[NH][16];
     {
-      float pv[8];
+      float pv[8], qk[16];
+      acc_ld32q(C0, q, cs, qk);
       acc_ld_t<NH>(C3, q, cs, rk);
       tc5::tmem_ld_wait();
-      dots_t<NH>(rk, Ks, kr, cs, lane, pv);
-      c_rk[q * BT + gcol] = sum8_over_g(pv, g);
+      FragLoad fp;
+      fp.load(Ps, BT, q * 16, cs, lane);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float2 pl = fp.lo2(i), phi = fp.hi2(i);
+        pv[2 * i] = pl.x * qk[4 * i] + phi.x * qk[4 * i + 2];
+        pv[2 * i + 1] = pl.y * qk[4 * i + 1] + phi.y * qk[4 * i + 3];
+      }
+      c_rk[q * BT + gcol] = dk_dot + sum8_over_g(pv, g);
       if (MODE == kTurns) {
         if (!first) {
           float acc[NH][16];
@@ -643,10 +659,11 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
             asm volatile("st.local.v4.f32 [%0], {%1, %2, %3, %4};\n" ::"l"(dk_sum + 16 * e), "f"(rk[e / 4][4 * (e % 4)]),
                          "f"(rk[e / 4][4 * (e % 4) + 1]), "f"(rk[e / 4][4 * (e % 4) + 2]), "f"(rk[e / 4][4 * (e % 4) + 3])
                          : "memory");
-        } else if (a.rstd_k != nullptr) {   // the sum's dots, over a tile that a last head needs no more
-          dots_t<NH>(rk, Ks, kr, cs, lane, pv);
-          reinterpret_cast<float*>(Do)[q * BT + gcol] = sum8_over_g(pv, g);
         }
+      }
+      if (!GROUPED && last && a.rstd_k != nullptr) {   // <dk, k> for the norm's backward, over a tile that is needed no more
+        dots_t<NH>(rk, Ks, kr, cs, lane, pv);
+        reinterpret_cast<float*>(Vn)[q * BT + gcol] = sum8_over_g(pv, g);
       }
     }
     __syncthreads();
@@ -654,7 +671,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
       const int i = tid;
       auto sum4 = [&](const float* v) { return (v[i] + v[BT + i]) + (v[2 * BT + i] + v[3 * BT + i]); };
       const float rmk = r_mk[i] + r_mk[BT + i], ckbg = sum4(c_kbg);
-      float x = sum4(c_rq) - sum4(c_rk) + 2.f * (ckbg * bge[i] + bet[i] * rmk);
+      float x = sum4(c_rq) - sum4(c_rk) + (ckbg * bge[i] + bet[i] * rmk);
       if (i == cm.len - 1) {
         float sh = 0.f, sr = 0.f;
 #pragma unroll
@@ -681,7 +698,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
       dGs[i] = x;
     }
     if (!GROUPED && last) {
-      if (a.rstd_k != nullptr) l2_backward_t<NH>(rk, Ks, MODE == kTurns ? reinterpret_cast<float*>(Do) : c_rk, rsk, kr, cs, lane);
+      if (a.rstd_k != nullptr) l2_backward_t<NH>(rk, Ks, reinterpret_cast<float*>(Vn), rsk, kr, cs, lane);
       store_t<NH>(rk, reinterpret_cast<__nv_bfloat16*>(a.dk) + (row0 * a.H + hq) * DK + kr, (int64_t)a.H * DK, cs, cm.len, g, t);
     } else if (GROUPED) {
       // this head's dq and dk in fp32, token-major, over the dead tiles
