@@ -138,6 +138,12 @@ class ShortConvolution(nn.Conv1d):
         if B * T == N:   # decoding: one token per sequence, the cache (created when absent) is updated in place
             if cache is None:
                 cache = x.new_zeros(N, self.hidden_size, self.kernel_size[0])
+            elif T == 1 and x.is_cuda and cu_seqlens is None and self.activation in ('silu', 'swish'):
+                # nothing that causal_conv1d would check: a step of three of these costs the host more than the device
+                params = self._parameters
+                y, cache = _lib.host().conv(x, params['weight'], params['bias'], residual, cache, True, True, True,
+                                           tables_for(B, 1, None, None, x.device).native())
+                return y, (cache if output_final_state else None)
             y, cache = causal_conv1d(x, self.weight, self.bias, residual, cache, True, self.activation, cu_seqlens=cu_seqlens,
                                      inplace_state=True)
             return y, (cache if output_final_state else None)
@@ -180,5 +186,8 @@ class FusedRMSNormGated(nn.Module):
         self.register_parameter('bias', None)
 
     def forward(self, x, g, residual=None, prenorm=False, residual_in_fp32=False):
-        return rms_norm_gated(x, g, self.weight, self.bias, self.activation, residual=residual, eps=self.eps,
+        params = self._parameters
+        if x.is_cuda and residual is None and not prenorm:
+            return _lib.host().norm_gate(x, g, params['weight'], params['bias'], self.activation == 'sigmoid', self.eps)
+        return rms_norm_gated(x, g, params['weight'], params['bias'], self.activation, residual=residual, eps=self.eps,
                               prenorm=prenorm, residual_in_fp32=residual_in_fp32)

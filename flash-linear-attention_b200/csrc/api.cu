@@ -317,9 +317,9 @@ static int check_norm_gate_args(const b200gdn_norm_gate_args* a, const char* who
   if (a->D != 64 && a->D != 128 && a->D != 256 && a->D != 512)
     return set_error(B200GDN_ERR_UNSUPPORTED, "%s: D=%d (64, 128, 256 and 512 are built)", who, a->D);
   if (a->dtype < 0 || a->dtype > 2) return set_error(B200GDN_ERR_BAD_ARGUMENT, "%s: dtype code %d", who, a->dtype);
-  REQUIRE(a->x, who); REQUIRE(a->g, who); REQUIRE(a->rstd, who);
-  if (!bwd) { REQUIRE(a->y, who); }
-  else { REQUIRE(a->dy, who); REQUIRE(a->dx, who); REQUIRE(a->dg, who); REQUIRE(a->partials, who); }
+  REQUIRE(a->x, who); REQUIRE(a->g, who);
+  if (!bwd) { REQUIRE(a->y, who); }   // rstd may be NULL where no backward pass follows
+  else { REQUIRE(a->rstd, who); REQUIRE(a->dy, who); REQUIRE(a->dx, who); REQUIRE(a->dg, who); REQUIRE(a->partials, who); }
   return 0;
 }
 

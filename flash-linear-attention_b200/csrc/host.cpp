@@ -646,7 +646,8 @@ struct NormForward {
   int32_t param_dtype = 0;
 };
 
-NormForward norm_forward(const Tensor& x, const Tensor& g, const Tensor& weight, const Tensor& bias, bool sigmoid, double eps) {
+NormForward norm_forward(const Tensor& x, const Tensor& g, const Tensor& weight, const Tensor& bias, bool sigmoid, double eps,
+                         bool need_grad) {
   NormForward r;
   const at::Device dev = x.device();
   c10::cuda::CUDAGuard guard(dev);
@@ -659,7 +660,7 @@ NormForward norm_forward(const Tensor& x, const Tensor& g, const Tensor& weight,
   if (weight.defined() || bias.defined()) r.param_dtype = gate_types(r.w, r.b);
   const int64_t D = x.size(-1), rows = x.numel() / D;
   r.y = new_tensor(r.x.sizes(), t, dev);
-  r.rstd = new_tensor({rows}, at::kFloat, dev);
+  if (need_grad) r.rstd = new_tensor({rows}, at::kFloat, dev);
   b200gdn_norm_gate_args a{};
   a.D = (int32_t)D;
   a.rows = rows;
@@ -681,7 +682,7 @@ class NormFunction : public torch::autograd::Function<NormFunction> {
  public:
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& g, const std::optional<Tensor>& weight,
                         const std::optional<Tensor>& bias, bool sigmoid, double eps) {
-    NormForward r = norm_forward(x, g, val(weight), val(bias), sigmoid, eps);
+    NormForward r = norm_forward(x, g, val(weight), val(bias), sigmoid, eps, true);
     ctx->save_for_backward({r.x, r.g, r.w, r.b, r.rstd});
     auto ty = [](const Tensor& z) { return (int64_t)(z.defined() ? z.scalar_type() : at::kFloat); };
     ctx->saved_data["s"] = std::vector<int64_t>{sigmoid, r.param_dtype, ty(g), ty(val(weight)), ty(val(bias))};
@@ -879,7 +880,7 @@ PyObject* py_norm_gate(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   Tensor y;
   {
     NoGil nogil;
-    y = wants_grad({&x, &g, &w, &b}) ? NormFunction::apply(x, g, opt(w), opt(b), sigmoid, eps) : norm_forward(x, g, w, b, sigmoid, eps).y;
+    y = wants_grad({&x, &g, &w, &b}) ? NormFunction::apply(x, g, opt(w), opt(b), sigmoid, eps) : norm_forward(x, g, w, b, sigmoid, eps, false).y;
   }
   return wrap(y);
   END_HANDLE_TH_ERRORS

@@ -357,7 +357,7 @@ typedef struct b200gdn_norm_gate_args {
   const void* weight;            /* [D] or NULL, element type param_dtype */
   const void* bias;              /* [D] or NULL, element type param_dtype */
   void* y;                       /* [rows, D] (forward) */
-  float* rstd;                   /* [rows]: written by the forward pass, read by the backward pass */
+  float* rstd;                   /* [rows]: written by the forward pass (NULL: not wanted), read by the backward pass */
   const void* dy;
   void* dx;
   void* dg;
