@@ -121,6 +121,7 @@ __global__ void __launch_bounds__(2 * DK, 256 / DK) cp_prefix_kernel(const b200g
   constexpr int NB = DK / 32, RB = NB < 4 ? NB : 4;          // blocks of 32 columns of M; blocks held in registers
   constexpr int XS = DK * CP + (DK / 4) * 4;                 // x rows; four floats of padding after every four rows (banks)
   __shared__ __align__(16) float xs[2][XS];
+  wait_for_predecessor();
   const int V = a.V, hv = blockIdx.y, c0 = blockIdx.x * CP, chain = blockIdx.z;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int mg = lane & 7, r0 = (warp * 4 + (lane >> 3)) * 4;                      // columns 32 b + 4 mg + e of rows r0 .. r0 + 3
@@ -206,7 +207,7 @@ __global__ void __launch_bounds__(2 * DK, 256 / DK) cp_prefix_kernel(const b200g
 
 template <int DK>
 int launch_prefix(const b200gdn_prefix_args& a, cudaStream_t st) {
-  cp_prefix_kernel<DK><<<dim3(a.V / CP, a.HV, a.n_chains), 2 * DK, 0, st>>>(a);
+  launch_overlapped(true, cp_prefix_kernel<DK>, dim3(a.V / CP, a.HV, a.n_chains), 2 * DK, 0, st, a);
   return check_launch("cp_prefix");
 }
 

@@ -176,6 +176,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
   constexpr int NP = DK / 64;   // 64-column panels of a V-wide tile (V = K)
   constexpr int NH = DK / 64;   // 16-row halves of a transposed accumulator per warp
   extern __shared__ unsigned char smem_raw[];
+  wait_for_predecessor();
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   unsigned char *Ks = smem + S::o_k, *Do = smem + S::o_do, *Qs = Do, *Vn = smem + S::o_vn, *dUs = Vn, *H0 = smem + S::o_h0, *dWt = H0;
   unsigned char *H1 = smem + S::o_h1, *Vs = H1, *dAs = H1, *M2s = H1, *Ys = H1 + BT * 128;
@@ -823,14 +824,18 @@ int launch(const b200gdn_chunk_args& a, cudaStream_t st) {
   cfg.blockDim = dim3(NTHREADS);
   cfg.dynamicSmemBytes = S::bytes;
   cfg.stream = st;
-  cudaLaunchAttribute attr;
+  cudaLaunchAttribute attr[2];
+  cfg.attrs = attr;
+  cfg.numAttrs = 0;
+  if (overlaps(a)) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
   if (MODE == kCluster) {
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = 1;
-    attr.val.clusterDim.y = a.HV / a.H;
-    attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs].val.clusterDim.x = 1;
+    attr[cfg.numAttrs].val.clusterDim.y = a.HV / a.H;
+    attr[cfg.numAttrs++].val.clusterDim.z = 1;
   }
   cudaLaunchKernelEx(&cfg, bwd_local_kernel<DK, MODE>, a, m);
   if (int e = check_launch("bwd_local")) return e;

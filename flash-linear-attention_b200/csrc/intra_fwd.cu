@@ -148,6 +148,7 @@ __global__ void __launch_bounds__(NTHREADS, 4) intra_fwd_kernel(const b200gdn_ch
   using S = IntraSmem<DK, DV>;
   constexpr int KB = DK / 64, VB = DV / 64;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
+  wait_for_predecessor();
   unsigned char* smem = smem_raw;
   if ((tc5::smem_addr(smem) & 1023u) != 0) {   // the swizzled tiles need it; never seen, but never silently wrong either
     if (threadIdx.x == 0) atomicExch(&g_intra_timeout, 2);
@@ -491,7 +492,7 @@ int launch(const b200gdn_chunk_args& a, cudaStream_t st) {
   if (a.q) rc |= tma::encode_bf16_panels(&m.q, a.q, a.rows, pk, pk, BT, DK / 64); else m.q = m.k;
   if (rc != 0) return set_error(B200GDN_ERR_CUDA, "intra_fwd: cuTensorMapEncodeTiled failed (%d)", rc);
   dim3 grid(a.n_chunks, a.HV);
-  intra_fwd_kernel<DK, DV><<<grid, NTHREADS, S::bytes, st>>>(a, m, resident_ctas(intra_fwd_kernel<DK, DV>, NTHREADS, S::bytes));
+  launch_overlapped(overlaps(a), intra_fwd_kernel<DK, DV>, grid, NTHREADS, S::bytes, st, a, m, resident_ctas(intra_fwd_kernel<DK, DV>, NTHREADS, S::bytes));
   return check_launch("intra_fwd");
 }
 

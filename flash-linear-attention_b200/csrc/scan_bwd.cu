@@ -59,6 +59,7 @@ __global__ void __launch_bounds__(NTHREADS)
   using S = ScanBwdSmem<DK, NSTAGE, DVL>;
   constexpr int NH = DK / 64;
   extern __shared__ unsigned char smem_raw[];
+  wait_for_predecessor();
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   float* gam_all = reinterpret_cast<float*>(smem + S::o_gam);
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + S::o_bar);   // K, do, gamma (+ qk | dv_local): what a step needs first
@@ -413,7 +414,7 @@ int launch(const b200gdn_chunk_args& a, cudaStream_t st) {
   if (DVL) rc |= tma::encode_bf16_2d(&m.pq, a.qk, a.rows, (uint64_t)a.HV * BT, (uint64_t)a.HV * BT, BT); else m.pq = dummy;
   if (rc != 0) return set_error(B200GDN_ERR_CUDA, "scan_bwd: cuTensorMapEncodeTiled failed (%d)", rc);
   dim3 grid(DV / BV + (a.cp_dM != nullptr ? DK / BV : 0), a.HV, a.n_seq);
-  scan_bwd_kernel<DK, DV, NSTAGE, DVL><<<grid, NTHREADS, S::bytes, st>>>(a, m);
+  launch_overlapped(overlaps(a), scan_bwd_kernel<DK, DV, NSTAGE, DVL>, grid, NTHREADS, S::bytes, st, a, m);
   return check_launch(DVL ? "scan_dvl_bwd" : "scan_bwd");
 }
 

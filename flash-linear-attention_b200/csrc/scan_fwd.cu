@@ -78,6 +78,7 @@ __global__ void __launch_bounds__(threads_of(OUT), PRE ? 2 : 1)
   using S = ScanFwdSmem<DK, NSTAGE, OUT, PRE>;
   constexpr int NH = DK / 64;   // 16-row halves of the state per epilogue warp
   extern __shared__ unsigned char smem_raw[];
+  wait_for_predecessor();
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   float* gam_all = reinterpret_cast<float*>(smem + S::o_gam);
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + S::o_bar);   // W, U, gamma of a stage (what the step needs first)
@@ -500,7 +501,7 @@ int launch(const b200gdn_chunk_args& a, cudaStream_t st) {
   }
   if (rc != 0) return set_error(B200GDN_ERR_CUDA, "scan_fwd: cuTensorMapEncodeTiled failed (%d)", rc);
   dim3 grid(DV / BV + ((!OUT && a.cp_M != nullptr) ? DK / BV : 0), a.HV, a.n_seq);
-  scan_fwd_kernel<DK, DV, NSTAGE, OUT, PRE><<<grid, threads_of(OUT), S::bytes, st>>>(a, m);
+  launch_overlapped(overlaps(a), scan_fwd_kernel<DK, DV, NSTAGE, OUT, PRE>, grid, threads_of(OUT), S::bytes, st, a, m);
   return check_launch(OUT ? "scan_out_fwd" : "scan_fwd");
 }
 
