@@ -90,9 +90,9 @@ def staged_bytes(R, C, NS):
 # summarised in profiles/ (file and source revision below); a kernel missing here was not captured.  The constant goes
 # stale with every kernel change: refresh it together with the profile.
 NCU_TRAFFIC = {
-    'source': 'profiles/chunk_fwd_bwd_B4_T4096_H16_D128_tcgen05.md',
-    'kernel_sources_commit': 'fa829f3',
-    'bytes': {'intra_fwd': 359.5e6, 'scan_out_fwd': 536.9e6, 'scan_dvl_bwd': 472.7e6, 'bwd_dqk': 650.1e6, 'bwd_wy': 549.8e6},
+    'source': 'profiles/chunk_fwd_bwd_B4_T4096_H16_D128_four_kernels.md',
+    'kernel_sources_commit': 'db95f86',
+    'bytes': {'intra_fwd': 358.8e6, 'scan_out_fwd': 536.1e6, 'scan_dvl_bwd': 469.7e6, 'bwd_local': 891.8e6},
 }
 
 
