@@ -235,3 +235,57 @@ def test_native_host_path_declines_what_it_does_not_serve():
         host.recurrent(q)
     with pytest.raises(ValueError):
         host.chunk(q, q, q, g, g, None, None, None, 1.0, False, 0, object())
+
+
+class _Cuda(torch.Tensor):
+    """A CPU tensor that says it is on the device: what a module hands to the native host path can be looked at here."""
+    is_cuda = True
+
+
+def _reparametrize(module, how):
+    """`module` with its weight held by something else than the module's own parameter."""
+    if how == 'parametrize':
+        class Twice(torch.nn.Module):
+            def forward(self, w):
+                return 2 * w
+        torch.nn.utils.parametrize.register_parametrization(module, 'weight', Twice())
+    elif how == 'prune':
+        torch.nn.utils.prune.l1_unstructured(module, 'weight', amount=0.5)
+    elif how == 'replica':   # what torch.nn.parallel.replicate makes of a module: attributes instead of parameters
+        weight = module._parameters['weight'].detach().clone()
+        module = module._replicate_for_data_parallel()
+        module._parameters.clear()
+        module.weight, module.bias = weight, None
+    return module
+
+
+@pytest.mark.parametrize('how', ['plain', 'parametrize', 'prune', 'replica'])
+@pytest.mark.parametrize('kind', ['norm', 'conv_step'])
+def test_modules_use_the_weight_attribute(kind, how, monkeypatch):
+    """The kernels get what `module.weight` is, also where no registered parameter of that name exists."""
+    import torch.nn.utils.parametrize   # noqa: F401
+    import torch.nn.utils.prune   # noqa: F401
+    from b200gdn import _lib, modules
+    seen = []
+
+    class Host:
+        def norm_gate(self, x, g, weight, bias, sigmoid, eps):
+            seen.append((weight, bias))
+
+        def conv(self, x, weight, bias, *rest):
+            seen.append((weight, bias))
+            return x, None
+
+        def plan(self, *tables):
+            return None
+    monkeypatch.setattr(_lib, 'host', lambda: Host())
+    if kind == 'norm':
+        module = _reparametrize(modules.FusedRMSNormGated(64), how)
+        x = torch.zeros(2, 64).as_subclass(_Cuda)
+        module(x, x)
+    else:
+        module = _reparametrize(modules.ShortConvolution(8, 4), how)
+        x = torch.zeros(1, 1, 8).as_subclass(_Cuda)
+        module(x, cache=torch.zeros(1, 8, 4))
+    (weight, bias), = seen
+    assert bias is None and torch.equal(weight, module.weight)
