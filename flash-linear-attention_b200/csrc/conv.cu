@@ -68,11 +68,9 @@ __device__ __forceinline__ void store_pairs(void* base, int64_t idx, const uint6
 }
 
 // One CTA's share of a tile: `row` is its first token, `len` its token count, `pos` that token's place in its sequence,
-// `last` whether the share ends the sequence, `after` how many tokens of the sequence follow it (capped at 3, the
-// largest overlap needed).
+// `after` how many tokens of the sequence follow it (capped at 3, the largest overlap needed).
 struct Share {
   int n, row, len, pos, after;
-  bool last;
 };
 __device__ __forceinline__ Share load_share(const b200gdn_conv_args& a, int tile, int sub, int tokens) {
   const int4 m = reinterpret_cast<const int4*>(a.tile_meta)[tile];
@@ -84,7 +82,6 @@ __device__ __forceinline__ Share load_share(const b200gdn_conv_args& a, int tile
   s.len = m.z - start < tokens ? m.z - start : tokens;   // <= 0: nothing to do for this CTA
   s.pos = m.w * BT + start;
   const int rest = m.z - start - s.len;                  // tokens of the tile behind this share
-  s.last = m.w == ntiles - 1 && rest <= 0;
   int after = rest;
   if (after < 3 && m.w < ntiles - 1) after += a.tile_meta[4 * (tile + 1) + 2];
   s.after = after < 3 ? (after < 0 ? 0 : after) : 3;
@@ -138,6 +135,26 @@ __global__ void __launch_bounds__(CT, sizeof(T) == 4 ? 5 : 7) conv_fwd_kernel(co
   if (d0 >= a.D) return;
   const Share s = load_share(a, blockIdx.x, blockIdx.z, tokens);
   if (s.len <= 0) return;
+  uint64_t hist[W - 1][C / 2];
+#pragma unroll
+  for (int j = 0; j < W - 1; ++j) input_at<T, W>(a, s.n, s.row - s.pos, s.pos - (W - 1) + j, d0, hist[j]);
+  // The last inputs of a sequence are stored by the CTA of its FIRST share: the cache may be updated in place, and its
+  // entries are read by the threads of that share alone (as the tokens before it, and below where the sequence is shorter
+  // than W), each of which has read what it overwrites.
+  if (a.final_state != nullptr && s.pos == 0) {
+    const int ntiles = a.seq_meta[2 * s.n + 1], length = (ntiles - 1) * BT + a.tile_meta[4 * (blockIdx.x + ntiles - 1) + 2];
+    uint64_t fin[W][C / 2];
+#pragma unroll
+    for (int j = 0; j < W; ++j) input_at<T, W>(a, s.n, s.row, length - W + j, d0, fin[j]);
+#pragma unroll
+    for (int i = 0; i < C / 2; ++i)
+#pragma unroll
+      for (int j = 0; j < W; ++j) {
+        const float2 f = unpack2(fin[j][i]);
+        Io<T>::st(a.final_state, ((int64_t)s.n * a.D + d0 + 2 * i) * W + j, f.x);
+        Io<T>::st(a.final_state, ((int64_t)s.n * a.D + d0 + 2 * i + 1) * W + j, f.y);
+      }
+  }
   const int64_t base = (int64_t)s.row * a.D + d0;
   const T* const x = static_cast<const T*>(a.x) + base;
   T* const y_out = static_cast<T*>(a.y) + base;
@@ -157,9 +174,6 @@ __global__ void __launch_bounds__(CT, sizeof(T) == 4 ? 5 : 7) conv_fwd_kernel(co
   fetch(GRP, buf[1]);
   Taps<W> k;
   k.load(a, d0);
-  uint64_t hist[W - 1][C / 2];
-#pragma unroll
-  for (int j = 0; j < W - 1; ++j) input_at<T, W>(a, s.n, s.row - s.pos, s.pos - (W - 1) + j, d0, hist[j]);
   auto group = [&](int t0, Raw<T> (&r)[GRP], auto full) {
     T* p = y_out + (int64_t)t0 * a.D;
 #pragma unroll
@@ -197,19 +211,6 @@ __global__ void __launch_bounds__(CT, sizeof(T) == 4 ? 5 : 7) conv_fwd_kernel(co
       else if (t < s.len) group(t, buf[h], std::false_type{});
       fetch(t + 2 * GRP, buf[h]);
     }
-  }
-  if (a.final_state != nullptr && s.last) {
-    uint64_t fin[W][C / 2];   // read completely before it is written: the cache may be updated in place
-#pragma unroll
-    for (int j = 0; j < W; ++j) input_at<T, W>(a, s.n, s.row - s.pos, s.pos + s.len - W + j, d0, fin[j]);
-#pragma unroll
-    for (int i = 0; i < C / 2; ++i)
-#pragma unroll
-      for (int j = 0; j < W; ++j) {
-        const float2 f = unpack2(fin[j][i]);
-        Io<T>::st(a.final_state, ((int64_t)s.n * a.D + d0 + 2 * i) * W + j, f.x);
-        Io<T>::st(a.final_state, ((int64_t)s.n * a.D + d0 + 2 * i + 1) * W + j, f.y);
-      }
   }
 }
 

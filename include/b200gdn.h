@@ -326,7 +326,7 @@ typedef struct b200gdn_conv_args {
   const void* residual;          /* [rows, D] or NULL (forward) */
   const void* initial_state;     /* [n_seq, D, W] or NULL */
   void* y;                       /* [rows, D] (forward) */
-  void* final_state;             /* [n_seq, D, W] or NULL (forward) */
+  void* final_state;             /* [n_seq, D, W] or NULL (forward); may alias initial_state for an in-place update */
   /* backward */
   const void* dy;                /* [rows, D] */
   void* dx;                      /* [rows, D] */

@@ -200,3 +200,24 @@ def test_conv_forms_at_group_and_share_edges(act, with_residual, with_bias):
     O.assert_close('y', ref, y.double(), 1e-5)
     for i, (r, t) in enumerate(zip(torch.autograd.grad(ref, leaves, dy.double()), got)):
         O.assert_close(f'grad {i}', r.double(), t.double(), 1e-5)
+
+
+@pytest.mark.parametrize('W', [2, 3, 4])
+@pytest.mark.parametrize('dtype', [torch.bfloat16, torch.float32])
+def test_conv_cache_updated_in_place(W, dtype):
+    """Several tokens per sequence with the final state written over the cache: bit for bit what separate tensors give, for
+    sequences shorter than the kernel, of one share and of several shares and tiles."""
+    from b200gdn.modules import causal_conv1d
+    lens, D = [1, 2, 3, 5, 15, 16, 17, 31, 32, 33, 64, 65, 200], 520
+    cu = torch.tensor([0] + list(np.cumsum(lens)), dtype=torch.int32, device='cuda')
+    gen = torch.Generator(device='cuda').manual_seed(W)
+    rn = lambda *s: torch.randn(*s, device='cuda', generator=gen).to(dtype)   # noqa: E731
+    x, w, cache = rn(1, sum(lens), D), rn(D, W), rn(len(lens), D, W)
+    y, new = causal_conv1d(x, w, initial_state=cache, output_final_state=True, activation='silu', cu_seqlens=cu)
+    want = O.causal_conv1d_ref(x.double().cpu(), w.double().cpu(), None, None, cache.double().cpu(), 'silu', cu.tolist(), True)[1]
+    assert torch.equal(new.double().cpu(), want)   # inputs and cache entries, moved only
+    for _ in range(20):
+        own = cache.clone()
+        y2, new2 = causal_conv1d(x, w, initial_state=own, output_final_state=True, activation='silu', cu_seqlens=cu,
+                                 inplace_state=True)
+        assert new2.data_ptr() == own.data_ptr() and torch.equal(y2, y) and torch.equal(own, new)
