@@ -118,6 +118,7 @@ struct Plan : torch::CustomClassHolder {
   Tensor chunk_meta, seq_meta, seq_order;
   int32_t n_chunks = 0, n_seq = 0;   // n_seq counts pieces under a split
   bool covered = true, split = false;
+  bool empty_seqs = false;           // some sequence has no token
   Tensor chains, pre_fwd, pre_bwd, first_piece, last_piece;
   int32_t n_chains = 0, n_pre = 0;
 };
@@ -556,7 +557,9 @@ ConvForward conv_forward(const Tensor& x, const Tensor& weight, const Tensor& bi
       r.final_state = initial_state;   // the decode step updates the cache in place
       r.in_place = true;
     } else {
-      r.final_state = new_tensor({plan->n_seq, D, s->W}, t, dev);
+      // no tile, and so no thread, visits a sequence without tokens: its cache stays as it is
+      r.final_state = new_tensor({plan->n_seq, D, s->W}, t, dev, plan->empty_seqs && !r.h0.defined());
+      if (plan->empty_seqs && r.h0.defined()) r.final_state.copy_(r.h0);
     }
   }
   b200gdn_conv_args a{};
@@ -611,7 +614,7 @@ class ConvFunction : public torch::autograd::Function<ConvFunction> {
     Tensor dx = new_tensor(x.sizes(), t, dev, !plan.covered);
     Tensor dw = new_tensor(s.w_sizes, pt, dev), db, dh0;
     if (b.defined()) db = new_tensor({D}, pt, dev);
-    if (h0.defined()) dh0 = new_tensor({plan.n_seq, D, s.W}, t, dev);
+    if (h0.defined()) dh0 = new_tensor({plan.n_seq, D, s.W}, t, dev, plan.empty_seqs);   // zero where no tile visits
     const Tensor partials = new_tensor({2 * tiles * D * (s.W + 1)}, at::kFloat, dev);
     b200gdn_conv_args a{};
     a.rows = (int32_t)(x.size(0) * x.size(1));
@@ -886,21 +889,23 @@ PyObject* py_norm_gate(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   END_HANDLE_TH_ERRORS
 }
 
-// plan(chunk_meta, seq_meta, n_chunks, n_seq, covered, seq_order or None[, chains, pre_fwd, pre_bwd, first_piece, last_piece, n_chains, n_pre])
+// plan(chunk_meta, seq_meta, n_chunks, n_seq, covered, empty_seqs, seq_order or None
+//      [, chains, pre_fwd, pre_bwd, first_piece, last_piece, n_chains, n_pre])
 PyObject* py_plan(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
-  if (nargs != 6) NEED_ARGS(13);
+  if (nargs != 7) NEED_ARGS(14);
   auto p = c10::make_intrusive<Plan>();
-  bool ok = get(args[0], p->chunk_meta) && get(args[1], p->seq_meta) && get(args[5], p->seq_order);
+  bool ok = get(args[0], p->chunk_meta) && get(args[1], p->seq_meta) && get(args[6], p->seq_order);
   p->n_chunks = (int32_t)PyLong_AsLong(args[2]);
   p->n_seq = (int32_t)PyLong_AsLong(args[3]);
   p->covered = truth(args[4]);
-  if (nargs == 13) {
+  p->empty_seqs = truth(args[5]);
+  if (nargs == 14) {
     p->split = true;
-    ok = ok && get(args[6], p->chains) && get(args[7], p->pre_fwd) && get(args[8], p->pre_bwd) && get(args[9], p->first_piece) &&
-         get(args[10], p->last_piece);
-    p->n_chains = (int32_t)PyLong_AsLong(args[11]);
-    p->n_pre = (int32_t)PyLong_AsLong(args[12]);
+    ok = ok && get(args[7], p->chains) && get(args[8], p->pre_fwd) && get(args[9], p->pre_bwd) && get(args[10], p->first_piece) &&
+         get(args[11], p->last_piece);
+    p->n_chains = (int32_t)PyLong_AsLong(args[12]);
+    p->n_pre = (int32_t)PyLong_AsLong(args[13]);
   }
   if (!ok && !PyErr_Occurred()) PyErr_SetString(PyExc_TypeError, "plan: tensors expected");
   if (PyErr_Occurred()) return nullptr;

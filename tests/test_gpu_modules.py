@@ -221,3 +221,26 @@ def test_conv_cache_updated_in_place(W, dtype):
         y2, new2 = causal_conv1d(x, w, initial_state=own, output_final_state=True, activation='silu', cu_seqlens=cu,
                                  inplace_state=True)
         assert new2.data_ptr() == own.data_ptr() and torch.equal(y2, y) and torch.equal(own, new)
+
+
+@pytest.mark.parametrize('with_cache', [False, True])
+def test_conv_sequences_without_tokens(with_cache):
+    """An empty sequence of a packed batch keeps its cache (zeros without one) as its final state and takes no gradient; the
+    memory that the results come from is filled with NaN first."""
+    from b200gdn.modules import causal_conv1d
+    cu, D, W = [0, 0, 5, 5, 70, 70], 64, 4
+    gen = torch.Generator(device='cuda').manual_seed(3)
+    x, w, c = (torch.randn(*s, device='cuda', generator=gen) for s in ((1, 70, D), (D, W), (5, D, W)))
+    c = c.requires_grad_(True) if with_cache else None
+    want = O.causal_conv1d_ref(x.cpu(), w.cpu(), None, None, c.detach().cpu() if with_cache else None, None, cu, True)[1]
+    torch.cuda.synchronize()
+
+    def poison():
+        del (junk := [torch.full((5, D, W), float('nan'), device='cuda') for _ in range(64)])[:]
+    poison()
+    y, new = causal_conv1d(x, w, initial_state=c, output_final_state=True, cu_seqlens=torch.tensor(cu, device='cuda'))
+    assert torch.equal(new.cpu(), want)
+    if with_cache:
+        poison()
+        dc, = torch.autograd.grad(y.sum(), c)
+        assert torch.isfinite(dc).all() and torch.count_nonzero(dc[[0, 2, 4]]) == 0
