@@ -528,7 +528,7 @@ struct ConvForward {
 };
 
 ConvForward conv_forward(const Tensor& x, const Tensor& weight, const Tensor& bias, const Tensor& residual, const Tensor& initial_state,
-                         bool silu, bool output_final_state, bool inplace_state, const PlanPtr& plan) {
+                         bool silu, bool output_final_state, bool inplace_state, const PlanPtr& plan, bool need_grad) {
   ConvForward r;
   const at::Device dev = x.device();
   c10::cuda::CUDAGuard guard(dev);
@@ -580,7 +580,10 @@ ConvForward conv_forward(const Tensor& x, const Tensor& weight, const Tensor& bi
   a.initial_state = ptr(r.h0);
   a.y = ptr(r.y);
   a.final_state = ptr(r.final_state);
+  // the backward pass reads the cache as it was
+  const Tensor before = need_grad && r.in_place ? r.h0.clone() : r.h0;
   call("b200gdn_conv_fwd", b200gdn_conv_fwd, a);
+  r.h0 = before;
   r.saved = std::move(s);
   return r;
 }
@@ -590,7 +593,7 @@ class ConvFunction : public torch::autograd::Function<ConvFunction> {
   static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& weight, const std::optional<Tensor>& bias,
                                const std::optional<Tensor>& residual, const std::optional<Tensor>& initial_state, bool silu,
                                bool output_final_state, bool inplace_state, const PlanPtr& plan) {
-    ConvForward r = conv_forward(x, weight, val(bias), val(residual), val(initial_state), silu, output_final_state, inplace_state, plan);
+    ConvForward r = conv_forward(x, weight, val(bias), val(residual), val(initial_state), silu, output_final_state, inplace_state, plan, true);
     ctx->save_for_backward({r.x, r.w, r.b, r.h0});
     ctx->saved_data["s"] = at::IValue::make_capsule(r.saved);
     ctx->set_materialize_grads(false);
@@ -858,7 +861,7 @@ PyObject* py_conv(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
       y = out[0];
       if (out.size() > 1) fin = out[1];
     } else {
-      ConvForward r = conv_forward(x, w, b, res, h0, silu, out_state, inplace, plan);
+      ConvForward r = conv_forward(x, w, b, res, h0, silu, out_state, inplace, plan, false);
       if (r.in_place && !r.final_state.is_inference()) torch::autograd::impl::bump_version(r.final_state);
       y = r.y;
       fin = r.final_state;

@@ -244,3 +244,18 @@ def test_conv_sequences_without_tokens(with_cache):
         poison()
         dc, = torch.autograd.grad(y.sum(), c)
         assert torch.isfinite(dc).all() and torch.count_nonzero(dc[[0, 2, 4]]) == 0
+
+
+@pytest.mark.parametrize('lens', [[1, 1, 1], [1, 2, 20]])
+def test_conv_gradients_with_the_cache_updated_in_place(lens):
+    """The backward pass of a call that overwrote its cache uses the cache that the forward pass read."""
+    from b200gdn.modules import causal_conv1d
+    cu = torch.tensor([0] + list(np.cumsum(lens)), dtype=torch.int32, device='cuda')
+    gen = torch.Generator(device='cuda').manual_seed(8)
+    rn = lambda *s: torch.randn(*s, device='cuda', generator=gen)   # noqa: E731
+    x, w, c, dy = rn(1, sum(lens), 64).requires_grad_(True), rn(64, 4).requires_grad_(True), rn(3, 64, 4), rn(1, sum(lens), 64)
+    want = torch.autograd.grad(causal_conv1d(x, w, initial_state=c, output_final_state=True, activation='silu', cu_seqlens=cu)[0],
+                               (x, w), dy)
+    y, _ = causal_conv1d(x, w, initial_state=c.clone(), output_final_state=True, activation='silu', cu_seqlens=cu,
+                         inplace_state=True)
+    assert all(torch.equal(a, b) for a, b in zip(want, torch.autograd.grad(y, (x, w), dy)))
