@@ -59,6 +59,15 @@ def device_tables(bounds, device) -> Tables:
     return out
 
 
+def packed_bounds(cu_seqlens: torch.Tensor, cu_seqlens_cpu: Optional[torch.Tensor], rows: int):
+    """(start, end) of every sequence of a packed batch, none of them outside its ``rows`` token rows.  Costs one
+    device-to-host copy without ``cu_seqlens_cpu``."""
+    cu = (cu_seqlens_cpu if cu_seqlens_cpu is not None else cu_seqlens.cpu()).to(torch.int64).tolist()
+    if cu and (cu[0] < 0 or cu[-1] > rows):
+        raise ValueError(f'cu_seqlens [{cu[0]}, {cu[-1]}] reaches outside the {rows} token rows')
+    return list(zip(cu[:-1], cu[1:]))
+
+
 def tables_for(B: int, T: int, cu_seqlens: Optional[torch.Tensor], cu_seqlens_cpu: Optional[torch.Tensor],
                device: torch.device) -> Tables:
     """Device tables for a dense [B,T] batch or a packed batch; memoised by shape / by the identity of
@@ -75,11 +84,7 @@ def tables_for(B: int, T: int, cu_seqlens: Optional[torch.Tensor], cu_seqlens_cp
         hit = _cache.get(key)
         if hit is not None and hit[1] is cu_seqlens:
             return hit[0]
-        cpu = cu_seqlens_cpu if cu_seqlens_cpu is not None else cu_seqlens.cpu()
-        cu = cpu.to(torch.int64).tolist()
-        bounds = [(cu[i], cu[i + 1]) for i in range(len(cu) - 1)]
-        if cu and (cu[0] < 0 or cu[-1] > B * T):
-            raise ValueError(f'cu_seqlens [{cu[0]}, {cu[-1]}] reaches outside the {B * T} token rows')
+        bounds = packed_bounds(cu_seqlens, cu_seqlens_cpu, B * T)
     out = device_tables(bounds, device)
     out.covered = bool(bounds) and bounds[0][0] == 0 and bounds[-1][1] == B * T
     if len(_cache) > 64:
@@ -196,9 +201,7 @@ def split_plan_for(B: int, T: int, cu_seqlens, cu_seqlens_cpu, device, HV: int, 
         hit = _split_cache.get(key)
         if hit is not None and hit[1] is cu_seqlens:
             return hit[0]
-        cpu = cu_seqlens_cpu if cu_seqlens_cpu is not None else cu_seqlens.cpu()
-        cu = cpu.to(torch.int64).tolist()
-        bounds = [(cu[i], cu[i + 1]) for i in range(len(cu) - 1)]
+        bounds = packed_bounds(cu_seqlens, cu_seqlens_cpu, B * T)
     plan = split_plan(bounds, HV, slices, device, B * T)
     if len(_split_cache) > 64:
         _split_cache.clear()

@@ -259,6 +259,16 @@ def _reparametrize(module, how):
     return module
 
 
+@pytest.mark.parametrize('cu', [[0, 6400], [-64, 6336], [0, 64, 8000]])
+@pytest.mark.parametrize('heads', [1, 64])
+def test_sequences_outside_the_token_rows_are_refused(cu, heads):
+    """By the planner too, which sees them first where a sequence is worth cutting (one head) and where none is."""
+    from b200gdn.index import native_plan, piece_counts
+    assert (max(piece_counts([100], heads, 2)) > 1) == (heads == 1)
+    with pytest.raises(ValueError, match='reaches outside the 6336 token rows'):
+        native_plan(1, 6336, torch.tensor(cu), None, torch.device('cpu'), heads, 2)
+
+
 @pytest.mark.parametrize('how', ['plain', 'parametrize', 'prune', 'replica'])
 @pytest.mark.parametrize('kind', ['norm', 'conv_step'])
 def test_modules_use_the_weight_attribute(kind, how, monkeypatch):
