@@ -59,6 +59,12 @@ def device_tables(bounds, device) -> Tables:
     return out
 
 
+def content_version(cu_seqlens: torch.Tensor):
+    """Changes when the tensor is written in place, so that tables of its old contents are not used for the new ones
+    (a tensor made under inference_mode keeps no such count: there the caller passes another tensor)."""
+    return None if cu_seqlens.is_inference() else cu_seqlens._version
+
+
 def packed_bounds(cu_seqlens: torch.Tensor, cu_seqlens_cpu: Optional[torch.Tensor], rows: int):
     """(start, end) of every sequence of a packed batch, none of them outside its ``rows`` token rows.  Costs one
     device-to-host copy without ``cu_seqlens_cpu``."""
@@ -70,9 +76,10 @@ def packed_bounds(cu_seqlens: torch.Tensor, cu_seqlens_cpu: Optional[torch.Tenso
 
 def tables_for(B: int, T: int, cu_seqlens: Optional[torch.Tensor], cu_seqlens_cpu: Optional[torch.Tensor],
                device: torch.device) -> Tables:
-    """Device tables for a dense [B,T] batch or a packed batch; memoised by shape / by the identity of
-    ``cu_seqlens`` (the reference memoises its index tensors the same way, fla/utils/_decorators.py:33-80).
+    """Device tables for a dense [B,T] batch or a packed batch; memoised by shape / by the identity and version of
+    ``cu_seqlens`` (the reference memoises its index tensors by identity, fla/utils/_decorators.py:33-80).
     A packed batch without ``cu_seqlens_cpu`` costs one device-to-host copy on first use."""
+    version = None if cu_seqlens is None else content_version(cu_seqlens)
     if cu_seqlens is None:
         key = ('dense', B, T, device)
         hit = _cache.get(key)
@@ -82,14 +89,14 @@ def tables_for(B: int, T: int, cu_seqlens: Optional[torch.Tensor], cu_seqlens_cp
     else:
         key = ('varlen', id(cu_seqlens), B * T, device)
         hit = _cache.get(key)
-        if hit is not None and hit[1] is cu_seqlens:
+        if hit is not None and hit[1] is cu_seqlens and hit[2] == version:
             return hit[0]
         bounds = packed_bounds(cu_seqlens, cu_seqlens_cpu, B * T)
     out = device_tables(bounds, device)
     out.covered = bool(bounds) and bounds[0][0] == 0 and bounds[-1][1] == B * T
     if len(_cache) > 64:
         _cache.clear()
-    _cache[key] = (out, cu_seqlens)
+    _cache[key] = (out, cu_seqlens, version)
     return out
 
 
@@ -189,7 +196,8 @@ def split_plan(bounds, HV: int, slices: int, device, rows: int) -> Optional[Spli
 
 
 def split_plan_for(B: int, T: int, cu_seqlens, cu_seqlens_cpu, device, HV: int, slices: int) -> Optional[SplitPlan]:
-    """Memoised like tables_for (by shape, or by the identity of ``cu_seqlens``)."""
+    """Memoised like tables_for (by shape, or by the identity and version of ``cu_seqlens``)."""
+    version = None if cu_seqlens is None else content_version(cu_seqlens)
     if cu_seqlens is None:
         key = ('dense', B, T, HV, slices, FORCE_PIECES, device)
         hit = _split_cache.get(key)
@@ -199,13 +207,13 @@ def split_plan_for(B: int, T: int, cu_seqlens, cu_seqlens_cpu, device, HV: int, 
     else:
         key = ('varlen', id(cu_seqlens), B * T, HV, slices, FORCE_PIECES, device)
         hit = _split_cache.get(key)
-        if hit is not None and hit[1] is cu_seqlens:
+        if hit is not None and hit[1] is cu_seqlens and hit[2] == version:
             return hit[0]
         bounds = packed_bounds(cu_seqlens, cu_seqlens_cpu, B * T)
     plan = split_plan(bounds, HV, slices, device, B * T)
     if len(_split_cache) > 64:
         _split_cache.clear()
-    _split_cache[key] = (plan, cu_seqlens)
+    _split_cache[key] = (plan, cu_seqlens, version)
     return plan
 
 

@@ -269,6 +269,22 @@ def test_sequences_outside_the_token_rows_are_refused(cu, heads):
         native_plan(1, 6336, torch.tensor(cu), None, torch.device('cpu'), heads, 2)
 
 
+def test_tables_follow_cu_seqlens_written_in_place():
+    """A tensor of sequence bounds that is reused for the next batch gives that batch's tables and cuts."""
+    from b200gdn.index import split_plan_for, tables_for
+    dev, cu = torch.device('cpu'), torch.tensor([0, 3200, 6400])
+
+    def seen():
+        return (tables_for(1, 6400, cu, None, dev)[0][:, 2].tolist(), split_plan_for(1, 6400, cu, None, dev, 1, 2).tables[0].tolist())
+    first = seen()
+    assert seen() == first and tables_for(1, 6400, cu, None, dev) is tables_for(1, 6400, cu, None, dev)
+    cu[1] = 100
+    second = seen()
+    assert second[0] == [64, 36] + [64] * 98 + [28] and second[1] != first[1]
+    cu = cu.clone()
+    assert seen() == second
+
+
 @pytest.mark.parametrize('how', ['plain', 'parametrize', 'prune', 'replica'])
 @pytest.mark.parametrize('kind', ['norm', 'conv_step'])
 def test_modules_use_the_weight_attribute(kind, how, monkeypatch):
