@@ -90,10 +90,12 @@ int gate_types(Tensor& g, Tensor& beta) {
   beta = dense(beta);
   return code;
 }
+// whether the call has to go through its autograd node: for gradients, and for forward-mode tangents, which no node here
+// serves and which it therefore refuses (without it they would be dropped in silence)
 bool wants_grad(std::initializer_list<const Tensor*> xs) {
-  if (!at::GradMode::is_enabled()) return false;
+  const bool reverse = at::GradMode::is_enabled(), forward = c10::AutogradState::get_tls_state().get_fw_grad_mode();
   for (const Tensor* x : xs)
-    if (x->defined() && x->requires_grad()) return true;
+    if (x->defined() && ((reverse && x->requires_grad()) || (forward && x->_fw_grad(0).defined()))) return true;
   return false;
 }
 // autograd's apply() takes an absent tensor as an empty optional
