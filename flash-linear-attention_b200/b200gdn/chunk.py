@@ -13,6 +13,7 @@ import torch
 
 from . import _lib
 from .index import native_plan
+from .recorded import RecordedCall, tracing
 
 _SUPPORTED_HEAD_DIMS = ((64, 64), (128, 128))
 
@@ -192,6 +193,11 @@ def prefix_chains(plan, M, h, x0, out, K, V, reverse: bool, stream: int, last=No
     _lib.call('b200gdn_cp_prefix', a, stream)
 
 
+def _native_chunk(q, k, v, g, beta, initial_state, A_log, dt_bias, scale, output_final_state, options, cu_seqlens, cu_seqlens_cpu):
+    plan = native_plan(q.shape[0], q.shape[1], cu_seqlens, cu_seqlens_cpu, q.device, v.shape[2], v.shape[3] // 64)
+    return _lib.host().chunk(q, k, v, g, beta, initial_state, A_log, dt_bias, scale, output_final_state, options, plan)
+
+
 def chunk_gated_delta_rule(
     q: torch.Tensor,
     k: torch.Tensor,
@@ -304,9 +310,9 @@ def chunk_gated_delta_rule(
     # layout by the scans themselves.
     if not use_gate_in_kernel:
         A_log = dt_bias = None
-    plan = native_plan(B, T, cu_seqlens, cu_seqlens_cpu, q.device, HV, V // 64)
-    return _lib.host().chunk(q, k, v, g, beta, initial_state, A_log, dt_bias, scale, output_final_state,
-                             flags | (_lib.STATE_V_FIRST if state_v_first else 0), plan)
+    args = (q, k, v, g, beta, initial_state, A_log, dt_bias, scale, output_final_state,
+            flags | (_lib.STATE_V_FIRST if state_v_first else 0), cu_seqlens, cu_seqlens_cpu)
+    return RecordedCall.apply(_native_chunk, *args) if tracing() else _native_chunk(*args)
 
 
 chunk_gdn = chunk_gated_delta_rule

@@ -8,10 +8,12 @@ from typing import Optional
 import torch
 
 from . import _lib
+from .recorded import seen_by_trace, tracing
+
 
 class FusedRecurrentFunction(torch.autograd.Function):
-    """The node of a call whose inputs ask for gradients: the forward pass runs, the backward pass says that it does not
-    exist (as in the reference, fla/ops/gated_delta_rule/fused_recurrent.py:299-306)."""
+    """The node of a call whose inputs ask for gradients, or that a trace records: the forward pass runs, the backward pass
+    says that it does not exist (as in the reference, fla/ops/gated_delta_rule/fused_recurrent.py:299-306)."""
 
     @staticmethod
     def forward(ctx, q, k, v, g, beta, A_log, dt_bias, scale, initial_state, output_final_state, flags, cu_seqlens,
@@ -22,7 +24,8 @@ class FusedRecurrentFunction(torch.autograd.Function):
             raise _lib.B200GDNError('fused_recurrent_gated_delta_rule: tensors of unexpected shapes or devices')
         if out[1] is not None and out[1] is initial_state:
             ctx.mark_dirty(initial_state)   # updated in place and returned
-        return out
+            return out
+        return seen_by_trace(out)
 
     @staticmethod
     def backward(ctx, do, dht):
@@ -79,12 +82,13 @@ def fused_recurrent_gated_delta_rule(
     flags = ((_lib.REC_L2NORM if use_qk_l2norm_in_kernel else 0) | (_lib.REC_GATE if use_gate_in_kernel else 0)
              | (_lib.REC_BETA_SIGMOID if use_beta_sigmoid_in_kernel else 0) | (_lib.REC_NEG_EIGVAL if allow_neg_eigval else 0)
              | (_lib.REC_STATE_V_FIRST if state_v_first else 0))
-    if gk is None and gv is None:
+    if gk is None and gv is None and not tracing():
         out = (_lib._host or _lib.host()).recurrent(q, k, v, g, beta, A_log, dt_bias, scale, initial_state, output_final_state,
                                                     flags, cu_seqlens, inplace_state, state_indices)
         if out is not NotImplemented:
             return out
-    # not served by the direct call: say what is wrong, or record the node that has no backward pass
+    # not served by the direct call: say what is wrong, or record the node that has no backward pass (as a trace does, which
+    # sees nothing of a native call)
     if gk is not None or gv is not None:
         raise NotImplementedError('per-dimension decays gk / gv are not part of the gated delta rule path')
     if cu_seqlens is not None:

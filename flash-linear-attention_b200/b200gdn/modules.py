@@ -20,6 +20,7 @@ import torch.nn as nn
 
 from . import _lib
 from .index import tables_for
+from .recorded import RecordedCall, tracing
 
 
 def _param(module: nn.Module, name: str):
@@ -30,10 +31,14 @@ def _param(module: nn.Module, name: str):
     return params[name] if name in params else getattr(module, name)
 
 
-def _conv(x, weight, bias, residual, initial_state, activation, output_final_state, cu_seqlens, cu_seqlens_cpu, inplace_state):
+def _native_conv(x, weight, bias, residual, initial_state, activation, output_final_state, cu_seqlens, cu_seqlens_cpu, inplace_state):
     plan = tables_for(x.shape[0], x.shape[1], cu_seqlens, cu_seqlens_cpu, x.device).native()
     return _lib.host().conv(x, weight, bias, residual, initial_state, activation in ('silu', 'swish'), output_final_state,
                             inplace_state, plan)
+
+
+def _conv(*args):
+    return RecordedCall.apply(_native_conv, *args) if tracing() else _native_conv(*args)
 
 
 class _HaloExchange(torch.autograd.Function):
@@ -146,7 +151,7 @@ class ShortConvolution(nn.Conv1d):
         if B * T == N:   # decoding: one token per sequence, the cache (created when absent) is updated in place
             if cache is None:
                 cache = x.new_zeros(N, self.hidden_size, self.kernel_size[0])
-            elif T == 1 and x.is_cuda and cu_seqlens is None and self.activation in ('silu', 'swish'):
+            elif T == 1 and x.is_cuda and cu_seqlens is None and self.activation in ('silu', 'swish') and not tracing():
                 # nothing that causal_conv1d would check: a step of three of these costs the host more than the device
                 y, cache = _lib.host().conv(x, _param(self, 'weight'), _param(self, 'bias'), residual, cache, True, True, True,
                                            tables_for(B, 1, None, None, x.device).native())
@@ -173,7 +178,8 @@ def rms_norm_gated(x, g, weight, bias=None, activation: str = 'swish', residual=
         raise NotImplementedError('rms_norm_gated: the residual / prenorm form is not built (the layer does not use it)')
     if not x.is_cuda:
         raise _lib.B200GDNError('rms_norm_gated runs on a CUDA device only (no CPU path)')
-    return _lib.host().norm_gate(x, g, weight, bias, activation == 'sigmoid', eps)
+    args = (x, g, weight, bias, activation == 'sigmoid', eps)
+    return RecordedCall.apply(_lib.host().norm_gate, *args) if tracing() else _lib.host().norm_gate(*args)
 
 
 class FusedRMSNormGated(nn.Module):
@@ -194,7 +200,7 @@ class FusedRMSNormGated(nn.Module):
 
     def forward(self, x, g, residual=None, prenorm=False, residual_in_fp32=False):
         weight, bias = _param(self, 'weight'), _param(self, 'bias')
-        if x.is_cuda and residual is None and not prenorm:
+        if x.is_cuda and residual is None and not prenorm and not tracing():
             return _lib.host().norm_gate(x, g, weight, bias, self.activation == 'sigmoid', self.eps)
         return rms_norm_gated(x, g, weight, bias, self.activation, residual=residual, eps=self.eps,
                               prenorm=prenorm, residual_in_fp32=residual_in_fp32)

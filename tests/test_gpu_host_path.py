@@ -42,3 +42,35 @@ def test_forward_mode_tangents_are_refused(name, grad):
         with pytest.raises((NotImplementedError, RuntimeError), match='jvp'):
             call(fw.make_dual(first, torch.ones_like(first)), *rest)
         call(first, *rest)
+
+
+@pytest.mark.parametrize('grad', [False, True])
+@pytest.mark.parametrize('name', [n for n in NAMES if n != 'conv_step'])
+def test_a_trace_replays_the_operator(name, grad):
+    """torch.jit.trace keeps a call as an operation: other inputs, of another length too, give what the call gives."""
+    call, inputs = _operators()[name]
+
+    class Call(torch.nn.Module):   # the modules' weights belong to the traced module
+        def __init__(self):
+            super().__init__()
+            self.op = next((c.cell_contents for c in call.__closure__ or () if isinstance(c.cell_contents, torch.nn.Module)), None)
+
+        def forward(self, *args):
+            return call(*args)
+    with torch.set_grad_enabled(grad):
+        traced = torch.jit.trace(Call(), tuple(x.requires_grad_(grad) for x in inputs(70, 0)), check_trace=False)
+        for tokens in (70, 90):
+            args = [x.requires_grad_(grad) for x in inputs(tokens, 1)]
+            want, got = ([y] if torch.is_tensor(y) else list(y) for y in (call(*args), traced(*args)))
+            assert all(torch.equal(a, b) for a, b in zip(want, got)) and len(want) == len(got)
+            if grad and name != 'recurrent':
+                dy = torch.ones_like(want[0])
+                for a, b in zip(torch.autograd.grad(want[0], args, dy), torch.autograd.grad(got[0], args, dy)):
+                    assert torch.equal(a, b)
+
+
+def test_a_state_updated_in_place_is_not_recorded():
+    from b200gdn.modules import causal_conv1d
+    x, w, cache = (torch.ones(*s, device='cuda') for s in ((3, 1, 64), (64, 4), (3, 64, 4)))
+    with pytest.raises(RuntimeError, match='cannot be recorded'):
+        torch.jit.trace(lambda *a: causal_conv1d(*a, initial_state=cache, output_final_state=True, inplace_state=True), (x, w))
