@@ -661,6 +661,7 @@ NormForward norm_forward(const Tensor& x, const Tensor& g, const Tensor& weight,
   c10::cuda::CUDAGuard guard(dev);
   const at::ScalarType t = x.scalar_type();
   if (act_code(t) < 0) raise(std::string("rms_norm_gated: dtype ") + c10::toString(t) + " is not supported");
+  if (x.size(-1) == 0) raise("rms_norm_gated: rows without elements");
   r.x = dense(x);
   r.g = dense(g, t);
   r.w = weight;
@@ -854,6 +855,7 @@ PyObject* py_conv(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     return nullptr;
   }
   const bool silu = truth(args[5]), out_state = truth(args[6]), inplace = truth(args[7]);
+  if (PyErr_Occurred()) return nullptr;
   const PlanPtr plan = plan_of(args[8]);
   Tensor y, fin;
   {

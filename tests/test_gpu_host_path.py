@@ -74,3 +74,14 @@ def test_a_state_updated_in_place_is_not_recorded():
     x, w, cache = (torch.ones(*s, device='cuda') for s in ((3, 1, 64), (64, 4), (3, 64, 4)))
     with pytest.raises(RuntimeError, match='cannot be recorded'):
         torch.jit.trace(lambda *a: causal_conv1d(*a, initial_state=cache, output_final_state=True, inplace_state=True), (x, w))
+
+
+def test_sizes_of_zero_and_unclear_switches_raise():
+    """Mistakes that native code would end the process for, or notice too late."""
+    from b200gdn import B200GDNError
+    from b200gdn.modules import causal_conv1d, rms_norm_gated
+    with pytest.raises(B200GDNError, match='without elements'):
+        rms_norm_gated(torch.zeros(4, 0, device='cuda'), torch.zeros(4, 0, device='cuda'), None)
+    x, w = torch.zeros(1, 4, 64, device='cuda'), torch.zeros(64, 4, device='cuda')
+    with pytest.raises(RuntimeError, match='ambiguous'):
+        causal_conv1d(x, w, output_final_state=torch.ones(2))
