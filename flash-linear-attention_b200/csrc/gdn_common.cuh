@@ -129,25 +129,35 @@ int set_error(int code, const char* fmt, ...);
 int check_launch(const char* what);
 void reset_launch_count();
 
-// Whether this thread has set the attribute for (kernel, device) before: the driver call costs about half a microsecond,
+// The dynamic shared memory limit of a kernel, set once per thread and device: the driver call costs about half a microsecond,
 // which a decoding step would pay on every launch.
-inline bool smem_attr_set_before(const void* kern) {
+struct SmemLimits {
   struct Entry { const void* kern; int dev; };
-  static thread_local Entry seen[64];
-  static thread_local int n = 0;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  for (int i = 0; i < n; ++i)
-    if (seen[i].kern == kern && seen[i].dev == dev) return true;
-  if (n < 64) seen[n++] = Entry{kern, dev};
-  return false;
+  Entry set[64];
+  int n = 0;
+  bool has(const void* kern, int dev) const {
+    for (int i = 0; i < n; ++i)
+      if (set[i].kern == kern && set[i].dev == dev) return true;
+    return false;
+  }
+  void add(const void* kern, int dev) {
+    if (n < 64) set[n++] = Entry{kern, dev};
+  }
+};
+inline SmemLimits& smem_limits() {
+  static thread_local SmemLimits limits;
+  return limits;
 }
 
 template <typename Kern>
 int ensure_smem(Kern kern, size_t bytes) {   // `bytes` is a constant of the kernel's instantiation
-  if (smem_attr_set_before(reinterpret_cast<const void*>(kern))) return 0;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  if (e != cudaSuccess) return set_error(B200GDN_ERR_CUDA, "cudaFuncSetAttribute(%zu B): %s", bytes, cudaGetErrorString(e));
+  int dev = 0;
+  cudaGetDevice(&dev);
+  const void* key = reinterpret_cast<const void*>(kern);
+  if (smem_limits().has(key, dev)) return 0;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess)
+    return set_error(B200GDN_ERR_CUDA, "cudaFuncSetAttribute(%zu B): %s", bytes, cudaGetErrorString(cudaGetLastError()));
+  smem_limits().add(key, dev);
   return 0;
 }
 

@@ -67,6 +67,23 @@ def test_argument_errors_without_gpu():
     assert lib.b200gdn_bwd_workspace_bytes(64, 2, 4, 128, 128, 1) > 0
 
 
+def test_a_failed_kernel_setup_is_reported_every_time():
+    """Without a device the first call that a kernel's setup makes fails; the next attempt says the same and does not go on
+    as if the setup had been done."""
+    import torch
+    from b200gdn import _lib
+    if torch.cuda.is_available():
+        pytest.skip('needs a machine without a device')
+    lib, a = _lib.load(), _lib.ChunkArgs()
+    a.struct_bytes = ctypes.sizeof(a)
+    a.rows, a.H, a.HV, a.K, a.V, a.n_seq, a.n_chunks, a.stage_mask = 64, 1, 1, 128, 128, 1, 1, _lib.FWD_INTRA
+    for name in ('chunk_meta', 'seq_meta', 'k', 'v', 'g', 'beta', 'gamma', 'A', 'w', 'u'):
+        setattr(a, name, 256)   # never followed: nothing is launched
+    for _ in range(3):
+        assert lib.b200gdn_chunk_fwd(ctypes.byref(a), None) == -3
+        assert b'cudaFuncSetAttribute' in lib.b200gdn_last_error()
+
+
 def test_product_does_not_import_oracle():
     """Nothing under the package may import, read or run the oracle."""
     pkg = os.path.join(ROOT, 'flash-linear-attention_b200')
