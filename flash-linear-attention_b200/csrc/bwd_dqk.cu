@@ -479,7 +479,7 @@ int launch(const b200gdn_chunk_args& a, cudaStream_t st) {
   rc |= tma::encode_bf16_2d(&m.dh, a.dh, hrows, DV, DV, DK);
   if (rc != 0) return set_error(B200GDN_ERR_CUDA, "bwd_dqk: cuTensorMapEncodeTiled failed (%d)", rc);
   dim3 grid(a.n_chunks, a.H);
-  bwd_dqk_kernel<DK, DV, GROUPED><<<grid, NTHREADS, S::bytes, st>>>(a, m, resident_ctas(bwd_dqk_kernel<DK, DV, GROUPED>, NTHREADS, S::bytes));
+  bwd_dqk_kernel<DK, DV, GROUPED><<<grid, NTHREADS, S::bytes, st>>>(a, m, resident_ctas<bwd_dqk_kernel<DK, DV, GROUPED>>(NTHREADS, S::bytes));
   return check_launch("bwd_dqk");
 }
 

@@ -172,7 +172,7 @@ int launch(const b200gdn_chunk_args& a, cudaStream_t st) {
   rc |= tma::encode_bf16_panels(&m.dv2, a.dv2, a.rows, pv, pv, BT, DV / 64);
   if (rc != 0) return set_error(B200GDN_ERR_CUDA, "dv_local: cuTensorMapEncodeTiled failed (%d)", rc);
   dim3 grid(a.n_chunks, a.HV);
-  dv_local_kernel<DK, DV><<<grid, NTHREADS, S::bytes, st>>>(a, m, resident_ctas(dv_local_kernel<DK, DV>, NTHREADS, S::bytes));
+  dv_local_kernel<DK, DV><<<grid, NTHREADS, S::bytes, st>>>(a, m, resident_ctas<dv_local_kernel<DK, DV>>(NTHREADS, S::bytes));
   return check_launch("dv_local");
 }
 

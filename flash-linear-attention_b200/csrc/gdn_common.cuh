@@ -7,6 +7,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "../../include/b200gdn.h"
 
 namespace gdn {
@@ -181,17 +183,18 @@ void launch_overlapped(bool overlap, void (*kern)(P...), dim3 grid, int threads,
   cudaLaunchKernelEx(&cfg, kern, P(args)...);
 }
 
-// CTAs of `kern` resident on the whole device at once (SMs x CTAs per SM); cached per instantiation and device.
-template <typename Kern>
-int resident_ctas(Kern kern, int threads, size_t smem) {
-  static int cached[64] = {0};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev >= 0 && dev < 64 && cached[dev] > 0) return cached[dev];
-  int per_sm = 1, sms = 148;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem) != cudaSuccess || per_sm < 1) per_sm = 1;
-  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) sms = 148;
-  if (dev >= 0 && dev < 64) cached[dev] = per_sm * sms;
-  return per_sm * sms;
+// CTAs of a kernel resident on the whole device at once (SMs x CTAs per SM); looked up once per kernel and device.
+template <auto KERN>
+int resident_ctas(int threads, size_t smem) {
+  static std::atomic<int> known[64];
+  int dev = 0, per_sm = 1, sms = 148;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = -1;
+  const int hit = dev >= 0 ? known[dev].load(std::memory_order_relaxed) : 0;
+  if (hit > 0) return hit;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, KERN, threads, smem) != cudaSuccess || per_sm < 1) per_sm = 1;
+  if (dev < 0 || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) sms = 148;
+  const int ctas = per_sm * sms;
+  if (dev >= 0) known[dev].store(ctas, std::memory_order_relaxed);
+  return ctas;
 }
 }  // namespace gdn

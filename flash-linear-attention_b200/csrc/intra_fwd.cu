@@ -492,7 +492,7 @@ int launch(const b200gdn_chunk_args& a, cudaStream_t st) {
   if (a.q) rc |= tma::encode_bf16_panels(&m.q, a.q, a.rows, pk, pk, BT, DK / 64); else m.q = m.k;
   if (rc != 0) return set_error(B200GDN_ERR_CUDA, "intra_fwd: cuTensorMapEncodeTiled failed (%d)", rc);
   dim3 grid(a.n_chunks, a.HV);
-  launch_overlapped(overlaps(a), intra_fwd_kernel<DK, DV>, grid, NTHREADS, S::bytes, st, a, m, resident_ctas(intra_fwd_kernel<DK, DV>, NTHREADS, S::bytes));
+  launch_overlapped(overlaps(a), intra_fwd_kernel<DK, DV>, grid, NTHREADS, S::bytes, st, a, m, resident_ctas<intra_fwd_kernel<DK, DV>>(NTHREADS, S::bytes));
   return check_launch("intra_fwd");
 }
 

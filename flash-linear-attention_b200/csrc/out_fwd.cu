@@ -224,7 +224,7 @@ int launch(const b200gdn_chunk_args& a, cudaStream_t st) {
   rc |= tma::encode_bf16_panels(&m.o, a.o, a.rows, pv, pv, BT, DV / 64);
   if (rc != 0) return set_error(B200GDN_ERR_CUDA, "out_fwd: cuTensorMapEncodeTiled failed (%d)", rc);
   dim3 grid(a.n_chunks, a.HV);
-  out_fwd_kernel<DK, DV><<<grid, NTHREADS, S::bytes, st>>>(a, m, resident_ctas(out_fwd_kernel<DK, DV>, NTHREADS, S::bytes));
+  out_fwd_kernel<DK, DV><<<grid, NTHREADS, S::bytes, st>>>(a, m, resident_ctas<out_fwd_kernel<DK, DV>>(NTHREADS, S::bytes));
   return check_launch("out_fwd");
 }
 
