@@ -107,7 +107,6 @@ def tables_for(B: int, T: int, cu_seqlens: Optional[torch.Tensor], cu_seqlens_cp
 # its affine map, a prefix chain turns the maps into the start state of every piece, and the regular scan then runs
 # over all pieces at once.  Pieces are whole numbers of chunks, so the chunking (and every chunk-local kernel) is
 # unchanged.
-SM_COUNT = 148
 FORCE_PIECES = None          # tests: cut every sequence into (up to) this many pieces regardless of the heuristic
 _split_cache: dict = {}
 
@@ -126,7 +125,11 @@ class SplitPlan:
         return self._native
 
 
-def piece_counts(chunks_per_seq, HV: int, slices: int):
+def sm_count(device) -> int:
+    return torch.cuda.get_device_properties(device).multi_processor_count if device.type == 'cuda' else 148
+
+
+def piece_counts(chunks_per_seq, HV: int, slices: int, sms: int = 148):
     """How many pieces each sequence is cut into (equal pieces, so the longest sequences into the most): the cut with the
     least time by the model below, in microseconds as measured on a B200 with heads of 128 and 64; none unless it saves
     a twentieth.  A scan CTA takes `step` per chunk and the pre-scan, which runs beside twice as many transition-matrix
@@ -137,19 +140,19 @@ def piece_counts(chunks_per_seq, HV: int, slices: int):
     uncut = [1] * len(chunks_per_seq)
     lens = [int(c) for c in chunks_per_seq if c > 0]
     per_seq = max(1, slices * HV)                    # scan CTAs of a piece
-    if not lens or per_seq * (len(lens) + 2) > SM_COUNT:
+    if not lens or per_seq * (len(lens) + 2) > sms:
         return uncut
     longest, step, chain = max(lens), 1.27 if slices > 1 else 1.06, 1.5 if slices > 1 else 0.65
-    if 8 * slices * HV * len(lens) > SM_COUNT:       # the chains' CTAs, eight columns each, share SMs
+    if 8 * slices * HV * len(lens) > sms:       # the chains' CTAs, eight columns each, share SMs
         chain *= 1.8
     best, length = 0.95 * (3.5 + step * longest), None
-    for pieces in range(3, min(longest, SM_COUNT // per_seq - len(lens) + 1) + 1):
+    for pieces in range(3, min(longest, sms // per_seq - len(lens) + 1) + 1):
         n = -(-longest // pieces)
         total = sum(-(-c // n) for c in lens)
         pre = (total - len(lens)) * 2 * per_seq      # pre-scan CTAs
-        if total * per_seq > SM_COUNT:
+        if total * per_seq > sms:
             continue
-        rounds = (-(-pre // SM_COUNT) - (-pre // (2 * SM_COUNT))) / 2
+        rounds = (-(-pre // sms) - (-pre // (2 * sms))) / 2
         cost = 12. + step * n * (1 + 0.92 * rounds) + chain * (-(-longest // n) - 1)
         if cost < best:
             best, length = cost, n
@@ -160,7 +163,7 @@ def split_plan(bounds, HV: int, slices: int, device, rows: int) -> Optional[Spli
     """None when no sequence is worth cutting; otherwise the plan (device tensors) for these bounds."""
     bounds = [(int(s), int(e)) for s, e in bounds]
     chunks = [(e - s + CHUNK - 1) // CHUNK for s, e in bounds]
-    pieces = piece_counts(chunks, HV, slices)
+    pieces = piece_counts(chunks, HV, slices, sm_count(device))
     if max(pieces, default=1) <= 1:
         return None
     vbounds, chains, pre_fwd, pre_bwd, first_piece, last_piece = [], [], [], [], [], []

@@ -847,7 +847,7 @@ int launch(const b200gdn_chunk_args& a, cudaStream_t st) {
 // against 242 at B4 T4096 8/16 heads of 128), but has G times as many CTAs, so it stays where turns would leave
 // the device to a few: two fit on an SM, and the rounds of CTAs decide.  Both add the heads in the same order and precision.
 bool in_turns(const b200gdn_chunk_args& a) {
-  constexpr int64_t slots = 2 * 148;
+  const int64_t slots = 2 * sm_count();
   const int64_t G = a.HV / a.H, turns = G * ((a.n_chunks * (int64_t)a.H + slots - 1) / slots),
                 cluster = (a.n_chunks * (int64_t)a.HV + slots - 1) / slots;
   return 4 * turns <= 5 * cluster;

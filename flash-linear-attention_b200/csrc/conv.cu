@@ -455,7 +455,7 @@ __global__ void __launch_bounds__(32 * RW) conv_param_reduce_kernel(const b200gd
 int share_tokens(const b200gdn_conv_args& a, int least) {
   int64_t warps = (int64_t)a.n_tiles * ((a.D / C + 31) / 32);
   int tokens = 64;
-  for (; tokens > least && warps < 148 * 12; warps *= 2) tokens /= 2;
+  for (; tokens > least && warps < 12 * sm_count(); warps *= 2) tokens /= 2;
   return tokens;
 }
 

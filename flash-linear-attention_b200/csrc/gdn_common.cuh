@@ -183,17 +183,27 @@ void launch_overlapped(bool overlap, void (*kern)(P...), dim3 grid, int threads,
   cudaLaunchKernelEx(&cfg, kern, P(args)...);
 }
 
+// Streaming multiprocessors of the current device (148 where there is none to ask), looked up once per device.
+inline int sm_count() {
+  static std::atomic<int> known[64];
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = -1;
+  if (dev >= 0 && (sms = known[dev].load(std::memory_order_relaxed)) > 0) return sms;
+  if (dev < 0 || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) return 148;
+  known[dev].store(sms, std::memory_order_relaxed);
+  return sms;
+}
+
 // CTAs of a kernel resident on the whole device at once (SMs x CTAs per SM); looked up once per kernel and device.
 template <auto KERN>
 int resident_ctas(int threads, size_t smem) {
   static std::atomic<int> known[64];
-  int dev = 0, per_sm = 1, sms = 148;
+  int dev = 0, per_sm = 1;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = -1;
   const int hit = dev >= 0 ? known[dev].load(std::memory_order_relaxed) : 0;
   if (hit > 0) return hit;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, KERN, threads, smem) != cudaSuccess || per_sm < 1) per_sm = 1;
-  if (dev < 0 || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) sms = 148;
-  const int ctas = per_sm * sms;
+  const int ctas = per_sm * sm_count();
   if (dev >= 0) known[dev].store(ctas, std::memory_order_relaxed);
   return ctas;
 }

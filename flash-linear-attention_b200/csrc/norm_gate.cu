@@ -329,14 +329,14 @@ int launch_d(const b200gdn_norm_gate_args& a, cudaStream_t st, bool bwd, int n_c
 
 // CTAs of the backward kernel for a row count (one partial row each): as many as fit on the device at once
 int norm_gate_grid(int64_t rows) {
-  const int64_t want = (rows + NT / 32 - 1) / (NT / 32), most = BWD_CTAS * 148;
+  const int64_t want = (rows + NT / 32 - 1) / (NT / 32), most = BWD_CTAS * sm_count();
   return (int)(want < 1 ? 1 : (want > most ? most : want));
 }
 
 int launch_norm_gate(const b200gdn_norm_gate_args& a, cudaStream_t st, bool bwd) {
   int n = norm_gate_grid(a.rows);
   if (!bwd) {
-    const int64_t want = (a.rows + NT / 32 - 1) / (NT / 32), most = FWD_CTAS * 148;
+    const int64_t want = (a.rows + NT / 32 - 1) / (NT / 32), most = FWD_CTAS * sm_count();
     n = (int)(want < 1 ? 1 : (want > most ? most : want));
   }
   return a.dtype == 0 ? launch_d<__nv_bfloat16>(a, st, bwd, n) : a.dtype == 1 ? launch_d<__half>(a, st, bwd, n) : launch_d<float>(a, st, bwd, n);

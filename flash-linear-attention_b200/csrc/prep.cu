@@ -198,8 +198,8 @@ template <typename T>
 int launch_vec(const b200gdn_prep_args& a, cudaStream_t st, bool bwd) {
   if (!bwd) {
     const int64_t n = (int64_t)a.rows * a.HV;
-    const int64_t want = (n + 255) / 256;
-    const int blocks = (int)(want < 148 * 8 ? want : 148 * 8);
+    const int64_t want = (n + 255) / 256, most = 8 * sm_count();
+    const int blocks = (int)(want < most ? want : most);
     gate_beta_fwd_kernel<T><<<blocks, 256, 0, st>>>(a);
     return check_launch("gate_beta_fwd");
   }

@@ -634,10 +634,7 @@ int launch(const b200gdn_recurrent_args& a, cudaStream_t st) {
     if (!(a.flags & B200GDN_REC_STATE_V_FIRST) && (a.V == 64 || a.V == 128) && a.T == 1 && a.cu_seqlens == nullptr &&
         a.h0 != nullptr && a.ht != nullptr && (int64_t)a.n_seq * a.HV * DK * a.V >= kStreamElements &&
         (reinterpret_cast<uintptr_t>(a.h0) & 15) == 0 && (reinterpret_cast<uintptr_t>(a.ht) & 15) == 0) {
-      int dev = 0, sms = 148;
-      cudaGetDevice(&dev);
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-      const int n_items = a.n_seq * a.HV;
+      const int n_items = a.n_seq * a.HV, sms = sm_count();
       auto stream = [&](auto* kernel, size_t bytes) -> int {
         if (int e = ensure_smem(kernel, bytes)) return e;
         kernel<<<n_items < sms ? n_items : sms, kStreamThreads, bytes, st>>>(a, n_items);

@@ -269,6 +269,17 @@ def test_sequences_outside_the_token_rows_are_refused(cu, heads):
         native_plan(1, 6336, torch.tensor(cu), None, torch.device('cpu'), heads, 2)
 
 
+@pytest.mark.parametrize('sms', [74, 148, 160])
+def test_pieces_fit_the_device(sms):
+    """The scans of all pieces run at once on the SMs that the device has."""
+    from b200gdn.index import piece_counts
+    for chunks in ([512], [3000], [400, 100, 700], [64] * 4):
+        for heads in (1, 2, 4, 8, 16):
+            pieces = piece_counts(chunks, heads, 2, sms)
+            assert max(pieces) == 1 or sum(pieces) * heads * 2 <= sms
+    assert sum(piece_counts([3000], 2, 2, 74)) < sum(piece_counts([3000], 2, 2, 148)) < sum(piece_counts([3000], 2, 2, 160))
+
+
 def test_tables_follow_cu_seqlens_written_in_place():
     """A tensor of sequence bounds that is reused for the next batch gives that batch's tables and cuts."""
     from b200gdn.index import split_plan_for, tables_for
