@@ -313,13 +313,9 @@ class ChunkGatedDeltaRuleCPFunction(torch.autograd.Function):
             rows = B * T
             dob = do.to(torch.bfloat16).contiguous()
             bf16, f32 = torch.bfloat16, torch.float32
-            grouped = HV > H
-            dq, dk, dv, dg, dbeta, dh, dv2, dG, dk_part, dq_acc = carve(
+            dq, dk, dv, dg, dbeta, dh, dv2 = carve(
                 dev, zero, ((B, T, H, K), bf16), ((B, T, H, K), bf16), ((B, T, HV, V), bf16), ((B, T, HV), f32), ((B, T, HV), f32),
-                ((n_chunks, HV, K, V), bf16), ((rows, HV, V), bf16), ((rows, HV), f32),
-                ((rows, H, K) if grouped else (0,), f32), ((rows, H, K) if grouped else (0,), f32))
-            if not grouped:
-                dk_part = dq_acc = None
+                ((n_chunks, HV, K, V), bf16), ((rows, HV, V), bf16))
             st = _stream(qb)
             tables = (chunk_meta, seq_meta, (n_chunks, n_seq))
 
@@ -363,8 +359,7 @@ class ChunkGatedDeltaRuleCPFunction(torch.autograd.Function):
             a.beta, a.gamma, a.A, a.qk, a.w, a.h, a.v_new = (x.data_ptr() for x in (bf, gamma, A, qk, w, h, v_new))
             a.d_o, a.dht = dob.data_ptr(), _lib.ptr(dht)
             a.dq, a.dk, a.dv, a.dg, a.dbeta = dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), dg.data_ptr(), dbeta.data_ptr()
-            a.dh, a.dv2, a.dk_part, a.dG, a.dq_acc = dh.data_ptr(), dv2.data_ptr(), \
-                _lib.ptr(dk_part), dG.data_ptr(), _lib.ptr(dq_acc)
+            a.dh, a.dv2 = dh.data_ptr(), dv2.data_ptr()
             a.stage_mask = 0
             with _Phase('bwd_main', dev):
                 _lib.call('b200gdn_chunk_bwd', a, st)

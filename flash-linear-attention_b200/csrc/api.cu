@@ -129,7 +129,7 @@ int b200gdn_chunk_bwd(const b200gdn_chunk_args* a, void* stream) {
       if (int e = launch_scan_bwd(*a, st)) return e;
     }
   }
-  if ((m & B200GDN_BWD_DQKWG) && (m & B200GDN_BWD_WY) && bwd_local_serves(*a)) {
+  if ((m & B200GDN_BWD_DQKWG) && (m & B200GDN_BWD_WY)) {
     // both chunk-local stages in one kernel: neither the chunk-local part of dk nor dG leaves the chip
     REQUIRE(a->q, "chunk_bwd"); REQUIRE(a->k, "chunk_bwd"); REQUIRE(a->v, "chunk_bwd"); REQUIRE(a->v_new, "chunk_bwd");
     REQUIRE(a->beta, "chunk_bwd"); REQUIRE(a->gamma, "chunk_bwd"); REQUIRE(a->A, "chunk_bwd"); REQUIRE(a->h, "chunk_bwd");
@@ -228,8 +228,8 @@ int64_t b200gdn_bwd_workspace_bytes(int32_t rows, int32_t H, int32_t HV, int32_t
   int64_t r = rows, hv = HV;
   return (int64_t)n_chunks * hv * K * V * 2 /* dh */
          + r * hv * V * 2                    /* dv2 */
-         + r * hv * 4                        /* dG */
-         + (HV > H ? 2 * r * H * K * 4 : 0); /* dq_acc, dk_part: fp32 sums over a group of value heads */
+         + r * hv * 4                        /* dG (single stages) */
+         + (HV > H ? 2 * r * H * K * 4 : 0); /* dq_acc, dk_part (single stages): fp32 sums over a group of value heads */
 }
 
 static int check_prep_args(const b200gdn_prep_args* a, const char* who, bool bwd) {

@@ -12,6 +12,8 @@
 // eight warps (warps w and w+4 share TMEM quadrant w&3 and split the columns).  h and dh are streamed in
 // 64-column panels through one buffer pair, which keeps the CTA at ~106 KiB of shared memory, so two CTAs
 // per SM overlap each other's phases.
+//
+// Runs where B200GDN_BWD_DQKWG is asked for by itself; with B200GDN_BWD_WY, and so in a whole pass, bwd_local_kernel does both.
 #include "tc5_tile.cuh"
 #include "tma.cuh"
 

@@ -845,10 +845,15 @@ int launch(const b200gdn_chunk_args& a, cudaStream_t st) {
 // Several value heads per q/k head: in turn in one CTA, or a CTA each and the sums of dq and dk through a cluster.  A cluster
 // costs about a quarter more per head (it holds its CTAs until the slowest has arrived and its sums have been read: 272 us
 // against 242 at B4 T4096 8/16 heads of 128), but has G times as many CTAs, so it stays where turns would leave
-// the device to a few: two fit on an SM, and the rounds of CTAs decide.  Both add the heads in the same order and precision.
+// the device to a few: two fit on an SM, and the rounds of CTAs decide.  Group sizes other than two, four
+// and eight are taken in turns always (the two kernels of the single stages, which such groups used where there are few chunks, also
+// take heads in turn: 1 x 2048 tokens, 2/12 heads of 128: 122 us, 90 here; 1/3 heads of 64: 34, 32).  Both forms add the heads
+// in the same order and precision.
 bool in_turns(const b200gdn_chunk_args& a) {
   const int64_t slots = 2 * sm_count();
-  const int64_t G = a.HV / a.H, turns = G * ((a.n_chunks * (int64_t)a.H + slots - 1) / slots),
+  const int64_t G = a.HV / a.H;
+  if (G != 2 && G != 4 && G != 8) return true;
+  const int64_t turns = G * ((a.n_chunks * (int64_t)a.H + slots - 1) / slots),
                 cluster = (a.n_chunks * (int64_t)a.HV + slots - 1) / slots;
   return 4 * turns <= 5 * cluster;
 }
@@ -861,15 +866,11 @@ int launch_heads(const b200gdn_chunk_args& a, cudaStream_t st) {
 
 }  // namespace
 
-// (group sizes beyond those that are legal cluster sizes are served in turns only)
-bool bwd_local_serves(const b200gdn_chunk_args& a) {
-  const int G = a.HV / a.H;
-  return a.K == a.V && (a.K == 64 || a.K == 128) && (G == 1 || G == 2 || G == 4 || G == 8 || in_turns(a));
-}
-
 int launch_bwd_local(const b200gdn_chunk_args& a, cudaStream_t st) {
   if (int e = check_gate_args(a, "bwd_local")) return e;
-  return a.K == 128 ? launch_heads<128>(a, st) : launch_heads<64>(a, st);
+  if (a.K == 128 && a.V == 128) return launch_heads<128>(a, st);
+  if (a.K == 64 && a.V == 64) return launch_heads<64>(a, st);
+  return set_error(B200GDN_ERR_UNSUPPORTED, "bwd_local: K=%d V=%d not built (64/64 and 128/128 are)", a.K, a.V);
 }
 
 // Reads and clears the flag a bounded device wait raises when it expires (synchronises with the device).

@@ -18,6 +18,8 @@
 // CUDA-core work on 64-row tiles, so they are spread over eight warps (warps w and w+4 share TMEM
 // quadrant w&3 and split the columns); all tiles arrive by TMA issued from one thread.  256 TMEM columns
 // and ~100 KiB of shared memory: two CTAs per SM overlap each other's phases.
+//
+// Runs where B200GDN_BWD_WY is asked for by itself; with B200GDN_BWD_DQKWG, and so in a whole pass, bwd_local_kernel does both.
 #include "tc5_tile.cuh"
 #include "tma.cuh"
 

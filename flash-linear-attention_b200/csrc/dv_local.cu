@@ -4,6 +4,8 @@
 // value head) on tcgen05 tensor cores: TMA brings Q, K, do and gamma; P = Q K^T in TMEM; the masked, gated
 // and scaled P goes to shared memory as bf16 and is used transposed (MN-major) for dv = P^T do; the result
 // leaves through one TMA store into the dv2 buffer, which the reverse scan then completes in place.
+//
+// Runs where B200GDN_BWD_DVLOCAL is asked for without B200GDN_BWD_SCAN; in a whole pass the reverse scan forms it.
 #include "tc5_tile.cuh"
 #include "tma.cuh"
 

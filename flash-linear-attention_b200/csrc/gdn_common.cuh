@@ -107,7 +107,6 @@ int launch_scan_dvl_bwd(const b200gdn_chunk_args& a, cudaStream_t st);
 int launch_bwd_dqk(const b200gdn_chunk_args& a, cudaStream_t st);
 int launch_bwd_wy(const b200gdn_chunk_args& a, cudaStream_t st);
 int launch_bwd_local(const b200gdn_chunk_args& a, cudaStream_t st);
-bool bwd_local_serves(const b200gdn_chunk_args& a);
 int launch_gate_reduce(const b200gdn_chunk_args& a, cudaStream_t st);
 int check_gate_args(const b200gdn_chunk_args& a, const char* who);
 int launch_recurrent(const b200gdn_recurrent_args& a, cudaStream_t st);

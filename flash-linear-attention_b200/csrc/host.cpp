@@ -421,9 +421,7 @@ class ChunkFunction : public torch::autograd::Function<ChunkFunction> {
     c10::cuda::CUDAGuard guard(dev);
     const bool zero = !plan.covered, gate = s.options & B200GDN_PREP_GATE;
     b200gdn_chunk_args a = chunk_args(q, k, v, s.scale, plan);
-    const int64_t rows = a.rows, H = a.H, HV = a.HV, K = a.K, V = a.V, C = a.n_chunks, N = a.n_seq;
-    const int64_t G = HV / H;
-    const bool grouped = G > 1 && G != 2 && G != 4 && G != 8;   // group sums through HBM (other sizes stay on the chip)
+    const int64_t rows = a.rows, HV = a.HV, K = a.K, V = a.V, C = a.n_chunks, N = a.n_seq;
     const Tensor d_o = grads[0].defined() ? dense(grads[0], at::kBFloat16) : new_tensor(v.sizes(), at::kBFloat16, dev, true);
     Tensor dht = grads.size() > 1 ? dense(grads[1], at::kFloat) : Tensor();
     if (s.transpose_states && dht.defined()) dht = dht.transpose(-1, -2).contiguous();
@@ -440,8 +438,7 @@ class ChunkFunction : public torch::autograd::Function<ChunkFunction> {
       if (dt_bias.defined()) ddt_bias = new_tensor({HV}, at::kFloat, dev);
     }
     Slab slots;
-    const int64_t o_dh = slots.add(C * HV * K * V * 2), o_dv2 = slots.add(rows * HV * V * 2), o_dG = slots.add(rows * HV * 4);
-    const int64_t o_dkp = slots.add(grouped ? rows * H * K * 4 : 0), o_dqa = slots.add(grouped ? rows * H * K * 4 : 0);
+    const int64_t o_dh = slots.add(C * HV * K * V * 2), o_dv2 = slots.add(rows * HV * V * 2);
     const int64_t o_gp = slots.add(gate ? C * HV * 2 * 4 : 0);
     const Tensor ws = slots.make(dev, zero);
     a.options = s.options;
@@ -465,9 +462,6 @@ class ChunkFunction : public torch::autograd::Function<ChunkFunction> {
     a.dh0 = fptr(dh0);
     a.dh = piece(ws, o_dh);
     a.dv2 = piece(ws, o_dv2);
-    a.dG = static_cast<float*>(piece(ws, o_dG));
-    a.dk_part = static_cast<float*>(piece(ws, o_dkp));
-    a.dq_acc = static_cast<float*>(piece(ws, o_dqa));
     if (gate) {
       a.g = ptr(g);
       a.A_log = fptr(A_log);

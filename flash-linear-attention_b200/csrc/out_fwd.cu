@@ -7,6 +7,8 @@
 //   phase 1b: O = Q h;        epilogue: O rows scaled by 2^gamma_i in place (tcgen05.ld / tcgen05.st);
 //   phase 2 : O += P v_new;   epilogue: scale, bf16, one TMA store (plain predicated stores for a ragged chunk).
 // 128 TMEM columns and ~73 KiB of shared memory per CTA: three CTAs per SM hide each other's latencies.
+//
+// Runs where B200GDN_FWD_OUT is asked for without B200GDN_FWD_SCAN; in a whole pass the scan forms the output.
 #include "tc5_tile.cuh"
 #include "tma.cuh"
 

@@ -108,6 +108,7 @@ typedef struct b200gdn_chunk_args {
   void* dh;                      /* bf16 [n_chunks,HV,K,V] */
   void* dv2;                     /* bf16 [rows,HV,V] */
   void* dw;                      /* unused (dw = -dv2 h^T stays on chip); may be NULL */
+  /* only for B200GDN_BWD_DQKWG and B200GDN_BWD_WY in calls of their own (together they are one kernel): */
   float* dk_part;                /* [rows,H,K], only read/written when HV > H (fp32 sum over a group's heads) */
   float* dG;                     /* [rows,HV] */
   float* dq_acc;                 /* [rows,H,K], only read/written when HV > H */
@@ -370,7 +371,8 @@ int b200gdn_norm_gate_fwd(const b200gdn_norm_gate_args* args, void* stream);
 int b200gdn_norm_gate_bwd(const b200gdn_norm_gate_args* args, void* stream);
 int b200gdn_norm_gate_ctas(int64_t rows);
 
-/* Bytes of forward-saved tensors and of backward workspace for a problem (what the caller allocates). */
+/* Bytes of forward-saved tensors and of backward workspace for a problem (what the caller allocates; the latter with what
+ * single stages of the backward pass need). */
 int64_t b200gdn_saved_bytes(int32_t rows, int32_t H, int32_t HV, int32_t K, int32_t V, int32_t n_chunks);
 int64_t b200gdn_bwd_workspace_bytes(int32_t rows, int32_t H, int32_t HV, int32_t K, int32_t V, int32_t n_chunks);
 

@@ -631,12 +631,12 @@ def test_trailing_empty_sequence():
     b200gdn.device_status()
 
 
-@pytest.mark.parametrize('K,H,HV,more', [(64, 2, 2, 0), (64, 1, 8, 0), (128, 1, 3, 0), (128, 2, 4, 0), (128, 2, 8, 0), (128, 1, 8, 0),
+@pytest.mark.parametrize('K,H,HV,more', [(64, 2, 2, 0), (64, 1, 8, 0), (64, 2, 12, 0), (128, 1, 3, 0), (128, 1, 16, 0), (128, 2, 4, 0), (128, 2, 8, 0), (128, 1, 8, 0),
                                          (64, 1, 3, 280), (128, 2, 4, 140), (128, 1, 3, 280)])
 def test_chunk_local_backward_by_group_size(K, H, HV, more):
-    """Up to eight value heads per key head sum their dq and dk in a cluster, any number in turn where there are many
-    chunks (here `more` sequences of one token), other group sizes take the separate kernels; sequences of one token up
-    to one past a tile, with and without the layer's options."""
+    """Two, four or eight value heads per key head sum their dq and dk in a cluster, any number in turn where there are many
+    chunks (here `more` sequences of one token), other group sizes in turn always; sequences of one token up to one past a
+    tile, with and without the layer's options."""
     cu = [0, 1, 64, 129, 192, 255, 300] + [301 + i for i in range(more)]
     d = O.make_inputs(1, cu[-1], H, HV, K, K, seed=17, cu_seqlens=cu)
     bf = {n: d[n].to(torch.bfloat16) for n in ('q', 'k', 'v', 'do')}
