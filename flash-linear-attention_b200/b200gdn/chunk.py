@@ -163,26 +163,6 @@ def carve(dev, zero, *specs):
     return out
 
 
-class Slab:
-    """One device allocation cut into pieces that are only ever handed to the kernels as addresses: ``nbytes`` per piece
-    (0 = no such piece, address 0), every piece on a 256-byte boundary.  Unlike ``carve`` it builds no tensor view per
-    piece (three torch calls each), which is most of what an allocation-heavy step costs on the host."""
-    __slots__ = ('buf', 'offs')
-
-    def __init__(self, dev, zero, nbytes):
-        offs, total = [], 0
-        for n in nbytes:
-            offs.append(total if n > 0 else -1)
-            total += (int(n) + 255) // 256 * 256
-        self.offs = offs
-        self.buf = (torch.zeros if zero else torch.empty)(max(total, 256), dtype=torch.uint8, device=dev)
-
-    @staticmethod
-    def addresses(buf, offs):
-        base = buf.data_ptr()
-        return [base + o if o >= 0 else 0 for o in offs]
-
-
 def prefix_chains(plan, M, h, x0, out, K, V, reverse: bool, stream: int, last=None, identity: bool = False) -> None:
     """b200gdn_cp_prefix over the chains of a split plan: the start state (reverse: the end gradient) of every piece."""
     a = _lib.PrefixArgs()

@@ -111,7 +111,8 @@ struct Slab {
     total += (bytes + 255) / 256 * 256;
     return off;
   }
-  Tensor make(const at::Device& dev, bool zero) const { return new_tensor({total > 256 ? total : 256}, at::kByte, dev, zero); }
+  int64_t bytes() const { return total > 256 ? total : 256; }   // never an empty allocation
+  Tensor make(const at::Device& dev, bool zero) const { return new_tensor({bytes()}, at::kByte, dev, zero); }
 };
 void* piece(const Tensor& buf, int64_t off) { return off < 0 ? nullptr : static_cast<char*>(buf.data_ptr()) + off; }
 
@@ -916,6 +917,18 @@ PyObject* py_plan(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   END_HANDLE_TH_ERRORS
 }
 
+// slab(bytes, bytes, ...) -> (bytes in all, offset, offset, ...): where the pieces of a workspace lie (-1: no such piece)
+PyObject* py_slab(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  Slab slab;
+  PyObject* r = PyTuple_New(nargs + 1);
+  if (r == nullptr) return nullptr;
+  for (Py_ssize_t i = 0; i < nargs; ++i) PyTuple_SET_ITEM(r, i + 1, PyLong_FromLongLong(slab.add(PyLong_AsLongLong(args[i]))));
+  PyTuple_SET_ITEM(r, 0, PyLong_FromLongLong(slab.bytes()));
+  if (!PyErr_Occurred()) return r;
+  Py_DECREF(r);
+  return nullptr;
+}
+
 PyObject* py_launch_count(PyObject*, PyObject*) { return PyLong_FromLongLong(g_launches.load(std::memory_order_relaxed)); }
 
 PyObject* py_set_error_class(PyObject*, PyObject* cls) {
@@ -931,6 +944,7 @@ PyMethodDef methods[] = {
     {"conv", FAST(py_conv), "short causal convolution, differentiable"},
     {"norm_gate", FAST(py_norm_gate), "gated RMS norm, differentiable"},
     {"plan", FAST(py_plan), "chunk tables (and split plan) of a shape as one handle"},
+    {"slab", FAST(py_slab), "layout of a workspace"},
     {"launch_count", py_launch_count, METH_NOARGS, "kernels enqueued through this module"},
     {"set_error_class", py_set_error_class, METH_O, "class raised when a library call fails"},
     {nullptr, nullptr, 0, nullptr}};

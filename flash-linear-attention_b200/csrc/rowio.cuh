@@ -79,37 +79,6 @@ __device__ __forceinline__ void store8(void* base, int64_t idx, const float (&x)
   }
 }
 
-// the same for C = 4 or 8 consecutive elements
-template <typename T, int C>
-__device__ __forceinline__ void load_c(const void* base, int64_t idx, float (&x)[C]) {
-  static_assert(C == 4 || C == 8, "four or eight elements");
-  if constexpr (C == 8) {
-    load8<T>(base, idx, x);
-  } else if constexpr (sizeof(T) == 2) {
-    const uint2 u = *reinterpret_cast<const uint2*>(static_cast<const T*>(base) + idx);
-    float y[8];
-    unpack8<T>(make_uint4(u.x, u.y, 0u, 0u), y);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) x[i] = y[i];
-  } else {
-    const float4 a = *reinterpret_cast<const float4*>(static_cast<const float*>(base) + idx);
-    x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w;
-  }
-}
-template <typename T, int C>
-__device__ __forceinline__ void store_c(void* base, int64_t idx, const float (&x)[C]) {
-  static_assert(C == 4 || C == 8, "four or eight elements");
-  if constexpr (C == 8) {
-    store8<T>(base, idx, x);
-  } else if constexpr (sizeof(T) == 2) {
-    const float y[8] = {x[0], x[1], x[2], x[3], 0.f, 0.f, 0.f, 0.f};
-    const uint4 u = pack8<T>(y);
-    *reinterpret_cast<uint2*>(static_cast<T*>(base) + idx) = make_uint2(u.x, u.y);
-  } else {
-    *reinterpret_cast<float4*>(static_cast<float*>(base) + idx) = make_float4(x[0], x[1], x[2], x[3]);
-  }
-}
-
 // ---- two fp32 operations in one instruction (channel or row pairs; each half rounds like the scalar instruction) ------
 __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
   uint64_t d;
@@ -158,15 +127,8 @@ __device__ __forceinline__ uint32_t narrow2(uint64_t v) {
   }
 }
 
-// sigmoid with two MUFU instructions (ex2.approx.ftz, rcp.approx.ftz: about 2 ulp each; the library forms of exp and
-// division add range handling that costs more instructions than the rest of an element's work in these kernels)
-__device__ __forceinline__ float fast_sigmoid(float x) {
-  float e, r;
-  asm("ex2.approx.ftz.f32 %0, %1;\n" : "=f"(e) : "f"(x * -1.4426950408889634f));
-  asm("rcp.approx.ftz.f32 %0, %1;\n" : "=f"(r) : "f"(1.f + e));
-  return r;
-}
-// the same for a pair
+// sigmoids of a pair with two MUFU instructions each (ex2.approx.ftz, rcp.approx.ftz: about 2 ulp each; the library forms of
+// exp and division add range handling that costs more instructions than the rest of an element's work in these kernels)
 __device__ __forceinline__ uint64_t fast_sigmoid2(uint64_t x) {
   const float2 z = unpack2(mul2(x, pack2(-1.4426950408889634f, -1.4426950408889634f)));
   float2 e, r;

@@ -204,23 +204,21 @@ def test_install_and_uninstall_against_the_reference_registry():
 
 def test_slab_hands_out_aligned_addresses_and_null_for_absent_pieces():
     """The step's workspace is one allocation known to the host only as addresses: every piece on a 256-byte boundary,
-    pieces of zero bytes get the null address, pieces do not overlap, and the addresses can be rebuilt from the saved
-    tensor and offsets (what the backward pass does)."""
-    import torch
-    from b200gdn.chunk import Slab
+    pieces of zero bytes get none (a null address), pieces do not overlap, and the offsets depend on the sizes alone (the
+    backward pass rebuilds the addresses from the saved tensor and its offsets)."""
+    from b200gdn import _lib
     sizes = (1000, 0, 256, 77, 0, 4096)
-    slab = Slab(torch.device('cpu'), True, sizes)
-    addr = Slab.addresses(slab.buf, slab.offs)
-    base = slab.buf.data_ptr()
-    assert [a == 0 for a in addr] == [n == 0 for n in sizes]
-    live = [(a - base, n) for a, n in zip(addr, sizes) if n]
+    total, *offs = _lib.host().slab(*sizes)
+    assert [o < 0 for o in offs] == [n == 0 for n in sizes]
+    live = [(o, n) for o, n in zip(offs, sizes) if n]
     assert all(off % 256 == 0 for off, _ in live)
     for (o0, n0), (o1, _) in zip(live, live[1:]):
         assert o0 + n0 <= o1
-    assert live[-1][0] + live[-1][1] <= slab.buf.numel()
-    assert Slab.addresses(slab.buf, list(slab.offs)) == addr
-    assert int(slab.buf.sum()) == 0                      # zero=True fills the allocation
-    assert Slab(torch.device('cpu'), False, (0, 0)).buf.numel() >= 256   # never an empty allocation
+    assert live[-1][0] + live[-1][1] <= total
+    assert _lib.host().slab(*sizes) == (total, *offs)
+    assert _lib.host().slab(0, 0)[0] >= 256   # never an empty allocation
+    with pytest.raises(TypeError):
+        _lib.host().slab('x')
 
 
 def test_native_host_path_declines_what_it_does_not_serve():
