@@ -76,31 +76,6 @@ class AffineArgs(C.Structure):
     ]
 
 
-class ConvArgs(C.Structure):
-    _fields_ = [
-        ('struct_bytes', C.c_int32), ('rows', C.c_int32), ('D', C.c_int32), ('W', C.c_int32),
-        ('n_seq', C.c_int32), ('n_tiles', C.c_int32), ('flags', C.c_uint32), ('dtype', C.c_int32),
-        ('tile_meta', _p), ('seq_meta', _p), ('x', _p), ('weight', _p), ('bias', _p), ('residual', _p),
-        ('initial_state', _p), ('y', _p), ('final_state', _p),
-        ('dy', _p), ('dx', _p), ('dweight', _p), ('dbias', _p), ('dinitial_state', _p), ('partials', _p),
-        ('param_dtype', C.c_int32),
-    ]
-
-
-class NormGateArgs(C.Structure):
-    _fields_ = [
-        ('struct_bytes', C.c_int32), ('D', C.c_int32), ('rows', C.c_int64), ('flags', C.c_uint32),
-        ('dtype', C.c_int32), ('eps', C.c_float),
-        ('x', _p), ('g', _p), ('weight', _p), ('bias', _p), ('y', _p), ('rstd', _p),
-        ('dy', _p), ('dx', _p), ('dg', _p), ('dweight', _p), ('dbias', _p), ('partials', _p),
-        ('param_dtype', C.c_int32),
-    ]
-
-
-CONV_SILU = 1
-NORM_GATE_SIGMOID = 1
-
-
 class PrefixArgs(C.Structure):
     _fields_ = [
         ('struct_bytes', C.c_int32), ('HV', C.c_int32), ('K', C.c_int32), ('V', C.c_int32),

@@ -60,12 +60,6 @@ __device__ __forceinline__ void st_param(void* p, int64_t i, int code, float x) 
   else static_cast<__half*>(p)[i] = __float2half_rn(x);
 }
 
-// Shared address of the 16-byte chunk holding (row r, columns col8 .. col8+7) of a bf16 tile of `rows` rows in the
-// 128-byte-swizzled panel layout (what TMA writes and the tensor cores read).
-__device__ __forceinline__ uint32_t swz_chunk_addr(uint32_t tile, int rows, int r, int col8) {
-  return tile + (col8 >> 6) * (rows * 128) + r * 128 + ((((col8 >> 3) & 7) ^ (r & 7)) << 4);
-}
-
 // gamma is stored per chunk, [n_chunks][HV][64] fp32, entries past the chunk's valid length repeating the
 // last valid value (so 2^(gamma_last - gamma_i) is 1 there): a chunk's 64 values are 256 contiguous,
 // 256-byte aligned bytes that one bulk copy or one coalesced load brings in.
