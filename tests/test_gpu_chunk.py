@@ -816,3 +816,31 @@ def test_planned_cuts_equal_the_uncut_scan(D, HV, lens):
     o_r, ht_r = fused_recurrent_gated_delta_rule(q, k, v, g, beta=beta, initial_state=h0, output_final_state=True, cu_seqlens=cu_t)
     O.assert_close('o vs recurrent', o_r.float().cpu(), out[None][0].float().cpu(), 0.005)
     O.assert_close('ht vs recurrent', ht_r.cpu(), out[None][1].cpu(), 0.005)
+
+
+@pytest.mark.parametrize('D,H,limit_dg,limit_sum', [(128, 1, 0.0040, 0.008), (64, 4, 0.0043, 0.011)])
+def test_gate_gradients_keep_their_distance_from_fp64(D, H, limit_dg, limit_sum):
+    """dg, and its sums over a sequence (dA_log and ddt_bias are such sums, of terms that cancel), with the layer's options
+    against the fp64 recurrence, over twelve seeds.  Measured: 0.00378 and 0.0051 (128, group of four), 0.00392 and 0.0088
+    (64); with the WY terms of dk inside the dots of the gate's gradient, whose bf16 operands do not cancel, 0.00417 and
+    0.0116, 0.00470 and 0.0148.  The limits lie between; results are the same from run to run."""
+    from b200gdn import chunk_gated_delta_rule
+    HV, T, errs, sums = 4, 384, [], []
+    for seed in range(12):
+        gen = torch.Generator().manual_seed(seed)
+        rn = lambda *s: torch.randn(*s, generator=gen)   # noqa: E731
+        q, k, v, do = (rn(1, T, h, D).to(torch.bfloat16) for h in (H, H, HV, HV))
+        g, b = rn(1, T, HV), rn(1, T, HV)
+        log_a, dt = (torch.rand(HV, generator=gen) * 15 + 1).log(), torch.rand(HV, generator=gen) * 0.1
+        dt = dt + torch.log(-torch.expm1(-dt))
+        opts = dict(use_qk_l2norm_in_kernel=True, use_gate_in_kernel=True, use_beta_sigmoid_in_kernel=True)
+        wide = [x.double().requires_grad_(True) for x in (q, k, v, g, b, log_a, dt)]
+        ro, _ = O.recurrent_step_options(*wide[:5], scale=D ** -0.5, A_log=wide[5], dt_bias=wide[6], dtype=torch.float64, **opts)
+        ref_g, ref_dt = torch.autograd.grad(ro, [wide[3], wide[6]], do.double())
+        leaves = [x.cuda().requires_grad_(True) for x in (q, k, v, g, b, log_a, dt)]
+        o, _ = chunk_gated_delta_rule(*leaves[:5], A_log=leaves[5], dt_bias=leaves[6], **opts)
+        got_g, got_dt = (x.double().cpu() for x in torch.autograd.grad(o, [leaves[3], leaves[6]], do.cuda()))
+        errs.append((got_g - ref_g).norm() / ref_g.norm())
+        sums.append((got_dt - ref_dt) / ref_g[0].norm(dim=0))
+    assert torch.stack(errs).mean() <= limit_dg
+    assert torch.stack(sums).square().mean().sqrt() <= limit_sum
