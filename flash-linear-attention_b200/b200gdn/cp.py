@@ -237,6 +237,7 @@ class ChunkGatedDeltaRuleCPFunction(torch.autograd.Function):
             plan = split_plan_for(B, T, cp_context.cu_seqlens, cp_context.cu_seqlens_cpu, dev, HV, V // 64)
             tables = plan.tables if plan is not None else tables_for(B, T, cp_context.cu_seqlens, cp_context.cu_seqlens_cpu, dev)
             chunk_meta, seq_meta, (n_chunks, n_seq) = tables      # n_seq counts pieces under a split plan
+            _lib.host().in_use((plan or tables).native())
             rows = B * T
             bf16, f32 = torch.bfloat16, torch.float32
             zero = not tables.covered
@@ -295,7 +296,7 @@ class ChunkGatedDeltaRuleCPFunction(torch.autograd.Function):
                 _lib.call('b200gdn_chunk_fwd', a, st)
         ctx.save_for_backward(qb, kb, vb, bf, gamma, A, qk, w, h, v_new, chunk_meta, seq_meta)
         ctx.meta = (scale, n_chunks, n_seq, in_dtypes, zero)
-        ctx.cp_context, ctx.plan = cp_context, plan
+        ctx.cp_context, ctx.plan, ctx.tables = cp_context, plan, tables
         return o.to(q.dtype)
 
     @staticmethod
@@ -308,6 +309,7 @@ class ChunkGatedDeltaRuleCPFunction(torch.autograd.Function):
         rank = dist.get_rank(group=group)
         dev = qb.device
         with torch.cuda.device(dev):
+            _lib.host().in_use((plan or ctx.tables).native())
             B, T, H, K = qb.shape
             HV, V = vb.shape[2], vb.shape[3]
             rows = B * T

@@ -19,12 +19,14 @@ class Tables(tuple):
     caller zero-fills its intermediates then.  ``native()`` is the same as one handle for the native host path."""
     covered = True
     empty_seqs = False   # some sequence has no token (and so no tile)
+    stream = 0           # the stream whose memory the tables are
     order = None      # int32 [n_seq]: sequences by falling length, None when all are of one length
     _native = None
 
     def native(self):
         if self._native is None:
-            self._native = _lib.host().plan(self[0], self[1], self[2][0], self[2][1], self.covered, self.empty_seqs, self.order)
+            self._native = _lib.host().plan(self[0], self[1], self[2][0], self[2][1], self.covered, self.empty_seqs,
+                                            self.stream, self.order)
         return self._native
 
 
@@ -53,6 +55,8 @@ def device_tables(bounds, device) -> Tables:
     so with more CTAs than SMs a long sequence that starts late is what everything else waits for."""
     cm, sm = build_tables(bounds)
     out = Tables((torch.from_numpy(cm).to(device), torch.from_numpy(sm).to(device), (cm.shape[0], sm.shape[0])))
+    if out[0].is_cuda:
+        out.stream = torch.cuda.current_stream(out[0].device).cuda_stream
     out.empty_seqs = bool((sm[:, 1] == 0).any())
     if len(sm) > 1 and (sm[:, 1] != sm[0, 1]).any():
         out.order = torch.from_numpy(np.argsort(-sm[:, 1], kind='stable').astype(np.int32)).to(device)
@@ -120,8 +124,8 @@ class SplitPlan:
         """The plan as one handle for the native host path."""
         if self._native is None:
             t = self.tables
-            self._native = _lib.host().plan(t[0], t[1], t[2][0], t[2][1], t.covered, t.empty_seqs, t.order, self.chains, self.pre_fwd,
-                                            self.pre_bwd, self.first_piece, self.last_piece, self.n_chains, self.n_pre)
+            self._native = _lib.host().plan(t[0], t[1], t[2][0], t[2][1], t.covered, t.empty_seqs, t.stream, t.order, self.chains,
+                                            self.pre_fwd, self.pre_bwd, self.first_piece, self.last_piece, self.n_chains, self.n_pre)
         return self._native
 
 

@@ -12,6 +12,7 @@
 
 #include <ATen/ATen.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
@@ -20,7 +21,9 @@
 #include <torch/custom_class.h>
 
 #include <atomic>
+#include <mutex>
 #include <string>
+#include <vector>
 
 #include "../../include/b200gdn.h"
 
@@ -124,7 +127,12 @@ struct Plan : torch::CustomClassHolder {
   bool empty_seqs = false;           // some sequence has no token
   Tensor chains, pre_fwd, pre_bwd, first_piece, last_piece;
   int32_t n_chains = 0, n_pre = 0;
+  cudaStream_t made_on = nullptr;    // the stream whose memory the tables are
+  static std::atomic<long> alive;
+  Plan() { alive.fetch_add(1, std::memory_order_relaxed); }
+  ~Plan() override { alive.fetch_sub(1, std::memory_order_relaxed); }
 };
+std::atomic<long> Plan::alive{0};
 using PlanPtr = c10::intrusive_ptr<Plan>;
 constexpr const char* kPlanName = "b200gdn.plan";
 
@@ -132,6 +140,61 @@ PlanPtr plan_of(PyObject* o) {
   auto* p = static_cast<Plan*>(PyCapsule_GetPointer(o, kPlanName));
   if (p == nullptr) throw python_error();
   return PlanPtr::reclaim_copy(p);
+}
+
+// References that captured graphs held on plans: the end of a graph may come on a thread that must not call CUDA, so they wait
+// here until the next plan is made.  Never destroyed, since graphs may outlive this module.
+struct Released {
+  std::mutex lock;
+  std::vector<PlanPtr> plans;
+  void add(PlanPtr p) {
+    std::lock_guard<std::mutex> g(lock);
+    plans.push_back(std::move(p));
+  }
+  void drop() {
+    std::vector<PlanPtr> old;
+    std::lock_guard<std::mutex> g(lock);
+    old.swap(plans);
+  }
+};
+Released& released() {
+  static Released* r = new Released;
+  return *r;
+}
+
+// Called before kernels that read a plan's tables are launched on the current stream.  The tables are kept in a bounded cache
+// and may leave it at any time: their memory must not be handed on before kernels on another stream than their own are done
+// with it, and a graph that captures the kernels holds the plan for as long as it can be replayed.
+void in_use(const PlanPtr& plan) {
+  if (!plan->chunk_meta.defined() || !plan->chunk_meta.is_cuda()) return;
+  const c10::cuda::CUDAStream stream = c10::cuda::getCurrentCUDAStream();
+  if (stream.stream() != plan->made_on)
+    for (const Tensor* t : {&plan->chunk_meta, &plan->seq_meta, &plan->seq_order, &plan->chains, &plan->pre_fwd, &plan->pre_bwd,
+                            &plan->first_piece, &plan->last_piece})
+      if (t->defined()) c10::cuda::CUDACachingAllocator::recordStream(t->storage().data_ptr(), stream);
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  cudaGraph_t graph = nullptr;
+  if (cudaStreamGetCaptureInfo(stream.stream(), &status, nullptr, &graph) != cudaSuccess) {
+    (void)cudaGetLastError();   // the legacy stream while another one is being captured
+    return;
+  }
+  if (status != cudaStreamCaptureStatusActive) return;
+  auto* held = new PlanPtr(plan);
+  auto end = [](void* p) {
+    auto* h = static_cast<PlanPtr*>(p);
+    released().add(std::move(*h));
+    delete h;
+  };
+  cudaUserObject_t obj = nullptr;
+  if (cudaUserObjectCreate(&obj, held, end, 1, cudaUserObjectNoDestructorSync) != cudaSuccess) {
+    delete held;
+    raise(std::string("cudaUserObjectCreate: ") + cudaGetErrorString(cudaGetLastError()));
+  }
+  if (cudaGraphRetainUserObject(graph, obj, 1, cudaGraphUserObjectMove) != cudaSuccess) {
+    const std::string what = cudaGetErrorString(cudaGetLastError());
+    cudaUserObjectRelease(obj, 1);
+    raise("cudaGraphRetainUserObject: " + what);
+  }
 }
 
 // ---- recurrent (decode) --------------------------------------------------------------------------------------
@@ -253,6 +316,7 @@ ChunkForward chunk_forward(const Tensor& q_in, const Tensor& k_in, const Tensor&
   ChunkForward r;
   const at::Device dev = q_in.device();
   c10::cuda::CUDAGuard guard(dev);
+  in_use(plan);
   auto s = c10::make_intrusive<ChunkSaved>();
   s->qt = q_in.scalar_type();
   s->kt = k_in.scalar_type();
@@ -420,6 +484,7 @@ class ChunkFunction : public torch::autograd::Function<ChunkFunction> {
     const Plan& plan = *s.plan;
     const at::Device dev = q.device();
     c10::cuda::CUDAGuard guard(dev);
+    in_use(s.plan);
     const bool zero = !plan.covered, gate = s.options & B200GDN_PREP_GATE;
     b200gdn_chunk_args a = chunk_args(q, k, v, s.scale, plan);
     const int64_t rows = a.rows, HV = a.HV, K = a.K, V = a.V, C = a.n_chunks, N = a.n_seq;
@@ -577,6 +642,7 @@ ConvForward conv_forward(const Tensor& x, const Tensor& weight, const Tensor& bi
   a.initial_state = ptr(r.h0);
   a.y = ptr(r.y);
   a.final_state = ptr(r.final_state);
+  if (a.rows != a.n_tiles || a.n_seq != a.n_tiles || a.n_seq > 65535) in_use(plan);   // a decoding step reads no table
   // the backward pass reads the cache as it was
   const Tensor before = need_grad && r.in_place ? r.h0.clone() : r.h0;
   call("b200gdn_conv_fwd", b200gdn_conv_fwd, a);
@@ -608,6 +674,7 @@ class ConvFunction : public torch::autograd::Function<ConvFunction> {
     const Plan& plan = *s.plan;
     const at::Device dev = x.device();
     c10::cuda::CUDAGuard guard(dev);
+    in_use(s.plan);
     const at::ScalarType t = x.scalar_type(), pt = w.scalar_type();
     const int64_t D = x.size(2), tiles = plan.n_chunks;
     const Tensor dy = grads[0].defined() ? dense(grads[0], t) : new_tensor(x.sizes(), t, dev, true);
@@ -891,23 +958,25 @@ PyObject* py_norm_gate(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   END_HANDLE_TH_ERRORS
 }
 
-// plan(chunk_meta, seq_meta, n_chunks, n_seq, covered, empty_seqs, seq_order or None
+// plan(chunk_meta, seq_meta, n_chunks, n_seq, covered, empty_seqs, stream, seq_order or None
 //      [, chains, pre_fwd, pre_bwd, first_piece, last_piece, n_chains, n_pre])
 PyObject* py_plan(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
-  if (nargs != 7) NEED_ARGS(14);
+  if (nargs != 8) NEED_ARGS(15);
+  released().drop();
   auto p = c10::make_intrusive<Plan>();
-  bool ok = get(args[0], p->chunk_meta) && get(args[1], p->seq_meta) && get(args[6], p->seq_order);
+  bool ok = get(args[0], p->chunk_meta) && get(args[1], p->seq_meta) && get(args[7], p->seq_order);
   p->n_chunks = (int32_t)PyLong_AsLong(args[2]);
   p->n_seq = (int32_t)PyLong_AsLong(args[3]);
   p->covered = truth(args[4]);
   p->empty_seqs = truth(args[5]);
-  if (nargs == 14) {
+  p->made_on = static_cast<cudaStream_t>(PyLong_AsVoidPtr(args[6]));
+  if (nargs == 15) {
     p->split = true;
-    ok = ok && get(args[7], p->chains) && get(args[8], p->pre_fwd) && get(args[9], p->pre_bwd) && get(args[10], p->first_piece) &&
-         get(args[11], p->last_piece);
-    p->n_chains = (int32_t)PyLong_AsLong(args[12]);
-    p->n_pre = (int32_t)PyLong_AsLong(args[13]);
+    ok = ok && get(args[8], p->chains) && get(args[9], p->pre_fwd) && get(args[10], p->pre_bwd) && get(args[11], p->first_piece) &&
+         get(args[12], p->last_piece);
+    p->n_chains = (int32_t)PyLong_AsLong(args[13]);
+    p->n_pre = (int32_t)PyLong_AsLong(args[14]);
   }
   if (!ok && !PyErr_Occurred()) PyErr_SetString(PyExc_TypeError, "plan: tensors expected");
   if (PyErr_Occurred()) return nullptr;
@@ -929,6 +998,20 @@ PyObject* py_slab(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   return nullptr;
 }
 
+// the streams and graphs of callers that launch kernels on a plan's tables themselves
+PyObject* py_in_use(PyObject*, PyObject* plan) {
+  HANDLE_TH_ERRORS
+  const PlanPtr p = plan_of(plan);
+  if (p->chunk_meta.defined() && p->chunk_meta.is_cuda()) {
+    c10::cuda::CUDAGuard guard(p->chunk_meta.device());
+    in_use(p);
+  }
+  Py_RETURN_NONE;
+  END_HANDLE_TH_ERRORS
+}
+
+PyObject* py_plans_alive(PyObject*, PyObject*) { return PyLong_FromLong(Plan::alive.load(std::memory_order_relaxed)); }
+
 PyObject* py_launch_count(PyObject*, PyObject*) { return PyLong_FromLongLong(g_launches.load(std::memory_order_relaxed)); }
 
 PyObject* py_set_error_class(PyObject*, PyObject* cls) {
@@ -944,6 +1027,8 @@ PyMethodDef methods[] = {
     {"conv", FAST(py_conv), "short causal convolution, differentiable"},
     {"norm_gate", FAST(py_norm_gate), "gated RMS norm, differentiable"},
     {"plan", FAST(py_plan), "chunk tables (and split plan) of a shape as one handle"},
+    {"in_use", py_in_use, METH_O, "the tables of a plan are about to be read on the current stream"},
+    {"plans_alive", py_plans_alive, METH_NOARGS, "plans that are cached, saved for a backward pass or held by a graph"},
     {"slab", FAST(py_slab), "layout of a workspace"},
     {"launch_count", py_launch_count, METH_NOARGS, "kernels enqueued through this module"},
     {"set_error_class", py_set_error_class, METH_O, "class raised when a library call fails"},

@@ -85,3 +85,75 @@ def test_sizes_of_zero_and_unclear_switches_raise():
     x, w = torch.zeros(1, 4, 64, device='cuda'), torch.zeros(64, 4, device='cuda')
     with pytest.raises(RuntimeError, match='ambiguous'):
         causal_conv1d(x, w, output_final_state=torch.ones(2))
+
+
+def _forget_tables():
+    """Everything that the package keeps about sequences is dropped and the memory it was in is written over."""
+    import gc
+    from b200gdn import index
+    index._cache.clear()
+    index._split_cache.clear()
+    gc.collect()
+    return [torch.zeros(128, dtype=torch.int32, device='cuda') for _ in range(4096)]
+
+
+@pytest.mark.parametrize('name', ['chunk', 'conv'])
+@pytest.mark.parametrize('pieces', [None, 3])
+def test_a_captured_graph_keeps_its_tables(name, pieces):
+    """A graph is replayed after the tables of its sequences have left the cache; its end gives them back."""
+    from b200gdn import _lib, index
+    call, inputs = _operators()[name]
+    args = [x.requires_grad_(True) for x in inputs(200, 0)]
+
+    def step():
+        out = call(*args)[0]
+        return (out.detach(), *torch.autograd.grad(out, args, torch.ones_like(out)))
+    index.FORCE_PIECES = pieces
+    try:
+        _forget_tables()
+        before = _lib.host().plans_alive()
+        side = torch.cuda.Stream()
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            step()
+        torch.cuda.current_stream().wait_stream(side)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            got = step()
+        graph.replay()
+        want = [x.clone() for x in got]
+        torch.cuda.synchronize()
+        kept = _forget_tables()
+        assert _lib.host().plans_alive() > before
+        for x in got:
+            x.fill_(float('nan'))
+        graph.replay()
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, b) for a, b in zip(want, got))
+        del graph, kept
+        torch.cuda.synchronize()
+        _forget_tables()
+        call(*inputs(7, 0))   # makes a plan, which drops what ended graphs held
+        _forget_tables()
+        assert _lib.host().plans_alive() == before
+    finally:
+        index.FORCE_PIECES = None
+
+
+@pytest.mark.parametrize('name', ['chunk', 'conv'])
+def test_tables_outlast_their_use_on_another_stream(name):
+    """The tables leave the cache while a stream other than the one they were made on has yet to read them."""
+    call, inputs = _operators()[name]
+    args = inputs(200, 0)
+    with torch.no_grad():
+        want = call(*args)
+        _forget_tables()
+        call(*args)              # the tables are made here
+        torch.cuda.synchronize()
+        side = torch.cuda.Stream()
+        with torch.cuda.stream(side):
+            torch.cuda._sleep(20_000_000)
+            got = call(*args)
+        kept = _forget_tables()
+        side.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(want, got)) and len(kept)
