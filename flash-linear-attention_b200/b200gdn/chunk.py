@@ -13,7 +13,7 @@ import torch
 
 from . import _lib
 from .index import native_plan
-from .recorded import RecordedCall, tracing
+from .recorded import RecordedCall, recorded
 
 _SUPPORTED_HEAD_DIMS = ((64, 64), (128, 128))
 
@@ -292,7 +292,7 @@ def chunk_gated_delta_rule(
         A_log = dt_bias = None
     args = (q, k, v, g, beta, initial_state, A_log, dt_bias, scale, output_final_state,
             flags | (_lib.STATE_V_FIRST if state_v_first else 0), cu_seqlens, cu_seqlens_cpu)
-    return RecordedCall.apply(_native_chunk, *args) if tracing() else _native_chunk(*args)
+    return RecordedCall.apply(_native_chunk, *args) if recorded(q) else _native_chunk(*args)
 
 
 chunk_gdn = chunk_gated_delta_rule

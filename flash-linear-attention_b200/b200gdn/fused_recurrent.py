@@ -8,7 +8,7 @@ from typing import Optional
 import torch
 
 from . import _lib
-from .recorded import seen_by_trace, tracing
+from .recorded import seen_by_trace, untraced
 
 
 class FusedRecurrentFunction(torch.autograd.Function):
@@ -18,8 +18,9 @@ class FusedRecurrentFunction(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, k, v, g, beta, A_log, dt_bias, scale, initial_state, output_final_state, flags, cu_seqlens,
                 inplace_state, state_indices=None):
-        out = _lib.host().recurrent(q, k, v, g, beta, A_log, dt_bias, scale, initial_state, output_final_state, flags,
-                                    cu_seqlens, inplace_state, state_indices)
+        with untraced():
+            out = _lib.host().recurrent(q, k, v, g, beta, A_log, dt_bias, scale, initial_state, output_final_state, flags,
+                                        cu_seqlens, inplace_state, state_indices)
         if out is NotImplemented:
             raise _lib.B200GDNError('fused_recurrent_gated_delta_rule: tensors of unexpected shapes or devices')
         if out[1] is not None and out[1] is initial_state:
@@ -82,7 +83,7 @@ def fused_recurrent_gated_delta_rule(
     flags = ((_lib.REC_L2NORM if use_qk_l2norm_in_kernel else 0) | (_lib.REC_GATE if use_gate_in_kernel else 0)
              | (_lib.REC_BETA_SIGMOID if use_beta_sigmoid_in_kernel else 0) | (_lib.REC_NEG_EIGVAL if allow_neg_eigval else 0)
              | (_lib.REC_STATE_V_FIRST if state_v_first else 0))
-    if gk is None and gv is None and not tracing():
+    if gk is None and gv is None:
         out = (_lib._host or _lib.host()).recurrent(q, k, v, g, beta, A_log, dt_bias, scale, initial_state, output_final_state,
                                                     flags, cu_seqlens, inplace_state, state_indices)
         if out is not NotImplemented:

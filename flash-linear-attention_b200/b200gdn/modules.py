@@ -20,15 +20,7 @@ import torch.nn as nn
 
 from . import _lib
 from .index import tables_for
-from .recorded import RecordedCall, tracing
-
-
-def _param(module: nn.Module, name: str):
-    """``module.name`` for a parameter.  Registered parameters are read from their dictionary, which spares a decoding step the
-    attribute protocol of nn.Module (0.11 against 0.31 us); where something else holds the name (a parametrization, pruning or
-    weight norm, the replica of a data-parallel step) the attribute is what counts."""
-    params = module._parameters
-    return params[name] if name in params else getattr(module, name)
+from .recorded import RecordedCall, recorded
 
 
 def _native_conv(x, weight, bias, residual, initial_state, activation, output_final_state, cu_seqlens, cu_seqlens_cpu, inplace_state):
@@ -37,8 +29,8 @@ def _native_conv(x, weight, bias, residual, initial_state, activation, output_fi
                             inplace_state, plan)
 
 
-def _conv(*args):
-    return RecordedCall.apply(_native_conv, *args) if tracing() else _native_conv(*args)
+def _conv(x, *args):
+    return RecordedCall.apply(_native_conv, x, *args) if recorded(x) else _native_conv(x, *args)
 
 
 class _HaloExchange(torch.autograd.Function):
@@ -151,9 +143,18 @@ class ShortConvolution(nn.Conv1d):
         if B * T == N:   # decoding: one token per sequence, the cache (created when absent) is updated in place
             if cache is None:
                 cache = x.new_zeros(N, self.hidden_size, self.kernel_size[0])
-            elif T == 1 and x.is_cuda and cu_seqlens is None and self.activation in ('silu', 'swish') and not tracing():
-                # nothing that causal_conv1d would check: a step of three of these costs the host more than the device
-                y, cache = _lib.host().conv(x, _param(self, 'weight'), _param(self, 'bias'), residual, cache, True, True, True,
+            elif type(T) is int and T == 1 and x.is_cuda and cu_seqlens is None and self.activation in ('silu', 'swish'):
+                # nothing that causal_conv1d would check (lengths that are no plain numbers are those of a recorded trace):
+                # a step of three of these costs the host more than the device.
+                # Registered parameters are read from their dictionary, which spares the step nn.Module's attribute protocol
+                # (0.2 us each); where something else holds a name (a parametrization, pruning or weight norm, the replica of
+                # a data-parallel step) the attribute is what counts.
+                params = self._parameters
+                try:
+                    weight, bias = params['weight'], params['bias']
+                except KeyError:
+                    weight, bias = self.weight, self.bias
+                y, cache = _lib.host().conv(x, weight, bias, residual, cache, True, True, True,
                                            tables_for(B, 1, None, None, x.device).native())
                 return y, (cache if output_final_state else None)
             y, cache = causal_conv1d(x, self.weight, self.bias, residual, cache, True, self.activation, cu_seqlens=cu_seqlens,
@@ -179,7 +180,8 @@ def rms_norm_gated(x, g, weight, bias=None, activation: str = 'swish', residual=
     if not x.is_cuda:
         raise _lib.B200GDNError('rms_norm_gated runs on a CUDA device only (no CPU path)')
     args = (x, g, weight, bias, activation == 'sigmoid', eps)
-    return RecordedCall.apply(_lib.host().norm_gate, *args) if tracing() else _lib.host().norm_gate(*args)
+    y = _lib.host().norm_gate(*args)
+    return RecordedCall.apply(_lib.host().norm_gate, *args) if y is NotImplemented else y
 
 
 class FusedRMSNormGated(nn.Module):
@@ -199,8 +201,14 @@ class FusedRMSNormGated(nn.Module):
         self.register_parameter('bias', None)
 
     def forward(self, x, g, residual=None, prenorm=False, residual_in_fp32=False):
-        weight, bias = _param(self, 'weight'), _param(self, 'bias')
-        if x.is_cuda and residual is None and not prenorm and not tracing():
-            return _lib.host().norm_gate(x, g, weight, bias, self.activation == 'sigmoid', self.eps)
+        params = self._parameters
+        try:   # as in ShortConvolution.forward
+            weight, bias = params['weight'], params['bias']
+        except KeyError:
+            weight, bias = self.weight, self.bias
+        if x.is_cuda and residual is None and not prenorm:
+            y = _lib.host().norm_gate(x, g, weight, bias, self.activation == 'sigmoid', self.eps)
+            if y is not NotImplemented:
+                return y
         return rms_norm_gated(x, g, weight, bias, self.activation, residual=residual, eps=self.eps,
                               prenorm=prenorm, residual_in_fp32=residual_in_fp32)

@@ -11,6 +11,7 @@
 #include <Python.h>
 
 #include <ATen/ATen.h>
+#include <ATen/TracerMode.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
@@ -97,8 +98,10 @@ int gate_types(Tensor& g, Tensor& beta) {
 // serves and which it therefore refuses (without it they would be dropped in silence)
 bool wants_grad(std::initializer_list<const Tensor*> xs) {
   const bool reverse = at::GradMode::is_enabled(), forward = c10::AutogradState::get_tls_state().get_fw_grad_mode();
-  for (const Tensor* x : xs)
-    if (x->defined() && ((reverse && x->requires_grad()) || (forward && x->_fw_grad(0).defined()))) return true;
+  for (const Tensor* x : xs) {
+    if (!x->defined() || x->unsafeGetTensorImpl()->autograd_meta() == nullptr) continue;
+    if ((reverse && x->requires_grad()) || (forward && x->_fw_grad(0).defined())) return true;
+  }
   return false;
 }
 // autograd's apply() takes an absent tensor as an empty optional
@@ -827,6 +830,8 @@ PyObject* wrap_pair(const Tensor& a, const Tensor& b) {
   return r;
 }
 bool on_device(const Tensor& t, const at::Device& dev) { return !t.defined() || t.device() == dev; }
+// while torch.jit.trace records, a call is left to the Python wrapper, which makes an operation of it
+bool tracing() { return at::tracer::impl::is_dispatch_enabled(); }
 bool truth(PyObject* o) { return o == Py_True || (o != Py_False && o != Py_None && PyObject_IsTrue(o) > 0); }
 
 #define NEED_ARGS(n)                                                                                            \
@@ -840,6 +845,7 @@ bool truth(PyObject* o) { return o == Py_True || (o != Py_False && o != Py_None 
 PyObject* py_recurrent(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
   NEED_ARGS(14);
+  if (tracing()) Py_RETURN_NOTIMPLEMENTED;
   Tensor q, k, v, g, beta, A, bias, h0, cu, idx;
   if (!get(args[0], q) || !get(args[1], k) || !get(args[2], v) || !get(args[3], g) || !get(args[4], beta) || !get(args[5], A) ||
       !get(args[6], bias) || !get(args[8], h0) || !get(args[11], cu) || !get(args[13], idx))
@@ -937,10 +943,11 @@ PyObject* py_conv(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   END_HANDLE_TH_ERRORS
 }
 
-// norm_gate(x, g, weight, bias, sigmoid, eps) -> y
+// norm_gate(x, g, weight, bias, sigmoid, eps) -> y or NotImplemented (while a trace is recorded)
 PyObject* py_norm_gate(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
   NEED_ARGS(6);
+  if (tracing()) Py_RETURN_NOTIMPLEMENTED;
   Tensor x, g, w, b;
   if (!get(args[0], x) || !get(args[1], g) || !get(args[2], w) || !get(args[3], b) || !x.defined() || !g.defined()) {
     PyErr_SetString(PyExc_TypeError, "rms_norm_gated: a tensor is expected");
