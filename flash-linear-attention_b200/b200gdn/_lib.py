@@ -14,7 +14,7 @@ import threading
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, 'libb200gdn.so')
 
-ABI_VERSION = 1
+ABI_VERSION = 2
 
 FWD_INTRA, FWD_SCAN, FWD_OUT = 1, 2, 4
 BWD_DVLOCAL, BWD_SCAN, BWD_DQKWG, BWD_WY = 1, 2, 4, 8

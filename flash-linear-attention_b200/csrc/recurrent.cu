@@ -391,7 +391,7 @@ __global__ void __launch_bounds__(NTHREADS) recurrent_kernel(const b200gdn_recur
 
 // Single-token decode at large batch as a stream: the step kernel loads a state, computes and stores it, so the memory pipe
 // of an SM idles while its CTAs compute.  Here one persistent CTA per SM walks its (sequence, head) items through a ring of
-// states in shared memory: a mover thread brings and takes away each 64 KiB state (one contiguous bulk copy each way), two
+// states in shared memory: a mover thread brings and takes away each 64 KiB state (one contiguous bulk copy each way), three
 // warps prepare the tokens (q and k as fp32 with their norms' factors, v, the activated gate scalars) for the same ring, and
 // eight consumer warps only compute, shared memory to shared memory.  Bound by HBM (one read and one write of every state).
 // 256 sequences x 16 heads, K = V = 128: 91 us, 5.9 TB/s (100 with the tokens fetched and the gates activated by the thread that

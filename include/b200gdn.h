@@ -14,7 +14,8 @@
  *  - token-major layout of the reference ([B,T,H,...], head_first is not supported) flattened to rows:
  *    q,k [rows,H,K]; v,o,do [rows,HV,V]; g,beta [rows,HV]; states [n_seq,HV,K,V] fp32;
  *    rows = B*T (dense) or the packed token count (cu_seqlens input, B == 1);
- *  - q/k/v/o/do and the saved tensors are bf16; gates, beta and states are fp32;
+ *  - q/k/v/o/do and the saved tensors are bf16; states are fp32; gates, beta and small parameters have an element type of
+ *    their own (B200GDN_F32 / BF16 / F16 below);
  *  - chunking (64 tokens, restarting at every sequence start) is described by two int32 tables that the
  *    host builds once per shape (fla/ops/utils/index.py:155-172 computes the same information):
  *      chunk_meta[n_chunks][4] = { sequence id, first row, valid rows (1..64), chunk index inside its sequence }
@@ -34,7 +35,9 @@
 extern "C" {
 #endif
 
-#define B200GDN_ABI_VERSION 1
+/* 2: element types of gates, betas and of the convolution's and norm's parameters (gb_dtype, param_dtype); the L2 norm in the
+ * forward chunk pass (qn, kn); the order of the sequences (seq_order).  Argument blocks changed size with it. */
+#define B200GDN_ABI_VERSION 2
 #define B200GDN_CHUNK 64
 
 /* element type of small per-head / per-channel tensors that are read (or written) in the caller's own precision:
@@ -334,7 +337,7 @@ typedef struct b200gdn_conv_args {
   void* dweight;                 /* [D, W] or NULL, element type param_dtype */
   void* dbias;                   /* [D] or NULL, element type param_dtype */
   void* dinitial_state;          /* [n_seq, D, W] or NULL */
-  float* partials;               /* workspace fp32 [2 n_tiles, D, W + 1]; required with dweight */
+  float* partials;               /* workspace fp32 [2 n_tiles, W + 1, D]; required with dweight */
   int32_t param_dtype;           /* B200GDN_F32 / BF16 / F16 */
 } b200gdn_conv_args;
 int b200gdn_conv_fwd(const b200gdn_conv_args* args, void* stream);
