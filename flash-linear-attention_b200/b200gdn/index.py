@@ -2,6 +2,7 @@
 prepare_chunk_offsets, in the form the kernels read)."""
 from __future__ import annotations
 
+import functools
 from typing import Optional, Sequence, Tuple
 
 import numpy as np
@@ -11,6 +12,7 @@ from . import _lib
 
 CHUNK = 64
 _cache: dict = {}
+_bounds_cache: dict = {}
 
 
 class Tables(tuple):
@@ -69,13 +71,20 @@ def content_version(cu_seqlens: torch.Tensor):
     return None if cu_seqlens.is_inference() else cu_seqlens._version
 
 
-def packed_bounds(cu_seqlens: torch.Tensor, cu_seqlens_cpu: Optional[torch.Tensor], rows: int):
-    """(start, end) of every sequence of a packed batch, none of them outside its ``rows`` token rows.  Costs one
-    device-to-host copy without ``cu_seqlens_cpu``."""
-    cu = (cu_seqlens_cpu if cu_seqlens_cpu is not None else cu_seqlens.cpu()).to(torch.int64).tolist()
-    if cu and (cu[0] < 0 or cu[-1] > rows):
-        raise ValueError(f'cu_seqlens [{cu[0]}, {cu[-1]}] reaches outside the {rows} token rows')
-    return list(zip(cu[:-1], cu[1:]))
+def packed_bounds(cu_seqlens: torch.Tensor, cu_seqlens_cpu: Optional[torch.Tensor], rows: int, version):
+    """(start, end) of every sequence of a packed batch, none of them outside its ``rows`` token rows.  The device-to-host copy
+    that this costs without ``cu_seqlens_cpu`` (17 us) is made once for the tables, the planner and the convolutions."""
+    hit = _bounds_cache.get(id(cu_seqlens))
+    if hit is None or hit[1] is not cu_seqlens or hit[2] != version:
+        cu = (cu_seqlens_cpu if cu_seqlens_cpu is not None else cu_seqlens.cpu()).tolist()
+        hit = ([(int(s), int(e)) for s, e in zip(cu[:-1], cu[1:])], cu_seqlens, version)
+        if len(_bounds_cache) > 64:
+            _bounds_cache.clear()
+        _bounds_cache[id(cu_seqlens)] = hit
+    bounds = hit[0]
+    if bounds and (bounds[0][0] < 0 or bounds[-1][1] > rows):
+        raise ValueError(f'cu_seqlens [{bounds[0][0]}, {bounds[-1][1]}] reaches outside the {rows} token rows')
+    return bounds
 
 
 def tables_for(B: int, T: int, cu_seqlens: Optional[torch.Tensor], cu_seqlens_cpu: Optional[torch.Tensor],
@@ -95,7 +104,7 @@ def tables_for(B: int, T: int, cu_seqlens: Optional[torch.Tensor], cu_seqlens_cp
         hit = _cache.get(key)
         if hit is not None and hit[1] is cu_seqlens and hit[2] == version:
             return hit[0]
-        bounds = packed_bounds(cu_seqlens, cu_seqlens_cpu, B * T)
+        bounds = packed_bounds(cu_seqlens, cu_seqlens_cpu, B * T, version)
     out = device_tables(bounds, device)
     out.covered = bool(bounds) and bounds[0][0] == 0 and bounds[-1][1] == B * T
     if len(_cache) > 64:
@@ -129,6 +138,7 @@ class SplitPlan:
         return self._native
 
 
+@functools.lru_cache(maxsize=None)
 def sm_count(device) -> int:
     return torch.cuda.get_device_properties(device).multi_processor_count if device.type == 'cuda' else 148
 
@@ -165,7 +175,6 @@ def piece_counts(chunks_per_seq, HV: int, slices: int, sms: int = 148):
 
 def split_plan(bounds, HV: int, slices: int, device, rows: int) -> Optional[SplitPlan]:
     """None when no sequence is worth cutting; otherwise the plan (device tensors) for these bounds."""
-    bounds = [(int(s), int(e)) for s, e in bounds]
     chunks = [(e - s + CHUNK - 1) // CHUNK for s, e in bounds]
     pieces = piece_counts(chunks, HV, slices, sm_count(device))
     if max(pieces, default=1) <= 1:
@@ -216,7 +225,7 @@ def split_plan_for(B: int, T: int, cu_seqlens, cu_seqlens_cpu, device, HV: int, 
         hit = _split_cache.get(key)
         if hit is not None and hit[1] is cu_seqlens and hit[2] == version:
             return hit[0]
-        bounds = packed_bounds(cu_seqlens, cu_seqlens_cpu, B * T)
+        bounds = packed_bounds(cu_seqlens, cu_seqlens_cpu, B * T, version)
     plan = split_plan(bounds, HV, slices, device, B * T)
     if len(_split_cache) > 64:
         _split_cache.clear()

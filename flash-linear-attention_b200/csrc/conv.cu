@@ -14,9 +14,9 @@
 // gradient of the cache for a sequence's first share, and leaves per-share sums of dweight / dbias that a second kernel
 // adds in a fixed order (no atomics: results are bit-reproducible).
 // One token per sequence (a decoding step) has a kernel of its own: no walk, the cache as whole words.
-// bf16, W = 4, SiLU, [4, 4096, 2048]: forward 27.9 us (4.8 TB/s of x and y; 35.3 with scalar instructions behind a ring of
-// asynchronous copies, 32.1 with the activation, the residual and every token's place decided at run time), backward 55.8 us
-// (80.9, 61.4) + 4.2 (6.7) for the parameter sums.  What is left to the copy rate is instruction issue (half of the cycles)
+// bf16, W = 4, SiLU, [4, 4096, 2048]: forward 27.3 us (4.9 TB/s of x and y; 35.3 with scalar instructions behind a ring of
+// asynchronous copies, 32.1 with the activation, the residual and every token's place decided at run time), backward 54.8 us
+// (80.9, 61.4) + 4.1 (6.7) for the parameter sums.  What is left to the copy rate is instruction issue (half of the cycles)
 // and latency at the warps that the registers allow (an eighth forward or a fifth backward CTA spills: 28.1 and 80.6 us;
 // 16-byte accesses with eight channels a thread: 40.9).  A decoding step of 32 users: 2.3 us (4.9).
 #include <type_traits>

@@ -19,7 +19,8 @@
 // merges, 4-byte stores of qk and A and a zero fill of the inverse, 5.8 k wavefronts a CTA).  So every merge has one operand
 // at an address that is uniform over the warp (one wavefront) and 16-byte reads along rows for the other, skips what is
 // zero by triangularity, and nothing is filled with zeros first.
-// B4 T4096 H16 K=V=128: 86 us (105); with the L2 norm, gate and beta options 120 us (108 + 47 for a norm pass of its own).
+// B4 T4096 H16 K=V=128: 87 us inside a step (105), 94 by itself between two events; with the L2 norm, gate and beta options
+// 120 us (108 + 47 for a norm pass of its own).
 #include "tc5_tile.cuh"
 #include "tma.cuh"
 
