@@ -104,6 +104,14 @@ bool wants_grad(std::initializer_list<const Tensor*> xs) {
   }
   return false;
 }
+// a tensor (or none) of which the kernels read `n` elements on `dev`: nothing on the device would notice that it is shorter
+void check(const char* what, const Tensor& x, int64_t n, const at::Device& dev) {
+  if (!x.defined()) return;
+  if (x.device() != dev) raise(std::string(what) + " is on " + x.device().str() + " where " + dev.str() + " is expected");
+  if (x.numel() < n)
+    raise(std::string(what) + " has " + std::to_string(x.numel()) + " elements where " + std::to_string(n) + " are expected");
+}
+bool holds(const Tensor& x, int64_t n) { return !x.defined() || x.numel() >= n; }
 // autograd's apply() takes an absent tensor as an empty optional
 std::optional<Tensor> opt(const Tensor& t) { return t.defined() ? std::optional<Tensor>(t) : std::nullopt; }
 Tensor val(const std::optional<Tensor>& t) { return t.has_value() ? *t : Tensor(); }
@@ -870,6 +878,10 @@ PyObject* py_recurrent(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   } else if (cu.defined() && h0.defined() && h0.size(0) != n_seq) {
     Py_RETURN_NOTIMPLEMENTED;
   }
+  const int64_t tokens = q.size(0) * q.size(1), HV = v.size(2), states = idx.defined() ? h0.size(0) : n_seq;
+  if (!holds(k, q.numel()) || !holds(v, tokens * HV * v.size(3)) || !holds(g, tokens * HV) || !holds(beta, tokens * HV) ||
+      ((flags & B200GDN_REC_GATE) && (!holds(A, HV) || !holds(bias, HV))) || !holds(h0, states * HV * q.size(3) * v.size(3)))
+    Py_RETURN_NOTIMPLEMENTED;
   if (wants_grad({&q, &k, &v, &g, &beta, &A, &bias, &h0})) Py_RETURN_NOTIMPLEMENTED;
   std::pair<Tensor, Tensor> r;
   {
@@ -902,6 +914,15 @@ PyObject* py_chunk(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
       if (act_code(q.scalar_type()) < 0 || k.scalar_type() != q.scalar_type())
         raise(std::string("q/k dtypes ") + c10::toString(q.scalar_type()) + "/" + c10::toString(k.scalar_type()) +
               " are not supported by the L2-norm option");
+    const at::Device dev = q.device();
+    const int64_t tokens = q.size(0) * q.size(1), HV = v.size(2), seqs = plan->split ? plan->n_chains : plan->n_seq;
+    check("k", k, q.numel(), dev);
+    check("v", v, tokens * HV * v.size(3), dev);
+    check("g", g, tokens * HV, dev);
+    check("beta", beta, tokens * HV, dev);
+    check("initial_state", h0, seqs * HV * q.size(3) * v.size(3), dev);
+    check("A_log", A, HV, dev);
+    check("dt_bias", bias, HV, dev);
     if (wants_grad({&q, &k, &v, &g, &beta, &h0, &A, &bias})) {
       out = ChunkFunction::apply(q, k, v, g, beta, opt(h0), opt(A), opt(bias), scale, out_state, options, plan);
     } else {
@@ -928,6 +949,12 @@ PyObject* py_conv(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   Tensor y, fin;
   {
     NoGil nogil;
+    const at::Device dev = x.device();
+    const int64_t D = x.size(2), W = w.size(-1);
+    check("weight", w, D * W, dev);
+    check("bias", b, D, dev);
+    check("residual", res, x.numel(), dev);
+    check("initial_state", h0, plan->n_seq * D * W, dev);
     if (wants_grad({&x, &w, &b, &res, &h0})) {
       variable_list out = ConvFunction::apply(x, w, opt(b), opt(res), opt(h0), silu, out_state, inplace, plan);
       y = out[0];
@@ -959,6 +986,9 @@ PyObject* py_norm_gate(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   Tensor y;
   {
     NoGil nogil;
+    check("g", g, x.numel(), x.device());
+    check("weight", w, x.size(-1), x.device());
+    check("bias", b, x.size(-1), x.device());
     y = wants_grad({&x, &g, &w, &b}) ? NormFunction::apply(x, g, opt(w), opt(b), sigmoid, eps) : norm_forward(x, g, w, b, sigmoid, eps, false).y;
   }
   return wrap(y);

@@ -157,3 +157,35 @@ def test_tables_outlast_their_use_on_another_stream(name):
         kept = _forget_tables()
         side.synchronize()
     assert all(torch.equal(a, b) for a, b in zip(want, got)) and len(kept)
+
+
+def test_tensors_too_short_or_elsewhere_are_refused():
+    """The kernels take their sizes from q and v (x): another tensor that is shorter, or not on the device, is refused before
+    anything is launched."""
+    from b200gdn import B200GDNError, chunk_gated_delta_rule, fused_recurrent_gated_delta_rule
+    from b200gdn.modules import causal_conv1d, rms_norm_gated
+    z = lambda *s, **kw: torch.zeros(*s, device='cuda', **kw)   # noqa: E731
+    q, v, g, state = z(2, 65, 2, 64), z(2, 65, 4, 64), z(2, 65, 4), z(2, 4, 64, 64)
+    good = dict(k=q, v=v, g=g, beta=g, initial_state=state, A_log=z(4), dt_bias=z(4))
+    gate = dict(use_gate_in_kernel=True, output_final_state=True)
+
+    def variants(args, **short):
+        for name, x in short.items():
+            for bad in (x, args[name].cpu()):
+                yield name, {**args, name: bad}
+    for op in (chunk_gated_delta_rule, fused_recurrent_gated_delta_rule):
+        op(q, **good, **gate)
+        for name, args in variants(good, k=q[:1], v=v[:1], g=g[:, :64], beta=g[:1], initial_state=state[:1], dt_bias=z(3)):
+            with pytest.raises(B200GDNError, match='expected'):
+                op(q, **args, **gate)
+    x = z(2, 65, 64)
+    conv = dict(weight=z(64, 4), bias=z(64), residual=x, initial_state=z(2, 64, 4))
+    causal_conv1d(x, **conv)
+    for name, args in variants(conv, weight=z(32, 4), bias=z(63), residual=x[:, :64], initial_state=z(1, 64, 4)):
+        with pytest.raises(B200GDNError, match=f'{name} .* expected'):
+            causal_conv1d(x, **args)
+    norm = dict(g=x, weight=z(64), bias=z(64))
+    rms_norm_gated(x, **norm)
+    for name, args in variants(norm, g=x[:1], weight=z(63), bias=z(1)):
+        with pytest.raises(B200GDNError, match=f'{name} .* expected'):
+            rms_norm_gated(x, **args)
