@@ -97,10 +97,10 @@ int gate_types(Tensor& g, Tensor& beta) {
 // whether the call has to go through its autograd node: for gradients, and for forward-mode tangents, which no node here
 // serves and which it therefore refuses (without it they would be dropped in silence)
 bool wants_grad(std::initializer_list<const Tensor*> xs) {
-  const bool reverse = at::GradMode::is_enabled(), forward = c10::AutogradState::get_tls_state().get_fw_grad_mode();
   for (const Tensor* x : xs) {
-    if (!x->defined() || x->unsafeGetTensorImpl()->autograd_meta() == nullptr) continue;
-    if ((reverse && x->requires_grad()) || (forward && x->_fw_grad(0).defined())) return true;
+    if (!x->defined() || x->unsafeGetTensorImpl()->autograd_meta() == nullptr) continue;   // neither
+    const auto& mode = c10::AutogradState::get_tls_state();
+    if ((mode.get_grad_mode() && x->requires_grad()) || (mode.get_fw_grad_mode() && x->_fw_grad(0).defined())) return true;
   }
   return false;
 }
@@ -878,9 +878,10 @@ PyObject* py_recurrent(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   } else if (cu.defined() && h0.defined() && h0.size(0) != n_seq) {
     Py_RETURN_NOTIMPLEMENTED;
   }
-  const int64_t tokens = q.size(0) * q.size(1), HV = v.size(2), states = idx.defined() ? h0.size(0) : n_seq;
-  if (!holds(k, q.numel()) || !holds(v, tokens * HV * v.size(3)) || !holds(g, tokens * HV) || !holds(beta, tokens * HV) ||
-      ((flags & B200GDN_REC_GATE) && (!holds(A, HV) || !holds(bias, HV))) || !holds(h0, states * HV * q.size(3) * v.size(3)))
+  const at::IntArrayRef qs = q.sizes(), vs = v.sizes();
+  const int64_t tokens = qs[0] * qs[1], HV = vs[2], states = idx.defined() ? h0.size(0) : n_seq;
+  if (!holds(k, q.numel()) || !holds(v, tokens * HV * vs[3]) || !holds(g, tokens * HV) || !holds(beta, tokens * HV) ||
+      ((flags & B200GDN_REC_GATE) && (!holds(A, HV) || !holds(bias, HV))) || !holds(h0, states * HV * qs[3] * vs[3]))
     Py_RETURN_NOTIMPLEMENTED;
   if (wants_grad({&q, &k, &v, &g, &beta, &A, &bias, &h0})) Py_RETURN_NOTIMPLEMENTED;
   std::pair<Tensor, Tensor> r;
