@@ -3,33 +3,39 @@
 // (fla/ops/common/chunk_o.py:172-342), prepare_wy_repr_bwd_kernel (fla/ops/gated_delta_rule/wy_fast.py:123-251) and the
 // reverse chunk-local cumsum of dg (gated_delta_rule/chunk.py:244-246).
 //
-//     dP   = tril(do v_new^T 2^(gamma_i - gamma_j)) scale            do_s = do scale 2^gamma_i          dU = dv2
-//     dq^T = h do_s^T + K^T dP^T                                     dW^T = -h dU^T
-//     dA   = strict_tril((dW K^T) (beta 2^gamma)_j + (dU V^T) beta_j)
-//     M2   = -strict_tril(A^T dA A^T) 2^(gamma_i - gamma_j) beta_i
-//     dk^T = (dh v_new^T) 2^(gamma_last - gamma_j) + q^T dP + dW^T A_b + K^T M2^T + K^T M2,   A_b = A (beta 2^gamma)_col
-//     dv^T = (dU^T A) beta_j
-//     dbeta= c_kbg 2^gamma + c_vb + r_mk,   c_kbg = colsum(A . dW K^T), c_vb = colsum(A . dU V^T), r_mk = rowsum(M . K K^T)
-//     dG_i = <dq_i,q_i> - <dk_loc_i,k_i> + c_kbg beta 2^gamma + beta r_mk - c_mk
-//            (+ at the last valid row: 2^gamma_last <h,dh> + sum_j <dk_state_j, k_j>);     dg = reverse cumsum of dG
+// With X the right-hand side of v_new = A X (X_i = beta_i (v_i - 2^gamma_i S^T k_i), A = (I + L)^-1), the adjoint of the triangular
+// solve is Z = A^T dv_new, dX = Z, dL = -strict_tril(Z v_new^T): one product each, where dA = dv_new X^T and -A^T dA A^T through
+// dW and dU took four in sequence (and rounded each of them to bf16).
+//     Z    = A^T dU      dU = dv2                                   dP   = tril(do v_new^T 2^(gamma_i - gamma_j)) scale
+//     dq^T = h do_s^T + K^T dP^T                                    do_s = do scale 2^gamma_i
+//     M    = -strict_tril(Z v_new^T) 2^(gamma_i - gamma_j)          M2   = M beta_i
+//     dk^T = (dh v_new^T) 2^(gamma_last - gamma_j) + q^T dP - (h Z^T) (beta 2^gamma)_j + K^T M2^T + K^T M2
+//     dv   = beta Z
+//     dbeta= c_kz 2^gamma + <Z_i,v_i> + r_mk,   c_kz_i = -<h Z_i, k_i>,  r_mk = rowsum(M . K K^T)
+//     dG_i = <dq_i,q_i> - <dk_loc_i,k_i> + c_kz beta 2^gamma + beta r_mk - c_mk
+//            (+ at the last valid row: 2^gamma_last <h,dh> + sum_j <dk_state_j, k_j>):     dg = reverse cumsum of dG
 // with dk_loc the first two terms of dk, <dk_loc_j,k_j> = <dk_state_j,k_j> + colsum(dP . Q K^T)_j, c_mk = colsum(M2 . K K^T).
-// (The WY terms of dk contribute c_kbg beta 2^gamma + beta r_mk + c_mk to <dk_i,k_i>, so dG could be had from the finished dk
+// (The other terms of dk contribute c_kz beta 2^gamma + beta r_mk + c_mk to <dk_i,k_i>, so dG could be had from the finished dk
 // without Q K^T and c_mk; but then the bf16 operands of those terms do not cancel against the fp32 sums, and the sums of dg
-// over a sequence, dA_log and ddt_bias, were twice as far from fp64 as with the terms kept apart: 0.016 against 0.008.)
+// over a sequence, dA_log and ddt_bias, were twice as far from fp64 as with the terms kept apart: 0.016 against 0.008.
+// Likewise dbeta = <Z_i, v_new_i> / beta_i, but v_new has been rounded as a difference: 0.0034 from fp64 against 0.0022.)
 //
-// As two kernels (dq and the chunk-local part of dk; the WY backward) k, h and that part of dk went through HBM twice:
-// 296 KiB per chunk and head at K = V = 128, 216 now, and nine dependent tensor-core phases are six.  Products with a
-// K- or V-wide result are formed TRANSPOSED ([K x 64 tokens], M = 128): the same tcgen05 instruction then does twice the
-// work of an M = 64 one, an accumulator takes 64 TMEM columns instead of 128, and every lane of a TMEM load carries data.
-// Tiles leave token-major straight from registers (movmatrix, then 16-byte words).
-// One CTA of eight warps; 256 TMEM columns (C0: dP, dq^T, dU V^T, K K^T, Q K^T; C1: the sum of dq over a group; C2: dW^T, dW K^T, Y, X,
-// dv^T; C3: dk^T) and ~111 KiB of shared memory whose regions change hands, so two CTAs per SM overlap each other's phases:
-//   R1: K      R2: do -> q      R3: v_new -> dU      R4: dh panel 0 -> h panel 0 -> dW^T
-//   R5: dh panel 1 -> h panel 1 -> V -> dA | Y -> M2 | Y
+// Products with a K- or V-wide result are formed TRANSPOSED ([K x 64 tokens], M = 128): the same tcgen05 instruction then does
+// twice the work of an M = 64 one, an accumulator takes 64 TMEM columns instead of 128, and every lane of a TMEM load carries
+// data.  dq, dk and dv go through a shared tile (stmatrix with a transpose) and leave by TMA.  <h,dh> is the diagonal of h dh^T in
+// 16 x 16 blocks by mma.sync, straight from the bf16 tiles: a tenth of the instructions of unpacking and multiplying.
+// What bounds it is the latency of the phases at two CTAs per SM, i.e. the instructions of an epilogue (39 % of issue slots, DRAM
+// 54 % of its peak rate), so epilogues work on fp32 pairs and skip blocks above the diagonal.
+// B4 T4096 H16 K=V=128: 186 us inside a step (228 with the solve's adjoint by way of dW, dU and dA, six dependent tensor-core phases
+// where there are three now; 213 with three, but element-wise stores and scalar epilogues).
+// One CTA of eight warps; 256 TMEM columns (C0: dP, dq^T, K K^T; C1: Z v_new^T, Q K^T; C2: Z^T; C3: dk_state^T, h Z^T, the rest of
+// dk^T) and ~111 KiB of shared memory whose regions change hands, so two CTAs per SM overlap each other's phases:
+//   R1: K   R2: do -> q   R3: v_new -> V   R4: dU -> Z^T -> dq   R5: dh -> h -> M2 | dv -> dk | dv   R6: A -> dP
 // Grouped value heads, many chunks: a CTA takes the heads of a group in turn, K stays, the tiles of the next head are fetched
-// under the last epilogue; the sum of dq waits in C1, that of dk in local memory (TMEM is full; 32 KiB per CTA that stay in L2).
+// under the last epilogue; the sums of dq and dk wait in local memory (TMEM is full; 64 KiB per CTA that stay in L2).
 // Few chunks: a CTA per head, the CTAs of a group form a cluster; each leaves its fp32 dq and dk in shared memory and adds up
 // a share of the rows over distributed shared memory.  Both add in head order (no atomics, no fp32 tensors in HBM).
+#include "rowio.cuh"
 #include "tc5_tile.cuh"
 #include "tma.cuh"
 
@@ -42,10 +48,11 @@ __device__ int g_local_timeout = 0;
 template <int DK>
 struct LocalSmem {
   static constexpr size_t tile = BT * DK * 2;                       // [64][DK] bf16 = [DK][64] bf16
-  static constexpr size_t o_k = 0, o_do = tile, o_vn = 2 * tile, o_h0 = 3 * tile, o_h1 = 4 * tile;
-  static constexpr size_t h1_bytes = tile > 2 * BT * 128 ? tile : 2 * BT * 128;
-  static constexpr size_t o_a = o_h1 + h1_bytes, o_ps = o_a + BT * 128, o_ab = o_ps + BT * 128;
-  static constexpr size_t o_vec = o_ab + BT * 128;
+  static constexpr size_t o_k = 0, o_do = tile, o_vn = 2 * tile, o_z = 3 * tile, o_h = 4 * tile;
+  static constexpr size_t h_bytes = DK * 128 + (DK * 128 > tile ? DK * 128 : tile);   // h; later M2 (then dk) | dv
+  static_assert(h_bytes >= DK * DK * 2, "every panel of h fits");
+  static constexpr size_t o_a = o_h + h_bytes;
+  static constexpr size_t o_vec = o_a + BT * 128;
   static constexpr int LDS = DK + 4;                                // fp32 row stride of the group-sum staging
   static constexpr size_t stage = (size_t)BT * LDS * 4;             // dq, then dk, from R2 on
   static constexpr size_t bytes = o_vec + 29 * BT * 4 + 160 + 1024; // + vectors, barriers, alignment slack
@@ -53,7 +60,7 @@ struct LocalSmem {
 };
 
 struct LocalMaps {
-  CUtensorMap q, k, v, d_o, vn, du, a, h, dh;
+  CUtensorMap q, k, v, d_o, vn, du, a, h, dh, dq, dk, dv;
 };
 
 // eight values per lane, each to be summed over the eight row-lanes of the warp (bits 2..4): recursive halving, 7 shuffles;
@@ -91,44 +98,98 @@ __device__ __forceinline__ void add_t(float (&r)[NH][16], const float (&before)[
 #pragma unroll
     for (int e = 0; e < 16; ++e) r[hf][e] = before[hf][e] + r[hf][e];
 }
+// ... tokens cs + 8 i + 2 t + {0, 1} of it times a factor per token; the same added to another block
+template <int NH>
+__device__ __forceinline__ void scale_t(float (&r)[NH][16], int i, float2 f) {
+  const uint64_t f2 = pack2(f.x, f.y);
+#pragma unroll
+  for (int hf = 0; hf < NH; ++hf)
+#pragma unroll
+    for (int e = 4 * i; e < 4 * i + 4; e += 2) {
+      const float2 x = unpack2(mul2(pack2(r[hf][e], r[hf][e + 1]), f2));
+      r[hf][e] = x.x;
+      r[hf][e + 1] = x.y;
+    }
+}
+template <int NH>
+__device__ __forceinline__ void scale_add_t(float (&to)[NH][16], const float (&r)[NH][16], int i, float2 f) {
+  const uint64_t f2 = pack2(f.x, f.y);
+#pragma unroll
+  for (int hf = 0; hf < NH; ++hf)
+#pragma unroll
+    for (int e = 4 * i; e < 4 * i + 4; e += 2) {
+      const float2 x = unpack2(fma2(pack2(r[hf][e], r[hf][e + 1]), f2, pack2(to[hf][e], to[hf][e + 1])));
+      to[hf][e] = x.x;
+      to[hf][e + 1] = x.y;
+    }
+}
 // ... its dot products with the same block of a [token][column] tile, added over the rows: value 2 i + p of the result
 // belongs to token 8 i + 2 t + p and still has to be summed over g
 template <int NH>
 __device__ __forceinline__ void dots_t(const float (&r)[NH][16], const unsigned char* tile, int row0, int cs, int lane, float (&pv)[8]) {
-#pragma unroll
-  for (int e = 0; e < 8; ++e) pv[e] = 0.f;
+  uint64_t p2[4] = {0ull, 0ull, 0ull, 0ull};
 #pragma unroll
   for (int hf = 0; hf < NH; ++hf) {
     FragLoadT f;
     f.load(tile, BT, cs, row0 + 16 * hf, lane);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const float2 x = f.lo2(i), y = f.hi2(i);
-      pv[2 * i] += r[hf][4 * i] * x.x + r[hf][4 * i + 2] * y.x;
-      pv[2 * i + 1] += r[hf][4 * i + 1] * x.y + r[hf][4 * i + 3] * y.y;
+      p2[i] = fma2(pack2(r[hf][4 * i], r[hf][4 * i + 1]), widen2<__nv_bfloat16>(f.lo[i]), p2[i]);
+      p2[i] = fma2(pack2(r[hf][4 * i + 2], r[hf][4 * i + 3]), widen2<__nv_bfloat16>(f.hi[i]), p2[i]);
     }
   }
-}
-// ... and its way to token-major global memory (`base`: row 0 of the chunk, this warp's first column)
-template <int NH>
-__device__ __forceinline__ void store_t(const float (&r)[NH][16], __nv_bfloat16* base, int64_t stride, int cs, int len, int g, int t) {
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    uint32_t w[4];
-#pragma unroll
-    for (int hf = 0; hf < NH; ++hf) {
-      w[2 * hf] = transpose8(pack_bf16(r[hf][4 * i], r[hf][4 * i + 1]));
-      w[2 * hf + 1] = transpose8(pack_bf16(r[hf][4 * i + 2], r[hf][4 * i + 3]));
-    }
-    const int tok = cs + 8 * i + g;
-    if constexpr (NH == 2) {
-      const uint4 v = quad_words(w, t);
-      if (tok < len) *reinterpret_cast<uint4*>(base + tok * stride + 8 * t) = v;
-    } else if (tok < len) {
-      *reinterpret_cast<uint32_t*>(base + tok * stride + 2 * t) = w[0];
-      *reinterpret_cast<uint32_t*>(base + tok * stride + 8 + 2 * t) = w[1];
-    }
+    const float2 x = unpack2(p2[i]);
+    pv[2 * i] = x.x;
+    pv[2 * i + 1] = x.y;
   }
+}
+// ... and its way into a token-major bf16 tile
+template <int NH>
+__device__ __forceinline__ void stage_t(const float (&r)[NH][16], unsigned char* tile, int row0, int cs, int lane) {
+#pragma unroll
+  for (int hf = 0; hf < NH; ++hf) {
+    FragStore fs;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) fs.set(i, r[hf][4 * i], r[hf][4 * i + 1], r[hf][4 * i + 2], r[hf][4 * i + 3]);
+    fs.store_trans(tile, BT, cs, row0 + 16 * hf, lane);
+  }
+}
+// ... and to and from local memory (written out: as an array the compiler would hold it in registers)
+template <int NH>
+__device__ __forceinline__ void st_local(const float (&r)[NH][16], uint64_t at) {
+#pragma unroll
+  for (int e = 0; e < NH * 4; ++e)
+    asm volatile("st.local.v4.f32 [%0], {%1, %2, %3, %4};\n" ::"l"(at + 16 * e), "f"(r[e / 4][4 * (e % 4)]), "f"(r[e / 4][4 * (e % 4) + 1]),
+                 "f"(r[e / 4][4 * (e % 4) + 2]), "f"(r[e / 4][4 * (e % 4) + 3])
+                 : "memory");
+}
+template <int NH>
+__device__ __forceinline__ void add_local(float (&r)[NH][16], uint64_t at) {
+  float x[NH][16];
+#pragma unroll
+  for (int e = 0; e < NH * 4; ++e)
+    asm volatile("ld.local.v4.f32 {%0, %1, %2, %3}, [%4];\n"
+                 : "=f"(x[e / 4][4 * (e % 4)]), "=f"(x[e / 4][4 * (e % 4) + 1]), "=f"(x[e / 4][4 * (e % 4) + 2]), "=f"(x[e / 4][4 * (e % 4) + 3])
+                 : "l"(at + 16 * e)
+                 : "memory");
+  add_t<NH>(r, x);
+}
+
+// 16 x 16 block `b` (row blocks first) of a swizzled [rows][rows] bf16 tile: words {rows 0-7, 8-15} x {columns 0-7, 8-15} in the order
+// of the first operand of mma.m16n8k16; words {0, 2} and {1, 3} are the second operand for the block's rows 0-7 and 8-15
+__device__ __forceinline__ void load_block16(uint32_t tile, int rows, int b, int lane, uint32_t (&x)[4]) {
+  const int per_row = rows / 16;
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];\n"
+               : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3])
+               : "r"(tile + tc5::swz_offset((b / per_row) * 16 + (lane & 15), (b % per_row) * 16 + 8 * (lane >> 4), rows))
+               : "memory");
+}
+__device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};\n"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
 // backward of the L2 norm on such a block: x = d w.r.t. the normalised row -> (x - y <x,y>) rstd, with y the tile, the dots in
@@ -178,22 +239,21 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
   extern __shared__ unsigned char smem_raw[];
   wait_for_predecessor();
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  unsigned char *Ks = smem + S::o_k, *Do = smem + S::o_do, *Qs = Do, *Vn = smem + S::o_vn, *dUs = Vn, *H0 = smem + S::o_h0, *dWt = H0;
-  unsigned char *H1 = smem + S::o_h1, *Vs = H1, *dAs = H1, *M2s = H1, *Ys = H1 + BT * 128;
-  unsigned char *As = smem + S::o_a, *Ps = smem + S::o_ps, *Abs = smem + S::o_ab;
+  unsigned char *Ks = smem + S::o_k, *Do = smem + S::o_do, *Qs = Do, *Vn = smem + S::o_vn, *Vs = Vn, *dUs = smem + S::o_z, *Zt = dUs;
+  unsigned char *Hs = smem + S::o_h, *M2s = Hs, *Dks = Hs, *Dvs = Hs + DK * 128, *Dqs = Zt, *As = smem + S::o_a, *Ps = As;
   float* const gs2 = reinterpret_cast<float*>(smem + S::o_vec);   // [2][64]: a head's and the next one's
   float *bet = gs2 + 2 * BT, *bge = bet + BT, *eg = bge + BT, *sgm = eg + BT, *gx = sgm + BT, *gv = gx + BT, *dGs = gv + BT, *rsq = dGs + BT, *rsk = rsq + BT;
   // sums over rows: each of the four row-quadrant warps leaves its partial in its own slot and the consumer adds the four in
   // a fixed order (no atomics: results are bit-reproducible)
   float* c_rq = rsk + BT;        // [4][64] <dq_i, q_i>
   float* c_rk = c_rq + 4 * BT;   // [4][64] <dk_loc_i, k_i> + c_mk
-  float* c_kbg = c_rk + 4 * BT;  // [4][64] colsum(A . dW K^T)
-  float* c_vb = c_kbg + 4 * BT;  // [4][64] colsum(A . dU V^T)
+  float* c_kz = c_rk + 4 * BT;   // [4][64] -<h Z_i, k_i>
+  float* c_vb = c_kz + 4 * BT;   // [4][64] <Z_i, v_i>
   float* r_mk = c_vb + 4 * BT;   // [2][64] rowsum(M . K K^T), two column halves
   float* red = r_mk + 2 * BT;    // [0..7] <h,dh> per warp, [8..15] sum of <dk_state, k> per warp, [16..19] gate sums
   uint64_t* bar = reinterpret_cast<uint64_t*>(red + 20);
-  uint64_t *bar_a = bar + 1, *bar_k = bar + 2, *bar_b = bar + 3, *bar_c = bar + 4;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar + 5);
+  uint64_t *bar_a = bar + 1, *bar_b = bar + 2, *bar_c = bar + 3;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar + 4);
 
   const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int q = warp & 3, hc = warp >> 2, g = lane >> 2, t = lane & 3;
@@ -203,26 +263,27 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
   const int64_t row0 = cm.row;
   const int r_lo = q * 16 + g, r_hi = r_lo + 8, cs = hc * 32;   // this warp's block of a [64][64] tile
   const int kr = (DK / 4) * q;                                  // ... and its first row of a transposed accumulator
+  const bool live = q * 16 + 15 >= cs;                          // some of that block is on or below the diagonal
   const int gcol = cs + 8 * (g >> 1) + 2 * t + (g & 1);         // the column whose sum sum8_over_g leaves in this lane
 
-  // one thread: what a head's first phases need, and the rest into L2
+  // one thread: what a head's first phase needs, and the rest into L2
   auto load_head = [&](int hv, bool first) {
     const int hrow = (c * a.HV + hv) * DK;   // the head's state snapshot in the [.., V] view
-    tc5::mbar_expect_tx(bar_a, (uint32_t)(2 * S::tile + NP * DK * 128 + BT * 4));
+    tc5::mbar_expect_tx(bar_a, (uint32_t)((first ? 4 : 3) * S::tile + DK * DK * 2 + BT * 128 + BT * 4));
     tma::load_3d(Do, &maps.d_o, cm.row, (hv * DK) / 64, bar_a);
     tma::load_3d(Vn, &maps.vn, cm.row, (hv * DK) / 64, bar_a);
+    tma::load_3d(dUs, &maps.du, cm.row, (hv * DK) / 64, bar_a);
+    tma::load_2d(As, &maps.a, hv * BT, cm.row, bar_a);
     tma::load_1d(gs2 + ((hv - hv0) & 1) * BT, gamma_ptr(a.gamma, c, a.HV, hv), BT * 4, bar_a);
-    for (int p = 0; p < NP; ++p) tma::load_2d(p ? H1 : H0, &maps.dh, p * 64, hrow, bar_a);
-    tc5::mbar_expect_tx(bar_k, (uint32_t)((first ? S::tile : 0) + BT * 128));
-    if (first) tma::load_3d(Ks, &maps.k, cm.row, (hq * DK) / 64, bar_k);
-    tma::load_2d(As, &maps.a, hv * BT, cm.row, bar_k);
+    if (first) tma::load_3d(Ks, &maps.k, cm.row, (hq * DK) / 64, bar_a);
+    else tma::store_wait_read<0>();   // dv of the head before leaves from this place
+    for (int p = 0; p < NP; ++p) tma::load_2d(Hs + p * DK * 128, &maps.dh, p * 64, hrow, bar_a);
     for (int p = 0; p < NP; ++p) tma::prefetch_2d(&maps.h, p * 64, hrow);
-    tma::prefetch_3d(&maps.du, cm.row, (hv * DK) / 64);
     if (first) tma::prefetch_3d(&maps.q, cm.row, (hq * DK) / 64);
     tma::prefetch_3d(&maps.v, cm.row, (hv * DK) / 64);
   };
   if (tid == 0) {
-    for (int i = 0; i < 5; ++i) tc5::mbar_init(bar + i, 1);
+    for (int i = 0; i < 4; ++i) tc5::mbar_init(bar + i, 1);
     tc5::fence_mbar_init();
     load_head(hv0, true);
   }
@@ -259,14 +320,13 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
   const uint32_t tm = *tmem_slot;
   const uint32_t C0 = tm, C1 = tm + 64, C2 = tm + 128, C3 = tm + 192;
   PhaseBarrier ph{bar, 0u, &g_local_timeout};
-  const uint32_t sK = tc5::smem_addr(Ks), sDo = tc5::smem_addr(Do), sVn = tc5::smem_addr(Vn), sH0 = tc5::smem_addr(H0), sH1 = tc5::smem_addr(H1);
-  const uint32_t sA = tc5::smem_addr(As), sP = tc5::smem_addr(Ps), sAb = tc5::smem_addr(Abs);
+  const uint32_t sK = tc5::smem_addr(Ks), sDo = tc5::smem_addr(Do), sVn = tc5::smem_addr(Vn), sZ = tc5::smem_addr(Zt), sH = tc5::smem_addr(Hs);
+  const uint32_t sA = tc5::smem_addr(As);
   const Operand opK_k{sK, BT, 0}, opK_mn{sK, BT, 1};      // K as (rows = token, contraction = key dim), and the reverse
-  const Operand opA_k{sA, BT, 0}, opA_mn{sA, BT, 1};
   bool failed = false;
-  // turns: this thread's part of the sum of dk over the heads, in local memory between them
-  __align__(16) float dk_local[MODE == kTurns ? 16 * NH : 4];
-  const uint64_t dk_sum = __cvta_generic_to_local(dk_local);
+  // several heads: this thread's part of dq and (turns) of the sums of dq and dk so far, in local memory between their uses
+  __align__(16) float sums_local[MODE != kOne ? 32 * NH : 4];
+  const uint64_t dq_sum = __cvta_generic_to_local(sums_local), dk_sum = dq_sum + 64 * NH;
 
   for (int hh = 0; hh < n_heads; ++hh) {
     const int hv = hv0 + hh, hrow = (c * a.HV + hv) * DK;
@@ -277,54 +337,61 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
     if (cm.len < BT) {   // ragged chunk: the extra rows of the boxes belong to the next sequence
       zero_tail_rows<BT, DK>(Do, cm.len, tid, NTHREADS);
       zero_tail_rows<BT, DK>(Vn, cm.len, tid, NTHREADS);
+      zero_tail_rows<BT, DK>(dUs, cm.len, tid, NTHREADS);
+      zero_tail_rows<BT, BT>(As, cm.len, tid, NTHREADS);
+      if (first) zero_tail_rows<BT, DK>(Ks, cm.len, tid, NTHREADS);
       tc5::fence_async_smem();
     }
     if (__syncthreads_or(failed)) { failed = true; break; }
 
-    // ---- phase 1: dP = do v_new^T | dk_state^T = dh v_new^T (column factor later)
+    // ---- phase 1: Z^T = dU^T A | dP = do v_new^T | dk_state^T = dh v_new^T (column factor later)
     if (warp == 0) {
       tc5::fence_after_sync();
+      issue_mma_t<BT / 16>(C2, Operand{sZ, BT, 1}, Operand{sA, BT, 1}, DK, 64, 0);
       issue_mma_t<DK / 16>(C0, Operand{sDo, BT, 0}, Operand{sVn, BT, 0}, 64, 64, 0);
 #pragma unroll
       for (int p = 0; p < NP; ++p)
-        issue_mma_t<4>(C3, Operand{p ? sH1 : sH0, DK, 0}, Operand{sVn + p * BT * 128, BT, 0}, DK, 64, p > 0);
+        issue_mma_t<4>(C3, Operand{sH + p * DK * 128, DK, 0}, Operand{sVn + p * BT * 128, BT, 0}, DK, 64, p > 0);
       ph.commit();
     }
+    // dh into registers (for <h,dh>) meanwhile
+    constexpr int ND = DK * DK / 256 / 8;   // 16 x 16 blocks per warp
+    uint32_t dhr[ND][4];
+#pragma unroll
+    for (int n = 0; n < ND; ++n) load_block16(sH, DK, warp * ND + n, lane, dhr[n]);
     const float g_lo = gs[r_lo], g_hi = gs[r_hi], glast = gs[BT - 1];
     if (tid < BT) {
       const float e = fast_exp2(gs[tid]);
       eg[tid] = e;
       bge[tid] = bet[tid] * e;
     }
-    if (!tc5::mbar_wait(bar_k, par)) failed = true;
-    if (cm.len < BT) {
-      if (first) zero_tail_rows<BT, DK>(Ks, cm.len, tid, NTHREADS);
-      zero_tail_rows<BT, BT>(As, cm.len, tid, NTHREADS);
-      tc5::fence_async_smem();
-    }
-    if (__syncthreads_or(failed || !ph.wait())) { failed = true; break; }
-
-    // ---- epilogue 1: dh into registers (for <h,dh>), then h takes its place and dU the place of v_new
-    constexpr int ND = DK * 8 * NP / NTHREADS;
-    uint4 dhr[ND];
-#pragma unroll
-    for (int n = 0; n < ND; ++n) {
-      const int idx = tid + n * NTHREADS;   // 16-byte words of both panels; the same positions are read in h
-      dhr[n] = *reinterpret_cast<const uint4*>((idx < DK * 8 ? H0 : H1 - DK * 128) + idx * 16);
-    }
     // the reads above are only issued: without this fence the copy of h can overtake those still queued
     tc5::fence_async_smem();
-    __syncthreads();
+    if (__syncthreads_or(!ph.wait())) { failed = true; break; }
+
+    // ---- epilogue 1: h takes the place of dh, Z^T that of dU, dP~ that of A
     if (tid == 0) {
-      tc5::mbar_expect_tx(bar_b, (uint32_t)(NP * DK * 128 + S::tile));
-      for (int p = 0; p < NP; ++p) tma::load_2d(p ? H1 : H0, &maps.h, p * 64, hrow, bar_b);
-      tma::load_3d(dUs, &maps.du, cm.row, (hv * DK) / 64, bar_b);
+      tc5::mbar_expect_tx(bar_b, (uint32_t)(DK * DK * 2));
+      for (int p = 0; p < NP; ++p) tma::load_2d(Hs + p * DK * 128, &maps.h, p * 64, hrow, bar_b);
+    }
+    {   // Z -> shared; it stays in C2 as well
+      float r[NH][16];
+      acc_ld_t<NH>(C2, q, cs, r);
+      tc5::tmem_ld_wait();
+#pragma unroll
+      for (int hf = 0; hf < NH; ++hf) {
+        FragStore fs;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) fs.set(i, r[hf][4 * i], r[hf][4 * i + 1], r[hf][4 * i + 2], r[hf][4 * i + 3]);
+        fs.store(Zt, DK, kr + 16 * hf, cs, lane);
+      }
     }
     {   // dP~ -> shared
       float r[16];
+      FragStore fs = {};
+      if (live) {
       acc_ld32q(C0, q, cs, r);
       tc5::tmem_ld_wait();
-      FragStore fs;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int j0 = cs + i * 8 + 2 * t;
@@ -336,6 +403,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
           v[e] = (ii >= jj) ? r[4 * i + e] * a.scale * fast_exp2(((e & 2) ? g_hi : g_lo) - ((e & 1) ? gj.y : gj.x)) : 0.f;
         }
         fs.set(i, v[0], v[1], v[2], v[3]);
+      }
       }
       fs.store(Ps, BT, q * 16, cs, lane);
     }
@@ -353,92 +421,90 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
       }
       *po = x;
     }
-    float dk_dot;   // this lane's part of c_rk
-    {   // dk_state^T: column factors, the sum of its dots with k, back to TMEM where the other terms of dk accumulate
-      float r[NH][16];
-      acc_ld_t<NH>(C3, q, cs, r);
+    float dk_dot;       // this lane's part of c_rk
+    float rk[NH][16];   // dk as far as it is known
+    {   // dk_state^T: column factors, the sum of its dots with k
+      acc_ld_t<NH>(C3, q, cs, rk);
       tc5::tmem_ld_wait();
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const float2 gj = *reinterpret_cast<const float2*>(&gs[cs + i * 8 + 2 * t]);
-        const float e0 = fast_exp2(glast - gj.x), e1 = fast_exp2(glast - gj.y);
-#pragma unroll
-        for (int hf = 0; hf < NH; ++hf) {
-          r[hf][4 * i] *= e0; r[hf][4 * i + 1] *= e1; r[hf][4 * i + 2] *= e0; r[hf][4 * i + 3] *= e1;
-        }
+        scale_t<NH>(rk, i, make_float2(fast_exp2(glast - gj.x), fast_exp2(glast - gj.y)));
       }
-#pragma unroll
-      for (int hf = 0; hf < NH; ++hf) tc5::tmem_st_16x256b_x4(C3 + ((uint32_t)(32 * q + 16 * hf) << 16) + cs, r[hf]);
       float pv[8];
-      dots_t<NH>(r, Ks, kr, cs, lane, pv);
+      dots_t<NH>(rk, Ks, kr, cs, lane, pv);
       dk_dot = sum8_over_g(pv, g);
       const float rs = warp_sum(dk_dot);
       if (lane == 0) red[8 + warp] = rs;
-      tc5::tmem_st_wait();
     }
     if (!tc5::mbar_wait(bar_b, par)) failed = true;
-    if (cm.len < BT) zero_tail_rows<BT, DK>(dUs, cm.len, tid, NTHREADS);
     {
-      float hd = 0.f;
+      float d0[4] = {0.f, 0.f, 0.f, 0.f}, d1[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
       for (int n = 0; n < ND; ++n) {
-        const int idx = tid + n * NTHREADS;
-        const uint4 x = *reinterpret_cast<const uint4*>((idx < DK * 8 ? H0 : H1 - DK * 128) + idx * 16);
-        const uint32_t xu[4] = {x.x, x.y, x.z, x.w}, yu[4] = {dhr[n].x, dhr[n].y, dhr[n].z, dhr[n].w};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float2 p = unpack_bf16(xu[e]), y = unpack_bf16(yu[e]);
-          hd += p.x * y.x + p.y * y.y;
-        }
+        uint32_t x[4];
+        load_block16(sH, DK, warp * ND + n, lane, x);
+        mma16816(d0, dhr[n], x[0], x[2]);
+        mma16816(d1, dhr[n], x[1], x[3]);
       }
-      hd = warp_sum(hd);
+      const float hd = warp_sum((g == 2 * t ? d0[0] + d1[2] : 0.f) + (g == 2 * t + 1 ? d0[1] + d1[3] : 0.f));
       if (lane == 0) red[warp] = hd;
     }
     tc5::fence_async_smem();
     tc5::fence_before_sync();
     if (__syncthreads_or(failed)) { failed = true; break; }
 
-    // ---- phase 2: dq^T = h do_s^T + K^T dP~^T | dW^T = -h dU^T
+    // ---- phase 2: ZV = Z v_new^T | -h Z^T | dq^T = h do_s^T + K^T dP~^T
     if (warp == 0) {
       tc5::fence_after_sync();
+      issue_mma_t<DK / 16>(C1, Operand{sZ, DK, 1}, Operand{sVn, BT, 0}, 64, 64, 0);
 #pragma unroll
       for (int p = 0; p < NP; ++p) {
-        issue_mma_t<4>(C2, Operand{p ? sH1 : sH0, DK, 0}, Operand{sVn + p * BT * 128, BT, 0}, DK, 64, p > 0, /*neg_a=*/1);
-        issue_mma_t<4>(C0, Operand{p ? sH1 : sH0, DK, 0}, Operand{sDo + p * BT * 128, BT, 0}, DK, 64, p > 0);
+        issue_mma_t<4>(C3, Operand{sH + p * DK * 128, DK, 0}, Operand{sZ + p * BT * 128, DK, 1}, DK, 64, p > 0, /*neg_a=*/1);
+        issue_mma_t<4>(C0, Operand{sH + p * DK * 128, DK, 0}, Operand{sDo + p * BT * 128, BT, 0}, DK, 64, p > 0);
       }
-      issue_mma_t<4>(C0, opK_mn, Operand{sP, BT, 0}, DK, 64, 1);
+      issue_mma_t<4>(C0, opK_mn, Operand{sA, BT, 0}, DK, 64, 1);
       ph.commit();
-    }
-    {   // A with its columns scaled by beta 2^gamma, while phase 2 runs
-      FragLoad fa;
-      fa.load(As, BT, q * 16, cs, lane);
-      FragStore fs;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float2 sc = *reinterpret_cast<const float2*>(&bge[cs + i * 8 + 2 * t]);
-        const float2 al = fa.lo2(i), ah = fa.hi2(i);
-        fs.set(i, al.x * sc.x, al.y * sc.y, ah.x * sc.x, ah.y * sc.y);
-      }
-      fs.store(Abs, BT, q * 16, cs, lane);
     }
     if (__syncthreads_or(!ph.wait())) { failed = true; break; }
 
-    // ---- epilogue 2: q takes the place of do, V that of the second h panel; dW^T -> shared (over the first)
+    // ---- epilogue 2: q takes the place of do, V that of v_new; M2 -> shared (over h)
     if (tid == 0) {
       tc5::mbar_expect_tx(bar_c, (uint32_t)(2 * S::tile));
-      tma::load_3d(Vs, &maps.v, cm.row, (hv * DK) / 64, bar_c);
       tma::load_3d(Qs, &maps.q, cm.row, (hq * DK) / 64, bar_c);
+      tma::load_3d(Vs, &maps.v, cm.row, (hv * DK) / 64, bar_c);
     }
+    float m[16];   // M, later its products with K K^T
     {
-      float r[NH][16];
-      acc_ld_t<NH>(C2, q, cs, r);
+      FragStore fs = {};
+      if (live) {
+        const float b_lo = bet[r_lo], b_hi = bet[r_hi];
+        acc_ld32q(C1, q, cs, m);
+        tc5::tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int col = cs + i * 8 + 2 * t;
+          const float2 gj = *reinterpret_cast<const float2*>(&gs[col]);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int ii = (e & 2) ? r_hi : r_lo, jj = col + (e & 1);
+            m[4 * i + e] = (ii > jj) ? -m[4 * i + e] * fast_exp2(((e & 2) ? g_hi : g_lo) - ((e & 1) ? gj.y : gj.x)) : 0.f;
+          }
+          fs.set(i, m[4 * i] * b_lo, m[4 * i + 1] * b_lo, m[4 * i + 2] * b_hi, m[4 * i + 3] * b_hi);
+        }
+      }
+      fs.store(M2s, BT, q * 16, cs, lane);
+    }
+    {   // -h Z^T: its dots with k; into dk with the factor beta 2^gamma
+      float r[NH][16], pv[8];
+      acc_ld_t<NH>(C3, q, cs, r);
       tc5::tmem_ld_wait();
+      dots_t<NH>(r, Ks, kr, cs, lane, pv);
+      c_kz[q * BT + gcol] = sum8_over_g(pv, g);
 #pragma unroll
-      for (int hf = 0; hf < NH; ++hf) {
-        FragStore fs;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) fs.set(i, r[hf][4 * i], r[hf][4 * i + 1], r[hf][4 * i + 2], r[hf][4 * i + 3]);
-        fs.store(dWt, DK, kr + 16 * hf, cs, lane);
+      for (int i = 0; i < 4; ++i) {
+        const float2 bg = *reinterpret_cast<const float2*>(&bge[cs + i * 8 + 2 * t]);
+        scale_add_t<NH>(rk, r, i, bg);
       }
     }
     float rq[NH][16];   // dq: C0 is phase 3's
@@ -453,226 +519,117 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
     tc5::fence_before_sync();
     if (__syncthreads_or(failed)) { failed = true; break; }
 
-    // ---- phase 3: dA1 = dW K^T | dA2 = dU V^T
+    // ---- phase 3: the rest of dk^T = q^T dP~ + K^T M2^T + K^T M2 | KK = K K^T | QK = Q K^T
     if (warp == 0) {
       tc5::fence_after_sync();
-      issue_mma_t<DK / 16>(C2, Operand{sH0, DK, 1}, opK_k, 64, 64, 0);
-      issue_mma_t<DK / 16>(C0, Operand{sVn, BT, 0}, Operand{sH1, BT, 0}, 64, 64, 0);
+      issue_mma_t<BT / 16>(C3, opK_mn, Operand{sH, BT, 0}, DK, 64, 0);
+      issue_mma_t<BT / 16>(C3, opK_mn, Operand{sH, BT, 1}, DK, 64, 1);
+      issue_mma_t<BT / 16>(C3, Operand{sDo, BT, 1}, Operand{sA, BT, 1}, DK, 64, 1);
+      issue_mma_t<DK / 16>(C0, opK_k, opK_k, 64, 64, 0);
+      issue_mma_t<DK / 16>(C1, Operand{sDo, BT, 0}, opK_k, 64, 64, 0);
       ph.commit();
     }
-    {   // dq: its dots with q, the sum over the heads (C1); ungrouped heads, and the last one in turn: it leaves
+    {   // dq: its dots with q, the sum over the heads; ungrouped heads, and the last one in turn: on its way out, over Z^T
       float pv[8];
       dots_t<NH>(rq, Qs, kr, cs, lane, pv);
       c_rq[q * BT + gcol] = sum8_over_g(pv, g);
-      if (!first) {
-        float acc[NH][16];
-        acc_ld_t<NH>(C1, q, cs, acc);
-        tc5::tmem_ld_wait();
-        add_t<NH>(rq, acc);
-      }
+      if (!first) add_local<NH>(rq, dq_sum);
       if (GROUPED || !last) {
-#pragma unroll
-        for (int hf = 0; hf < NH; ++hf) tc5::tmem_st_16x256b_x4(C1 + ((uint32_t)(32 * q + 16 * hf) << 16) + cs, rq[hf]);
-        tc5::tmem_st_wait();
+        st_local<NH>(rq, dq_sum);
       } else {
         if (a.rstd_q != nullptr) {
           float* dots = c_rq;
-          if (MODE == kTurns) {   // of the sum; c_kbg is free until epilogue 3
-            dots = c_kbg;
+          if (MODE == kTurns) {   // of the sum; c_rk is free until epilogue 3
+            dots = c_rk;
             dots_t<NH>(rq, Qs, kr, cs, lane, pv);
             dots[q * BT + gcol] = sum8_over_g(pv, g);
           }
           __syncthreads();
           l2_backward_t<NH>(rq, Qs, dots, rsq, kr, cs, lane);
         }
-        store_t<NH>(rq, reinterpret_cast<__nv_bfloat16*>(a.dq) + (row0 * a.H + hq) * DK + kr, (int64_t)a.H * DK, cs, cm.len, g, t);
+        stage_t<NH>(rq, Dqs, kr, cs, lane);
       }
     }
-    if (__syncthreads_or(!ph.wait())) { failed = true; break; }
-
-    // ---- epilogue 3: dA -> shared (over V)
-    {
-      float r[16], dA2[16];
-      acc_ld32q(C2, q, cs, r);
-      acc_ld32q(C0, q, cs, dA2);
+    {   // Z: its dots with v; dv = beta Z on its way out, over the second panel of h
+      float z[NH][16], pv[8];
+      acc_ld_t<NH>(C2, q, cs, z);
       tc5::tmem_ld_wait();
-      FragStore fs;
+      dots_t<NH>(z, Vs, kr, cs, lane, pv);
+      c_vb[q * BT + gcol] = sum8_over_g(pv, g);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int col = cs + i * 8 + 2 * t;
-        const float2 bg = *reinterpret_cast<const float2*>(&bge[col]), bj = *reinterpret_cast<const float2*>(&bet[col]);
-        float v[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int ii = (e & 2) ? r_hi : r_lo, jj = col + (e & 1);
-          v[e] = (ii > jj) ? r[4 * i + e] * ((e & 1) ? bg.y : bg.x) + dA2[4 * i + e] * ((e & 1) ? bj.y : bj.x) : 0.f;
-        }
-        fs.set(i, v[0], v[1], v[2], v[3]);
-      }
-      fs.store(dAs, BT, q * 16, cs, lane);
-      tc5::fence_async_smem();
-      tc5::fence_before_sync();
-      __syncthreads();
-      // ---- phase 4: Y = dA A^T (all the chain waits for) | KK = K K^T
-      if (warp == 0) {
-        tc5::fence_after_sync();
-        issue_mma_t<BT / 16>(C2, Operand{sH1, BT, 0}, opA_k, 64, 64, 0);
-        ph.commit();
-        issue_mma_t<DK / 16>(C0, opK_k, opK_k, 64, 64, 0);
-      }
-      FragLoad fa;
-      fa.load(As, BT, q * 16, cs, lane);
-      float pv[8], pw[8];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float2 al = fa.lo2(i), ah = fa.hi2(i);
-        pv[2 * i] = al.x * r[4 * i] + ah.x * r[4 * i + 2];
-        pv[2 * i + 1] = al.y * r[4 * i + 1] + ah.y * r[4 * i + 3];
-        pw[2 * i] = al.x * dA2[4 * i] + ah.x * dA2[4 * i + 2];
-        pw[2 * i + 1] = al.y * dA2[4 * i + 1] + ah.y * dA2[4 * i + 3];
-      }
-      c_kbg[q * BT + gcol] = sum8_over_g(pv, g);
-      c_vb[q * BT + gcol] = sum8_over_g(pw, g);
+      for (int i = 0; i < 4; ++i) scale_t<NH>(z, i, *reinterpret_cast<const float2*>(&bet[cs + i * 8 + 2 * t]));
+      stage_t<NH>(z, Dvs, kr, cs, lane);
     }
-    if (__syncthreads_or(!ph.wait())) { failed = true; break; }
-
-    // ---- epilogue 4: Y -> shared
-    {
-      float r[16];
-      acc_ld32q(C2, q, cs, r);
-      tc5::tmem_ld_wait();
-      FragStore fs;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) fs.set(i, r[4 * i], r[4 * i + 1], r[4 * i + 2], r[4 * i + 3]);
-      fs.store(Ys, BT, q * 16, cs, lane);
-    }
-    tc5::fence_async_smem();
+    FragLoad fp;
+    fp.load(Ps, BT, q * 16, cs, lane);
+    tc5::fence_async_smem();   // the staged tiles are read, and what was read here is overwritten, by bulk copies
     tc5::fence_before_sync();
-    __syncthreads();
-
-    // ---- phase 5: X = A^T Y (all the chain waits for) | dk^T += q^T dP~ + dW^T A_b
-    if (warp == 0) {
-      tc5::fence_after_sync();
-      issue_mma_t<BT / 16>(C2, opA_mn, Operand{sH1 + BT * 128, BT, 1}, 64, 64, 0);
-      ph.commit();
-      issue_mma_t<BT / 16>(C3, Operand{sDo, BT, 1}, Operand{sP, BT, 1}, DK, 64, 1);
-      issue_mma_t<BT / 16>(C3, Operand{sH0, DK, 0}, Operand{sAb, BT, 1}, DK, 64, 1);
-    }
     if (__syncthreads_or(!ph.wait())) { failed = true; break; }
+    if (cm.len == BT) {
+      if (tid == 0) {
+        tma::store_3d(&maps.dv, cm.row, (hv * DK) / 64, Dvs);
+        if (!GROUPED && last) tma::store_3d(&maps.dq, cm.row, (hq * DK) / 64, Dqs);
+        tma::store_commit();
+      }
+    } else {
+      store_tile_swz<BT, DK, NTHREADS>(reinterpret_cast<__nv_bfloat16*>(a.dv) + (row0 * a.HV + hv) * DK, (int64_t)a.HV * DK, Dvs, cm.len, tid);
+      if (!GROUPED && last)
+        store_tile_swz<BT, DK, NTHREADS>(reinterpret_cast<__nv_bfloat16*>(a.dq) + (row0 * a.H + hq) * DK, (int64_t)a.H * DK, Dqs, cm.len, tid);
+      if (!last) {
+        tc5::fence_async_smem();
+        __syncthreads();
+      }
+    }
+    if (!last && tid == 0) load_head(hv + 1, false);   // every tile but K is dead
 
-    // ---- epilogue 5: M2 -> shared
+    // ---- epilogue 3: dk and the gate and beta gradients
     {
-      const float b_lo = bet[r_lo], b_hi = bet[r_hi];
-      float m[16], kk[16];
-      acc_ld32q(C2, q, cs, m);
+      float kk[16], qk[16], pv[8], rmk_lo = 0.f, rmk_hi = 0.f;   // (blocks above the diagonal hold zeros)
+      if (live) {
       acc_ld32q(C0, q, cs, kk);
+      acc_ld32q(C1, q, cs, qk);
       tc5::tmem_ld_wait();
-      FragStore fs;
-      float rmk_lo = 0.f, rmk_hi = 0.f, pv[8];
+      const float b_lo = bet[r_lo], b_hi = bet[r_hi];
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const int col = cs + i * 8 + 2 * t;
-        const float2 gj = *reinterpret_cast<const float2*>(&gs[col]);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int ii = (e & 2) ? r_hi : r_lo, jj = col + (e & 1);
-          m[4 * i + e] = (ii > jj) ? -m[4 * i + e] * fast_exp2(((e & 2) ? g_hi : g_lo) - ((e & 1) ? gj.y : gj.x)) : 0.f;
-        }
-        rmk_lo += m[4 * i] * kk[4 * i] + m[4 * i + 1] * kk[4 * i + 1];
-        rmk_hi += m[4 * i + 2] * kk[4 * i + 2] + m[4 * i + 3] * kk[4 * i + 3];
-        m[4 * i] *= b_lo; m[4 * i + 1] *= b_lo; m[4 * i + 2] *= b_hi; m[4 * i + 3] *= b_hi;
-        pv[2 * i] = m[4 * i] * kk[4 * i] + m[4 * i + 2] * kk[4 * i + 2];
-        pv[2 * i + 1] = m[4 * i + 1] * kk[4 * i + 1] + m[4 * i + 3] * kk[4 * i + 3];
-        fs.set(i, m[4 * i], m[4 * i + 1], m[4 * i + 2], m[4 * i + 3]);
+        for (int e = 0; e < 4; ++e) m[4 * i + e] *= kk[4 * i + e];
+        rmk_lo += m[4 * i] + m[4 * i + 1];
+        rmk_hi += m[4 * i + 2] + m[4 * i + 3];
+        const float2 pl = fp.lo2(i), phi = fp.hi2(i);
+        pv[2 * i] = (m[4 * i] * b_lo + m[4 * i + 2] * b_hi) + (pl.x * qk[4 * i] + phi.x * qk[4 * i + 2]);
+        pv[2 * i + 1] = (m[4 * i + 1] * b_lo + m[4 * i + 3] * b_hi) + (pl.y * qk[4 * i + 1] + phi.y * qk[4 * i + 3]);
       }
       dk_dot += sum8_over_g(pv, g);
-      fs.store(M2s, BT, q * 16, cs, lane);
       rmk_lo = sum_over_t(rmk_lo);
       rmk_hi = sum_over_t(rmk_hi);
+      }
+      c_rk[q * BT + gcol] = dk_dot;
       if (t == 0) {
         r_mk[hc * BT + r_lo] = rmk_lo;
         r_mk[hc * BT + r_hi] = rmk_hi;
       }
-    }
-    tc5::fence_async_smem();
-    tc5::fence_before_sync();
-    __syncthreads();
-
-    // ---- phase 6: dv^T = dU^T A | dk^T += K^T M2^T + K^T M2 | QK = Q K^T
-    if (warp == 0) {
-      tc5::fence_after_sync();
-      issue_mma_t<BT / 16>(C2, Operand{sVn, BT, 1}, opA_mn, DK, 64, 0);
-      ph.commit();
-      issue_mma_t<BT / 16>(C3, opK_mn, Operand{sH1, BT, 0}, DK, 64, 1);
-      issue_mma_t<BT / 16>(C3, opK_mn, Operand{sH1, BT, 1}, DK, 64, 1);
-      issue_mma_t<DK / 16>(C0, Operand{sDo, BT, 0}, opK_k, 64, 64, 0);
-    }
-    if (__syncthreads_or(!ph.wait())) { failed = true; break; }
-    if (warp == 0) ph.commit();   // ... of the rest
-    {
       float r[NH][16];
-      acc_ld_t<NH>(C2, q, cs, r);
+      acc_ld_t<NH>(C3, q, cs, r);
       tc5::tmem_ld_wait();
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float2 bj = *reinterpret_cast<const float2*>(&bet[cs + i * 8 + 2 * t]);
-#pragma unroll
-        for (int hf = 0; hf < NH; ++hf) {
-          r[hf][4 * i] *= bj.x; r[hf][4 * i + 1] *= bj.y; r[hf][4 * i + 2] *= bj.x; r[hf][4 * i + 3] *= bj.y;
-        }
-      }
-      store_t<NH>(r, reinterpret_cast<__nv_bfloat16*>(a.dv) + (row0 * a.HV + hv) * DK + kr, (int64_t)a.HV * DK, cs, cm.len, g, t);
-    }
-    if (__syncthreads_or(!ph.wait())) { failed = true; break; }
-    if (!last && tid == 0) load_head(hv + 1, false);   // every tile but K is dead
-
-    // ---- epilogue 6: dk and the gate and beta gradients
-    float rk[NH][16];
-    {
-      float pv[8], qk[16];
-      acc_ld32q(C0, q, cs, qk);
-      acc_ld_t<NH>(C3, q, cs, rk);
-      tc5::tmem_ld_wait();
-      FragLoad fp;
-      fp.load(Ps, BT, q * 16, cs, lane);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float2 pl = fp.lo2(i), phi = fp.hi2(i);
-        pv[2 * i] = pl.x * qk[4 * i] + phi.x * qk[4 * i + 2];
-        pv[2 * i + 1] = pl.y * qk[4 * i + 1] + phi.y * qk[4 * i + 3];
-      }
-      c_rk[q * BT + gcol] = dk_dot + sum8_over_g(pv, g);
+      add_t<NH>(rk, r);
       if (MODE == kTurns) {
-        if (!first) {
-          float acc[NH][16];
-#pragma unroll
-          for (int e = 0; e < NH * 4; ++e)
-            asm volatile("ld.local.v4.f32 {%0, %1, %2, %3}, [%4];\n"
-                         : "=f"(acc[e / 4][4 * (e % 4)]), "=f"(acc[e / 4][4 * (e % 4) + 1]), "=f"(acc[e / 4][4 * (e % 4) + 2]),
-                           "=f"(acc[e / 4][4 * (e % 4) + 3])
-                         : "l"(dk_sum + 16 * e)
-                         : "memory");
-          add_t<NH>(rk, acc);
-        }
-        if (!last) {
-#pragma unroll
-          for (int e = 0; e < NH * 4; ++e)
-            asm volatile("st.local.v4.f32 [%0], {%1, %2, %3, %4};\n" ::"l"(dk_sum + 16 * e), "f"(rk[e / 4][4 * (e % 4)]),
-                         "f"(rk[e / 4][4 * (e % 4) + 1]), "f"(rk[e / 4][4 * (e % 4) + 2]), "f"(rk[e / 4][4 * (e % 4) + 3])
-                         : "memory");
-        }
+        if (!first) add_local<NH>(rk, dk_sum);
+        if (!last) st_local<NH>(rk, dk_sum);
       }
       if (!GROUPED && last && a.rstd_k != nullptr) {   // <dk, k> for the norm's backward, over a tile that is needed no more
         dots_t<NH>(rk, Ks, kr, cs, lane, pv);
-        reinterpret_cast<float*>(Vn)[q * BT + gcol] = sum8_over_g(pv, g);
+        reinterpret_cast<float*>(Ps)[q * BT + gcol] = sum8_over_g(pv, g);
       }
     }
+    if (GROUPED && tid == 0) tma::store_wait_read<0>();   // the sums are staged over dv
+    tc5::fence_before_sync();   // the next head's first phase writes what was read here
     __syncthreads();
     if (tid < BT) {
       const int i = tid;
       auto sum4 = [&](const float* v) { return (v[i] + v[BT + i]) + (v[2 * BT + i] + v[3 * BT + i]); };
-      const float rmk = r_mk[i] + r_mk[BT + i], ckbg = sum4(c_kbg);
-      float x = sum4(c_rq) - sum4(c_rk) + (ckbg * bge[i] + bet[i] * rmk);
+      const float rmk = r_mk[i] + r_mk[BT + i], ckz = sum4(c_kz);
+      float x = sum4(c_rq) - sum4(c_rk) + (ckz * bge[i] + bet[i] * rmk);
       if (i == cm.len - 1) {
         float sh = 0.f, sr = 0.f;
 #pragma unroll
@@ -683,7 +640,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
         x += fast_exp2(glast) * sh + sr;
       }
       if (i < cm.len) {
-        float db = ckbg * eg[i] + sum4(c_vb) + rmk;
+        float db = ckz * eg[i] + sum4(c_vb) + rmk;
         if (a.options & B200GDN_PREP_BETA_SIGMOID)   // chain rule through (1|2) sigmoid
           db *= ((a.options & B200GDN_PREP_NEG_EIGVAL) ? 2.f : 1.f) * sgm[i] * (1.f - sgm[i]);
         st_param(a.dbeta, (row0 + i) * a.HV + hv, a.gb_dtype, db);
@@ -699,15 +656,15 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
       dGs[i] = x;
     }
     if (!GROUPED && last) {
-      if (a.rstd_k != nullptr) l2_backward_t<NH>(rk, Ks, reinterpret_cast<float*>(Vn), rsk, kr, cs, lane);
-      store_t<NH>(rk, reinterpret_cast<__nv_bfloat16*>(a.dk) + (row0 * a.H + hq) * DK + kr, (int64_t)a.H * DK, cs, cm.len, g, t);
+      if (a.rstd_k != nullptr) l2_backward_t<NH>(rk, Ks, reinterpret_cast<float*>(Ps), rsk, kr, cs, lane);
+      stage_t<NH>(rk, Dks, kr, cs, lane);   // over M2
+      tc5::fence_async_smem();
     } else if (GROUPED) {
       // this head's dq and dk in fp32, token-major, over the dead tiles
       float* sq = reinterpret_cast<float*>(smem + S::o_do);
       float* sk = reinterpret_cast<float*>(smem + S::o_do + S::stage);
-      float r[NH][16];
-      acc_ld_t<NH>(C1, q, cs, r);
-      tc5::tmem_ld_wait();
+      float r[NH][16] = {};
+      add_local<NH>(r, dq_sum);
 #pragma unroll
       for (int hf = 0; hf < NH; ++hf)
 #pragma unroll
@@ -720,6 +677,16 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
           }
     }
     __syncthreads();
+    if (!GROUPED && last) {
+      if (cm.len == BT) {
+        if (tid == 0) {
+          tma::store_3d(&maps.dk, cm.row, (hq * DK) / 64, Dks);
+          tma::store_commit();
+        }
+      } else {
+        store_tile_swz<BT, DK, NTHREADS>(reinterpret_cast<__nv_bfloat16*>(a.dk) + (row0 * a.H + hq) * DK, (int64_t)a.H * DK, Dks, cm.len, tid);
+      }
+    }
     if (!(a.options & B200GDN_PREP_GATE)) {
       if (tid < cm.len) st_param(a.dg, (row0 + tid) * a.HV + hv, a.gb_dtype, dGs[tid] + (tid < 32 ? dGs[32] : 0.f));
     } else {
@@ -795,6 +762,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
     }
     cluster_sync();   // shared memory must outlive the peers that read it
   }
+  if (tid == 0) tma::store_wait_read<0>();   // shared memory must outlive the bulk stores that read it
   if (failed && tid == 0) atomicExch(&g_local_timeout, 1);
   tc5::fence_before_sync();
   __syncthreads();
@@ -815,6 +783,9 @@ int launch(const b200gdn_chunk_args& a, cudaStream_t st) {
   rc |= tma::encode_bf16_panels(&m.d_o, a.d_o, a.rows, pv, pv, BT, DK / 64);
   rc |= tma::encode_bf16_panels(&m.vn, a.v_new, a.rows, pv, pv, BT, DK / 64);
   rc |= tma::encode_bf16_panels(&m.du, a.dv2, a.rows, pv, pv, BT, DK / 64);
+  rc |= tma::encode_bf16_panels(&m.dq, a.dq, a.rows, pk, pk, BT, DK / 64);
+  rc |= tma::encode_bf16_panels(&m.dk, a.dk, a.rows, pk, pk, BT, DK / 64);
+  rc |= tma::encode_bf16_panels(&m.dv, a.dv, a.rows, pv, pv, BT, DK / 64);
   rc |= tma::encode_bf16_2d(&m.a, a.A, a.rows, (uint64_t)a.HV * BT, (uint64_t)a.HV * BT, BT);
   rc |= tma::encode_bf16_2d(&m.h, a.h, hrows, DK, DK, DK);
   rc |= tma::encode_bf16_2d(&m.dh, a.dh, hrows, DK, DK, DK);

@@ -58,6 +58,17 @@ struct FragStore {
                  "r"(hi[1]), "r"(hi[2]), "r"(hi[3])
                  : "memory");
   }
+  // the block's TRANSPOSE into a tile [token][column] of `rows` rows: the block's rows become the columns col0 .. col0 + 15, its
+  // columns the tokens tok0 .. tok0 + 31
+  __device__ __forceinline__ void store_trans(unsigned char* tile, int rows, int tok0, int col0, int lane) const {
+    const uint32_t base = tc5::smem_addr(tile);
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};\n" ::"r"(base + tc5::swz_offset(tok0 + lane, col0, rows)),
+                 "r"(lo[0]), "r"(lo[1]), "r"(lo[2]), "r"(lo[3])
+                 : "memory");
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};\n" ::"r"(base + tc5::swz_offset(tok0 + lane, col0 + 8, rows)),
+                 "r"(hi[0]), "r"(hi[1]), "r"(hi[2]), "r"(hi[3])
+                 : "memory");
+  }
 };
 
 // The reverse: one 16-row x 32-column block of a swizzled bf16 tile into the accumulator-fragment layout with two
