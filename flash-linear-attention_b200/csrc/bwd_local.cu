@@ -26,13 +26,17 @@
 // 16 x 16 blocks by mma.sync, straight from the bf16 tiles: a tenth of the instructions of unpacking and multiplying.
 // What bounds it is the latency of the phases at two CTAs per SM, i.e. the instructions of an epilogue (39 % of issue slots, DRAM
 // 54 % of its peak rate), so epilogues work on fp32 pairs and skip blocks above the diagonal.
-// B4 T4096 H16 K=V=128: 186 us inside a step (228 with the solve's adjoint by way of dW, dU and dA, six dependent tensor-core phases
-// where there are three now; 213 with three, but element-wise stores and scalar epilogues).
+// The CTAs of a chunk are neighbours in launch order: a row of q, k, v or do is then read as a whole at about one time, which DRAM
+// pages like better than 256 bytes of every row (chunks first: 187 us for 179, grouped heads in turn 226 for 217).  Pulling the
+// next head's tiles into L2 while a head is worked on was slower (244 for 226).
+// B4 T4096 H16 K=V=128: 179 us inside a step (228 with the solve's adjoint by way of dW, dU and dA, six dependent tensor-core phases
+// where there are three now; 213 with three, but element-wise stores and scalar epilogues); 8/16 heads 217 (242).
 // One CTA of eight warps; 256 TMEM columns (C0: dP, dq^T, K K^T; C1: Z v_new^T, Q K^T; C2: Z^T; C3: dk_state^T, h Z^T, the rest of
 // dk^T) and ~111 KiB of shared memory whose regions change hands, so two CTAs per SM overlap each other's phases:
 //   R1: K   R2: do -> q   R3: v_new -> V   R4: dU -> Z^T -> dq   R5: dh -> h -> M2 | dv -> dk | dv   R6: A -> dP
 // Grouped value heads, many chunks: a CTA takes the heads of a group in turn, K stays, the tiles of the next head are fetched
-// under the last epilogue; the sums of dq and dk wait in local memory (TMEM is full; 64 KiB per CTA that stay in L2).
+// under the last epilogue; the sum of dq waits in C1 (Z in registers and Z v_new^T in C2 instead), that of dk in local memory (TMEM
+// is full; 32 KiB per CTA that stay in L2).
 // Few chunks: a CTA per head, the CTAs of a group form a cluster; each leaves its fp32 dq and dk in shared memory and adds up
 // a share of the rows over distributed shared memory.  Both add in head order (no atomics, no fp32 tensors in HBM).
 #include "rowio.cuh"
@@ -232,7 +236,7 @@ enum Heads { kOne, kCluster, kTurns };
 
 template <int DK, Heads MODE>
 __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_chunk_args a, const __grid_constant__ LocalMaps maps) {
-  constexpr bool GROUPED = MODE == kCluster;
+  constexpr bool GROUPED = MODE == kCluster, TURNS = MODE == kTurns;
   using S = LocalSmem<DK>;
   constexpr int NP = DK / 64;   // 64-column panels of a V-wide tile (V = K)
   constexpr int NH = DK / 64;   // 16-row halves of a transposed accumulator per warp
@@ -257,8 +261,9 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
 
   const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int q = warp & 3, hc = warp >> 2, g = lane >> 2, t = lane & 3;
-  const int c = blockIdx.x, G = a.HV / a.H, hq = MODE == kTurns ? blockIdx.y : blockIdx.y / G;
-  const int hv0 = MODE == kTurns ? hq * G : blockIdx.y, n_heads = MODE == kTurns ? G : 1;
+  const int per_chunk = TURNS ? a.H : a.HV, c = blockIdx.x / per_chunk, head = blockIdx.x % per_chunk;
+  const int G = a.HV / a.H, hq = TURNS ? head : head / G;
+  const int hv0 = TURNS ? hq * G : head, n_heads = TURNS ? G : 1;
   const ChunkMeta cm = load_chunk_meta(a.chunk_meta, c);
   const int64_t row0 = cm.row;
   const int r_lo = q * 16 + g, r_hi = r_lo + 8, cs = hc * 32;   // this warp's block of a [64][64] tile
@@ -288,10 +293,16 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
     load_head(hv0, true);
   }
   if (warp == 1) tc5::tmem_alloc(tmem_slot, 256);
-  auto head_vectors = [&](int hv) {   // beta and, with the gate option, the gate's value and derivative
+  // beta and, with the gate option, the gate's value and derivative: the loads, and what becomes of them
+  auto head_raw = [&](int hv) {
+    const bool beta = tid < BT, gate = (a.options & B200GDN_PREP_GATE) && tid >= 2 * BT && tid < 3 * BT;
+    const int r = beta ? tid : tid - 2 * BT;
+    return (beta || gate) && r < cm.len ? ld_param(beta ? a.beta : a.g, (row0 + r) * a.HV + hv, a.gb_dtype) : 0.f;
+  };
+  auto head_vectors = [&](int hv, float raw) {
     if (tid < BT) {
       const bool ok = tid < cm.len;
-      float b = ok ? ld_param(a.beta, (row0 + tid) * a.HV + hv, a.gb_dtype) : 0.f;
+      float b = raw;
       if (a.options & B200GDN_PREP_BETA_SIGMOID) {   // raw beta: the kernels work with (1|2) sigmoid(beta)
         const float sg = 1.f / (1.f + expf(-b));
         sgm[tid] = sg;
@@ -302,13 +313,13 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
     if ((a.options & B200GDN_PREP_GATE) && tid >= 2 * BT && tid < 3 * BT) {
       // fused gate: g = -exp(A_log) softplus(x), x = g_raw + dt_bias; its value and derivative, while the tiles are on their way
       const int r = tid - 2 * BT;
-      const float x = (r < cm.len ? ld_param(a.g, (row0 + r) * a.HV + hv, a.gb_dtype) : 0.f) + (a.dt_bias ? a.dt_bias[hv] : 0.f);
+      const float x = raw + (a.dt_bias ? a.dt_bias[hv] : 0.f);
       const float negA = -expf(a.A_log[hv]);
       gx[r] = negA / (1.f + expf(-x));
       gv[r] = negA * (x > 20.f ? x : log1pf(expf(x)));
     }
   };
-  head_vectors(hv0);
+  head_vectors(hv0, head_raw(hv0));
   if (!GROUPED && tid >= BT && tid < 2 * BT) {   // L2-norm option: reciprocal norms of the rows
     const int r = tid - BT;
     if (a.rstd_q != nullptr) rsq[r] = r < cm.len ? a.rstd_q[(row0 + r) * a.H + hq] : 0.f;
@@ -324,14 +335,16 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
   const uint32_t sA = tc5::smem_addr(As);
   const Operand opK_k{sK, BT, 0}, opK_mn{sK, BT, 1};      // K as (rows = token, contraction = key dim), and the reverse
   bool failed = false;
-  // several heads: this thread's part of dq and (turns) of the sums of dq and dk so far, in local memory between their uses
-  __align__(16) float sums_local[MODE != kOne ? 32 * NH : 4];
-  const uint64_t dq_sum = __cvta_generic_to_local(sums_local), dk_sum = dq_sum + 64 * NH;
+  // several heads: this thread's part of the sum of dk so far (turns) or of dq (cluster), in local memory between its uses
+  __align__(16) float part_local[MODE != kOne ? 16 * NH : 4];
+  const uint64_t part = __cvta_generic_to_local(part_local);
+  // one head: Z waits in C2 for V, and Z v_new^T takes C1; turns: the sum of dq has C1, so Z waits in registers
+  const uint32_t CZ = TURNS ? C2 : C1;
 
   for (int hh = 0; hh < n_heads; ++hh) {
     const int hv = hv0 + hh, hrow = (c * a.HV + hv) * DK;
     const uint32_t par = hh & 1;
-    const bool first = MODE != kTurns || hh == 0, last = MODE != kTurns || hh + 1 == n_heads;
+    const bool first = !TURNS || hh == 0, last = !TURNS || hh + 1 == n_heads;
     const float* gs = gs2 + par * BT;
     if (!tc5::mbar_wait(bar_a, par)) failed = true;
     if (cm.len < BT) {   // ragged chunk: the extra rows of the boxes belong to the next sequence
@@ -450,6 +463,11 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
       const float hd = warp_sum((g == 2 * t ? d0[0] + d1[2] : 0.f) + (g == 2 * t + 1 ? d0[1] + d1[3] : 0.f));
       if (lane == 0) red[warp] = hd;
     }
+    float z[NH][16];
+    if (TURNS) {
+      acc_ld_t<NH>(C2, q, cs, z);
+      tc5::tmem_ld_wait();
+    }
     tc5::fence_async_smem();
     tc5::fence_before_sync();
     if (__syncthreads_or(failed)) { failed = true; break; }
@@ -457,7 +475,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
     // ---- phase 2: ZV = Z v_new^T | -h Z^T | dq^T = h do_s^T + K^T dP~^T
     if (warp == 0) {
       tc5::fence_after_sync();
-      issue_mma_t<DK / 16>(C1, Operand{sZ, DK, 1}, Operand{sVn, BT, 0}, 64, 64, 0);
+      issue_mma_t<DK / 16>(CZ, Operand{sZ, DK, 1}, Operand{sVn, BT, 0}, 64, 64, 0);
 #pragma unroll
       for (int p = 0; p < NP; ++p) {
         issue_mma_t<4>(C3, Operand{sH + p * DK * 128, DK, 0}, Operand{sZ + p * BT * 128, DK, 1}, DK, 64, p > 0, /*neg_a=*/1);
@@ -479,7 +497,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
       FragStore fs = {};
       if (live) {
         const float b_lo = bet[r_lo], b_hi = bet[r_hi];
-        acc_ld32q(C1, q, cs, m);
+        acc_ld32q(CZ, q, cs, m);
         tc5::tmem_ld_wait();
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -507,9 +525,21 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
         scale_add_t<NH>(rk, r, i, bg);
       }
     }
+    auto finish_z = [&] {   // Z: its dots with v; dv = beta Z on its way out, over the second panel of h
+      float pv[8];
+      dots_t<NH>(z, Vs, kr, cs, lane, pv);   // (rows past a ragged chunk's end are not used)
+      c_vb[q * BT + gcol] = sum8_over_g(pv, g);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) scale_t<NH>(z, i, *reinterpret_cast<const float2*>(&bet[cs + i * 8 + 2 * t]));
+      stage_t<NH>(z, Dvs, kr, cs, lane);
+    };
     float rq[NH][16];   // dq: C0 is phase 3's
-    acc_ld_t<NH>(C0, q, cs, rq);
+    if (!TURNS) acc_ld_t<NH>(C0, q, cs, rq);
     if (!tc5::mbar_wait(bar_c, par)) failed = true;
+    if (TURNS) {
+      finish_z();
+      acc_ld_t<NH>(C0, q, cs, rq);
+    }
     if (cm.len < BT) {
       zero_tail_rows<BT, DK>(Qs, cm.len, tid, NTHREADS);
       zero_tail_rows<BT, DK>(Vs, cm.len, tid, NTHREADS);
@@ -526,20 +556,29 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
       issue_mma_t<BT / 16>(C3, opK_mn, Operand{sH, BT, 1}, DK, 64, 1);
       issue_mma_t<BT / 16>(C3, Operand{sDo, BT, 1}, Operand{sA, BT, 1}, DK, 64, 1);
       issue_mma_t<DK / 16>(C0, opK_k, opK_k, 64, 64, 0);
-      issue_mma_t<DK / 16>(C1, Operand{sDo, BT, 0}, opK_k, 64, 64, 0);
+      issue_mma_t<DK / 16>(CZ, Operand{sDo, BT, 0}, opK_k, 64, 64, 0);
       ph.commit();
     }
     {   // dq: its dots with q, the sum over the heads; ungrouped heads, and the last one in turn: on its way out, over Z^T
       float pv[8];
       dots_t<NH>(rq, Qs, kr, cs, lane, pv);
       c_rq[q * BT + gcol] = sum8_over_g(pv, g);
-      if (!first) add_local<NH>(rq, dq_sum);
-      if (GROUPED || !last) {
-        st_local<NH>(rq, dq_sum);
+      if (!first) {
+        float acc[NH][16];
+        acc_ld_t<NH>(C1, q, cs, acc);
+        tc5::tmem_ld_wait();
+        add_t<NH>(rq, acc);
+      }
+      if (GROUPED) {
+        st_local<NH>(rq, part);
+      } else if (!last) {
+#pragma unroll
+        for (int hf = 0; hf < NH; ++hf) tc5::tmem_st_16x256b_x4(C1 + ((uint32_t)(32 * q + 16 * hf) << 16) + cs, rq[hf]);
+        tc5::tmem_st_wait();
       } else {
         if (a.rstd_q != nullptr) {
           float* dots = c_rq;
-          if (MODE == kTurns) {   // of the sum; c_rk is free until epilogue 3
+          if (TURNS) {   // of the sum; c_rk is free until epilogue 3
             dots = c_rk;
             dots_t<NH>(rq, Qs, kr, cs, lane, pv);
             dots[q * BT + gcol] = sum8_over_g(pv, g);
@@ -550,16 +589,12 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
         stage_t<NH>(rq, Dqs, kr, cs, lane);
       }
     }
-    {   // Z: its dots with v; dv = beta Z on its way out, over the second panel of h
-      float z[NH][16], pv[8];
+    if (!TURNS) {
       acc_ld_t<NH>(C2, q, cs, z);
       tc5::tmem_ld_wait();
-      dots_t<NH>(z, Vs, kr, cs, lane, pv);
-      c_vb[q * BT + gcol] = sum8_over_g(pv, g);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) scale_t<NH>(z, i, *reinterpret_cast<const float2*>(&bet[cs + i * 8 + 2 * t]));
-      stage_t<NH>(z, Dvs, kr, cs, lane);
+      finish_z();
     }
+    const float raw_next = last ? 0.f : head_raw(hv + 1);
     FragLoad fp;
     fp.load(Ps, BT, q * 16, cs, lane);
     tc5::fence_async_smem();   // the staged tiles are read, and what was read here is overwritten, by bulk copies
@@ -587,7 +622,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
       float kk[16], qk[16], pv[8], rmk_lo = 0.f, rmk_hi = 0.f;   // (blocks above the diagonal hold zeros)
       if (live) {
       acc_ld32q(C0, q, cs, kk);
-      acc_ld32q(C1, q, cs, qk);
+      acc_ld32q(CZ, q, cs, qk);
       tc5::tmem_ld_wait();
       const float b_lo = bet[r_lo], b_hi = bet[r_hi];
 #pragma unroll
@@ -613,9 +648,9 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
       acc_ld_t<NH>(C3, q, cs, r);
       tc5::tmem_ld_wait();
       add_t<NH>(rk, r);
-      if (MODE == kTurns) {
-        if (!first) add_local<NH>(rk, dk_sum);
-        if (!last) st_local<NH>(rk, dk_sum);
+      if (TURNS) {
+        if (!first) add_local<NH>(rk, part);
+        if (!last) st_local<NH>(rk, part);
       }
       if (!GROUPED && last && a.rstd_k != nullptr) {   // <dk, k> for the norm's backward, over a tile that is needed no more
         dots_t<NH>(rk, Ks, kr, cs, lane, pv);
@@ -664,7 +699,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
       float* sq = reinterpret_cast<float*>(smem + S::o_do);
       float* sk = reinterpret_cast<float*>(smem + S::o_do + S::stage);
       float r[NH][16] = {};
-      add_local<NH>(r, dq_sum);
+      add_local<NH>(r, part);
 #pragma unroll
       for (int hf = 0; hf < NH; ++hf)
 #pragma unroll
@@ -716,7 +751,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
     }
     if (!last) {
       __syncthreads();   // the vectors have been read
-      head_vectors(hv + 1);
+      head_vectors(hv + 1, raw_next);
     }
   }
 
@@ -791,7 +826,7 @@ int launch(const b200gdn_chunk_args& a, cudaStream_t st) {
   rc |= tma::encode_bf16_2d(&m.dh, a.dh, hrows, DK, DK, DK);
   if (rc != 0) return set_error(B200GDN_ERR_CUDA, "bwd_local: cuTensorMapEncodeTiled failed (%d)", rc);
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(a.n_chunks, MODE == kTurns ? a.H : a.HV);
+  cfg.gridDim = dim3((unsigned)a.n_chunks * (MODE == kTurns ? a.H : a.HV));
   cfg.blockDim = dim3(NTHREADS);
   cfg.dynamicSmemBytes = S::bytes;
   cfg.stream = st;
@@ -804,8 +839,8 @@ int launch(const b200gdn_chunk_args& a, cudaStream_t st) {
   }
   if (MODE == kCluster) {
     attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
-    attr[cfg.numAttrs].val.clusterDim.x = 1;
-    attr[cfg.numAttrs].val.clusterDim.y = a.HV / a.H;
+    attr[cfg.numAttrs].val.clusterDim.x = a.HV / a.H;
+    attr[cfg.numAttrs].val.clusterDim.y = 1;
     attr[cfg.numAttrs++].val.clusterDim.z = 1;
   }
   cudaLaunchKernelEx(&cfg, bwd_local_kernel<DK, MODE>, a, m);
