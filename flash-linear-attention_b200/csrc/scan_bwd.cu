@@ -12,7 +12,8 @@
 // a ring of stages with TMA (Q, K, W tiles, the do slice, gamma; the qk tile with DVL, the dv_local slice without);
 // the chain MMA warp issues  acc = K dS_bf16  and  dS += Q^T do_s - W^T dv2  with accumulators in TMEM; a store warp
 // issues the TMA stores of dh_c and dv2; eight epilogue warps move dS between TMEM and shared memory and form dv2.
-// B4 T4096 H16 K=V=128: 95 us (107 with products and stores issued by one thread in turn).
+// B4 T4096 H16 K=V=128: 94 us (107 with products and stores issued by one thread in turn; 96 with the 80 registers that two CTAs per SM
+// would allow, of which shared memory has room for one).
 // DVL: the chain MMA warp also issues  L = qk^T do  of the NEXT chunk right after a step's last product (it only needs
 // loaded tiles and runs while the epilogue warps convert dS); qk = tril(Q K^T 2^(gamma_i-gamma_j)) comes ready-made
 // from the forward pass; the epilogue warps add scale L where they form dv2.
@@ -54,7 +55,7 @@ struct ScanBwdMaps {
 };
 
 template <int DK, int DV, int NSTAGE, bool DVL>
-__global__ void __launch_bounds__(NTHREADS)
+__global__ void __launch_bounds__(NTHREADS, 1)
     scan_bwd_kernel(const b200gdn_chunk_args a, const __grid_constant__ ScanBwdMaps maps) {
   using S = ScanBwdSmem<DK, NSTAGE, DVL>;
   constexpr int NH = DK / 64;
