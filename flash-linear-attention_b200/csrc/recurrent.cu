@@ -2,10 +2,11 @@
 //     S *= exp(g);  r = beta (v - S^T k);  S += k r^T;  o = S^T (scale q)
 // Replaces fused_recurrent_gated_delta_rule_fwd_kernel (fla/ops/gated_delta_rule/fused_recurrent.py:30-181),
 // including its in-kernel options (q/k L2 norm, -exp(A_log) softplus(g + dt_bias) gate, sigmoid beta,
-// V-first state layout).  fp32 arithmetic throughout.  Three kernels:
+// V-first state layout).  fp32 arithmetic throughout.  Four kernels:
 //   recurrent_step_kernel   one token per sequence, small and middling batches: latency of one pass over the state
 //   decode_stream_kernel    one token per sequence, large batches: pure state traffic (read + write K*V fp32)
-//   recurrent_kernel        several tokens per sequence: latency of the per-token chain
+//   recurrent_few_kernel    a few tokens per sequence: latency of the per-token chain
+//   recurrent_pairs_kernel  more tokens per sequence: the same chain for two tokens at a time
 #include "gdn_common.cuh"
 #include "rowio.cuh"
 #include "tc5.cuh"
@@ -158,12 +159,14 @@ struct WarpState {
 };
 
 // e^g and beta of one token with the layer's activations
-__device__ __forceinline__ void gate_beta(const b200gdn_recurrent_args& a, int64_t row, int hv, float& dec, float& beta) {
-  float gg = a.g ? ld_param(a.g, row * a.HV + hv, a.gb_dtype) : 0.f;
-  float bb = ld_param(a.beta, row * a.HV + hv, a.gb_dtype);
+__device__ __forceinline__ void load_gate_beta(const b200gdn_recurrent_args& a, int64_t row, int hv, float& gg, float& bb) {
+  gg = a.g ? ld_param(a.g, row * a.HV + hv, a.gb_dtype) : 0.f;
+  bb = ld_param(a.beta, row * a.HV + hv, a.gb_dtype);
+}
+__device__ __forceinline__ void activate(const b200gdn_recurrent_args& a, float A_log, float dt_bias, float gg, float bb, float& dec, float& beta) {
   if (a.flags & B200GDN_REC_GATE) {
-    if (a.dt_bias) gg += a.dt_bias[hv];
-    gg = -expf(a.A_log[hv]) * softplus_f(gg);
+    gg += dt_bias;
+    gg = -expf(A_log) * softplus_f(gg);
   }
   if (a.flags & B200GDN_REC_BETA_SIGMOID) {
     bb = 1.f / (1.f + expf(-bb));
@@ -171,6 +174,12 @@ __device__ __forceinline__ void gate_beta(const b200gdn_recurrent_args& a, int64
   }
   dec = expf(gg);
   beta = bb;
+}
+__device__ __forceinline__ void gate_beta(const b200gdn_recurrent_args& a, int64_t row, int hv, float& dec, float& beta) {
+  float gg, bb;
+  load_gate_beta(a, row, hv, gg, bb);
+  const bool gate = a.flags & B200GDN_REC_GATE;
+  activate(a, gate ? a.A_log[hv] : 0.f, gate && a.dt_bias ? a.dt_bias[hv] : 0.f, gg, bb, dec, beta);
 }
 
 // One token per sequence: a CTA of four warps owns 32 value channels of one (sequence, head).  Every lane loads its own rows
@@ -280,14 +289,14 @@ __global__ void __launch_bounds__(NTHREADS, DK <= 128 ? 7 : 3) recurrent_step_ke
   if (a.ht != nullptr && writeback) w.store(a.ht + (slot * a.HV + hv) * DK * DV, r0, c0, DV);
 }
 
-// Several tokens per sequence: a CTA of four warps owns 32 value channels of one (sequence, head).  q, k and v of TB tokens
+// A few tokens per sequence: a CTA of four warps owns 32 value channels of one (sequence, head).  q, k and v of TB tokens
 // at a time reach shared memory as they are by asynchronous 16-byte copies, one block ahead (two buffers); the norms,
 // <k,q>, e^g and beta of a block are formed once by the CTA; then every warp walks the block without a barrier.
 // Bound by the latency of the per-token chain (K/32 multiply-adds, five shuffles in sequence, K/32 multiply-adds), about
-// 0.26 us a token at K = 64 and 0.45 at K = 128.  4 sequences x 16 heads x 37 tokens, K = V = 128: 20.3 us (77.5 with the
-// channels combined through shared memory, five barriers a token); 128 x 16 x 4: 75.8 (110.6).
+// 0.26 us a token at K = 64 and 0.45 at K = 128.  128 sequences x 16 heads x 4 tokens, K = V = 128: 75.8 us (110.6 with the
+// channels combined through shared memory, five barriers a token).
 template <int DK, bool VFIRST, typename T>
-__global__ void __launch_bounds__(NTHREADS) recurrent_kernel(const b200gdn_recurrent_args a) {
+__global__ void __launch_bounds__(NTHREADS) recurrent_few_kernel(const b200gdn_recurrent_args a) {
   using W = WarpState<DK, VFIRST>;
   constexpr int TB = 2048 / DK < 32 ? 2048 / DK : 32;   // tokens per block
   constexpr int E16 = 16 / (int)sizeof(T);              // elements of one 16-byte copy
@@ -387,6 +396,304 @@ __global__ void __launch_bounds__(NTHREADS) recurrent_kernel(const b200gdn_recur
     __syncthreads();   // the next block's scalars and the copies after it overwrite what was read here
   }
   if (a.ht != nullptr && writeback) w.store(a.ht + (slot * a.HV + hv) * DK * DV, r0, c0, DV);
+}
+
+// ---- several tokens per sequence: tokens in pairs ---------------------------------------------------------------------
+constexpr int NT = 2;
+
+// What a token of a pair needs besides its rows; kn k and qn q are the rows with the factors of their norms (and the scale).
+struct __align__(16) PairToken {
+  float k, q;          // e^g from before the pair to the token, times kn | qn
+  float decay, last;   // the same alone; e^g from the token to the pair's end, times kn
+  float kk;            // second token: e^g <kn k, kn k of the first>
+  float kq0, kq1;      // <qn q, kn k> with the first token's k (second token: times e^g; first: not used) and the second's
+  float beta;
+};
+
+// The state of one warp: eight value channels with ALL K rows.  Lane l keeps, of channels 2 (l / 8) and + 1, the rows 32 m + 4 (l % 8)
+// .. + 3 as pairs: a row of k is read once for two channels, and a reduction over the rows is three shuffles for both channels of
+// S^T k and S^T q together.
+template <int DK, bool VFIRST>
+struct PairState {
+  static constexpr int NM = DK / 32;
+  uint64_t st[2 * NM][2];   // st[2 m + e][j]: rows (32 m + 4 (l % 8) + 2 e, + 1), channel c0 + j
+  __device__ __forceinline__ void load(const float* h, int s, int c0, int DV) {
+#pragma unroll
+    for (int m = 0; m < NM; ++m) {
+      const int r = 32 * m + 4 * s;
+      if (h == nullptr) {
+#pragma unroll
+        for (int e = 0; e < 2; ++e) st[2 * m + e][0] = st[2 * m + e][1] = 0ull;
+      } else if (VFIRST) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const float4 x = *reinterpret_cast<const float4*>(h + (int64_t)(c0 + j) * DK + r);
+          st[2 * m][j] = pack2(x.x, x.y);
+          st[2 * m + 1][j] = pack2(x.z, x.w);
+        }
+      } else {
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const float2 x = *reinterpret_cast<const float2*>(h + (int64_t)(r + 2 * e) * DV + c0);
+          const float2 y = *reinterpret_cast<const float2*>(h + (int64_t)(r + 2 * e + 1) * DV + c0);
+          st[2 * m + e][0] = pack2(x.x, y.x);
+          st[2 * m + e][1] = pack2(x.y, y.y);
+        }
+      }
+    }
+  }
+  __device__ __forceinline__ void store(float* h, int s, int c0, int DV) const {
+#pragma unroll
+    for (int m = 0; m < NM; ++m) {
+      const int r = 32 * m + 4 * s;
+      if (VFIRST) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const float2 x = unpack2(st[2 * m][j]), y = unpack2(st[2 * m + 1][j]);
+          *reinterpret_cast<float4*>(h + (int64_t)(c0 + j) * DK + r) = make_float4(x.x, x.y, y.x, y.y);
+        }
+      } else {
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const float2 x = unpack2(st[2 * m + e][0]), y = unpack2(st[2 * m + e][1]);
+          *reinterpret_cast<float2*>(h + (int64_t)(r + 2 * e) * DV + c0) = make_float2(x.x, y.x);
+          *reinterpret_cast<float2*>(h + (int64_t)(r + 2 * e + 1) * DV + c0) = make_float2(x.y, y.y);
+        }
+      }
+    }
+  }
+  // Two tokens.  Every reduction is taken from the state before them,
+  //     r_t = beta_t (v_t - D kn_t S^T k_t - sum_{s<t} kk_ts r_s);   o_t = D qn_t S^T q_t + sum_{s<=t} kq_ts r_s;
+  //     S <- D S + sum_s D(end, s) kn_s k_s r_s^T,
+  // so one round of shuffles in sequence serves both.  k, q: this lane's rows of the first token in shared memory; v: the first
+  // token's channel of this lane, c0 + ((lane >> 1) & 1).  o: of the same channel, right in lanes with bit 2 set.
+  template <typename T>
+  __device__ __forceinline__ void pair(const float* k, const float* q, const T* v, const PairToken* c, int lane, float (&o)[NT]) {
+    const bool b4 = lane & 4, b2 = lane & 2;
+    uint64_t k2[NT][2 * NM];
+    float z[NT];
+#pragma unroll
+    for (int u = 0; u < NT; ++u) {
+      uint64_t ad[2] = {0ull, 0ull}, aq[2] = {0ull, 0ull};
+#pragma unroll
+      for (int m = 0; m < NM; ++m) {
+        const float4 kf = *reinterpret_cast<const float4*>(k + u * DK + 32 * m), qf = *reinterpret_cast<const float4*>(q + u * DK + 32 * m);
+        k2[u][2 * m] = pack2(kf.x, kf.y);
+        k2[u][2 * m + 1] = pack2(kf.z, kf.w);
+        const uint64_t q0 = pack2(qf.x, qf.y), q1 = pack2(qf.z, qf.w);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          ad[j] = fma2(st[2 * m][j], k2[u][2 * m], ad[j]);
+          aq[j] = fma2(st[2 * m][j], q0, aq[j]);
+          ad[j] = fma2(st[2 * m + 1][j], k2[u][2 * m + 1], ad[j]);
+          aq[j] = fma2(st[2 * m + 1][j], q1, aq[j]);
+        }
+      }
+      // afterwards a lane holds the sum (bit 2: 0 = S^T k, 1 = S^T q) of channel (bit 1) of its two
+      float x[2];
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const float2 d = unpack2(ad[j]), e = unpack2(aq[j]);
+        const float sd = d.x + d.y, sq = e.x + e.y;
+        x[j] = (b4 ? sq : sd) + __shfl_xor_sync(0xffffffffu, b4 ? sd : sq, 4);
+      }
+      z[u] = (b2 ? x[1] : x[0]) + __shfl_xor_sync(0xffffffffu, b2 ? x[0] : x[1], 2);
+      z[u] += __shfl_xor_sync(0xffffffffu, z[u], 1);
+    }
+    // of the lane's channel; right in the lanes that hold S^T k
+    const float ra = c[0].beta * (Io<T>::ld(v, 0) - c[0].k * z[0]);
+    const float rb = c[1].beta * (Io<T>::ld(v, VS) - (c[1].k * z[1] + c[1].kk * ra));
+    const int k_lane = lane & 24;
+    const float a0 = __shfl_sync(0xffffffffu, ra, k_lane), a1 = __shfl_sync(0xffffffffu, ra, k_lane | 2);
+    const float b0 = __shfl_sync(0xffffffffu, rb, k_lane), b1 = __shfl_sync(0xffffffffu, rb, k_lane | 2);
+    const uint64_t dec2 = pack2(c[1].decay, c[1].decay);
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const float x = (j ? a1 : a0) * c[0].last, y = (j ? b1 : b0) * c[1].last;
+      const uint64_t xx = pack2(x, x), yy = pack2(y, y);
+#pragma unroll
+      for (int i = 0; i < 2 * NM; ++i) st[i][j] = fma2(st[i][j], dec2, fma2(k2[0][i], xx, mul2(k2[1][i], yy)));
+    }
+    const float oa = b2 ? a1 : a0, ob = b2 ? b1 : b0;
+    o[0] = c[0].q * z[0] + c[0].kq0 * oa;
+    o[1] = c[1].q * z[1] + (c[1].kq0 * oa + c[1].kq1 * ob);
+  }
+};
+
+// A CTA of four warps owns 32 value channels of one (sequence, head).  q, k and v of TB tokens at a time reach shared memory as they
+// are by asynchronous 16-byte copies, one block ahead (two buffers).  Half a warp then turns the q and k of a pair into fp32 and forms
+// what its tokens are to one another (norms, <k,k>, <k,q>, decays; PairToken), once for the CTA, and every warp walks the block pair
+// by pair without a barrier.
+// Bound by issue and latency at two warps a scheduler: 220 instructions a pair and warp, half of them fma.f32x2 at two cycles, 1000
+// cycles a pair, and 1900 a block for its preparation (clock stamps).  A fifth warp that prepares a block ahead took as long as the
+// walk (64 tokens 22.9 us for 21.0), groups of four tokens cost more in preparation than they save (22.7 for 19.0).
+// 4 sequences x 16 heads x 37 tokens, K = V = 128: 19.0 us (21.1 token by token); 1 x 16 x 64: 21.0 (26.4); 2 x 8 x 64, K = V = 64:
+// 15.9 (20.5).
+template <int DK, bool VFIRST, typename T>
+__global__ void __launch_bounds__(NTHREADS) recurrent_pairs_kernel(const b200gdn_recurrent_args a) {
+  constexpr int TB = 2048 / DK < 32 ? 2048 / DK : 32;   // tokens per block
+  constexpr int E16 = 16 / (int)sizeof(T);              // elements of one 16-byte copy
+  constexpr int RPL = DK / 16, RP2 = RPL / 2;           // rows of q and k per lane while pairs are prepared
+  constexpr int PASS = NTHREADS / 16 * NT, NPASS = (TB + PASS - 1) / PASS;   // tokens prepared at once
+  constexpr bool WIDEN = sizeof(T) == 2;
+  static_assert(TB % NT == 0, "whole pairs");
+  __shared__ __align__(16) T qs[2][TB * DK];
+  __shared__ __align__(16) T ks[2][TB * DK];
+  __shared__ __align__(16) T vs[2][TB * VS];
+  __shared__ __align__(16) float qw[WIDEN ? TB * DK : 4], kw[WIDEN ? TB * DK : 4];   // the block in fp32
+  __shared__ PairToken tok[TB];
+  __shared__ float dots[NTHREADS / 16][8];
+
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int v0 = blockIdx.x * VS, hv = blockIdx.y, n = blockIdx.z, hq = hv / (a.HV / a.H), DV = a.V;
+  int64_t bos;
+  int len;
+  if (a.cu_seqlens != nullptr) {
+    bos = a.cu_seqlens[n];
+    len = a.cu_seqlens[n + 1] - (int)bos;
+  } else {
+    bos = (int64_t)n * a.T;
+    len = a.T;
+  }
+  const bool wide = ((reinterpret_cast<uintptr_t>(a.q) | reinterpret_cast<uintptr_t>(a.k) | reinterpret_cast<uintptr_t>(a.v)) & 15) == 0;
+  auto fetch = [&](int t0, int buf) {
+    const int nt = len - t0 < TB ? len - t0 : TB;
+    if (nt & 1) {   // a last pair that is not full: a token of zeros, which changes nothing
+      for (int i = tid; i < DK; i += NTHREADS) qs[buf][nt * DK + i] = ks[buf][nt * DK + i] = T(0.f);
+      if (tid < VS) vs[buf][nt * VS + tid] = T(0.f);
+    }
+    if (wide) {
+      for (int i = tid; i < nt * (DK / E16); i += NTHREADS) {
+        const int t = i / (DK / E16), c = (i % (DK / E16)) * E16;
+        const int64_t at = ((bos + t0 + t) * a.H + hq) * DK + c;
+        cp_async16(&qs[buf][t * DK + c], static_cast<const T*>(a.q) + at);
+        cp_async16(&ks[buf][t * DK + c], static_cast<const T*>(a.k) + at);
+      }
+      for (int i = tid; i < nt * (VS / E16); i += NTHREADS) {
+        const int t = i / (VS / E16), c = (i % (VS / E16)) * E16;
+        cp_async16(&vs[buf][t * VS + c], static_cast<const T*>(a.v) + ((bos + t0 + t) * a.HV + hv) * DV + v0 + c);
+      }
+    } else {
+      for (int i = tid; i < nt * DK; i += NTHREADS) {
+        const int64_t at = ((bos + t0 + i / DK) * a.H + hq) * DK + i % DK;
+        qs[buf][i] = static_cast<const T*>(a.q)[at];
+        ks[buf][i] = static_cast<const T*>(a.k)[at];
+      }
+      for (int i = tid; i < nt * VS; i += NTHREADS)
+        vs[buf][i] = static_cast<const T*>(a.v)[((bos + t0 + i / VS) * a.HV + hv) * DV + v0 + i % VS];
+    }
+    cp_async_commit();
+  };
+  // g and beta of the tokens that this lane will prepare the scalars of: lanes 0 and 1 of a half-warp, one token of its pair each
+  const int l16 = lane & 15, half = tid >> 4;
+  float g_raw[NPASS], b_raw[NPASS];
+  auto fetch_gates = [&](int t0) {
+#pragma unroll
+    for (int p = 0; p < NPASS; ++p) {
+      const int t = t0 + p * PASS + half * NT + l16;
+      if (l16 < NT && p * PASS + half * NT < TB && t < len) load_gate_beta(a, bos + t, hv, g_raw[p], b_raw[p]);
+    }
+  };
+  const bool gate = a.flags & B200GDN_REC_GATE, l2 = a.flags & B200GDN_REC_L2NORM;
+  float A_log = 0.f, dt_bias = 0.f;
+  if (gate && l16 < NT) {
+    A_log = a.A_log[hv];
+    if (a.dt_bias) dt_bias = a.dt_bias[hv];
+  }
+  fetch_gates(0);
+  fetch(0, 0);
+  bool writeback;
+  const int64_t slot = state_slot(a, n, &writeback);   // which state of the pool this sequence uses
+  const int s = lane & 7, cl = warp * 8 + (lane >> 3) * 2, c0 = v0 + cl, ch = (lane >> 1) & 1;
+  PairState<DK, VFIRST> w;
+  w.load(a.h0 ? a.h0 + (slot * a.HV + hv) * DK * DV : nullptr, s, c0, DV);
+
+  for (int t0 = 0, buf = 0; t0 < len; t0 += TB, buf ^= 1) {
+    const int nt = len - t0 < TB ? len - t0 : TB;
+    cp_async_wait<0>();
+    __syncthreads();   // ... and every warp has walked the block before
+    if (t0 + TB < len) fetch(t0 + TB, buf ^ 1);
+#pragma unroll
+    for (int p = 0; p < NPASS; ++p) {
+      const int t = p * PASS + half * NT;   // this half-warp's pair
+      if (p * PASS + (half & ~1) * NT >= nt) break;   // (the same for both halves)
+      const bool live = t < nt;
+      uint64_t k[NT][RP2], q[NT][RP2];
+#pragma unroll
+      for (int u = 0; u < NT; ++u) {
+        const int at = (live ? t + u : u) * DK + l16 * RPL;
+        load_pairs<T, RPL>(ks[buf], at, true, k[u]);
+        load_pairs<T, RPL>(qs[buf], at, true, q[u]);
+        if (WIDEN && live) {
+#pragma unroll
+          for (int i = 0; i < RP2; ++i) {
+            *reinterpret_cast<uint64_t*>(&kw[at + 2 * i]) = k[u][i];
+            *reinterpret_cast<uint64_t*>(&qw[at + 2 * i]) = q[u][i];
+          }
+        }
+      }
+      uint64_t x2[8] = {};
+#pragma unroll
+      for (int i = 0; i < RP2; ++i) {
+        x2[0] = fma2(k[0][i], k[0][i], x2[0]);
+        x2[1] = fma2(k[1][i], k[1][i], x2[1]);
+        x2[2] = fma2(q[0][i], q[0][i], x2[2]);
+        x2[3] = fma2(q[1][i], q[1][i], x2[3]);
+        x2[4] = fma2(k[1][i], k[0][i], x2[4]);
+        x2[5] = fma2(q[0][i], k[0][i], x2[5]);
+        x2[6] = fma2(q[1][i], k[0][i], x2[6]);
+        x2[7] = fma2(q[1][i], k[1][i], x2[7]);
+      }
+      float x[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const float2 f = unpack2(x2[e]);
+        x[e] = f.x + f.y;
+      }
+      // summed over the sixteen lanes by recursive halving: lane l ends with value l / 2
+#pragma unroll
+      for (int h = 4; h > 0; h >>= 1)
+#pragma unroll
+        for (int e = 0; e < h; ++e)
+          x[e] = (l16 & 2 * h ? x[e + h] : x[e]) + __shfl_xor_sync(0xffffffffu, l16 & 2 * h ? x[e] : x[e + h], 2 * h);
+      x[0] += __shfl_xor_sync(0xffffffffu, x[0], 1);
+      if (!(l16 & 1)) dots[half][l16 >> 1] = x[0];
+      __syncwarp();
+      float dec = 1.f, beta = 0.f;   // (a token past the end)
+      if (l16 < NT && t + l16 < nt) activate(a, A_log, dt_bias, g_raw[p], b_raw[p], dec, beta);
+      const float other = __shfl_xor_sync(0xffffffffu, dec, 1);   // of the pair's other token
+      if (l16 < NT && live) {
+        const float* d = dots[half];
+        const float kn0 = l2 ? rsqrtf(d[0] + 1e-6f) : 1.f, kn1 = l2 ? rsqrtf(d[1] + 1e-6f) : 1.f;
+        const float qn = l2 ? a.scale * rsqrtf(d[2 + l16] + 1e-6f) : a.scale;
+        PairToken g;
+        g.decay = l16 ? dec * other : dec;
+        g.k = g.decay * (l16 ? kn1 : kn0);
+        g.q = g.decay * qn;
+        g.last = l16 ? kn1 : other * kn0;
+        g.kk = dec * d[4] * kn0 * kn1;
+        g.kq0 = (l16 ? dec * d[6] : d[5]) * kn0 * qn;
+        g.kq1 = d[7] * kn1 * qn;
+        g.beta = beta;
+        tok[t + l16] = g;
+      }
+    }
+    __syncthreads();
+    fetch_gates(t0 + TB);
+    const float* kf = reinterpret_cast<const float*>(WIDEN ? static_cast<const void*>(kw) : ks[buf]);
+    const float* qf = reinterpret_cast<const float*>(WIDEN ? static_cast<const void*>(qw) : qs[buf]);
+    T* out = static_cast<T*>(a.o) + ((bos + t0) * a.HV + hv) * DV + c0 + ch;
+    for (int t = 0; t < nt; t += NT) {
+      float o[NT];
+      w.template pair<T>(kf + t * DK + 4 * s, qf + t * DK + 4 * s, &vs[buf][t * VS + cl + ch], &tok[t], lane, o);
+      if ((lane & 5) == 4) {
+        Io<T>::st(out, 0, o[0]);
+        if (t + 1 < nt) Io<T>::st(out, (int64_t)a.HV * DV, o[1]);
+      }
+      out += (int64_t)NT * a.HV * DV;
+    }
+  }
+  if (a.ht != nullptr && writeback) w.store(a.ht + (slot * a.HV + hv) * DK * DV, s, c0, DV);
 }
 
 // Single-token decode at large batch as a stream: the step kernel loads a state, computes and stores it, so the memory pipe
@@ -656,8 +963,15 @@ int launch(const b200gdn_recurrent_args& a, cudaStream_t st) {
   dim3 grid(a.V / VS, a.HV, a.n_seq);
   const bool vf = a.flags & B200GDN_REC_STATE_V_FIRST;
   const bool step = a.T == 1 && a.cu_seqlens == nullptr;   // one token per sequence: no block of tokens to stage
-  auto run = [&](auto* one, auto* many) { (step ? one : many)<<<grid, NTHREADS, 0, st>>>(a); };
-#define RUN(VF, TY) run(recurrent_step_kernel<DK, VF, TY>, recurrent_kernel<DK, VF, TY>)
+  // Tokens per sequence (on average) from which they are taken in pairs.  Measured, one by one / in pairs, K = V = 128 bf16: 1 x 16
+  // heads, 8 tokens 6.2 / 6.3 us, 12 tokens 7.4 / 7.1, 24 tokens 12.1 / 10.6; 16 x 32 heads (2048 CTAs), 16 tokens 46.7 / 48.9, 24
+  // tokens 66.9 / 64.8, 64 tokens 158 / 139 (fp32: 33 tokens 89.8 / 91.8, 64 tokens 156 / 147); K = V = 64: 8 tokens 5.7 / 5.0 and
+  // 13.1 / 13.6, 12 tokens 6.7 / 5.6 and 16.4 / 15.7.
+  const int tokens = a.T / (a.cu_seqlens != nullptr && a.n_seq > 0 ? a.n_seq : 1);
+  const bool many_ctas = (int64_t)grid.x * grid.y * grid.z > 4 * sm_count();
+  const bool pairs = tokens >= (DK >= 128 && many_ctas ? 40 : 12);
+  auto run = [&](auto* one, auto* few, auto* many) { (step ? one : pairs ? many : few)<<<grid, NTHREADS, 0, st>>>(a); };
+#define RUN(VF, TY) run(recurrent_step_kernel<DK, VF, TY>, recurrent_few_kernel<DK, VF, TY>, recurrent_pairs_kernel<DK, VF, TY>)
   switch (a.qkv_dtype) {
     case 0: if (vf) RUN(true, __nv_bfloat16); else RUN(false, __nv_bfloat16); break;
     case 1: if (vf) RUN(true, __half); else RUN(false, __half); break;

@@ -267,3 +267,31 @@ def test_single_token_steps_around_the_streaming_size(K, V, N, HV):
     rest = torch.ones(slots, dtype=torch.bool, device='cuda')
     rest[at[used].long()] = False
     assert torch.equal(pool[rest], before[rest]), 'a slot that no sequence uses was written'
+
+
+@pytest.mark.parametrize('K,V', [(32, 32), (64, 64), (128, 128), (256, 64)])
+@pytest.mark.parametrize('lens,v_first', [([12], False), ([13, 12], True), ([16, 17, 7, 33], False), ([64, 0, 31, 1], True), ([65, 32], False)])
+def test_tokens_in_pairs(K, V, lens, v_first):
+    """Enough tokens to be taken in pairs: odd and even lengths, blocks that are full, nearly full and just exceeded, a sequence of one
+    token and one of none beside longer ones; fp32, where the recurrence's own tolerance (1e-5) holds."""
+    from b200gdn import fused_recurrent_gated_delta_rule
+    H, HV, dev, T, N = 2, 4, 'cuda', sum(lens), len(lens)
+    cu = torch.tensor([0] + lens).cumsum(0)
+    q, k, v, graw, braw, A_log, dt_bias, gen = _inputs(1, T, H, HV, K, V, 31, torch.float32)
+    h0 = torch.randn(N, HV, *((V, K) if v_first else (K, V)), generator=gen) * 0.5
+    ref_o, ref_ht = [], []
+    for i in range(N):
+        rows = slice(int(cu[i]), int(cu[i + 1]))
+        if lens[i] == 0:
+            ref_ht.append(h0[i:i + 1])
+            continue
+        ro, rs = O.recurrent_step_options(q[:, rows], k[:, rows], v[:, rows], graw[:, rows], braw[:, rows], None, h0[i:i + 1], True, True, True,
+                                          A_log, dt_bias, True, True, v_first)
+        ref_o.append(ro)
+        ref_ht.append(rs)
+    o, ht = fused_recurrent_gated_delta_rule(
+        *(x.to(dev) for x in (q, k, v, graw)), beta=braw.to(dev), initial_state=h0.to(dev), output_final_state=True,
+        use_qk_l2norm_in_kernel=True, use_gate_in_kernel=True, A_log=A_log.to(dev), dt_bias=dt_bias.to(dev),
+        use_beta_sigmoid_in_kernel=True, allow_neg_eigval=True, state_v_first=v_first, cu_seqlens=cu.to(dev))
+    O.assert_close('o', torch.cat(ref_o, 1), o.cpu(), 1e-5)
+    O.assert_close('ht', torch.cat(ref_ht, 0), ht.cpu(), 1e-5)
