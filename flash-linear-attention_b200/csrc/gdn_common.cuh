@@ -67,6 +67,34 @@ __device__ __forceinline__ const float* gamma_ptr(const float* gamma, int c, int
   return gamma + ((int64_t)c * HV + hv) * BT;
 }
 
+// bounds of the chunks' state transitions (option TRANSITION_BOUNDS), [n_chunks][HV] behind gamma
+__device__ __forceinline__ float* bounds_ptr(float* gamma, int n_chunks, int HV) { return gamma + (int64_t)n_chunks * HV * BT; }
+
+// How many chunks of [c_first, c_first + nc), counted from the end (`step` -1: a forward scan's) or from the start (+1), have
+// transitions whose product is at most 2^-128: what lies beyond them does not reach a state of fp32 there (gate factors below 2^-126
+// are flushed to zero within a chunk as well).  nc where there are none, or where a chunk beyond has values that are not finite and
+// so have to.  Executed by a whole warp; a sum of infinities or NaN compares as "no".
+constexpr float kNothingReaches = -128.f;
+__device__ __forceinline__ int chunks_that_reach(const float* bounds, int HV, int hv, int c_first, int nc, int step, int lane) {
+  int n = nc;
+  float sum = 0.f;
+  bool finite = true;
+  for (int j0 = 0; j0 < nc; j0 += 32) {
+    const int j = j0 + lane;
+    float b = j < nc ? bounds[(int64_t)(step > 0 ? c_first + j : c_first + nc - 1 - j) * HV + hv] : 0.f;
+    finite = finite && __all_sync(0xffffffffu, b < INFINITY);   // (false for NaN)
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float y = __shfl_up_sync(0xffffffffu, b, o);
+      if (lane >= o) b += y;
+    }
+    const unsigned enough = __ballot_sync(0xffffffffu, j < nc && sum + b < kNothingReaches);
+    if (n == nc && enough != 0) n = j0 + __ffs(enough);
+    sum += __shfl_sync(0xffffffffu, b, 31);
+  }
+  return finite ? n : nc;
+}
+
 // Look-ahead for the one-CTA-per-(chunk, head) kernels.  CTAs are dispatched in launch order (x fastest), so the
 // CTA that will take this one's place on the device is `dist` CTAs further on (dist = CTAs resident at once).
 // A CTA pulls that successor's tiles into L2 as it starts; the successor's own loads then see L2 latency

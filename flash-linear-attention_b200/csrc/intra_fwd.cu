@@ -19,6 +19,8 @@
 // merges, 4-byte stores of qk and A and a zero fill of the inverse, 5.8 k wavefronts a CTA).  So every merge has one operand
 // at an address that is uniform over the warp (one wavefront) and 16-byte reads along rows for the other, skips what is
 // zero by triangularity, and nothing is filled with zeros first.
+// Bounds of the chunk's state transition, where pre-scans will want them (TRANSITION_BOUNDS), cost 3 %: the squared norms of k are the
+// diagonal of K K^T, and the largest of W and U is taken from the accumulators on their way out.
 // B4 T4096 H16 K=V=128: 87 us inside a step (105), 94 by itself between two events; with the L2 norm, gate and beta options
 // 120 us (108 + 47 for a norm pass of its own).
 #include "tc5_tile.cuh"
@@ -143,6 +145,13 @@ __device__ __forceinline__ void normalise_rows(unsigned char* tile, int tid, int
   }
 }
 
+// the largest magnitude of three; NaN if one of them is
+__device__ __forceinline__ float max_abs3(float a, float b, float c) {
+  float d;
+  asm("max.NaN.abs.f32 %0, %1, %2, %3;\n" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+
 template <int DK, int DV>
 __global__ void __launch_bounds__(NTHREADS, 4) intra_fwd_kernel(const b200gdn_chunk_args a, const __grid_constant__ IntraMaps maps,
                                                                 const int pf_dist) {
@@ -183,6 +192,7 @@ __global__ void __launch_bounds__(NTHREADS, 4) intra_fwd_kernel(const b200gdn_ch
   // with q and a qk buffer the kernel also emits the gated causal q k^T tile that the scans use for the chunk-local
   // parts of o and dv (so that they neither form nor mask it on their serial chain)
   const bool with_qk = a.qk != nullptr && a.q != nullptr;
+  const bool bounds = a.options & B200GDN_TRANSITION_BOUNDS;
   unsigned char* Qs = smem + S::o_l;
 
   if (tid == 0) {
@@ -293,6 +303,7 @@ __global__ void __launch_bounds__(NTHREADS, 4) intra_fwd_kernel(const b200gdn_ch
         const float g_lo = gam[r_lo], g_hi = gam[r_hi];
         const float b_lo = bet[r_lo], b_hi = bet[r_hi];
         uint32_t p_lo[4], p_hi[4];
+        float kk_lo = 0.f, kk_hi = 0.f;   // |k|^2 of the two rows, where the diagonal is this thread's
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const int j0 = cs + i * 8 + 2 * t;
@@ -302,6 +313,7 @@ __global__ void __launch_bounds__(NTHREADS, 4) intra_fwd_kernel(const b200gdn_ch
           for (int e = 0; e < 4; ++e) {
             const int ii = (e & 2) ? r_hi : r_lo, jj = j0 + (e & 1);
             const float f = fast_exp2(((e & 2) ? g_hi : g_lo) - ((e & 1) ? gj.y : gj.x));
+            if (ii == jj) ((e & 2) ? kk_hi : kk_lo) = r[4 * i + e];
             v[e] = (ii > jj) ? r[4 * i + e] * ((e & 2) ? b_hi : b_lo) * f : 0.f;
             w4[e] = (with_qk && ii >= jj) ? pq[4 * i + e] * f : 0.f;
           }
@@ -310,14 +322,21 @@ __global__ void __launch_bounds__(NTHREADS, 4) intra_fwd_kernel(const b200gdn_ch
           p_lo[i] = pack_bf16(w4[0], w4[1]);
           p_hi[i] = pack_bf16(w4[2], w4[3]);
         }
+        if (bounds) {
+          float x = log2f(fmaxf(1.f, fabsf(1.f - b_lo * kk_lo))) + log2f(fmaxf(1.f, fabsf(1.f - b_hi * kk_hi)));
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+          if (lane == 0) graw[warp] = x;   // (the raw sums have been read)
+        }
         if (with_qk) {
           const uint4 lo = quad_words(p_lo, t), hi = quad_words(p_hi, t);
           if (r_lo < cm.len) *reinterpret_cast<uint4*>(Pg + r_lo * pstride) = lo;
           if (r_hi < cm.len) *reinterpret_cast<uint4*>(Pg + r_hi * pstride) = hi;
         }
-      } else if (with_qk) {
-        if (r_lo < cm.len) *reinterpret_cast<uint4*>(Pg + r_lo * pstride) = make_uint4(0, 0, 0, 0);
-        if (r_hi < cm.len) *reinterpret_cast<uint4*>(Pg + r_hi * pstride) = make_uint4(0, 0, 0, 0);
+      } else {
+        if (bounds && lane == 0) graw[warp] = 0.f;
+        if (with_qk && r_lo < cm.len) *reinterpret_cast<uint4*>(Pg + r_lo * pstride) = make_uint4(0, 0, 0, 0);
+        if (with_qk && r_hi < cm.len) *reinterpret_cast<uint4*>(Pg + r_hi * pstride) = make_uint4(0, 0, 0, 0);
       }
     }
     tc5::fence_before_sync();
@@ -420,6 +439,13 @@ __global__ void __launch_bounds__(NTHREADS, 4) intra_fwd_kernel(const b200gdn_ch
       tc5::tmem_ld_wait();
       tc5::fence_before_sync();
       __syncthreads();   // W has left tensor memory, K is no longer an operand
+      float size = 0.f;   // the largest of this thread's part of W and U; NaN if one of them is
+      if (bounds) {
+#pragma unroll
+        for (int b = 0; b < KB; ++b)
+#pragma unroll
+          for (int e = 0; e < 16; e += 2) size = max_abs3(size, rw[b][e], rw[b][e + 1]);
+      }
       // ---- U = Au V into the same columns, while W is converted and staged over the K tile
       if (warp == 0) {
         tc5::fence_after_sync();
@@ -450,6 +476,12 @@ __global__ void __launch_bounds__(NTHREADS, 4) intra_fwd_kernel(const b200gdn_ch
 #pragma unroll
         for (int b = 0; b < VB; ++b) acc_ld32q(tm, q, cv + b * 32, ru[b]);
         tc5::tmem_ld_wait();
+        if (bounds) {
+#pragma unroll
+          for (int b = 0; b < VB; ++b)
+#pragma unroll
+            for (int e = 0; e < 16; e += 2) size = max_abs3(size, ru[b][e], ru[b][e + 1]);
+        }
 #pragma unroll
         for (int b = 0; b < VB; ++b) {
           FragStore fs;
@@ -459,7 +491,13 @@ __global__ void __launch_bounds__(NTHREADS, 4) intra_fwd_kernel(const b200gdn_ch
         }
         tc5::fence_async_smem();
         tc5::fence_before_sync();
-        __syncthreads();
+        const int odd = __syncthreads_or(!(size < INFINITY));
+        if (bounds && tid == 0) {
+          float x = gam[BT - 1];
+#pragma unroll
+          for (int w = 0; w < NTHREADS / 32; ++w) x += graw[w];
+          bounds_ptr(a.gamma, a.n_chunks, a.HV)[(int64_t)c * a.HV + hv] = odd ? INFINITY : x;
+        }
         if (cm.len == BT) {
           if (tid == 32) {
             tma::store_3d(&maps.u, (int)cm.row, (hv * DV) / 64, Vs);

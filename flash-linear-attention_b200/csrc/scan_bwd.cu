@@ -24,6 +24,7 @@
 // for context parallelism (fla/ops/cp/chunk_delta_h.py:478-744).  When cp_dM is given the grid grows by K / 64 such
 // slices (either form), so that the shard's (dh_ext, dM) pair comes out of ONE launch.  Without DVL, d_o == NULL also
 // means zero do and dv_local, and dv2 is then not stored.
+// The pre-scan of a piece of a long sequence (TRANSITION_BOUNDS) walks only the chunks whose gradients reach the piece's start.
 #include "tc5_tile.cuh"
 #include "tma.cuh"
 
@@ -82,13 +83,38 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   const int v0 = (m_mode ? (int)blockIdx.x - DV / BV : (int)blockIdx.x) * BV, hv = blockIdx.y;
   const int n = a.seq_order != nullptr ? a.seq_order[blockIdx.z] : (int)blockIdx.z;   // longest sequences first
   const int G = a.HV / a.H, hq = hv / G;
-  const int c_first = a.seq_meta[2 * n], nc = a.seq_meta[2 * n + 1];
-  const int c_last = c_first + nc - 1;
+  const int c_first = a.seq_meta[2 * n];
+  int nc = a.seq_meta[2 * n + 1];
   const bool has_do = !m_mode && (DVL || a.d_o != nullptr);
   const bool has_dl = !m_mode && !DVL && a.d_o != nullptr;   // a dv_local slice comes in through the dv2 buffer
   const bool store_d2 = a.dv2 != nullptr && (dvl || has_dl);
   const bool st_dh = !m_mode && a.dh != nullptr;
   float* const dh0_out = m_mode ? a.cp_dM : a.dh0;
+  bool m_zero = false;   // the transition matrix is zero
+  if (DVL && a.dh == nullptr && a.dv2 == nullptr && (a.options & B200GDN_TRANSITION_BOUNDS)) {
+    int reach = chunks_that_reach(bounds_ptr(const_cast<float*>(a.gamma), a.n_chunks, a.HV), a.HV, hv, c_first, nc, 1, lane);
+    if (reach < nc && !m_mode) {
+      // an output gradient that is not finite reaches everything before it; those left out are looked at, which takes a twentieth of
+      // the time that walking them would
+      const ChunkMeta from = load_chunk_meta(a.chunk_meta, c_first + reach), last = load_chunk_meta(a.chunk_meta, c_first + nc - 1);
+      const int rows = last.row + last.len - from.row, row0 = warp * 4 + (lane >> 3);
+      const __nv_bfloat16* d_o = reinterpret_cast<const __nv_bfloat16*>(a.d_o) + ((int64_t)from.row * a.HV + hv) * DV + v0 + (lane & 7) * 8;
+      uint32_t odd = 0;
+#pragma unroll 8
+      for (int r = row0; r < rows; r += NTHREADS / 8) {
+        const uint4 w = __ldg(reinterpret_cast<const uint4*>(d_o + (int64_t)r * a.HV * DV));
+        const uint32_t u[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) odd |= ((u[e] & 0x7f800000u) == 0x7f800000u) | ((u[e] & 0x7f80u) == 0x7f80u);
+      }
+      if (__syncthreads_or(odd)) reach = nc;
+    }
+    if (reach < nc) {
+      m_zero = m_mode;
+      nc = m_mode ? 0 : reach;
+    }
+  }
+  const int c_last = c_first + nc - 1;
   const bool vfirst = !m_mode && (a.options & B200GDN_STATE_V_FIRST);   // dht and dh0 stored [V][K]
   constexpr uint32_t TMEM_COLS = DVL ? 256 : 128;   // DVL: 192 used; the allocation is a power of two
 
@@ -230,7 +256,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
           for (int e = 0; e < 4; ++e) {
             const int r = srow0 + 16 * hf + g + ((e >> 1) << 3);
             const int col = v0 + 32 * hc + 8 * i + 2 * t + (e & 1);
-            Sr[hf][4 * i + e] = dht ? (vfirst ? dht[(int64_t)col * DK + r] : dht[(int64_t)r * DV + col]) : ((m_mode && r == col) ? 1.f : 0.f);
+            Sr[hf][4 * i + e] = dht ? (vfirst ? dht[(int64_t)col * DK + r] : dht[(int64_t)r * DV + col]) : ((m_mode && !m_zero && r == col) ? 1.f : 0.f);
           }
     }
 

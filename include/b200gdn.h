@@ -70,6 +70,12 @@ typedef enum b200gdn_status {
 #define B200GDN_PREP_BETA_SIGMOID 4u
 #define B200GDN_PREP_NEG_EIGVAL 8u
 #define B200GDN_STATE_V_FIRST 16u /* chunk passes: h0, ht, dht and dh0 are stored [N,HV,V,K] (the reference's state_v_first) */
+/* chunk passes: `gamma` is followed by n_chunks * HV floats more, bounds of the chunks' state transitions.  The transition of a chunk is
+ * prod_i 2^(g_i log2 e) (I - beta_i k_i k_i^T), so its norm is at most two to the power of
+ *     gamma_last + sum_i log2 max(1, |1 - beta_i |k_i|^2|),
+ * which the intra stage writes (+infinity where w or u of the chunk is not finite).  A pre-scan (a scan that stores nothing but its
+ * final state and the transition matrix) leaves out the chunks from which no more than 2^-128 reaches the end of its sequence. */
+#define B200GDN_TRANSITION_BOUNDS 32u
 typedef struct b200gdn_chunk_args {
   int32_t struct_bytes;          /* = sizeof(b200gdn_chunk_args), checked */
   int32_t rows, H, HV, K, V;

@@ -745,6 +745,47 @@ def test_sequence_split_equals_the_unsplit_scan(pieces):
         O.assert_close(f'{n} split vs unsplit', p_, s_, 0.004)
 
 
+@pytest.mark.parametrize('D', [64, 128])
+@pytest.mark.parametrize('odd', [None, 'v', 'do'])
+def test_pre_scans_leave_out_what_does_not_reach(D, odd):
+    """Long pieces whose heads forget nothing, part of a piece, all but two chunks of it, and grow: against the uncut run.  Each of the two
+    is within REF_TOL of the exact result, so they are within twice that of one another (heads that forget nothing use most of it, with
+    and without anything left out: up to 0.0067 for dk); what a head that forgets shows of the cut is far less.  A value or an output gradient that is not finite in a chunk that is left out still reaches everything that
+    it reaches in the uncut run."""
+    from b200gdn import chunk_gated_delta_rule, index
+    dev, T, H, HV = 'cuda', 64 * 60 + 37, 2, 4
+    d = O.make_inputs(1, T, H, HV, D, D, seed=37)
+    rate = torch.tensor([-1e-4, -0.2, -1.5, 2e-3])
+    g = rate * (0.5 + torch.rand(1, T, HV, generator=torch.Generator().manual_seed(1)))
+    v, do = d['v'].clone(), d['do'].clone()
+    if odd == 'v':
+        v[0, 70, 2, 5] = float('nan')
+    if odd == 'do':
+        do[0, T - 80, 2, 5] = float('inf')
+
+    def run(pieces):
+        index.FORCE_PIECES = pieces
+        index._split_cache.clear()
+        try:
+            leaves = [x.to(dev).to(torch.bfloat16).requires_grad_(True) for x in (d['q'], d['k'], v)]
+            leaves += [x.to(dev).requires_grad_(True) for x in (g, d['beta'], d['h0'])]
+            o, ht = chunk_gated_delta_rule(*leaves[:5], initial_state=leaves[5], output_final_state=True)
+            torch.autograd.backward([o, ht], [do.to(dev).to(torch.bfloat16), d['dht'].to(dev)])
+            return [o.float().cpu(), ht.cpu()] + [x.grad.float().cpu() for x in leaves]
+        finally:
+            index.FORCE_PIECES = None
+            index._split_cache.clear()
+    names = ('o', 'ht', 'dq', 'dk', 'dv', 'dg', 'dbeta', 'dh0')
+    for n, a, b in zip(names, run(1), run(3)):
+        if odd is not None:
+            bad = ~torch.isfinite(a)
+            assert torch.equal(bad, ~torch.isfinite(b)), n
+            a, b = a.masked_fill(bad, 0), b.masked_fill(bad, 0)
+        O.assert_close(f'{n} cut vs uncut', a, b, 2 * REF_TOL[n])
+        if n in ('o', 'dv') and odd is None:
+            O.assert_close(f'{n} cut vs uncut, heads that forget', a[:, :, 1:3], b[:, :, 1:3], 1e-3)
+
+
 @pytest.mark.parametrize('pieces', [None, 3])
 def test_state_v_first_layout(pieces):
     """states stored [N,HV,V,K] (the reference's state_v_first, tests/ops/test_gdn.py:385-461): the scans read h0 / dht
