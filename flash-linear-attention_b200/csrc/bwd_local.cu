@@ -27,10 +27,10 @@
 // What bounds it is the latency of the phases at two CTAs per SM, i.e. the instructions of an epilogue (39 % of issue slots, DRAM
 // 54 % of its peak rate), so epilogues work on fp32 pairs and skip blocks above the diagonal.
 // The CTAs of a chunk are neighbours in launch order: a row of q, k, v or do is then read as a whole at about one time, which DRAM
-// pages like better than 256 bytes of every row (chunks first: 187 us for 179, grouped heads in turn 226 for 217).  Pulling the
+// pages like better than 256 bytes of every row (chunks first: 187 us for 179, grouped heads in turn 226 for 217 at the time).  Pulling the
 // next head's tiles into L2 while a head is worked on was slower (244 for 226).
 // B4 T4096 H16 K=V=128: 179 us inside a step (228 with the solve's adjoint by way of dW, dU and dA, six dependent tensor-core phases
-// where there are three now; 213 with three, but element-wise stores and scalar epilogues); 8/16 heads 217 (242).
+// where there are three now; 213 with three, but element-wise stores and scalar epilogues); 8/16 heads 201 (242; 217 with the load of dh waiting for the copy of dv to leave at once).
 // One CTA of eight warps; 256 TMEM columns (C0: dP, dq^T, K K^T; C1: Z v_new^T, Q K^T; C2: Z^T; C3: dk_state^T, h Z^T, the rest of
 // dk^T) and ~111 KiB of shared memory whose regions change hands, so two CTAs per SM overlap each other's phases:
 //   R1: K   R2: do -> q   R3: v_new -> V   R4: dU -> Z^T -> dq   R5: dh -> h -> M2 | dv -> dk | dv   R6: A -> dP
@@ -271,6 +271,9 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
   const bool live = q * 16 + 15 >= cs;                          // some of that block is on or below the diagonal
   const int gcol = cs + 8 * (g >> 1) + 2 * t + (g & 1);         // the column whose sum sum8_over_g leaves in this lane
 
+  auto load_dh = [&](int hv) {
+    for (int p = 0; p < NP; ++p) tma::load_2d(Hs + p * DK * 128, &maps.dh, p * 64, (c * a.HV + hv) * DK, bar_a);
+  };
   // one thread: what a head's first phase needs, and the rest into L2
   auto load_head = [&](int hv, bool first) {
     const int hrow = (c * a.HV + hv) * DK;   // the head's state snapshot in the [.., V] view
@@ -281,9 +284,11 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
     tma::load_2d(As, &maps.a, hv * BT, cm.row, bar_a);
     tma::load_1d(gs2 + ((hv - hv0) & 1) * BT, gamma_ptr(a.gamma, c, a.HV, hv), BT * 4, bar_a);
     if (first) tma::load_3d(Ks, &maps.k, cm.row, (hq * DK) / 64, bar_a);
-    else tma::store_wait_read<0>();   // dv of the head before leaves from this place
-    for (int p = 0; p < NP; ++p) tma::load_2d(Hs + p * DK * 128, &maps.dh, p * 64, hrow, bar_a);
-    for (int p = 0; p < NP; ++p) tma::prefetch_2d(&maps.h, p * 64, hrow);
+    if (first) load_dh(hv);
+    for (int p = 0; p < NP; ++p) {
+      if (!first) tma::prefetch_2d(&maps.dh, p * 64, hrow);
+      tma::prefetch_2d(&maps.h, p * 64, hrow);
+    }
     if (first) tma::prefetch_3d(&maps.q, cm.row, (hq * DK) / 64);
     tma::prefetch_3d(&maps.v, cm.row, (hv * DK) / 64);
   };
@@ -750,6 +755,10 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
       }
     }
     if (!last) {
+      if (tid == 0) {   // dv of this head leaves from the place of dh; waited for here, where the copy has long been read
+        tma::store_wait_read<0>();
+        load_dh(hv + 1);
+      }
       __syncthreads();   // the vectors have been read
       head_vectors(hv + 1, raw_next);
     }
@@ -849,11 +858,10 @@ int launch(const b200gdn_chunk_args& a, cudaStream_t st) {
 }
 
 // Several value heads per q/k head: in turn in one CTA, or a CTA each and the sums of dq and dk through a cluster.  A cluster
-// costs about a quarter more per head (it holds its CTAs until the slowest has arrived and its sums have been read: 272 us
-// against 242 at B4 T4096 8/16 heads of 128), but has G times as many CTAs, so it stays where turns would leave
+// costs more per head (it holds its CTAs until the slowest has arrived and its sums have been read: 260 us against 201 at B4 T4096
+// 8/16 heads of 128, but 78 against 87 at B1 T3300 4/16 heads, whose turns are four rounds and whose clusters three), but has G times as many CTAs, so it stays where turns would leave
 // the device to a few: two fit on an SM, and the rounds of CTAs decide.  Group sizes other than two, four
-// and eight are taken in turns always (the two kernels of the single stages, which such groups used where there are few chunks, also
-// take heads in turn: 1 x 2048 tokens, 2/12 heads of 128: 122 us, 90 here; 1/3 heads of 64: 34, 32).  Both forms add the heads
+// and eight are taken in turns always.  Both forms add the heads
 // in the same order and precision.
 bool in_turns(const b200gdn_chunk_args& a) {
   const int64_t slots = 2 * sm_count();
