@@ -23,6 +23,7 @@
 // diagonal of K K^T, and the largest of W and U is taken from the accumulators on their way out.
 // B4 T4096 H16 K=V=128: 87 us inside a step (105), 94 by itself between two events; with the L2 norm, gate and beta options
 // 120 us (108 + 47 for a norm pass of its own).
+#include "rowio.cuh"
 #include "tc5_tile.cuh"
 #include "tma.cuh"
 
@@ -116,8 +117,7 @@ template <int DK>
 __device__ __forceinline__ void normalise_rows(unsigned char* tile, int tid, int len, float* rstd, int64_t rstride, __nv_bfloat16* out,
                                                int64_t ostride) {
   const int r = tid >> 2, seg = tid & 3;
-  float2 x[DK / 32][4];
-  float ss = 0.f;
+  uint64_t x[DK / 32][4], s2[2] = {0ull, 0ull};   // pairs
   auto chunk = [&](int i) {   // the lane's i-th 16-byte word of the row
     const int c = seg + 4 * i;
     return reinterpret_cast<uint4*>(tile + (c >> 3) * (BT * 128) + r * 128 + (((c & 7) ^ (r & 7)) << 4));
@@ -128,18 +128,21 @@ __device__ __forceinline__ void normalise_rows(unsigned char* tile, int tid, int
     const uint32_t u[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      x[i][e] = unpack_bf16(u[e]);
-      ss += x[i][e].x * x[i][e].x + x[i][e].y * x[i][e].y;
+      x[i][e] = widen2<__nv_bfloat16>(u[e]);
+      s2[e & 1] = fma2(x[i][e], x[i][e], s2[e & 1]);
     }
   }
+  const float2 s = unpack2(add2(s2[0], s2[1]));
+  float ss = s.x + s.y;
   ss += __shfl_xor_sync(0xffffffffu, ss, 1);
   ss += __shfl_xor_sync(0xffffffffu, ss, 2);
   const float y = 1.f / sqrtf(ss + 1e-6f);
+  const uint64_t y2 = pack2(y, y);
   if (rstd != nullptr && seg == 0 && r < len) rstd[r * rstride] = y;
 #pragma unroll
   for (int i = 0; i < DK / 32; ++i) {
-    const uint4 w = make_uint4(pack_bf16(x[i][0].x * y, x[i][0].y * y), pack_bf16(x[i][1].x * y, x[i][1].y * y),
-                               pack_bf16(x[i][2].x * y, x[i][2].y * y), pack_bf16(x[i][3].x * y, x[i][3].y * y));
+    const uint4 w = make_uint4(narrow2<__nv_bfloat16>(mul2(x[i][0], y2)), narrow2<__nv_bfloat16>(mul2(x[i][1], y2)),
+                               narrow2<__nv_bfloat16>(mul2(x[i][2], y2)), narrow2<__nv_bfloat16>(mul2(x[i][3], y2)));
     *chunk(i) = w;
     if (out != nullptr && r < len) *reinterpret_cast<uint4*>(out + r * ostride + (seg + 4 * i) * 8) = w;
   }
