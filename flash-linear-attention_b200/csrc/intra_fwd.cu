@@ -56,7 +56,7 @@ struct IntraSmem {
 };
 
 struct IntraMaps {
-  CUtensorMap k, v, w, u, q;
+  CUtensorMap k, v, w, u, q, kn, qn;
 };
 
 // A21 = -A22 (L21 A11) for an N x N block below the diagonal whose corner is (r0, c0), T = L21 A11 going through a compact
@@ -261,12 +261,13 @@ __global__ void __launch_bounds__(NTHREADS, 4) intra_fwd_kernel(const b200gdn_ch
   }
   if ((a.options & B200GDN_PREP_L2NORM) && !failed) {   // q and k are the raw tensors; the scans read the normalised ones
     const bool lead = hv % G == 0;   // one of the value heads that share these q and k
+    const bool rows_out = lead && cm.len < BT;   // whole tiles leave by TMA below
     const int64_t at = row0 * a.H + hq, st = (int64_t)a.H * DK;
     if (cm.len < BT) __syncthreads();   // the zeroed tail of K
     normalise_rows<DK>(Ks, tid, cm.len, lead && a.rstd_k ? a.rstd_k + at : nullptr, a.H,
-                       lead ? reinterpret_cast<__nv_bfloat16*>(a.kn) + at * DK : nullptr, st);
+                       rows_out ? reinterpret_cast<__nv_bfloat16*>(a.kn) + at * DK : nullptr, st);
     if (with_qk) normalise_rows<DK>(Qs, tid, cm.len, lead && a.rstd_q ? a.rstd_q + at : nullptr, a.H,
-                                    lead ? reinterpret_cast<__nv_bfloat16*>(a.qn) + at * DK : nullptr, st);
+                                    rows_out ? reinterpret_cast<__nv_bfloat16*>(a.qn) + at * DK : nullptr, st);
     tc5::fence_async_smem();
   }
   if (__syncthreads_or(failed)) {
@@ -278,6 +279,12 @@ __global__ void __launch_bounds__(NTHREADS, 4) intra_fwd_kernel(const b200gdn_ch
       if (with_qk) issue_mma_t<DK / 16>(tm + 64, Operand{tc5::smem_addr(Qs), BT, 0}, Operand{tc5::smem_addr(Ks), BT, 0}, 64, 64, 0);
       ph.commit();
     }
+    const bool tiles_out = (a.options & B200GDN_PREP_L2NORM) && hv % G == 0 && cm.len == BT;
+    if (tiles_out && tid == 32) {   // the normalised tiles leave while the products run
+      if (with_qk) tma::store_3d(&maps.qn, (int)cm.row, (hq * DK) / 64, Qs);
+      tma::store_3d(&maps.kn, (int)cm.row, (hq * DK) / 64, Ks);
+      tma::store_commit();
+    }
     if (tid < BT) graw[tid] = (gam[tid] + (tid >= 32 ? gam[31] : 0.f)) * 1.4426950216f;
     __syncthreads();
     if (tid < BT) {
@@ -288,6 +295,7 @@ __global__ void __launch_bounds__(NTHREADS, 4) intra_fwd_kernel(const b200gdn_ch
       bge[tid] = bet[tid] * fast_exp2(gm);
       a.gamma[((int64_t)c * a.HV + hv) * BT + tid] = gm;   // padded rows carry the last valid value (their g is 0)
     }
+    if (tiles_out && tid == 32) tma::store_wait_read<0>();   // L takes the place of q
     if (!ph.sync_wait()) failed = true;
   }
 
@@ -532,6 +540,11 @@ int launch(const b200gdn_chunk_args& a, cudaStream_t st) {
   rc |= tma::encode_bf16_panels(&m.w, a.w, a.rows, pw, pw, BT, DK / 64);
   rc |= tma::encode_bf16_panels(&m.u, a.u, a.rows, pv, pv, BT, DV / 64);
   if (a.q) rc |= tma::encode_bf16_panels(&m.q, a.q, a.rows, pk, pk, BT, DK / 64); else m.q = m.k;
+  m.kn = m.qn = m.k;
+  if (a.options & B200GDN_PREP_L2NORM) {
+    rc |= tma::encode_bf16_panels(&m.kn, a.kn, a.rows, pk, pk, BT, DK / 64);
+    rc |= tma::encode_bf16_panels(&m.qn, a.qn, a.rows, pk, pk, BT, DK / 64);
+  }
   if (rc != 0) return set_error(B200GDN_ERR_CUDA, "intra_fwd: cuTensorMapEncodeTiled failed (%d)", rc);
   dim3 grid(a.n_chunks, a.HV);
   launch_overlapped(overlaps(a), intra_fwd_kernel<DK, DV>, grid, NTHREADS, S::bytes, st, a, m, resident_ctas<intra_fwd_kernel<DK, DV>>(NTHREADS, S::bytes));
