@@ -54,6 +54,7 @@ class RecurrentArgs(C.Structure):
 
 PREP_L2NORM, PREP_GATE, PREP_BETA_SIGMOID, PREP_NEG_EIGVAL = 1, 2, 4, 8
 TRANSITION_BOUNDS = 32   # chunk passes: gamma is followed by a bound of each chunk's state transition
+FORWARD_ONLY = 64   # forward pass: A is not written
 STATE_V_FIRST = 16   # chunk passes: h0, ht, dht, dh0 stored [N,HV,V,K]
 PREP_PART_ROWS = 128
 

@@ -80,7 +80,8 @@ int b200gdn_chunk_fwd(const b200gdn_chunk_args* a, void* stream) {
   const uint32_t m = a->stage_mask ? a->stage_mask : (B200GDN_FWD_INTRA | B200GDN_FWD_SCAN | B200GDN_FWD_OUT);
   if (m & B200GDN_FWD_INTRA) {
     REQUIRE(a->k, "chunk_fwd"); REQUIRE(a->v, "chunk_fwd"); REQUIRE(a->g, "chunk_fwd"); REQUIRE(a->beta, "chunk_fwd");
-    REQUIRE(a->gamma, "chunk_fwd"); REQUIRE(a->A, "chunk_fwd"); REQUIRE(a->w, "chunk_fwd"); REQUIRE(a->u, "chunk_fwd");
+    REQUIRE(a->gamma, "chunk_fwd"); REQUIRE(a->w, "chunk_fwd"); REQUIRE(a->u, "chunk_fwd");
+    if (!(a->options & B200GDN_FORWARD_ONLY)) { REQUIRE(a->A, "chunk_fwd"); }
     if (int e = launch_intra_fwd(*a, st)) return e;
   }
   if ((m & B200GDN_FWD_SCAN) && (m & B200GDN_FWD_OUT)) {

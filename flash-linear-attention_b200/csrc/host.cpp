@@ -402,7 +402,7 @@ ChunkForward chunk_forward(const Tensor& q_in, const Tensor& k_in, const Tensor&
   if (bounds) options |= B200GDN_TRANSITION_BOUNDS;
   s->options = options & ~B200GDN_PREP_L2NORM;
   s->off_gamma = slab.add(C * HV * (64 + (bounds ? 1 : 0)) * 4);
-  s->off_A = slab.add(rows * HV * 64 * 2);
+  s->off_A = slab.add(need_grad ? rows * HV * 64 * 2 : 0);
   s->off_qk = slab.add(rows * HV * 64 * 2);
   s->off_w = slab.add(rows * HV * K * 2);
   s->off_vnew = slab.add(need_grad ? rows * HV * V * 2 : 0);
@@ -416,7 +416,7 @@ ChunkForward chunk_forward(const Tensor& q_in, const Tensor& k_in, const Tensor&
     r.A_log = dense(A_log_in, at::kFloat);
     r.dt_bias = dense(dt_bias_in, at::kFloat);
   }
-  a.options = options;
+  a.options = options | (need_grad ? 0u : B200GDN_FORWARD_ONLY);
   a.gb_dtype = s->gb_dtype;
   a.g = ptr(g);
   a.beta = ptr(beta);

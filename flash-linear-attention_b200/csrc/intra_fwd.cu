@@ -421,9 +421,11 @@ __global__ void __launch_bounds__(NTHREADS, 4) intra_fwd_kernel(const b200gdn_ch
       // A itself goes straight to global memory, 64 contiguous bytes per row and quad
       __nv_bfloat16* Ag = reinterpret_cast<__nv_bfloat16*>(a.A) + (row0 * a.HV + hv) * BT + cs + 8 * t;
       const int64_t astride = (int64_t)a.HV * BT;
-      const uint4 lo = quad_words(fa.lo, t), hi = quad_words(fa.hi, t);
-      if (r_lo < cm.len) *reinterpret_cast<uint4*>(Ag + r_lo * astride) = lo;
-      if (r_hi < cm.len) *reinterpret_cast<uint4*>(Ag + r_hi * astride) = hi;
+      if (!(a.options & B200GDN_FORWARD_ONLY)) {
+        const uint4 lo = quad_words(fa.lo, t), hi = quad_words(fa.hi, t);
+        if (r_lo < cm.len) *reinterpret_cast<uint4*>(Ag + r_lo * astride) = lo;
+        if (r_hi < cm.len) *reinterpret_cast<uint4*>(Ag + r_hi * astride) = hi;
+      }
     }
     tc5::fence_async_smem();
     tc5::fence_before_sync();

@@ -76,6 +76,8 @@ typedef enum b200gdn_status {
  * which the intra stage writes (+infinity where w or u of the chunk is not finite).  A pre-scan (a scan that stores nothing but its
  * final state and the transition matrix) leaves out the chunks from which no more than 2^-128 reaches the end of its sequence. */
 #define B200GDN_TRANSITION_BOUNDS 32u
+/* b200gdn_chunk_fwd: no backward pass follows.  A, which only that reads, is not written and may be NULL. */
+#define B200GDN_FORWARD_ONLY 64u
 typedef struct b200gdn_chunk_args {
   int32_t struct_bytes;          /* = sizeof(b200gdn_chunk_args), checked */
   int32_t rows, H, HV, K, V;
