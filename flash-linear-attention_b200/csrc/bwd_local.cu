@@ -235,7 +235,8 @@ __device__ __forceinline__ void cluster_sync() {
 enum Heads { kOne, kCluster, kTurns };
 
 template <int DK, Heads MODE>
-__global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_chunk_args a, const __grid_constant__ LocalMaps maps) {
+__global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_chunk_args a, const __grid_constant__ LocalMaps maps,
+                                                                const bool out_maps) {
   constexpr bool GROUPED = MODE == kCluster, TURNS = MODE == kTurns;
   using S = LocalSmem<DK>;
   constexpr int NP = DK / 64;   // 64-column panels of a V-wide tile (V = K)
@@ -266,6 +267,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
   const int hv0 = TURNS ? hq * G : head, n_heads = TURNS ? G : 1;
   const ChunkMeta cm = load_chunk_meta(a.chunk_meta, c);
   const int64_t row0 = cm.row;
+  const bool by_tma = cm.len == BT && out_maps;   // how dq, dk and dv leave
   const int r_lo = q * 16 + g, r_hi = r_lo + 8, cs = hc * 32;   // this warp's block of a [64][64] tile
   const int kr = (DK / 4) * q;                                  // ... and its first row of a transposed accumulator
   const bool live = q * 16 + 15 >= cs;                          // some of that block is on or below the diagonal
@@ -605,7 +607,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
     tc5::fence_async_smem();   // the staged tiles are read, and what was read here is overwritten, by bulk copies
     tc5::fence_before_sync();
     if (__syncthreads_or(!ph.wait())) { failed = true; break; }
-    if (cm.len == BT) {
+    if (by_tma) {
       if (tid == 0) {
         tma::store_3d(&maps.dv, cm.row, (hv * DK) / 64, Dvs);
         if (!GROUPED && last) tma::store_3d(&maps.dq, cm.row, (hq * DK) / 64, Dqs);
@@ -718,7 +720,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) bwd_local_kernel(const b200gdn_ch
     }
     __syncthreads();
     if (!GROUPED && last) {
-      if (cm.len == BT) {
+      if (by_tma) {
         if (tid == 0) {
           tma::store_3d(&maps.dk, cm.row, (hq * DK) / 64, Dks);
           tma::store_commit();
@@ -827,9 +829,14 @@ int launch(const b200gdn_chunk_args& a, cudaStream_t st) {
   rc |= tma::encode_bf16_panels(&m.d_o, a.d_o, a.rows, pv, pv, BT, DK / 64);
   rc |= tma::encode_bf16_panels(&m.vn, a.v_new, a.rows, pv, pv, BT, DK / 64);
   rc |= tma::encode_bf16_panels(&m.du, a.dv2, a.rows, pv, pv, BT, DK / 64);
-  rc |= tma::encode_bf16_panels(&m.dq, a.dq, a.rows, pk, pk, BT, DK / 64);
-  rc |= tma::encode_bf16_panels(&m.dk, a.dk, a.rows, pk, pk, BT, DK / 64);
-  rc |= tma::encode_bf16_panels(&m.dv, a.dv, a.rows, pv, pv, BT, DK / 64);
+  // A tensor map costs the host 0.6 us: small problems, which wait for the host, store their results by rows
+  const bool out_maps = !overlaps(a);
+  m.dq = m.dk = m.dv = m.q;
+  if (out_maps) {
+    rc |= tma::encode_bf16_panels(&m.dq, a.dq, a.rows, pk, pk, BT, DK / 64);
+    rc |= tma::encode_bf16_panels(&m.dk, a.dk, a.rows, pk, pk, BT, DK / 64);
+    rc |= tma::encode_bf16_panels(&m.dv, a.dv, a.rows, pv, pv, BT, DK / 64);
+  }
   rc |= tma::encode_bf16_2d(&m.a, a.A, a.rows, (uint64_t)a.HV * BT, (uint64_t)a.HV * BT, BT);
   rc |= tma::encode_bf16_2d(&m.h, a.h, hrows, DK, DK, DK);
   rc |= tma::encode_bf16_2d(&m.dh, a.dh, hrows, DK, DK, DK);
@@ -852,7 +859,7 @@ int launch(const b200gdn_chunk_args& a, cudaStream_t st) {
     attr[cfg.numAttrs].val.clusterDim.y = 1;
     attr[cfg.numAttrs++].val.clusterDim.z = 1;
   }
-  cudaLaunchKernelEx(&cfg, bwd_local_kernel<DK, MODE>, a, m);
+  cudaLaunchKernelEx(&cfg, bwd_local_kernel<DK, MODE>, a, m, out_maps);
   if (int e = check_launch("bwd_local")) return e;
   return launch_gate_reduce(a, st);
 }

@@ -157,7 +157,7 @@ __device__ __forceinline__ float max_abs3(float a, float b, float c) {
 
 template <int DK, int DV>
 __global__ void __launch_bounds__(NTHREADS, 4) intra_fwd_kernel(const b200gdn_chunk_args a, const __grid_constant__ IntraMaps maps,
-                                                                const int pf_dist) {
+                                                                const int pf_dist, const bool out_maps) {
   using S = IntraSmem<DK, DV>;
   constexpr int KB = DK / 64, VB = DV / 64;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -261,7 +261,7 @@ __global__ void __launch_bounds__(NTHREADS, 4) intra_fwd_kernel(const b200gdn_ch
   }
   if ((a.options & B200GDN_PREP_L2NORM) && !failed) {   // q and k are the raw tensors; the scans read the normalised ones
     const bool lead = hv % G == 0;   // one of the value heads that share these q and k
-    const bool rows_out = lead && cm.len < BT;   // whole tiles leave by TMA below
+    const bool rows_out = lead && !(out_maps && cm.len == BT);   // whole tiles leave by TMA below
     const int64_t at = row0 * a.H + hq, st = (int64_t)a.H * DK;
     if (cm.len < BT) __syncthreads();   // the zeroed tail of K
     normalise_rows<DK>(Ks, tid, cm.len, lead && a.rstd_k ? a.rstd_k + at : nullptr, a.H,
@@ -279,7 +279,7 @@ __global__ void __launch_bounds__(NTHREADS, 4) intra_fwd_kernel(const b200gdn_ch
       if (with_qk) issue_mma_t<DK / 16>(tm + 64, Operand{tc5::smem_addr(Qs), BT, 0}, Operand{tc5::smem_addr(Ks), BT, 0}, 64, 64, 0);
       ph.commit();
     }
-    const bool tiles_out = (a.options & B200GDN_PREP_L2NORM) && hv % G == 0 && cm.len == BT;
+    const bool tiles_out = out_maps && hv % G == 0 && cm.len == BT;
     if (tiles_out && tid == 32) {   // the normalised tiles leave while the products run
       if (with_qk) tma::store_3d(&maps.qn, (int)cm.row, (hq * DK) / 64, Qs);
       tma::store_3d(&maps.kn, (int)cm.row, (hq * DK) / 64, Ks);
@@ -543,13 +543,14 @@ int launch(const b200gdn_chunk_args& a, cudaStream_t st) {
   rc |= tma::encode_bf16_panels(&m.u, a.u, a.rows, pv, pv, BT, DV / 64);
   if (a.q) rc |= tma::encode_bf16_panels(&m.q, a.q, a.rows, pk, pk, BT, DK / 64); else m.q = m.k;
   m.kn = m.qn = m.k;
-  if (a.options & B200GDN_PREP_L2NORM) {
+  const bool out_maps = (a.options & B200GDN_PREP_L2NORM) && !overlaps(a);   // (small problems wait for the host, and a map costs it 0.6 us)
+  if (out_maps) {
     rc |= tma::encode_bf16_panels(&m.kn, a.kn, a.rows, pk, pk, BT, DK / 64);
     rc |= tma::encode_bf16_panels(&m.qn, a.qn, a.rows, pk, pk, BT, DK / 64);
   }
   if (rc != 0) return set_error(B200GDN_ERR_CUDA, "intra_fwd: cuTensorMapEncodeTiled failed (%d)", rc);
   dim3 grid(a.n_chunks, a.HV);
-  launch_overlapped(overlaps(a), intra_fwd_kernel<DK, DV>, grid, NTHREADS, S::bytes, st, a, m, resident_ctas<intra_fwd_kernel<DK, DV>>(NTHREADS, S::bytes));
+  launch_overlapped(overlaps(a), intra_fwd_kernel<DK, DV>, grid, NTHREADS, S::bytes, st, a, m, resident_ctas<intra_fwd_kernel<DK, DV>>(NTHREADS, S::bytes), out_maps);
   return check_launch("intra_fwd");
 }
 

@@ -885,3 +885,32 @@ def test_gate_gradients_keep_their_distance_from_fp64(D, H, limit_dg, limit_sum)
         sums.append((got_dt - ref_dt) / ref_g[0].norm(dim=0))
     assert torch.stack(errs).mean() <= limit_dg
     assert torch.stack(sums).square().mean().sqrt() <= limit_sum
+
+
+@pytest.mark.parametrize('D', [64, 128])
+@pytest.mark.parametrize('H,HV,copies', [(2, 2, 1), (1, 2, 1), (1, 3, 1), (2, 4, 24)])
+def test_chunk_local_backward_at_chunk_edges(D, H, HV, copies):
+    """Chunks of 1, 2, 63 and 64 tokens next to one another, write strengths of exactly 0 and 1 among them, one head, groups that meet in a
+    cluster, groups that one CTA takes in turn (three heads, and many chunks): every gradient against the fp64 recurrence."""
+    from b200gdn import chunk_gated_delta_rule
+    lens = [1, 63, 64, 65, 130, 2] * copies
+    cu = [0] + [int(x) for x in np.cumsum(lens)]
+    T = cu[-1]
+    d = O.make_inputs(1, T, H, HV, D, D, seed=41, cu_seqlens=cu)
+    d['beta'][:, ::5] = 0.0
+    d['beta'][:, 3::7] = 1.0
+    bf = torch.bfloat16
+    leaves = [d[n].to('cuda').to(bf).requires_grad_(True) for n in ('q', 'k', 'v')]
+    leaves += [d[n].to('cuda').requires_grad_(True) for n in ('g', 'beta', 'h0')]
+    cu_t = torch.tensor(cu, dtype=torch.int32, device='cuda')
+    o, ht = chunk_gated_delta_rule(*leaves[:5], initial_state=leaves[5], output_final_state=True, cu_seqlens=cu_t)
+    torch.autograd.backward([o, ht], [d['do'].to('cuda').to(bf), d['dht'].to('cuda')])
+    with torch.no_grad():   # where A is not written
+        o_only, ht_only = chunk_gated_delta_rule(*leaves[:5], initial_state=leaves[5], output_final_state=True, cu_seqlens=cu_t)
+    assert torch.equal(o, o_only) and torch.equal(ht, ht_only)
+    ro, rht, rg = O.naive_with_grads(*(d[n].to(bf).float() for n in ('q', 'k', 'v')), d['g'], d['beta'], D ** -0.5, d['h0'],
+                                     d['do'].to(bf).float(), d['dht'], cu_seqlens=cu)
+    O.assert_close('o', ro.float(), o.detach().float().cpu(), REF_TOL['o'])
+    O.assert_close('ht', rht.float(), ht.detach().cpu(), REF_TOL['ht'])
+    for n, leaf in zip(('dq', 'dk', 'dv', 'dg', 'dbeta', 'dh0'), leaves):
+        O.assert_close(n, rg[n].float(), leaf.grad.float().cpu(), REF_TOL[n])
