@@ -45,16 +45,18 @@ import torch  # noqa: E402
 METRIC = 'tokens/s chunk_gated_delta_rule fwd+bwd (B4 T4096 H16 D128 bf16); % tensor peak'
 B, T, H, HV, K, V, BT = 4, 4096, 16, 16, 128, 128, 64
 
-# algorithmic FLOPs per (token, value head), dense-tile counting, no recomputation
+# FLOPs per (token, value head) of what the kernels form, dense-tile counting, no recomputation
 STAGE_FLOPS = {
     'intra_fwd': 2 * BT * (3 * K + V),                                 # K K^T, W, U | Q K^T
     'scan_out_fwd': 4 * K * V + 2 * K * V + 2 * BT * V,                # W S, K^T V~ | Q S, P V
     'scan_dvl_bwd': 6 * K * V + 2 * BT * (K + V),                      # K dS, Q^T do, W^T dv2 | P^T do (+ the Q K^T it does not redo)
-    # dP, do h^T, v dh^T, dP k, dP^T q | dv2 h^T + WY backward
-    'bwd_local': 6 * K * V + 2 * BT * (V + 2 * K) + 2 * BT * (5 * K + 2 * V + 2 * BT),
+    # do h^T, v dh^T, Z h^T | A^T dv2, dP, Z v^T | dP k, dP^T q, M k, M^T k, K K^T, Q K^T
+    'bwd_local': 6 * K * V + 2 * BT * (3 * V + 6 * K),
 }
+# algorithmic FLOPs of the passes: the WY backward counted as the reference forms it (dW, dU V^T, A^T dA A^T), which takes more
+# products than the adjoint of the solve that bwd_local uses
 F_FWD = STAGE_FLOPS['intra_fwd'] + STAGE_FLOPS['scan_out_fwd']
-F_BWD = STAGE_FLOPS['scan_dvl_bwd'] + STAGE_FLOPS['bwd_local']
+F_BWD = STAGE_FLOPS['scan_dvl_bwd'] + 6 * K * V + 2 * BT * (V + 2 * K) + 2 * BT * (5 * K + 2 * V + 2 * BT)
 assert F_FWD == 180224 and F_BWD == 409600
 
 
@@ -91,8 +93,8 @@ def staged_bytes(R, C, NS):
 # stale with every kernel change: refresh it together with the profile.
 NCU_TRAFFIC = {
     'source': 'profiles/chunk_fwd_bwd_B4_T4096_H16_D128_four_kernels.md',
-    'kernel_sources_commit': 'db95f86',
-    'bytes': {'intra_fwd': 358.8e6, 'scan_out_fwd': 536.1e6, 'scan_dvl_bwd': 469.7e6, 'bwd_local': 891.8e6},
+    'kernel_sources_commit': 'cc215a0',
+    'bytes': {'intra_fwd': 361.8e6, 'scan_out_fwd': 539.4e6, 'scan_dvl_bwd': 472.6e6, 'bwd_local': 886.8e6},
 }
 
 
