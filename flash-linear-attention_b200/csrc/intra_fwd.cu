@@ -155,7 +155,8 @@ __device__ __forceinline__ float max_abs3(float a, float b, float c) {
   return d;
 }
 
-template <int DK, int DV>
+// BOUNDS: option TRANSITION_BOUNDS (an instantiation of its own: a small pass was 1 % slower with the branches alone)
+template <int DK, int DV, bool BOUNDS>
 __global__ void __launch_bounds__(NTHREADS, 4) intra_fwd_kernel(const b200gdn_chunk_args a, const __grid_constant__ IntraMaps maps,
                                                                 const int pf_dist, const bool out_maps) {
   using S = IntraSmem<DK, DV>;
@@ -195,7 +196,7 @@ __global__ void __launch_bounds__(NTHREADS, 4) intra_fwd_kernel(const b200gdn_ch
   // with q and a qk buffer the kernel also emits the gated causal q k^T tile that the scans use for the chunk-local
   // parts of o and dv (so that they neither form nor mask it on their serial chain)
   const bool with_qk = a.qk != nullptr && a.q != nullptr;
-  const bool bounds = a.options & B200GDN_TRANSITION_BOUNDS;
+  constexpr bool bounds = BOUNDS;
   unsigned char* Qs = smem + S::o_l;
 
   if (tid == 0) {
@@ -314,7 +315,6 @@ __global__ void __launch_bounds__(NTHREADS, 4) intra_fwd_kernel(const b200gdn_ch
         const float g_lo = gam[r_lo], g_hi = gam[r_hi];
         const float b_lo = bet[r_lo], b_hi = bet[r_hi];
         uint32_t p_lo[4], p_hi[4];
-        float kk_lo = 0.f, kk_hi = 0.f;   // |k|^2 of the two rows, where the diagonal is this thread's
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const int j0 = cs + i * 8 + 2 * t;
@@ -324,7 +324,6 @@ __global__ void __launch_bounds__(NTHREADS, 4) intra_fwd_kernel(const b200gdn_ch
           for (int e = 0; e < 4; ++e) {
             const int ii = (e & 2) ? r_hi : r_lo, jj = j0 + (e & 1);
             const float f = fast_exp2(((e & 2) ? g_hi : g_lo) - ((e & 1) ? gj.y : gj.x));
-            if (ii == jj) ((e & 2) ? kk_hi : kk_lo) = r[4 * i + e];
             v[e] = (ii > jj) ? r[4 * i + e] * ((e & 2) ? b_hi : b_lo) * f : 0.f;
             w4[e] = (with_qk && ii >= jj) ? pq[4 * i + e] * f : 0.f;
           }
@@ -334,6 +333,13 @@ __global__ void __launch_bounds__(NTHREADS, 4) intra_fwd_kernel(const b200gdn_ch
           p_hi[i] = pack_bf16(w4[2], w4[3]);
         }
         if (bounds) {
+          float kk_lo = 0.f, kk_hi = 0.f;   // |k|^2 of the two rows, where the diagonal is this thread's
+#pragma unroll
+          for (int e = 0; e < 16; ++e) {
+            const int jj = cs + (e >> 2) * 8 + 2 * t + (e & 1);
+            if ((e & 2) && jj == r_hi) kk_hi = r[e];
+            if (!(e & 2) && jj == r_lo) kk_lo = r[e];
+          }
           float x = log2f(fmaxf(1.f, fabsf(1.f - b_lo * kk_lo))) + log2f(fmaxf(1.f, fabsf(1.f - b_hi * kk_hi)));
 #pragma unroll
           for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
@@ -504,7 +510,9 @@ __global__ void __launch_bounds__(NTHREADS, 4) intra_fwd_kernel(const b200gdn_ch
         }
         tc5::fence_async_smem();
         tc5::fence_before_sync();
-        const int odd = __syncthreads_or(!(size < INFINITY));
+        int odd = 0;
+        if (bounds) odd = __syncthreads_or(!(size < INFINITY));
+        else __syncthreads();
         if (bounds && tid == 0) {
           float x = gam[BT - 1];
 #pragma unroll
@@ -530,10 +538,10 @@ __global__ void __launch_bounds__(NTHREADS, 4) intra_fwd_kernel(const b200gdn_ch
   if (warp == 1) tc5::tmem_dealloc(tm, 128);
 }
 
-template <int DK, int DV>
+template <int DK, int DV, bool BOUNDS>
 int launch(const b200gdn_chunk_args& a, cudaStream_t st) {
   using S = IntraSmem<DK, DV>;
-  if (int e = ensure_smem(intra_fwd_kernel<DK, DV>, S::bytes)) return e;
+  if (int e = ensure_smem(intra_fwd_kernel<DK, DV, BOUNDS>, S::bytes)) return e;
   IntraMaps m;
   const uint64_t pk = (uint64_t)a.H * DK, pw = (uint64_t)a.HV * DK, pv = (uint64_t)a.HV * DV;
   int rc = 0;
@@ -550,7 +558,7 @@ int launch(const b200gdn_chunk_args& a, cudaStream_t st) {
   }
   if (rc != 0) return set_error(B200GDN_ERR_CUDA, "intra_fwd: cuTensorMapEncodeTiled failed (%d)", rc);
   dim3 grid(a.n_chunks, a.HV);
-  launch_overlapped(overlaps(a), intra_fwd_kernel<DK, DV>, grid, NTHREADS, S::bytes, st, a, m, resident_ctas<intra_fwd_kernel<DK, DV>>(NTHREADS, S::bytes), out_maps);
+  launch_overlapped(overlaps(a), intra_fwd_kernel<DK, DV, BOUNDS>, grid, NTHREADS, S::bytes, st, a, m, resident_ctas<intra_fwd_kernel<DK, DV, BOUNDS>>(NTHREADS, S::bytes), out_maps);
   return check_launch("intra_fwd");
 }
 
@@ -561,8 +569,9 @@ int launch_intra_fwd(const b200gdn_chunk_args& a, cudaStream_t st) {
     return set_error(B200GDN_ERR_BAD_ARGUMENT, "intra_fwd: the fused gate needs A_log");
   if ((a.options & B200GDN_PREP_L2NORM) && (a.qn == nullptr || a.kn == nullptr))
     return set_error(B200GDN_ERR_BAD_ARGUMENT, "intra_fwd: the fused L2 norm needs qn and kn");
-  if (a.K == 128 && a.V == 128) return launch<128, 128>(a, st);
-  if (a.K == 64 && a.V == 64) return launch<64, 64>(a, st);
+  const bool bounds = a.options & B200GDN_TRANSITION_BOUNDS;
+  if (a.K == 128 && a.V == 128) return bounds ? launch<128, 128, true>(a, st) : launch<128, 128, false>(a, st);
+  if (a.K == 64 && a.V == 64) return bounds ? launch<64, 64, true>(a, st) : launch<64, 64, false>(a, st);
   return set_error(B200GDN_ERR_UNSUPPORTED, "intra_fwd: K=%d V=%d not built (64/64 and 128/128 are)", a.K, a.V);
 }
 

@@ -55,7 +55,9 @@ struct ScanBwdMaps {
   CUtensorMap q, k, w, d_o, dv2, dh, pq;
 };
 
-template <int DK, int DV, int NSTAGE, bool DVL>
+// PRE: nothing stored but the final gradient (a pre-scan); an instantiation of its own, because the look at the bounds, not executed,
+// cost the main scan 5 us in 95
+template <int DK, int DV, int NSTAGE, bool DVL, bool PRE>
 __global__ void __launch_bounds__(NTHREADS, 1)
     scan_bwd_kernel(const b200gdn_chunk_args a, const __grid_constant__ ScanBwdMaps maps) {
   using S = ScanBwdSmem<DK, NSTAGE, DVL>;
@@ -91,7 +93,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   const bool st_dh = !m_mode && a.dh != nullptr;
   float* const dh0_out = m_mode ? a.cp_dM : a.dh0;
   bool m_zero = false;   // the transition matrix is zero
-  if (DVL && a.dh == nullptr && a.dv2 == nullptr && (a.options & B200GDN_TRANSITION_BOUNDS)) {
+  if (PRE && (a.options & B200GDN_TRANSITION_BOUNDS)) {
     int reach = chunks_that_reach(bounds_ptr(const_cast<float*>(a.gamma), a.n_chunks, a.HV), a.HV, hv, c_first, nc, 1, lane);
     if (reach < nc && !m_mode) {
       // an output gradient that is not finite reaches everything before it; those left out are looked at, which takes a twentieth of
@@ -419,13 +421,13 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   if (warp == 0) tc5::tmem_dealloc(tm, TMEM_COLS);
 }
 
-template <int DK, int DV, int NSTAGE, bool DVL>
+template <int DK, int DV, int NSTAGE, bool DVL, bool PRE = false>
 int launch(const b200gdn_chunk_args& a, cudaStream_t st) {
   using S = ScanBwdSmem<DK, NSTAGE, DVL>;
   static_assert(DV % BV == 0, "value dimension is processed in 64-column slices");
   static_assert(S::bytes <= 227 * 1024, "shared memory of one CTA");
   static_assert(DK == DV, "the transition-matrix slices reuse the value-slice code with V := K");
-  if (int e = ensure_smem(scan_bwd_kernel<DK, DV, NSTAGE, DVL>, S::bytes)) return e;
+  if (int e = ensure_smem(scan_bwd_kernel<DK, DV, NSTAGE, DVL, PRE>, S::bytes)) return e;
   ScanBwdMaps m;
   const uint64_t pk = (uint64_t)a.H * DK, pw = (uint64_t)a.HV * DK, pv = (uint64_t)a.HV * DV;
   int rc = 0;
@@ -441,7 +443,7 @@ int launch(const b200gdn_chunk_args& a, cudaStream_t st) {
   if (DVL) rc |= tma::encode_bf16_2d(&m.pq, a.qk, a.rows, (uint64_t)a.HV * BT, (uint64_t)a.HV * BT, BT); else m.pq = dummy;
   if (rc != 0) return set_error(B200GDN_ERR_CUDA, "scan_bwd: cuTensorMapEncodeTiled failed (%d)", rc);
   dim3 grid(DV / BV + (a.cp_dM != nullptr ? DK / BV : 0), a.HV, a.n_seq);
-  launch_overlapped(overlaps(a), scan_bwd_kernel<DK, DV, NSTAGE, DVL>, grid, NTHREADS, S::bytes, st, a, m);
+  launch_overlapped(overlaps(a), scan_bwd_kernel<DK, DV, NSTAGE, DVL, PRE>, grid, NTHREADS, S::bytes, st, a, m);
   return check_launch(DVL ? "scan_dvl_bwd" : "scan_bwd");
 }
 
@@ -458,8 +460,9 @@ int launch_scan_bwd(const b200gdn_chunk_args& a, cudaStream_t st) {
 // The reverse scan with dv_local formed on chip (needs d_o and the forward pass's qk; dv2 is an output only and may be NULL).
 int launch_scan_dvl_bwd(const b200gdn_chunk_args& a, cudaStream_t st) {
   if (a.d_o == nullptr || a.qk == nullptr) return set_error(B200GDN_ERR_BAD_ARGUMENT, "scan_dvl_bwd: d_o or qk is NULL");
-  if (a.K == 128 && a.V == 128) return launch<128, 128, 2, true>(a, st);
-  if (a.K == 64 && a.V == 64) return launch<64, 64, 3, true>(a, st);
+  const bool pre = a.dh == nullptr && a.dv2 == nullptr;
+  if (a.K == 128 && a.V == 128) return pre ? launch<128, 128, 2, true, true>(a, st) : launch<128, 128, 2, true>(a, st);
+  if (a.K == 64 && a.V == 64) return pre ? launch<64, 64, 3, true, true>(a, st) : launch<64, 64, 3, true>(a, st);
   return set_error(B200GDN_ERR_UNSUPPORTED, "scan_dvl_bwd: K=%d V=%d not built (64/64 and 128/128 are)", a.K, a.V);
 }
 
