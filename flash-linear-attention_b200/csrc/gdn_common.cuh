@@ -70,13 +70,19 @@ __device__ __forceinline__ const float* gamma_ptr(const float* gamma, int c, int
 // bounds of the chunks' state transitions (option TRANSITION_BOUNDS), [n_chunks][HV] behind gamma
 __device__ __forceinline__ float* bounds_ptr(float* gamma, int n_chunks, int HV) { return gamma + (int64_t)n_chunks * HV * BT; }
 
-// How many chunks of [c_first, c_first + nc), counted from the end (`step` -1: a forward scan's) or from the start (+1), have
-// transitions whose product is at most 2^-128: what lies beyond them does not reach a state of fp32 there (gate factors below 2^-126
-// are flushed to zero within a chunk as well).  nc where there are none, or where a chunk beyond has values that are not finite and
-// so have to.  Executed by a whole warp; a sum of infinities or NaN compares as "no".
+// Of the chunks of [c_first, c_first + nc), counted from the end (`step` -1: a forward scan's) or from the start (+1): `n`, as many as a
+// scan has to walk.  For each of the others the transitions of ALL chunks nearer the end have a product of at most 2^-128, so of what
+// it leaves in the state no more than that share arrives (gate factors below 2^-126 are flushed to zero within a chunk as well).  The
+// sums are not monotonous where gates grow, so what counts is the last one that is not below the line, not the first one that is.
+// `zero`: the product over all of them is at most 2^-128.  Where a chunk has values that are not finite nothing is left out.
+// Executed by a whole warp; a sum of infinities or NaN compares as "not below".
 constexpr float kNothingReaches = -128.f;
-__device__ __forceinline__ int chunks_that_reach(const float* bounds, int HV, int hv, int c_first, int nc, int step, int lane) {
-  int n = nc;
+struct Reach {
+  int n;
+  bool zero;
+};
+__device__ __forceinline__ Reach chunks_that_reach(const float* bounds, int HV, int hv, int c_first, int nc, int step, int lane) {
+  int n = nc < 1 ? nc : 1;
   float sum = 0.f;
   bool finite = true;
   for (int j0 = 0; j0 < nc; j0 += 32) {
@@ -88,11 +94,12 @@ __device__ __forceinline__ int chunks_that_reach(const float* bounds, int HV, in
       const float y = __shfl_up_sync(0xffffffffu, b, o);
       if (lane >= o) b += y;
     }
-    const unsigned enough = __ballot_sync(0xffffffffu, j < nc && sum + b < kNothingReaches);
-    if (n == nc && enough != 0) n = j0 + __ffs(enough);
+    // what lies beyond chunk j arrives: j + 2 chunks are walked at least
+    const unsigned arrives = __ballot_sync(0xffffffffu, j + 1 < nc && !(sum + b < kNothingReaches));
+    if (arrives != 0) n = j0 + 33 - __clz(arrives);
     sum += __shfl_sync(0xffffffffu, b, 31);
   }
-  return finite ? n : nc;
+  return finite ? Reach{n, sum < kNothingReaches} : Reach{nc, false};
 }
 
 // Look-ahead for the one-CTA-per-(chunk, head) kernels.  CTAs are dispatched in launch order (x fastest), so the

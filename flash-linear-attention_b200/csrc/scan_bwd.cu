@@ -94,11 +94,14 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   float* const dh0_out = m_mode ? a.cp_dM : a.dh0;
   bool m_zero = false;   // the transition matrix is zero
   if (PRE && (a.options & B200GDN_TRANSITION_BOUNDS)) {
-    int reach = chunks_that_reach(bounds_ptr(const_cast<float*>(a.gamma), a.n_chunks, a.HV), a.HV, hv, c_first, nc, 1, lane);
-    if (reach < nc && !m_mode) {
+    const Reach reach = chunks_that_reach(bounds_ptr(const_cast<float*>(a.gamma), a.n_chunks, a.HV), a.HV, hv, c_first, nc, 1, lane);
+    if (m_mode) {
+      m_zero = reach.zero;
+      if (m_zero) nc = 0;
+    } else if (reach.n < nc && a.dht == nullptr) {   // (an end gradient is not one of the chunks' values)
       // an output gradient that is not finite reaches everything before it; those left out are looked at, which takes a twentieth of
       // the time that walking them would
-      const ChunkMeta from = load_chunk_meta(a.chunk_meta, c_first + reach), last = load_chunk_meta(a.chunk_meta, c_first + nc - 1);
+      const ChunkMeta from = load_chunk_meta(a.chunk_meta, c_first + reach.n), last = load_chunk_meta(a.chunk_meta, c_first + nc - 1);
       const int rows = last.row + last.len - from.row, row0 = warp * 4 + (lane >> 3);
       const __nv_bfloat16* d_o = reinterpret_cast<const __nv_bfloat16*>(a.d_o) + ((int64_t)from.row * a.HV + hv) * DV + v0 + (lane & 7) * 8;
       uint32_t odd = 0;
@@ -109,11 +112,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 #pragma unroll
         for (int e = 0; e < 4; ++e) odd |= ((u[e] & 0x7f800000u) == 0x7f800000u) | ((u[e] & 0x7f80u) == 0x7f80u);
       }
-      if (__syncthreads_or(odd)) reach = nc;
-    }
-    if (reach < nc) {
-      m_zero = m_mode;
-      nc = m_mode ? 0 : reach;
+      if (!__syncthreads_or(odd)) nc = reach.n;
     }
   }
   const int c_last = c_first + nc - 1;

@@ -112,11 +112,13 @@ __global__ void __launch_bounds__(threads_of(OUT), PRE ? 2 : 1)
   int c_first = a.seq_meta[2 * n], nc = a.seq_meta[2 * n + 1];
   bool m_zero = false;   // the transition matrix is zero
   if (PRE && (a.options & B200GDN_TRANSITION_BOUNDS)) {
-    const int reach = chunks_that_reach(bounds_ptr(a.gamma, a.n_chunks, a.HV), a.HV, hv, c_first, nc, -1, lane);
-    if (reach < nc) {
-      m_zero = m_mode;
-      c_first += nc - (m_mode ? 0 : reach);
-      nc = m_mode ? 0 : reach;
+    const Reach reach = chunks_that_reach(bounds_ptr(a.gamma, a.n_chunks, a.HV), a.HV, hv, c_first, nc, -1, lane);
+    if (m_mode) {
+      m_zero = reach.zero;
+      if (m_zero) nc = 0;
+    } else if (a.h0 == nullptr) {   // (a start state is not one of the chunks' values)
+      c_first += nc - reach.n;
+      nc = reach.n;
     }
   }
   const bool has_u = !m_mode && a.u != nullptr;

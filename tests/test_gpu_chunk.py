@@ -786,6 +786,53 @@ def test_pre_scans_leave_out_what_does_not_reach(D, odd):
             O.assert_close(f'{n} cut vs uncut, heads that forget', a[:, :, 1:3], b[:, :, 1:3], 1e-3)
 
 
+@pytest.mark.parametrize('D', [64, 128])
+@pytest.mark.parametrize('reverse', [False, True])
+def test_pre_scans_where_gates_grow_and_decay(D, reverse):
+    """Pieces of 18 chunks whose state grows by 2^116 in nine of them and then decays by 2^129 (reverse: the other way round, so that the
+    gradient does, on its way back): what crosses a piece is 2^-13 of what entered it, although the product of its last (first) nine
+    transitions alone is below 2^-128.  Head 0 has a start state (end gradient) only, head 1 only what a chunk at the far end of each
+    piece adds; against the fp64 recurrence, each result in units of its own size."""
+    from b200gdn import chunk_gated_delta_rule, index
+    dev, n, pieces = 'cuda', 18 * 64, 3
+    T = n * pieces
+    d = O.make_inputs(1, T, 1, 2, D, D, seed=43)
+    grows, decays = torch.full((n // 2,), 0.14), torch.full((n // 2,), -0.155)
+    g = torch.cat([decays, grows] if reverse else [grows, decays]).repeat(pieces)[None, :, None].expand(1, T, 2).contiguous()
+    far = (torch.arange(T) % n >= n - 64) if reverse else (torch.arange(T) % n < 64)
+    beta, do, h0, dht = d['beta'].clone(), d['do'].clone(), d['h0'].clone(), d['dht'].clone()
+    beta[:, ~far] = 0
+    do[:, ~far] = 0
+    if reverse:
+        beta[:] = 0
+        do[:, :, 0] = 0
+        dht[:, 1] = 0
+    else:
+        beta[:, :, 0] = 0
+        h0[:, 1] = 0
+        do[:] = 0
+    bf = torch.bfloat16
+    q, k, v = (d[x].to(bf) for x in ('q', 'k', 'v'))
+    leaf = h0.to(dev).requires_grad_(reverse)
+    index.FORCE_PIECES = pieces
+    index._split_cache.clear()
+    try:
+        o, ht = chunk_gated_delta_rule(*(x.to(dev) for x in (q, k, v, g, beta)), initial_state=leaf, output_final_state=True)
+        if reverse:
+            torch.autograd.backward([o, ht], [do.to(dev).to(bf), dht.to(dev)])
+    finally:
+        index.FORCE_PIECES = None
+        index._split_cache.clear()
+    ro, rht, rg = O.naive_with_grads(q, k, v, g, beta, D ** -0.5, h0, do.to(bf), dht)
+    got, want = (leaf.grad.cpu(), rg['dh0']) if reverse else (ht.cpu(), rht)
+    for hv in range(2):
+        size = want[:, hv].abs().max()
+        O.assert_close(f'head {hv}', want[:, hv] / size, got[:, hv].double() / size, REF_TOL['dh0' if reverse else 'ht'])
+    if not reverse:
+        size = ro[:, -64:].abs().max()
+        O.assert_close('o', ro[:, -64:] / size, o[:, -64:].cpu().double() / size, REF_TOL['o'])
+
+
 @pytest.mark.parametrize('pieces', [None, 3])
 def test_state_v_first_layout(pieces):
     """states stored [N,HV,V,K] (the reference's state_v_first, tests/ops/test_gdn.py:385-461): the scans read h0 / dht
