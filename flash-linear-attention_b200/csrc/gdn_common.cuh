@@ -67,14 +67,19 @@ __device__ __forceinline__ const float* gamma_ptr(const float* gamma, int c, int
   return gamma + ((int64_t)c * HV + hv) * BT;
 }
 
-// bounds of the chunks' state transitions (option TRANSITION_BOUNDS), [n_chunks][HV] behind gamma
+// bounds of the chunks' state transitions (option TRANSITION_BOUNDS), [n_chunks][HV] behind gamma; +infinity (or NaN) where w or u of the
+// chunk is not finite.  The lowest bit says that the products of q and k are not: of no account for the state, but the gradient that
+// leaves the chunk is not finite then, whatever the output's gradient is.
 __device__ __forceinline__ float* bounds_ptr(float* gamma, int n_chunks, int HV) { return gamma + (int64_t)n_chunks * HV * BT; }
+
+__device__ __forceinline__ float tagged_bound(float x, bool q_odd) { return __uint_as_float((__float_as_uint(x) & ~1u) | (q_odd ? 1u : 0u)); }
 
 // Of the chunks of [c_first, c_first + nc), counted from the end (`step` -1: a forward scan's) or from the start (+1): `n`, as many as a
 // scan has to walk.  For each of the others the transitions of ALL chunks nearer the end have a product of at most 2^-128, so of what
 // it leaves in the state no more than that share arrives (gate factors below 2^-126 are flushed to zero within a chunk as well).  The
 // sums are not monotonous where gates grow, so what counts is the last one that is not below the line, not the first one that is.
-// `zero`: the product over all of them is at most 2^-128.  Where a chunk has values that are not finite nothing is left out.
+// `zero`: the product over all of them is at most 2^-128.  Where a chunk has values that are not finite (step +1: q among
+// them) nothing is left out.
 // Executed by a whole warp; a sum of infinities or NaN compares as "not below".
 constexpr float kNothingReaches = -128.f;
 struct Reach {
@@ -88,7 +93,7 @@ __device__ __forceinline__ Reach chunks_that_reach(const float* bounds, int HV, 
   for (int j0 = 0; j0 < nc; j0 += 32) {
     const int j = j0 + lane;
     float b = j < nc ? bounds[(int64_t)(step > 0 ? c_first + j : c_first + nc - 1 - j) * HV + hv] : 0.f;
-    finite = finite && __all_sync(0xffffffffu, b < INFINITY);   // (false for NaN)
+    finite = finite && __all_sync(0xffffffffu, b < INFINITY && !(step > 0 && (__float_as_uint(b) & 1u)));   // (false for NaN)
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const float y = __shfl_up_sync(0xffffffffu, b, o);

@@ -154,6 +154,8 @@ __device__ __forceinline__ float max_abs3(float a, float b, float c) {
   asm("max.NaN.abs.f32 %0, %1, %2, %3;\n" : "=f"(d) : "f"(a), "f"(b), "f"(c));
   return d;
 }
+// a magnitude that is a finite bf16 when rounded (false for NaN)
+__device__ __forceinline__ bool fits_bf16(float x) { return x <= 3.3895313892515355e38f; }
 
 // BOUNDS: option TRANSITION_BOUNDS (an instantiation of its own: a small pass was 1 % slower with the branches alone)
 template <int DK, int DV, bool BOUNDS>
@@ -315,6 +317,7 @@ __global__ void __launch_bounds__(NTHREADS, 4) intra_fwd_kernel(const b200gdn_ch
         const float g_lo = gam[r_lo], g_hi = gam[r_hi];
         const float b_lo = bet[r_lo], b_hi = bet[r_hi];
         uint32_t p_lo[4], p_hi[4];
+        float2 qk_lo[4], qk_hi[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const int j0 = cs + i * 8 + 2 * t;
@@ -331,6 +334,8 @@ __global__ void __launch_bounds__(NTHREADS, 4) intra_fwd_kernel(const b200gdn_ch
           *reinterpret_cast<float2*>(&Lf[r_hi * LDF + j0]) = make_float2(v[2], v[3]);
           p_lo[i] = pack_bf16(w4[0], w4[1]);
           p_hi[i] = pack_bf16(w4[2], w4[3]);
+          qk_lo[i] = make_float2(w4[0], w4[1]);
+          qk_hi[i] = make_float2(w4[2], w4[3]);
         }
         if (bounds) {
           float kk_lo = 0.f, kk_hi = 0.f;   // |k|^2 of the two rows, where the diagonal is this thread's
@@ -343,7 +348,18 @@ __global__ void __launch_bounds__(NTHREADS, 4) intra_fwd_kernel(const b200gdn_ch
           float x = log2f(fmaxf(1.f, fabsf(1.f - b_lo * kk_lo))) + log2f(fmaxf(1.f, fabsf(1.f - b_hi * kk_hi)));
 #pragma unroll
           for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-          if (lane == 0) graw[warp] = x;   // (the raw sums have been read)
+          // a value of q that is not finite makes its row's product with k, at least the one on the diagonal, not finite either
+          float s_lo = 0.f, s_hi = 0.f;
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            s_lo = max_abs3(s_lo, qk_lo[i].x, qk_lo[i].y);
+            s_hi = max_abs3(s_hi, qk_hi[i].x, qk_hi[i].y);
+          }
+          const bool odd = __any_sync(0xffffffffu, (r_lo < cm.len && !fits_bf16(s_lo)) || (r_hi < cm.len && !fits_bf16(s_hi)));
+          if (lane == 0) {   // (the raw sums have been read)
+            graw[warp] = x;
+            graw[NTHREADS / 32 + warp] = odd;
+          }
         }
         if (with_qk) {
           const uint4 lo = quad_words(p_lo, t), hi = quad_words(p_hi, t);
@@ -351,7 +367,7 @@ __global__ void __launch_bounds__(NTHREADS, 4) intra_fwd_kernel(const b200gdn_ch
           if (r_hi < cm.len) *reinterpret_cast<uint4*>(Pg + r_hi * pstride) = hi;
         }
       } else {
-        if (bounds && lane == 0) graw[warp] = 0.f;
+        if (bounds && lane == 0) graw[warp] = graw[NTHREADS / 32 + warp] = 0.f;
         if (with_qk && r_lo < cm.len) *reinterpret_cast<uint4*>(Pg + r_lo * pstride) = make_uint4(0, 0, 0, 0);
         if (with_qk && r_hi < cm.len) *reinterpret_cast<uint4*>(Pg + r_hi * pstride) = make_uint4(0, 0, 0, 0);
       }
@@ -511,13 +527,16 @@ __global__ void __launch_bounds__(NTHREADS, 4) intra_fwd_kernel(const b200gdn_ch
         tc5::fence_async_smem();
         tc5::fence_before_sync();
         int odd = 0;
-        if (bounds) odd = __syncthreads_or(!(size < INFINITY));
+        if (bounds) odd = __syncthreads_or(!fits_bf16(size));
         else __syncthreads();
         if (bounds && tid == 0) {
-          float x = gam[BT - 1];
+          float x = gam[BT - 1], q_odd = 0.f;
 #pragma unroll
-          for (int w = 0; w < NTHREADS / 32; ++w) x += graw[w];
-          bounds_ptr(a.gamma, a.n_chunks, a.HV)[(int64_t)c * a.HV + hv] = odd ? INFINITY : x;
+          for (int w = 0; w < NTHREADS / 32; ++w) {
+            x += graw[w];
+            q_odd += graw[NTHREADS / 32 + w];
+          }
+          bounds_ptr(a.gamma, a.n_chunks, a.HV)[(int64_t)c * a.HV + hv] = odd ? INFINITY : tagged_bound(x, q_odd != 0.f);
         }
         if (cm.len == BT) {
           if (tid == 32) {

@@ -73,7 +73,8 @@ typedef enum b200gdn_status {
 /* chunk passes: `gamma` is followed by n_chunks * HV floats more, bounds of the chunks' state transitions.  The transition of a chunk is
  * prod_i 2^(g_i log2 e) (I - beta_i k_i k_i^T), so its norm is at most two to the power of
  *     gamma_last + sum_i log2 max(1, |1 - beta_i |k_i|^2|),
- * which the intra stage writes (+infinity where w or u of the chunk is not finite).  A pre-scan (a scan that stores nothing but its
+ * which the intra stage writes (+infinity where w or u of the chunk is not finite; the lowest bit of the float is set where the chunk's
+ * products of q and k are not, which the gradient, but not the state, depends on).  A pre-scan (a scan that stores nothing but its
  * final state and the transition matrix) without a start state leaves out a chunk where the product of the transitions of all chunks
  * between it and the end of its sequence is at most 2^-128 and so is that of every chunk beyond it: of what these add to the state no
  * larger share arrives.  The transition matrix is zero where the product over the whole sequence is at most 2^-128. */

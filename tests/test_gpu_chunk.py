@@ -746,18 +746,20 @@ def test_sequence_split_equals_the_unsplit_scan(pieces):
 
 
 @pytest.mark.parametrize('D', [64, 128])
-@pytest.mark.parametrize('odd', [None, 'v', 'do'])
+@pytest.mark.parametrize('odd', [None, 'v', 'do', 'q'])
 def test_pre_scans_leave_out_what_does_not_reach(D, odd):
     """Long pieces whose heads forget nothing, part of a piece, all but two chunks of it, and grow: against the uncut run.  Each of the two
     is within REF_TOL of the exact result, so they are within twice that of one another (heads that forget nothing use most of it, with
-    and without anything left out: up to 0.0067 for dk); what a head that forgets shows of the cut is far less.  A value or an output gradient that is not finite in a chunk that is left out still reaches everything that
-    it reaches in the uncut run."""
+    and without anything left out: up to 0.0067 for dk); what a head that forgets shows of the cut is far less.  A value, an output gradient or a query that is not finite in a chunk that is left out still reaches everything
+    that it reaches in the uncut run."""
     from b200gdn import chunk_gated_delta_rule, index
     dev, T, H, HV = 'cuda', 64 * 60 + 37, 2, 4
     d = O.make_inputs(1, T, H, HV, D, D, seed=37)
     rate = torch.tensor([-1e-4, -0.2, -1.5, 2e-3])
     g = rate * (0.5 + torch.rand(1, T, HV, generator=torch.Generator().manual_seed(1)))
-    v, do = d['v'].clone(), d['do'].clone()
+    q, v, do = d['q'].clone(), d['v'].clone(), d['do'].clone()
+    if odd == 'q':
+        q[0, T - 80, 1, 5] = float('inf')
     if odd == 'v':
         v[0, 70, 2, 5] = float('nan')
     if odd == 'do':
@@ -767,7 +769,7 @@ def test_pre_scans_leave_out_what_does_not_reach(D, odd):
         index.FORCE_PIECES = pieces
         index._split_cache.clear()
         try:
-            leaves = [x.to(dev).to(torch.bfloat16).requires_grad_(True) for x in (d['q'], d['k'], v)]
+            leaves = [x.to(dev).to(torch.bfloat16).requires_grad_(True) for x in (q, d['k'], v)]
             leaves += [x.to(dev).requires_grad_(True) for x in (g, d['beta'], d['h0'])]
             o, ht = chunk_gated_delta_rule(*leaves[:5], initial_state=leaves[5], output_final_state=True)
             torch.autograd.backward([o, ht], [do.to(dev).to(torch.bfloat16), d['dht'].to(dev)])
