@@ -677,6 +677,7 @@ __global__ void __launch_bounds__(NTHREADS) recurrent_pairs_kernel(const b200gdn
         g.beta = beta;
         tok[t + l16] = g;
       }
+      __syncwarp();   // the next pass writes `dots` again
     }
     __syncthreads();
     fetch_gates(t0 + TB);

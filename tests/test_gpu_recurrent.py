@@ -295,3 +295,25 @@ def test_tokens_in_pairs(K, V, lens, v_first):
         use_beta_sigmoid_in_kernel=True, allow_neg_eigval=True, state_v_first=v_first, cu_seqlens=cu.to(dev))
     O.assert_close('o', torch.cat(ref_o, 1), o.cpu(), 1e-5)
     O.assert_close('ht', torch.cat(ref_ht, 0), ht.cpu(), 1e-5)
+
+
+@pytest.mark.parametrize('K', [32, 64])
+def test_pairs_of_a_block_are_prepared_in_two_passes(K):
+    """Blocks of 32 tokens, of which a warp prepares four at a time in two passes over the same scratch row: against the fp32
+    recurrence for every length from a first pass alone to several blocks, and the same bits every time."""
+    from b200gdn import fused_recurrent_gated_delta_rule
+    H, HV, N, dev = 2, 4, 48, 'cuda'
+    for T in (15, 17, 31, 32, 33, 64):
+        q, k, v, graw, braw, A_log, dt_bias, gen = _inputs(N, T, H, HV, K, K, 53, torch.float32)
+        h0 = torch.randn(N, HV, K, K, generator=gen) * 0.5
+        options = (True, True, True, A_log, dt_bias, True, True, False)
+        ref_o, ref_ht = O.recurrent_step_options(q, k, v, graw, braw, None, h0, *options)
+        args = [x.to(dev) for x in (q, k, v, graw)]
+        runs = [fused_recurrent_gated_delta_rule(
+            *args, beta=braw.to(dev), initial_state=h0.to(dev), output_final_state=True, use_qk_l2norm_in_kernel=True,
+            use_gate_in_kernel=True, A_log=A_log.to(dev), dt_bias=dt_bias.to(dev), use_beta_sigmoid_in_kernel=True,
+            allow_neg_eigval=True) for _ in range(8)]
+        for o, ht in runs[1:]:
+            assert torch.equal(o, runs[0][0]) and torch.equal(ht, runs[0][1])
+        O.assert_close(f'o T={T}', ref_o, runs[0][0].cpu(), 1e-5)
+        O.assert_close(f'ht T={T}', ref_ht, runs[0][1].cpu(), 1e-5)
