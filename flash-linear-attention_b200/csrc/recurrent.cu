@@ -967,10 +967,16 @@ int launch(const b200gdn_recurrent_args& a, cudaStream_t st) {
   // Tokens per sequence (on average) from which they are taken in pairs.  Measured, one by one / in pairs, K = V = 128 bf16: 1 x 16
   // heads, 8 tokens 6.2 / 6.3 us, 12 tokens 7.4 / 7.1, 24 tokens 12.1 / 10.6; 16 x 32 heads (2048 CTAs), 16 tokens 46.7 / 48.9, 24
   // tokens 66.9 / 64.8, 64 tokens 158 / 139 (fp32: 33 tokens 89.8 / 91.8, 64 tokens 156 / 147); K = V = 64: 8 tokens 5.7 / 5.0 and
-  // 13.1 / 13.6, 12 tokens 6.7 / 5.6 and 16.4 / 15.7.
+  // 13.1 / 13.6, 12 tokens 6.7 / 5.6 and 16.4 / 15.7.  [V,K] states gain more, at every K (K = V = 256, 4 x 16 heads, 12 tokens: 29.0 /
+  // 20.9; K = 32: a quarter).  K = 256 with [K,V] states starts late, its registers leave fewer CTAs per SM and a state comes in words
+  // of 8 bytes: 4 x 16 heads, V = 256, 12 tokens 21.4 / 28.3 us in bf16 and 22.6 / 27.4 in fp32, 64 tokens 80.0 / 90.9 and 85.2 / 86.8;
+  // V = 128 (256 CTAs) 64 tokens 47.2 / 48.9 and 51.6 / 46.4, 24 tokens in fp32 22.3 / 21.7; 1 x 16 heads (128 CTAs) 40 tokens in
+  // bf16 24.4 / 24.7, 64 tokens 36.8 / 36.3, in fp32 16 tokens 12.3 / 12.2, 24 tokens 16.6 / 15.5.
   const int tokens = a.T / (a.cu_seqlens != nullptr && a.n_seq > 0 ? a.n_seq : 1);
-  const bool many_ctas = (int64_t)grid.x * grid.y * grid.z > 4 * sm_count();
-  const bool pairs = tokens >= (DK >= 128 && many_ctas ? 40 : 12);
+  const int64_t ctas = (int64_t)grid.x * grid.y * grid.z, sms = sm_count();
+  const bool fp32 = a.qkv_dtype != 0 && a.qkv_dtype != 1;
+  const bool pairs = DK == 256 && !vf ? tokens >= (fp32 ? 24 : 64) && ctas <= (fp32 ? 2 : 1) * sms
+                                      : tokens >= (DK >= 128 && ctas > 4 * sms ? 40 : 12);
   auto run = [&](auto* one, auto* few, auto* many) { (step ? one : pairs ? many : few)<<<grid, NTHREADS, 0, st>>>(a); };
 #define RUN(VF, TY) run(recurrent_step_kernel<DK, VF, TY>, recurrent_few_kernel<DK, VF, TY>, recurrent_pairs_kernel<DK, VF, TY>)
   switch (a.qkv_dtype) {
