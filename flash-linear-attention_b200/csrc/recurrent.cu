@@ -163,11 +163,9 @@ __device__ __forceinline__ void load_gate_beta(const b200gdn_recurrent_args& a, 
   gg = a.g ? ld_param(a.g, row * a.HV + hv, a.gb_dtype) : 0.f;
   bb = ld_param(a.beta, row * a.HV + hv, a.gb_dtype);
 }
-__device__ __forceinline__ void activate(const b200gdn_recurrent_args& a, float A_log, float dt_bias, float gg, float bb, float& dec, float& beta) {
-  if (a.flags & B200GDN_REC_GATE) {
-    gg += dt_bias;
-    gg = -expf(A_log) * softplus_f(gg);
-  }
+template <typename Gate>   // the gate's value from its raw one, with the head's parameters
+__device__ __forceinline__ void activate(const b200gdn_recurrent_args& a, Gate&& gate, float gg, float bb, float& dec, float& beta) {
+  if (a.flags & B200GDN_REC_GATE) gg = gate(gg);
   if (a.flags & B200GDN_REC_BETA_SIGMOID) {
     bb = 1.f / (1.f + expf(-bb));
     if (a.flags & B200GDN_REC_NEG_EIGVAL) bb *= 2.f;
@@ -175,11 +173,16 @@ __device__ __forceinline__ void activate(const b200gdn_recurrent_args& a, float 
   dec = expf(gg);
   beta = bb;
 }
+// The parameters are loaded here, where the option is on: as arguments they are loaded ahead of the branch and held, which cost two
+// tokens of 16 x 32 heads, K = V = 128 with [V,K] states, 26.4 us for 25.2.
 __device__ __forceinline__ void gate_beta(const b200gdn_recurrent_args& a, int64_t row, int hv, float& dec, float& beta) {
   float gg, bb;
   load_gate_beta(a, row, hv, gg, bb);
-  const bool gate = a.flags & B200GDN_REC_GATE;
-  activate(a, gate ? a.A_log[hv] : 0.f, gate && a.dt_bias ? a.dt_bias[hv] : 0.f, gg, bb, dec, beta);
+  auto gate = [&](float x) {
+    if (a.dt_bias) x += a.dt_bias[hv];
+    return -expf(a.A_log[hv]) * softplus_f(x);
+  };
+  activate(a, gate, gg, bb, dec, beta);
 }
 
 // One token per sequence: a CTA of four warps owns 32 value channels of one (sequence, head).  Every lane loads its own rows
@@ -660,7 +663,7 @@ __global__ void __launch_bounds__(NTHREADS) recurrent_pairs_kernel(const b200gdn
       if (!(l16 & 1)) dots[half][l16 >> 1] = x[0];
       __syncwarp();
       float dec = 1.f, beta = 0.f;   // (a token past the end)
-      if (l16 < NT && t + l16 < nt) activate(a, A_log, dt_bias, g_raw[p], b_raw[p], dec, beta);
+      if (l16 < NT && t + l16 < nt) activate(a, [&](float x) { return -expf(A_log) * softplus_f(x + dt_bias); }, g_raw[p], b_raw[p], dec, beta);
       const float other = __shfl_xor_sync(0xffffffffu, dec, 1);   // of the pair's other token
       if (l16 < NT && live) {
         const float* d = dots[half];
