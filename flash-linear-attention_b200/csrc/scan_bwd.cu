@@ -13,7 +13,7 @@
 // the chain MMA warp issues  acc = K dS_bf16  and  dS += Q^T do_s - W^T dv2  with accumulators in TMEM; a store warp
 // issues the TMA stores of dh_c and dv2; eight epilogue warps move dS between TMEM and shared memory and form dv2.
 // B4 T4096 H16 K=V=128: 94 us (107 with products and stores issued by one thread in turn; 96 with the 80 registers that two CTAs per SM
-// would allow, of which shared memory has room for one).
+// would allow, of which shared memory has room for one; both K = 128).
 // DVL: the chain MMA warp also issues  L = qk^T do  of the NEXT chunk right after a step's last product (it only needs
 // loaded tiles and runs while the epilogue warps convert dS); qk = tril(Q K^T 2^(gamma_i-gamma_j)) comes ready-made
 // from the forward pass; the epilogue warps add scale L where they form dv2.
@@ -56,9 +56,11 @@ struct ScanBwdMaps {
 };
 
 // PRE: nothing stored but the final gradient (a pre-scan); an instantiation of its own, because the look at the bounds, not executed,
-// cost the main scan 5 us in 95
+// cost the main scan 5 us in 95.  At K = 64, which spills nothing at 80 registers, a pre-scan keeps to half of an SM's: with 111 the
+// chain's CTAs, launched early in small passes, found no place beside it (forward and backward, 8192 tokens, 4 heads: 113.3 us for 118.5;
+// 3000 tokens, 8 heads 85.5 for 88.3; the main scan is the faster one with 111)
 template <int DK, int DV, int NSTAGE, bool DVL, bool PRE>
-__global__ void __launch_bounds__(NTHREADS, 1)
+__global__ void __launch_bounds__(NTHREADS, DK == 64 && PRE ? 2 : 1)
     scan_bwd_kernel(const b200gdn_chunk_args a, const __grid_constant__ ScanBwdMaps maps) {
   using S = ScanBwdSmem<DK, NSTAGE, DVL>;
   constexpr int NH = DK / 64;
