@@ -835,6 +835,165 @@ def test_pre_scans_where_gates_grow_and_decay(D, reverse):
         O.assert_close('o', ro[:, -64:] / size, o[:, -64:].cpu().double() / size, REF_TOL['o'])
 
 
+def _walked(bounds, reverse):
+    """From the bounds [chunks] of one sequence: how many chunks a pre-scan walks, whether the whole transition counts as zero, how close a
+    sum comes to the line, and the first one below it (for the test's own sake)."""
+    sums = np.cumsum((bounds if reverse else bounds[::-1]).astype(np.float64))
+    above = np.nonzero(sums[:-1] >= -128)[0]
+    return (int(above[-1]) + 2 if len(above) else 1), bool(sums[-1] < -128), np.abs(sums + 128).min(), int((sums >= -128).argmin()) + 1
+
+
+@pytest.mark.parametrize('D', [64, 128])
+@pytest.mark.parametrize('reverse', [False, True])
+def test_pre_scan_against_itself(D, reverse):
+    """A pre-scan of 66 chunks with and without the transition bounds, through the C ABI, for heads that forget nothing, most of the
+    piece (the line is crossed in the second round of 32 chunks), part of it, all but two chunks, that grow, and that grow and decay in turn:
+    * the bounds are gamma_last + sum log2 max(1, |1 - beta |k|^2|), their lowest bits clear;
+    * results are the same up to the share that may be left out (2^-128 of values that are below 2^20, and again for what the changed
+      values round differently in bf16 on the way), so the same bits wherever they are above 2^-80;
+    * exactly the chunks are walked that the rule names: NaN in the operands of the others, written after their bounds, is not
+      seen, and in the last one of them it is;
+    * a start state (end gradient) is not left out, and values that are not finite more than 32 chunks away are not either.
+    The forward pass runs without A (B200GDN_FORWARD_ONLY)."""
+    from b200gdn import _lib
+    from b200gdn.chunk import new_chunk_args
+    from b200gdn.index import build_tables
+    H, HV, nc = 2, 6, 66
+    rows, dev, st = 64 * (nc - 1) + 21, 'cuda', torch.cuda.current_stream().cuda_stream
+    d = O.make_inputs(1, rows, H, HV, D, D, seed=47)
+    k = d['k'].clone()
+    k[:, ::64, 1] *= 1.6   # |1 - beta |k|^2| above one for some
+    in_turn = torch.cat([torch.full((9,), -0.17), torch.full((9,), 0.14)]).repeat(4)[:nc]   # nearest the scan's end first
+    in_turn = (in_turn if reverse else in_turn.flip(0)).repeat_interleave(64)[:rows]
+    g = torch.stack([torch.full((rows,), r) for r in (-1e-4, -0.03, -0.2, -1.5, 2e-3)] + [in_turn], 1)
+    cm, sm = (torch.from_numpy(x).to(dev) for x in build_tables([(0, rows)]))
+    bf, f32 = dict(dtype=torch.bfloat16, device=dev), dict(dtype=torch.float32, device=dev)
+    q0, k0, v0, do0 = (x.to(**bf).contiguous() for x in (d['q'], k, d['v'], d['do']))
+    g0, beta0 = g.to(**f32).contiguous(), d['beta'].to(**f32).contiguous()
+    state = (torch.randn(1, HV, D, D, generator=torch.Generator().manual_seed(3))).to(dev)
+
+    def intra(q, v):
+        a = new_chunk_args(q, k0, v, D ** -0.5, (cm, sm, (nc, 1)))
+        t = dict(gamma=torch.zeros(nc * HV * 65, **f32), qk=torch.zeros(rows, HV, 64, **bf), w=torch.zeros(rows, HV, D, **bf),
+                 u=torch.zeros(rows, HV, D, **bf))
+        a.g, a.beta, a.stage_mask, a.options = g0.data_ptr(), beta0.data_ptr(), _lib.FWD_INTRA, _lib.TRANSITION_BOUNDS | _lib.FORWARD_ONLY
+        for name, x in t.items():
+            setattr(a, name, x.data_ptr())
+        _lib.call('b200gdn_chunk_fwd', a, st)
+        return t
+
+    def scan(t, bounds, q=q0, v=v0, do=do0, start=None):
+        a = new_chunk_args(q, k0, v, D ** -0.5, (cm, sm, (nc, 1)))
+        out, M = torch.full((1, HV, D, D), float('nan'), **f32), torch.full((1, HV, D, D), float('nan'), **f32)
+        a.options = _lib.TRANSITION_BOUNDS if bounds else 0
+        a.gamma, a.w = t['gamma'].data_ptr(), t['w'].data_ptr()
+        if reverse:
+            a.qk, a.d_o, a.dht, a.dh0, a.cp_dM = t['qk'].data_ptr(), do.data_ptr(), _lib.ptr(start), out.data_ptr(), M.data_ptr()
+            a.stage_mask = _lib.BWD_DVLOCAL | _lib.BWD_SCAN
+            _lib.call('b200gdn_chunk_bwd', a, st)
+        else:
+            a.u, a.h0, a.ht, a.cp_M, a.stage_mask = t['u'].data_ptr(), _lib.ptr(start), out.data_ptr(), M.data_ptr(), _lib.FWD_SCAN
+            _lib.call('b200gdn_chunk_fwd', a, st)
+        return out[0].cpu(), M[0].cpu()
+
+    def same(x, y):
+        return bool(((x.double() - y.double()).abs() <= 2.0 ** -100).all())
+
+    t = intra(q0, v0)
+    bounds = t['gamma'][nc * HV * 64:].reshape(nc, HV).cpu()
+    assert not (bounds.view(torch.int32) & 1).any()
+    kk = k0[0].double().cpu().square().sum(-1).repeat_interleave(HV // H, 1)
+    growth = (1 - beta0[0].double().cpu() * kk).abs().clamp(min=1).log2()
+    pad = torch.zeros(64 * nc - rows, HV, dtype=torch.float64)
+    want = torch.cat([g.double() * O.RCP_LN2 + growth, pad]).reshape(nc, 64, HV).sum(1)
+    assert (want - bounds.double()).abs().max() < 1e-3
+    rule = [_walked(bounds[:, hv].numpy(), reverse) for hv in range(HV)]
+    assert min(r[2] for r in rule) > 0.01   # 66 fp32 values below 2^8 add up to within 0.001
+    assert rule[0][0] == nc and 32 < rule[1][0] < nc and rule[2][0] < 16 and rule[3][0] <= 2 and rule[4][0] == nc
+    assert rule[5][3] < 18 and 54 < rule[5][0] < nc
+    assert [r[1] for r in rule] == [False, True, True, True, False, True]
+
+    full, M_full = scan(t, False)
+    cut, M_cut = scan(t, True)
+    assert torch.isfinite(full).all() and same(full, cut) and same(M_full, M_cut)
+    assert [bool((M_cut[hv] == 0).all()) for hv in range(HV)] == [r[1] for r in rule]
+    for a, b in zip(scan(t, False, start=state), scan(t, True, start=state)):
+        assert same(a, b)
+    # operands of the chunks that are not walked, then of the farthest one that is
+    name = 'w' if reverse else 'u'
+    x = t[name].clone()
+    poisoned = {**t, name: x}
+    for hv in range(HV):
+        n = rule[hv][0]
+        x[slice(64 * n, None) if reverse else slice(0, 64 * (nc - n)), hv] = float('nan')
+    assert torch.equal(scan(poisoned, True)[0], cut)
+    for hv in range(HV):
+        c = rule[hv][0] - 1 if reverse else nc - rule[hv][0]
+        x[64 * c:64 * c + 64, hv] = float('nan')
+    assert not torch.isfinite(scan(poisoned, True)[0]).any(-1).any(-1).any()
+    # values that are not finite, far away
+    if reverse:
+        q1, do1 = q0.clone(), do0.clone()
+        q1[0, 64 * 60 + 3, :, 5] = float('nan')
+        do1[0, 64 * 60 + 3, :, 5] = float('inf')
+        t1 = intra(q1, v0)
+        odd = t1['gamma'][nc * HV * 64:].reshape(nc, HV).cpu().view(torch.int32) & 1
+        assert odd[60].all() and odd.sum() == HV
+        pairs = [[scan(t1, b, q=q1)[0] for b in (False, True)], [scan(t, b, do=do1)[0] for b in (False, True)]]
+    else:
+        v1 = v0.clone()
+        v1[0, 64 * 10 + 3, :, 5] = float('nan')
+        t1 = intra(q0, v1)
+        assert torch.isinf(t1['gamma'][nc * HV * 64:].reshape(nc, HV)[10]).all()
+        pairs = [[scan(t1, b, v=v1)[0] for b in (False, True)]]
+    for a, b in pairs:
+        bad = ~torch.isfinite(a)
+        assert bad.flatten(1).any(1).all() and torch.equal(bad, ~torch.isfinite(b))
+        assert same(a.masked_fill(bad, 0), b.masked_fill(bad, 0))
+
+
+@pytest.mark.parametrize('D,H,HV,options', [(128, 16, 16, True), (128, 8, 24, True), (128, 4, 16, True), (64, 16, 16, True), (64, 8, 24, True), (64, 8, 32, False)])
+def test_results_by_tma_equal_results_by_rows(D, H, HV, options):
+    """From 2049 chunk-heads on, whole chunks of the normalised q and k and of dq, dk and dv leave by TMA; below, and where a chunk is
+    ragged, by rows.  150 chunks of full and ragged sequences in one call against the sequences one by one (at most 50 chunks): the same bits.
+    8/24 heads: a CTA takes the heads of a group in turn, in both; 4/16: a cluster does, 150 x 4 CTAs in turn being the longer way; 8/32:
+    in turn in one call and a cluster in the others, which add in the same order."""
+    from b200gdn import chunk_gated_delta_rule, index
+    lens = [64 * 40, 64 * 30 + 1, 63, 64, 64 * 50, 64 * 26 + 33]
+    cu = [0] + [int(x) for x in np.cumsum(lens)]
+    T, N, dev, bf = cu[-1], len(lens), 'cuda', torch.bfloat16
+    gen = torch.Generator(device=dev).manual_seed(59)
+
+    def normal(*shape):
+        return torch.randn(*shape, generator=gen, device=dev)
+    q, k = (torch.nn.functional.normalize(normal(1, T, H, D), dim=-1) * (3 if options else 1) for _ in range(2))
+    data = [q.to(bf), k.to(bf), normal(1, T, HV, D).to(bf)]
+    data += [normal(1, T, HV).to(bf) for _ in range(2)] if options else [torch.nn.functional.logsigmoid(normal(1, T, HV)), torch.rand(1, T, HV, generator=gen, device=dev)]
+    h0, do, dht = normal(N, HV, D, D) * 0.1, normal(1, T, HV, D).to(bf), normal(N, HV, D, D) * 0.1
+    A_log, dt_bias = normal(HV) * 0.3, normal(HV) * 0.3
+    more = dict(use_qk_l2norm_in_kernel=True, use_gate_in_kernel=True, A_log=A_log, dt_bias=dt_bias, use_beta_sigmoid_in_kernel=True) if options else {}
+
+    def run(rows, seqs, cu_t):
+        leaves = [x[:, rows].contiguous().requires_grad_(True) for x in data] + [h0[seqs].contiguous().requires_grad_(True)]
+        o, ht = chunk_gated_delta_rule(*leaves[:5], initial_state=leaves[5], output_final_state=True, cu_seqlens=cu_t, **more)
+        grads = torch.autograd.grad([o, ht], leaves, [do[:, rows].contiguous(), dht[seqs].contiguous()])
+        return [x.detach() for x in (o, *grads[:5])], [x.detach() for x in (ht, grads[5])]
+    index.FORCE_PIECES = 1
+    index._split_cache.clear()
+    try:
+        by_row, by_seq = run(slice(0, T), slice(0, N), torch.tensor(cu, dtype=torch.int32, device=dev))
+        parts = [run(slice(cu[i], cu[i + 1]), slice(i, i + 1), None) for i in range(N)]
+    finally:
+        index.FORCE_PIECES = None
+        index._split_cache.clear()
+    for j, n in enumerate(('o', 'dq', 'dk', 'dv', 'dg', 'dbeta')):
+        for i in range(N):
+            assert torch.equal(by_row[j][:, cu[i]:cu[i + 1]], parts[i][0][j]), f'{n}, sequence {i}'
+    for j, n in enumerate(('ht', 'dh0')):
+        for i in range(N):
+            assert torch.equal(by_seq[j][i:i + 1], parts[i][1][j]), f'{n}, sequence {i}'
+
+
 @pytest.mark.parametrize('pieces', [None, 3])
 def test_state_v_first_layout(pieces):
     """states stored [N,HV,V,K] (the reference's state_v_first, tests/ops/test_gdn.py:385-461): the scans read h0 / dht
