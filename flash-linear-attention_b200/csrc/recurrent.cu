@@ -408,7 +408,7 @@ constexpr int NT = 2;
 struct __align__(16) PairToken {
   float k, q;          // e^g from before the pair to the token, times kn | qn
   float decay, last;   // the same alone; e^g from the token to the pair's end, times kn
-  float kk;            // second token: e^g <kn k, kn k of the first>
+  float kk;            // second token: e^g <kn k, kn k of the first>.  First: a factor of the state ahead of the pair, 1 as a rule
   float kq0, kq1;      // <qn q, kn k> with the first token's k (second token: times e^g; first: not used) and the second's
   float beta;
 };
@@ -473,6 +473,13 @@ struct PairState {
   template <typename T>
   __device__ __forceinline__ void pair(const float* k, const float* q, const T* v, const PairToken* c, int lane, float (&o)[NT]) {
     const bool b4 = lane & 4, b2 = lane & 2;
+    if (c[0].kk != 1.f) {
+      const uint64_t f2 = pack2(c[0].kk, c[0].kk);
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int i = 0; i < 2 * NM; ++i) st[i][j] = mul2(st[i][j], f2);
+    }
     uint64_t k2[NT][2 * NM];
     float z[NT];
 #pragma unroll
@@ -670,11 +677,14 @@ __global__ void __launch_bounds__(NTHREADS) recurrent_pairs_kernel(const b200gdn
         const float kn0 = l2 ? rsqrtf(d[0] + 1e-6f) : 1.f, kn1 = l2 ? rsqrtf(d[1] + 1e-6f) : 1.f;
         const float qn = l2 ? a.scale * rsqrtf(d[2 + l16] + 1e-6f) : a.scale;
         PairToken g;
-        g.decay = l16 ? dec * other : dec;
+        // the state takes the first token's e^g ahead of the pair where the two together are out of fp32's range (zero times an
+        // overflowed product is not zero, a large state times one that vanished is not either)
+        const float both = dec * other, ahead = both >= 1.17549435e-38f && both < INFINITY ? 1.f : l16 ? other : dec;
+        g.decay = ahead == 1.f ? (l16 ? both : dec) : l16 ? dec : 1.f;
         g.k = g.decay * (l16 ? kn1 : kn0);
         g.q = g.decay * qn;
         g.last = l16 ? kn1 : other * kn0;
-        g.kk = dec * d[4] * kn0 * kn1;
+        g.kk = l16 ? dec * d[4] * kn0 * kn1 : ahead;
         g.kq0 = (l16 ? dec * d[6] : d[5]) * kn0 * qn;
         g.kq1 = d[7] * kn1 * qn;
         g.beta = beta;

@@ -317,3 +317,29 @@ def test_pairs_of_a_block_are_prepared_in_two_passes(K):
             assert torch.equal(o, runs[0][0]) and torch.equal(ht, runs[0][1])
         O.assert_close(f'o T={T}', ref_o, runs[0][0].cpu(), 1e-5)
         O.assert_close(f'ht T={T}', ref_ht, runs[0][1].cpu(), 1e-5)
+
+
+@pytest.mark.parametrize('K,v_first', [(64, False), (128, False), (128, True)])
+@pytest.mark.parametrize('start', ['nothing', 'large'])
+def test_gates_of_a_pair_whose_product_leaves_fp32(K, v_first, start):
+    """Two gates of a pair that fp32 holds one by one but not as a product: e^50 twice on a state of zeros, which stays zero until the
+    first token has written, and e^-60 twice on a state of 1e30, which keeps 1e-22 (and comes back by e^45, the only token written out
+    then).  The second tokens of the pairs, and the pair that an odd length leaves, take part.  Tolerance of the fp32 recurrence."""
+    from b200gdn import fused_recurrent_gated_delta_rule
+    T, H, dev = 13, 2, 'cuda'
+    d = O.make_inputs(1, T, H, H, K, K, seed=7, h0_std=1.)
+    g, beta, h0 = d['g'], d['beta'], None
+    if start == 'nothing':
+        g[:, :2], g[:, 6:8] = 50., -50.
+    else:
+        g.zero_(), beta.zero_()
+        g[:, 2:4], g[:, 8], h0 = -60., 45., d['h0'] * 1e30
+    ref_o, ref_ht = O.naive_recurrent(d['q'], d['k'], d['v'], g, beta, None, h0, True, dtype=torch.float64)
+    flip = (lambda x: x.transpose(-1, -2).contiguous()) if v_first else (lambda x: x)
+    o, ht = fused_recurrent_gated_delta_rule(*(d[n].to(dev) for n in 'qkv'), g.to(dev), beta=beta.to(dev),
+                                             initial_state=None if h0 is None else flip(h0).to(dev), output_final_state=True,
+                                             state_v_first=v_first)
+    assert torch.isfinite(o).all() and torch.isfinite(ht).all()
+    for t in range(T):   # magnitudes differ by forty decades: token by token
+        O.assert_close(f'o {t}', ref_o[:, t], o[:, t].double().cpu(), 1e-5)
+    O.assert_close('ht', ref_ht, flip(ht).double().cpu(), 1e-5)
