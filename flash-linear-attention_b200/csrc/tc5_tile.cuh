@@ -123,13 +123,6 @@ struct FragLoadT {
   __device__ __forceinline__ float2 hi2(int i) const { return unpack_bf16(hi[i]); }
 };
 
-// transpose of an 8 x 8 matrix of 16-bit elements held one 32-bit word (two elements of a row) per lane
-__device__ __forceinline__ uint32_t transpose8(uint32_t x) {
-  uint32_t y;
-  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;\n" : "=r"(y) : "r"(x));
-  return y;
-}
-
 // Zero rows [valid, ROWS) of a swizzled [ROWS][COLS] tile (a ragged last chunk arrives by TMA as a full box
 // whose extra rows belong to the next sequence).  The caller fences and synchronises afterwards.
 template <int ROWS, int COLS>
