@@ -93,8 +93,8 @@ def staged_bytes(R, C, NS):
 # stale with every kernel change: refresh it together with the profile.
 NCU_TRAFFIC = {
     'source': 'profiles/chunk_fwd_bwd_B4_T4096_H16_D128_four_kernels.md',
-    'kernel_sources_commit': 'cc215a0',
-    'bytes': {'intra_fwd': 361.8e6, 'scan_out_fwd': 539.4e6, 'scan_dvl_bwd': 472.6e6, 'bwd_local': 886.8e6},
+    'kernel_sources_commit': '396d023',
+    'bytes': {'intra_fwd': 361.5e6, 'scan_out_fwd': 538.5e6, 'scan_dvl_bwd': 473.1e6, 'bwd_local': 886.9e6},
 }
 
 

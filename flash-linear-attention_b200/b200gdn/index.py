@@ -147,8 +147,8 @@ def piece_counts(chunks_per_seq, HV: int, slices: int, sms: int = 148):
     """How many pieces each sequence is cut into (equal pieces, so the longest sequences into the most): the cut with the
     least time by the model below, in microseconds as measured on a B200 with heads of 128 and 64; none unless it saves
     a twentieth.  A scan CTA takes `step` per chunk and the pre-scan, which runs beside twice as many transition-matrix
-    CTAs (two per SM forward, one backward), nearly as long; the prefix chain takes a step per piece.  Two pieces never
-    pay: pre-scan and scan together then walk as far as the uncut scan."""
+    CTAs (two per SM forward, one backward), nearly as long (heads that forget are pre-scanned in less, but a plan does not
+    see the gates); the prefix chain takes a step per piece.  Two pieces never pay: pre-scan and scan together then walk as far as the uncut scan."""
     if FORCE_PIECES is not None:
         return [max(1, min(int(FORCE_PIECES), int(c))) for c in chunks_per_seq]
     uncut = [1] * len(chunks_per_seq)

@@ -20,9 +20,11 @@
 // at an address that is uniform over the warp (one wavefront) and 16-byte reads along rows for the other, skips what is
 // zero by triangularity, and nothing is filled with zeros first.
 // Bounds of the chunk's state transition, where pre-scans will want them (TRANSITION_BOUNDS), cost 3 %: the squared norms of k are the
-// diagonal of K K^T, and the largest of W and U is taken from the accumulators on their way out.
+// diagonal of K K^T, and the largest of W and U is taken from the accumulators on their way out.  That is all they do where heads forget
+// nothing: B1 T65536 H16 K=V=128 972 us for 957, with the backward pass 2687 for 2673 (gates of logsigmoid(N(0,1)): 617 and 1890).
 // B4 T4096 H16 K=V=128: 87 us inside a step (105), 94 by itself between two events; with the L2 norm, gate and beta options
-// 120 us (108 + 47 for a norm pass of its own).
+// 115 us (108 + 47 for a norm pass of its own; 120 with the norm's sums in scalars and normalised rows stored from registers), 109 with
+// 8/16 heads.
 #include "rowio.cuh"
 #include "tc5_tile.cuh"
 #include "tma.cuh"
