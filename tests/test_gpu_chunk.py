@@ -746,20 +746,18 @@ def test_sequence_split_equals_the_unsplit_scan(pieces):
 
 
 @pytest.mark.parametrize('D', [64, 128])
-@pytest.mark.parametrize('odd', [None, 'v', 'do', 'q'])
+@pytest.mark.parametrize('odd', [None, 'v', 'do'])
 def test_pre_scans_leave_out_what_does_not_reach(D, odd):
     """Long pieces whose heads forget nothing, part of a piece, all but two chunks of it, and grow: against the uncut run.  Each of the two
     is within REF_TOL of the exact result, so they are within twice that of one another (heads that forget nothing use most of it, with
-    and without anything left out: up to 0.0067 for dk); what a head that forgets shows of the cut is far less.  A value, an output gradient or a query that is not finite in a chunk that is left out still reaches everything
-    that it reaches in the uncut run."""
+    and without anything left out: up to 0.0067 for dk); what a head that forgets shows of the cut is far less.  A value or an output gradient that is not finite in a chunk that is left out still reaches everything that
+    it reaches in the uncut run."""
     from b200gdn import chunk_gated_delta_rule, index
     dev, T, H, HV = 'cuda', 64 * 60 + 37, 2, 4
     d = O.make_inputs(1, T, H, HV, D, D, seed=37)
     rate = torch.tensor([-1e-4, -0.2, -1.5, 2e-3])
     g = rate * (0.5 + torch.rand(1, T, HV, generator=torch.Generator().manual_seed(1)))
-    q, v, do = d['q'].clone(), d['v'].clone(), d['do'].clone()
-    if odd == 'q':
-        q[0, T - 80, 1, 5] = float('inf')
+    v, do = d['v'].clone(), d['do'].clone()
     if odd == 'v':
         v[0, 70, 2, 5] = float('nan')
     if odd == 'do':
@@ -769,7 +767,7 @@ def test_pre_scans_leave_out_what_does_not_reach(D, odd):
         index.FORCE_PIECES = pieces
         index._split_cache.clear()
         try:
-            leaves = [x.to(dev).to(torch.bfloat16).requires_grad_(True) for x in (q, d['k'], v)]
+            leaves = [x.to(dev).to(torch.bfloat16).requires_grad_(True) for x in (d['q'], d['k'], v)]
             leaves += [x.to(dev).requires_grad_(True) for x in (g, d['beta'], d['h0'])]
             o, ht = chunk_gated_delta_rule(*leaves[:5], initial_state=leaves[5], output_final_state=True)
             torch.autograd.backward([o, ht], [do.to(dev).to(torch.bfloat16), d['dht'].to(dev)])
@@ -786,6 +784,37 @@ def test_pre_scans_leave_out_what_does_not_reach(D, odd):
         O.assert_close(f'{n} cut vs uncut', a, b, 2 * REF_TOL[n])
         if n in ('o', 'dv') and odd is None:
             O.assert_close(f'{n} cut vs uncut, heads that forget', a[:, :, 1:3], b[:, :, 1:3], 1e-3)
+
+
+@pytest.mark.parametrize('D', [64, 128])
+def test_a_query_that_is_not_finite_is_not_left_out(D):
+    """An infinite query in a chunk that the reverse pre-scan would leave out, of heads that forget part of a piece and all but two chunks of
+    it (and one that forgets nothing): in the cut run the same results are finite as in the uncut one, and these are the same within
+    twice the tolerance that each has to the exact result."""
+    from b200gdn import chunk_gated_delta_rule, index
+    dev, T, H, HV, bf = 'cuda', 64 * 60 + 37, 2, 4, torch.bfloat16
+    d = O.make_inputs(1, T, H, HV, D, D, seed=37)
+    rate = torch.tensor([-1e-4, -0.2, -1.5, -0.2])
+    g = rate * (0.5 + torch.rand(1, T, HV, generator=torch.Generator().manual_seed(1)))
+    q = d['q'].clone()
+    q[0, T - 80, 1, 5] = float('inf')
+
+    def run(pieces):
+        index.FORCE_PIECES = pieces
+        index._split_cache.clear()
+        try:
+            leaves = [x.to(dev).to(bf).requires_grad_(True) for x in (q, d['k'], d['v'])]
+            leaves += [x.to(dev).requires_grad_(True) for x in (g, d['beta'], d['h0'])]
+            o, ht = chunk_gated_delta_rule(*leaves[:5], initial_state=leaves[5], output_final_state=True)
+            return [x.detach().float().cpu() for x in (o, ht, *torch.autograd.grad([o, ht], leaves, [d['do'].to(dev).to(bf), d['dht'].to(dev)]))]
+        finally:
+            index.FORCE_PIECES = None
+            index._split_cache.clear()
+    for n, a, b in zip(('o', 'ht', 'dq', 'dk', 'dv', 'dg', 'dbeta', 'dh0'), run(1), run(3)):
+        bad = ~torch.isfinite(a)
+        assert torch.equal(bad, ~torch.isfinite(b)), n
+        assert bad.any() == (n not in ('ht', 'dq'))   # which do not depend on q
+        O.assert_close(f'{n} cut vs uncut', a.masked_fill(bad, 0), b.masked_fill(bad, 0), 2 * REF_TOL[n])
 
 
 @pytest.mark.parametrize('D', [64, 128])
